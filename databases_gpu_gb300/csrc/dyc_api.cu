@@ -236,7 +236,10 @@ dyc_status ensure_scratch(dyc_table *t, uint64_t n) {
     const size_t idx_bytes = t->kb == 8 ? (size_t)cap * 4 : 0;
     const size_t list_bytes = (size_t)n * t->slot_bytes;
     const size_t win_bytes = (size_t)(n / 32 + 1) * 4;
-    const size_t need = dedup_bytes + idx_bytes + 2 * list_bytes + win_bytes + 256 + 5 * 256;
+    const size_t lcnt_bytes = (size_t)(n / dyc::kLeftTile + 1) * 4;
+    const size_t bcnt_bytes = (size_t)(n / dyc::kBinSmallMean + 1) * 4;
+    const size_t need = dedup_bytes + idx_bytes + 2 * list_bytes + 2 * win_bytes + (size_t)n * 5 +
+                        lcnt_bytes + bcnt_bytes + 256 + 10 * 256;
     if (t->scratch && t->scratch_bytes >= need && t->S.list_cap >= n && t->S.dedup_cap >= cap)
         return DYC_OK;
     if (t->scratch) {
@@ -260,6 +263,11 @@ dyc_status ensure_scratch(dyc_table *t, uint64_t n) {
     t->S.list_cap = n;
     t->S.winbits = (uint32_t *)carve(win_bytes);
     t->S.dupseen = (uint32_t *)carve(4);
+    t->S.bin_count = (uint32_t *)carve(bcnt_bytes);
+    t->S.left_idx = (uint32_t *)carve((size_t)n * 4);
+    t->S.left_ops = (uint8_t *)carve((size_t)n);
+    t->S.left_bits = (uint32_t *)carve(win_bytes);
+    t->S.left_cnt = (uint32_t *)carve(lcnt_bytes);
     return DYC_OK;
 }
 
@@ -268,9 +276,8 @@ dyc_status reset_call_counters(dyc_table *t, cudaStream_t s) {
     return DYC_OK;
 }
 
-dyc_status read_counters(dyc_table *t, cudaStream_t s) {
-    CK(cudaMemcpyAsync(t->h_ctr, t->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+// The counters a finished chunk left in h_ctr: errors, and the table's size.
+dyc_status check_counters(dyc_table *t) {
     if (t->h_ctr->spill)
         return fail(DYC_EOVERFLOW, "internal list overflow (%llu entries)",
                     (unsigned long long)t->h_ctr->spill);
@@ -279,6 +286,12 @@ dyc_status read_counters(dyc_table *t, cudaStream_t s) {
                     (unsigned long long)t->h_ctr->timeouts);
     t->size = t->h_ctr->size;
     return DYC_OK;
+}
+
+dyc_status read_counters(dyc_table *t, cudaStream_t s) {
+    CK(cudaMemcpyAsync(t->h_ctr, t->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return check_counters(t);
 }
 
 // ---- entries held outside the table after a failed call -------------------
@@ -494,22 +507,76 @@ dyc_status dedup_chunk(dyc_table *t, const Scratch &S, const void *keys, uint64_
     return DYC_OK;
 }
 
-dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64_t n,
-                        uint32_t flags, cudaStream_t s) {
-    const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
-    const bool new_keys = (flags & DYC_FLAG_NEW_KEYS) != 0;
-    const Scratch S = chunk_scratch(t, n);
-    if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepLast, s));
-    else TRY(reset_call_counters(t, s));
-    cudaError_t e = KB_CALL(t, place, ctx(t, s), t->D, t->sb, S, use_dedup, new_keys, keys,
-                            vals, (uint32_t)t->vb, n, t->d_ctr);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "place kernel: %s", cudaGetErrorString(e));
-    // walks for the ops whose buckets were full: list_a -> list_b
-    e = KB_CALL(t, walk, ctx(t, s), t->D, t->sb, t->S.list_a, &t->d_ctr->pending, t->S.list_b,
-                &t->d_ctr->overflow, t->S.list_cap, t->cfg.max_evictions, true, t->d_ctr,
-                t->S.list_cap);
+// ---- chunks whose keys may repeat, by bins (dyc_bins.cuh) ------------------
+// The records of a chunk take the cells of the dedup table, which the general
+// path fills only after the ops that bins left over have been gathered. The
+// single bits of an insert or erase chunk are the winner bits the place and
+// erase kernels read.
+bool bins_ok(const dyc_table *t) { return t->D.l2_keep == 0u; }  // k_bin_small carries no L2 hints
+
+dyc::BinScratch chunk_bins(const dyc_table *t, uint64_t n, uint32_t *single) {
+    const bool small = n <= dyc::kBinSmallOps;
+    dyc::BinScratch B{};
+    B.rec = (unsigned long long *)t->S.dedup;
+    B.count = t->S.bin_count;
+    B.nbins = (uint32_t)(small ? (n + dyc::kBinSmallMean - 1) / dyc::kBinSmallMean
+                               : n / dyc::kBinMean);
+    B.cap = small ? dyc::kSmallCap : dyc::kBinCap;
+    B.single = small ? nullptr : single;
+    return B;
+}
+
+// Find the repeated keys of a chunk of more than kBinSmallOps ops.
+dyc_status bins_group(dyc_table *t, const dyc::BinScratch &B, const dyc::ApplyScratch &A, int mode,
+                      const uint8_t *ops, const void *keys, uint32_t *bits_out, uint64_t n,
+                      cudaStream_t s) {
+    const cudaError_t e = KB_CALL(t, bin_group, ctx(t, s), B, A, mode, ops, keys, bits_out, n,
+                                  t->d_ctr);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "bin kernels: %s", cudaGetErrorString(e));
+    return DYC_OK;
+}
+
+// Eviction walks of the entries the probe kernels left without a slot.
+dyc_status walk_pending(dyc_table *t, cudaStream_t s) {
+    const cudaError_t e = KB_CALL(t, walk, ctx(t, s), t->D, t->sb, t->S.list_a, &t->d_ctr->pending,
+                                  t->S.list_b, &t->d_ctr->overflow, t->S.list_cap,
+                                  t->cfg.max_evictions, true, t->d_ctr, t->S.list_cap);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "walk kernel: %s", cudaGetErrorString(e));
-    TRY(read_counters(t, s));
+    return DYC_OK;
+}
+
+// A batch of up to kBinSmallOps ops: one kernel, which leaves its counters in
+// h_ctr and places a few entries without a slot on its own; more of them take
+// a walk kernel.
+dyc_status bins_small(dyc_table *t, const dyc::BinScratch &B, int mode, const uint8_t *ops,
+                      const void *keys, const void *vals, void *vals_out, uint32_t *bits_out,
+                      uint64_t n, uint32_t flags, cudaStream_t s) {
+    const cudaError_t e = KB_CALL(t, bin_small, ctx(t, s), t->D, t->sb, t->S, B, mode, ops, keys,
+                                  vals, (uint32_t)t->vb, vals_out, bits_out, n, flags, t->d_ctr,
+                                  t->h_ctr);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "bin kernel: %s", cudaGetErrorString(e));
+    CK(cudaStreamSynchronize(s));
+    TRY(check_counters(t));
+    if (t->h_ctr->pending == 0) return DYC_OK;
+    TRY(walk_pending(t, s));
+    return read_counters(t, s);
+}
+
+// Gather the ops of the bins that went over, keys and values into list_b
+// (read before the eviction walks write there).
+dyc_status bins_left(dyc_table *t, const dyc::BinScratch &B, const uint8_t *ops, const void *keys,
+                     const void *vals, uint64_t n, void **lk, void **lv, cudaStream_t s) {
+    *lk = t->S.list_b;
+    *lv = (char *)t->S.list_b + (((size_t)t->S.list_cap * t->kb + 7) & ~(size_t)7);
+    const cudaError_t e = KB_CALL(t, left_gather, ctx(t, s), t->S, B, ops, keys, vals,
+                                  (uint32_t)t->vb, n, *lk, *lv);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "gather kernels: %s", cudaGetErrorString(e));
+    return DYC_OK;
+}
+
+// After the counters of an insert pass are in h_ctr: the call's stats, and the
+// entries whose walks reached their bound.
+dyc_status insert_finish(dyc_table *t, cudaStream_t s) {
     const Counters c = *t->h_ctr;
     dyc_op_stats &L = t->last;
     L.inserted += c.inserted;
@@ -527,18 +594,101 @@ dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64
     return DYC_OK;
 }
 
-dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits,
-                       uint32_t flags, cudaStream_t s) {
-    const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
+// One pass over n ops with the scratch S naming the op of each key that
+// counts (use_dedup) or with distinct keys; `left` ops are not its own.
+dyc_status insert_pass(dyc_table *t, const Scratch &S, const void *keys, const void *vals,
+                       uint64_t n, bool use_dedup, bool new_keys, cudaStream_t s) {
+    cudaError_t e = KB_CALL(t, place, ctx(t, s), t->D, t->sb, S, use_dedup, new_keys, keys,
+                            vals, (uint32_t)t->vb, n, t->d_ctr);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "place kernel: %s", cudaGetErrorString(e));
+    // walks for the ops whose buckets were full: list_a -> list_b
+    TRY(walk_pending(t, s));
+    TRY(read_counters(t, s));
+    t->h_ctr->superseded -= t->h_ctr->left;  // ops of bins that went over won nothing yet
+    return insert_finish(t, s);
+}
+
+// n ops by the batch dedup table, or with distinct keys.
+dyc_status insert_general(dyc_table *t, const void *keys, const void *vals, uint64_t n,
+                          bool use_dedup, bool new_keys, cudaStream_t s) {
     const Scratch S = chunk_scratch(t, n);
-    if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepFirst, s));
+    if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepLast, s));
     else TRY(reset_call_counters(t, s));
+    return insert_pass(t, S, keys, vals, n, use_dedup, new_keys, s);
+}
+
+// The scratch with the winner bits the bins left (no dedup table to look at).
+Scratch bins_scratch(const dyc_table *t) {
+    Scratch S = t->S;
+    S.dedup_cap = std::max(S.dedup_cap, dyc::kWinnersMinCap);
+    S.dupseen = nullptr;
+    return S;
+}
+
+dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64_t n,
+                        uint32_t flags, cudaStream_t s) {
+    const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
+    const bool new_keys = (flags & DYC_FLAG_NEW_KEYS) != 0;
+    if (!use_dedup || !bins_ok(t)) return insert_general(t, keys, vals, n, use_dedup, new_keys, s);
+    const dyc::BinScratch B = chunk_bins(t, n, t->S.winbits);
+    if (B.single == nullptr) {
+        TRY(bins_small(t, B, dyc::kBinModeInsert, nullptr, keys, vals, nullptr, nullptr, n,
+                       new_keys ? (uint32_t)dyc::kBinNewKeys : 0u, s));
+        TRY(insert_finish(t, s));
+    } else {
+        TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeInsert, nullptr, keys, nullptr, n, s));
+        TRY(insert_pass(t, bins_scratch(t), keys, vals, n, true, new_keys, s));
+    }
+    const uint64_t left = t->h_ctr->left;
+    if (left == 0) return DYC_OK;
+    void *lk, *lv;
+    TRY(bins_left(t, B, nullptr, keys, vals, n, &lk, &lv, s));
+    return insert_general(t, lk, lv, left, true, new_keys, s);
+}
+
+dyc_status erase_pass(dyc_table *t, const Scratch &S, const void *keys, uint64_t n, uint32_t *bits,
+                      bool use_dedup, cudaStream_t s) {
     cudaError_t e = KB_CALL(t, erase, ctx(t, s), t->D, t->sb, S, use_dedup, keys, n, bits,
                             t->d_ctr);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "erase kernel: %s", cudaGetErrorString(e));
     TRY(read_counters(t, s));
     t->last.erased += t->h_ctr->erased;
-    t->last.superseded += t->h_ctr->superseded;
+    t->last.superseded += t->h_ctr->superseded - t->h_ctr->left;
+    return DYC_OK;
+}
+
+dyc_status erase_general(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits,
+                         bool use_dedup, cudaStream_t s) {
+    const Scratch S = chunk_scratch(t, n);
+    if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepFirst, s));
+    else TRY(reset_call_counters(t, s));
+    return erase_pass(t, S, keys, n, bits, use_dedup, s);
+}
+
+dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits,
+                       uint32_t flags, cudaStream_t s) {
+    const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
+    if (!use_dedup || !bins_ok(t)) return erase_general(t, keys, n, bits, use_dedup, s);
+    const dyc::BinScratch B = chunk_bins(t, n, t->S.winbits);
+    if (B.single == nullptr) {
+        TRY(bins_small(t, B, dyc::kBinModeErase, nullptr, keys, nullptr, nullptr, bits, n, 0u, s));
+        t->last.erased += t->h_ctr->erased;
+        t->last.superseded += t->h_ctr->superseded;
+    } else {
+        TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeErase, nullptr, keys, nullptr, n, s));
+        TRY(erase_pass(t, bins_scratch(t), keys, n, bits, true, s));
+    }
+    const uint64_t left = t->h_ctr->left;
+    if (left == 0) return DYC_OK;
+    void *lk, *lv;
+    TRY(bins_left(t, B, nullptr, keys, nullptr, n, &lk, &lv, s));
+    TRY(erase_general(t, lk, left, bits ? t->S.left_bits : nullptr, true, s));
+    if (bits) {
+        const cudaError_t e = KB_CALL(t, left_return, ctx(t, s), t->S, left, nullptr,
+                                      (uint32_t)t->vb, nullptr, bits);
+        if (e != cudaSuccess) return fail(DYC_ECUDA, "return kernel: %s", cudaGetErrorString(e));
+        CK(cudaStreamSynchronize(s));
+    }
     return DYC_OK;
 }
 
@@ -1227,30 +1377,115 @@ dyc_status read_apply_counters(dyc_table *t, cudaStream_t s) {
     return DYC_OK;
 }
 
-// A chunk of n mixed ops: grouping, scatter and replay (dyc_apply.cuh), then
-// the table-set probe kernels (dyc_set.cuh) with this table's one-entry
-// descriptor array: the find of the distinct keys, one pass for the erases
-// and upserts, the eviction walks. Every kernel reads its item count on the
-// device, so the host reads the counters once, at the end. The upsize
-// policy (api.cpp:359-369: the size after the batch's erases plus its
+// How a chunk of mixed ops finds its repeated keys, and what resolves the
+// others.
+enum class ApplyPath {
+    kBins,    // k_bin_group lists the repeated keys; the one-pass kernel takes the others
+    kSingle,  // k_apply_group and compaction list them; the one-pass kernel takes the others
+    kAll      // k_apply_group and compaction list every key
+};
+
+// n mixed ops: the keys with several ops listed with their segments, the find
+// of those keys, the replays (dyc_apply.cuh), the one-pass kernel for every
+// other op (one probe of its key's buckets; it touches no key the others do),
+// then the erases and upserts of the listed keys and the eviction walks
+// (dyc_set.cuh, with this table's one-entry descriptor array). Every kernel
+// reads its item count on the device, so the host reads the counters once, at
+// the end (in h_ctr when this returns).
+// policy(upserts, erases): the upsize policy where the table must grow before
+// the batch (before); a counting pass over the other ops then runs first and
+// the host reads both kinds' counts. Ops of bins that went over are left
+// untouched, counted in h_ctr->left; with `before` nothing else has been
+// applied then.
+template <class F>
+dyc_status apply_kernels(dyc_table *t, ApplyPath path, const dyc::BinScratch &B, const uint8_t *ops,
+                         const void *keys, const void *vals, uint64_t n, void *vals_out,
+                         uint32_t *bits_out, bool before, cudaStream_t s, F &&policy) {
+    const dyc::ApplyScratch &A = t->A;
+    const LaunchCtx L = ctx(t, s);
+    const uint32_t vb = (uint32_t)t->vb;
+    const bool bins = path == ApplyPath::kBins;
+    dyc::ApplyScratch Ag = A;
+    if (path == ApplyPath::kSingle) {
+        // a batch in which no key repeats (k_apply_group sets the gate) skips
+        // compaction and the scatter; later kernels read counts left at 0
+        Ag.gate = &A.ctr[dyc::kCtrRepeat];
+        Ag.single_pass = 1u;
+    }
+    TRY(push_desc(t, s));
+    cudaError_t e = cudaSuccess;
+    if (bins) {
+        TRY(bins_group(t, B, A, dyc::kBinModeMixed, ops, keys, bits_out, n, s));
+    } else {
+        TRY(reset_call_counters(t, s));
+        CK(cudaMemsetAsync(A.cells, 0, (size_t)(2 * n) * (t->kb == 4 ? 8 : 16), s));  // 2n cells used
+        CK(cudaMemsetAsync(A.ctr, 0, dyc::kCtrSlots * sizeof(unsigned long long), s));
+        if (bits_out) CK(cudaMemsetAsync(bits_out, 0, (size_t)((n + 31) / 32) * 4, s));
+        e = KB_CALL(t, apply_group, L, Ag, keys, n);
+    }
+    // state of every listed key before the batch
+    if (e == cudaSuccess)
+        e = KB_CALL(t, set_find, L, t->d_desc, 1u, t->sb, A.dkey, nullptr,
+                    &A.ctr[dyc::kCtrDistinct], n, A.pre_val, vb, A.pre_hit, &A.ctr[dyc::kCtrBad],
+                    t->D.l2_keep != 0u);
+    if (e == cudaSuccess && !bins)
+        e = KB_CALL(t, apply_scatter, L, Ag, n, nullptr, ops, vals, vb, vals_out, bits_out);
+    if (e == cudaSuccess) e = KB_CALL(t, apply_replay, L, Ag, ops, vals, vb, vals_out, bits_out, n, n);
+    if (e == cudaSuccess && before) {
+        if (bins)
+            e = KB_CALL(t, apply_count, L, t->D, t->sb, ops, keys, vals, vb, n, B.single, t->d_ctr);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(t->h_actr, A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
+                                cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) return fail(DYC_ECUDA, "apply kernels: %s", cudaGetErrorString(e));
+        TRY(read_counters(t, s));
+        if (t->h_ctr->left) return DYC_OK;  // the policy needs every op's count
+        TRY(policy(t->h_actr[dyc::kCtrUp] + t->h_ctr->nins, t->h_actr[dyc::kCtrEr] + t->h_ctr->erased));
+        TRY(push_desc(t, s));
+        TRY(reset_call_counters(t, s));
+    }
+    if (e == cudaSuccess && path != ApplyPath::kAll)
+        e = KB_CALL(t, apply_unique, L, t->D, t->sb, t->S, ops, keys, vals, vb, vals_out, bits_out,
+                    n, t->d_ctr, bins ? B.single : A.single, Ag.gate,
+                    before ? (uint32_t)dyc::kBinSkipEqual : 0u);
+    if (e == cudaSuccess)
+        e = KB_CALL(t, set_mutate, L, t->d_desc, 1u, t->d_ctr, t->sb, A.er_key, nullptr,
+                    &A.ctr[dyc::kCtrEr], A.up_key, A.up_val, vb, nullptr, &A.ctr[dyc::kCtrUp], n,
+                    t->S.list_a, nullptr, t->S.list_cap, t->d_ctr, &A.ctr[dyc::kCtrBad], nullptr,
+                    t->D.l2_keep != 0u);
+    if (e == cudaSuccess)
+        e = KB_CALL(t, set_walk, L, t->d_desc, 1u, t->d_ctr, t->sb, t->S.list_a, nullptr,
+                    &t->d_ctr->pending, t->S.list_b, nullptr, &t->d_ctr->overflow,
+                    t->S.list_cap, t->cfg.max_evictions, t->d_ctr, t->S.list_cap,
+                    &A.ctr[dyc::kCtrBad]);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "apply kernels: %s", cudaGetErrorString(e));
+    CK(cudaMemcpyAsync(t->h_actr, A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
+                       cudaMemcpyDeviceToHost, s));
+    TRY(read_counters(t, s));
+    if (t->h_actr[dyc::kCtrBad])
+        return fail(DYC_ECUDA, "mixed batch: %llu device counts or ids out of range",
+                    t->h_actr[dyc::kCtrBad]);
+    return DYC_OK;
+}
+
+// A chunk of n mixed ops, by bins (dyc_bins.cuh); ops of bins that went over,
+// and the chunks of tables the bin kernels do not serve, by grouping. The
+// upsize policy (api.cpp:359-369: the size after the batch's erases plus its
 // inserts above upper bound x capacity) needs the batch's upsert and erase
 // counts: where even n inserts keep the table within deferred_fill() of its
 // slots it is applied after the batch with the same counts, so the capacity
 // ends as if it had run first (entries the fuller table could not place
-// take the overflow path); otherwise the host reads the counts after the
-// replay and upsizes first.
+// take the overflow path); otherwise the counts are taken first, the host
+// reads them and upsizes, and the batch is applied after that.
 dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const void *vals,
                        uint64_t n, void *vals_out, uint32_t *bits_out, uint32_t flags,
                        cudaStream_t s) {
-    const dyc::ApplyScratch &A = t->A;
-    const LaunchCtx L = ctx(t, s);
-    const uint32_t vb = (uint32_t)t->vb;
     const bool resize = t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE);
-    const bool deferred = !resize || (double)(t->size + n) <= deferred_fill(t) * (double)t->capacity;
+    const bool before = resize && (double)(t->size + n) > deferred_fill(t) * (double)t->capacity;
     const uint64_t size0 = t->size;
     bool grew = false;
     // nu upserts and ne erases of present keys
-    auto upsize_policy = [&](uint64_t nu, uint64_t ne) -> dyc_status {
+    auto policy = [&](uint64_t nu, uint64_t ne) -> dyc_status {
         int guard = 0;
         while (resize && nu &&
                (double)size0 - (double)ne + (double)nu > t->cfg.upper_load * (double)t->capacity &&
@@ -1260,74 +1495,66 @@ dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const
         }
         return DYC_OK;
     };
-    // With the policy deferred, keys with a single op in the chunk (most keys
-    // of a random batch) skip the per-key passes: compaction lists only keys
-    // with several ops, the find, scatter, replays and mutation handle those,
-    // and after the replays the one-pass kernel resolves every other op in
-    // one probe of its key's buckets (it touches no key the others do). A
-    // chunk in which no key repeats (k_apply_group sets the gate) skips
-    // compaction and the scatter altogether. The host reads nothing in
-    // between; later kernels read counts the skipped ones leave at 0.
-    dyc::ApplyScratch Ag = A;
-    if (deferred) {
-        Ag.gate = &A.ctr[dyc::kCtrRepeat];
-        Ag.single_pass = 1u;
-    }
-    TRY(push_desc(t, s));
-    TRY(reset_call_counters(t, s));
-    CK(cudaMemsetAsync(A.cells, 0, (size_t)(2 * n) * (t->kb == 4 ? 8 : 16), s));  // 2n cells used
-    CK(cudaMemsetAsync(A.ctr, 0, dyc::kCtrSlots * sizeof(unsigned long long), s));
-    if (bits_out) CK(cudaMemsetAsync(bits_out, 0, (size_t)((n + 31) / 32) * 4, s));
-    cudaError_t e = KB_CALL(t, apply_group, L, Ag, keys, n);
-    // state of every distinct key before the batch
-    if (e == cudaSuccess)
-        e = KB_CALL(t, set_find, L, t->d_desc, 1u, t->sb, A.dkey, nullptr,
-                    &A.ctr[dyc::kCtrDistinct], n, A.pre_val, vb, A.pre_hit, &A.ctr[dyc::kCtrBad],
-                    t->D.l2_keep != 0u);
-    if (e == cudaSuccess)
-        e = KB_CALL(t, apply_scatter, L, Ag, n, nullptr, ops, vals, vb, vals_out, bits_out);
-    if (e == cudaSuccess) e = KB_CALL(t, apply_replay, L, Ag, ops, vals, vb, vals_out, bits_out, n, n);
-    if (e == cudaSuccess && deferred)
-        e = KB_CALL(t, apply_unique, L, t->D, t->sb, t->S, ops, keys, vals, vb, vals_out, bits_out,
-                    n, t->d_ctr, A.single, Ag.gate);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "apply kernels: %s", cudaGetErrorString(e));
-    if (!deferred) {
-        TRY(read_apply_counters(t, s));
-        TRY(upsize_policy(t->h_actr[dyc::kCtrUp], t->h_actr[dyc::kCtrEr]));
-        if (grew) TRY(push_desc(t, s));
-    }
-    e = KB_CALL(t, set_mutate, L, t->d_desc, 1u, t->d_ctr, t->sb, A.er_key, nullptr,
-                &A.ctr[dyc::kCtrEr], A.up_key, A.up_val, vb, nullptr, &A.ctr[dyc::kCtrUp], n,
-                t->S.list_a, nullptr, t->S.list_cap, t->d_ctr, &A.ctr[dyc::kCtrBad], nullptr,
-                t->D.l2_keep != 0u);
-    if (e == cudaSuccess)
-        e = KB_CALL(t, set_walk, L, t->d_desc, 1u, t->d_ctr, t->sb, t->S.list_a, nullptr,
-                    &t->d_ctr->pending, t->S.list_b, nullptr, &t->d_ctr->overflow,
-                    t->S.list_cap, t->cfg.max_evictions, t->d_ctr, t->S.list_cap,
-                    &A.ctr[dyc::kCtrBad]);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "apply probe kernels: %s", cudaGetErrorString(e));
-    CK(cudaMemcpyAsync(t->h_actr, A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
-                       cudaMemcpyDeviceToHost, s));
-    TRY(read_counters(t, s));
-    if (t->h_actr[dyc::kCtrBad])
-        return fail(DYC_ECUDA, "mixed batch: %llu device counts or ids out of range",
-                    t->h_actr[dyc::kCtrBad]);
-    const Counters c = *t->h_ctr;
-    // both paths' upserts and erases of present keys, as the table counted
-    // them (the one-pass kernel counts an insert on a present key as an
-    // update even when the value is the same)
-    if (deferred) TRY(upsize_policy(c.inserted + c.updated, c.erased));
     dyc_op_stats &St = t->last;
+    const dyc::BinScratch B = chunk_bins(t, n, t->A.single);
+    bool bins = bins_ok(t);
+    if (bins && B.single == nullptr) {  // a small batch
+        if (before) {
+            TRY(bins_small(t, B, dyc::kBinModeCount, ops, keys, vals, nullptr, nullptr, n, 0u, s));
+            if (t->h_ctr->left) bins = false;  // the policy needs every op's count
+            else TRY(policy(t->h_ctr->nins, t->h_ctr->erased));
+        }
+        if (bins)
+            TRY(bins_small(t, B, dyc::kBinModeMixed, ops, keys, vals, vals_out, bits_out, n,
+                           before ? (uint32_t)dyc::kBinSkipEqual : 0u, s));
+    } else if (bins) {
+        TRY(apply_kernels(t, ApplyPath::kBins, B, ops, keys, vals, n, vals_out, bits_out, before, s,
+                          policy));
+        if (before && t->h_ctr->left) bins = false;
+    }
+    if (!bins)
+        TRY(apply_kernels(t, before ? ApplyPath::kAll : ApplyPath::kSingle, B, ops, keys, vals, n,
+                          vals_out, bits_out, before, s, policy));
+    Counters c = *t->h_ctr;
+    if (const uint64_t left = bins ? c.left : 0) {
+        if (c.overflow) {  // its list is used again below
+            St.overflowed += c.overflow;
+            TRY(drain(t, s, t->S.list_b, &t->d_ctr->overflow, t->S.list_a, &t->d_ctr->pending,
+                      t->S.list_cap, true, true));
+            grew = true;
+            c = *t->h_ctr;
+            c.overflow = 0;
+        }
+        void *lk, *lv, *lo = vals_out ? t->S.dedup : nullptr;
+        TRY(bins_left(t, B, ops, keys, vals, n, &lk, &lv, s));
+        TRY(apply_kernels(t, ApplyPath::kSingle, B, t->S.left_ops, lk, lv, left, lo,
+                          bits_out ? t->S.left_bits : nullptr, false, s,
+                          [](uint64_t, uint64_t) { return DYC_OK; }));
+        const cudaError_t e = KB_CALL(t, left_return, ctx(t, s), t->S, left, lo, (uint32_t)t->vb,
+                                      vals_out, bits_out);
+        if (e != cudaSuccess) return fail(DYC_ECUDA, "return kernel: %s", cudaGetErrorString(e));
+        CK(cudaStreamSynchronize(s));
+        c.inserted += t->h_ctr->inserted;
+        c.updated += t->h_ctr->updated;
+        c.erased += t->h_ctr->erased;
+        c.evict_steps += t->h_ctr->evict_steps;
+        c.overflow += t->h_ctr->overflow;
+    }
+    // both kinds of keys' upserts and erases of present keys, as the table
+    // counted them (an insert of the only op of its key counts as an update
+    // even when the value is the same)
+    if (!before) TRY(policy(c.inserted + c.updated, c.erased));
     St.inserted += c.inserted;
     St.updated += c.updated;
     St.erased += c.erased;
     St.evict_steps += c.evict_steps;
     St.overflowed += c.overflow;
     if (c.overflow) {
+        const Counters at = *t->h_ctr;
         TRY(drain(t, s, t->S.list_b, &t->d_ctr->overflow, t->S.list_a, &t->d_ctr->pending,
                   t->S.list_cap, true, !grew));
-        St.inserted += t->h_ctr->inserted - c.inserted;
-        St.evict_steps += t->h_ctr->evict_steps - c.evict_steps;
+        St.inserted += t->h_ctr->inserted - at.inserted;
+        St.evict_steps += t->h_ctr->evict_steps - at.evict_steps;
     }
     return DYC_OK;
 }

@@ -893,7 +893,7 @@ __global__ void __launch_bounds__(256) k_apply_unique(
     const uint8_t *__restrict__ ops, const void *__restrict__ keys,
     const void *__restrict__ vals, uint32_t vb, void *__restrict__ vals_out,
     uint32_t *__restrict__ bits_out, uint64_t n, Counters *ctr, const uint32_t *single,
-    const unsigned long long *gate) {
+    const unsigned long long *gate, uint32_t flags) {
     using T = SlotT<KB>;
     using Sl = typename T::S;
     using Gm = Geo<KB, SB>;
@@ -940,7 +940,9 @@ __global__ void __launch_bounds__(256) k_apply_unique(
         const uint64_t before = found1 ? r1.value : (found2 ? r2.value : 0ull);
         bool pend = false;
         if (ins) {
-            if (found1) {
+            if (present && (flags & kBinSkipEqual) && before == T::val(e)) {
+                // the key's value stays: neither written nor counted
+            } else if (found1) {
                 T::store(slot_ptr<KB, SB>(p1, r1.match), e);
                 ++n_upd;
             } else if (found2) {
@@ -991,6 +993,65 @@ __global__ void __launch_bounds__(256) k_apply_unique(
         if (s_sum[2]) atomicAdd(&ctr->erased, s_sum[2]);
         const long long net = (long long)s_sum[0] - (long long)s_sum[2];
         if (net) atomicAdd(&ctr->size, (unsigned long long)net);  // size += inserted - erased
+    }
+}
+
+// The upserts and erases k_apply_unique would make (with kBinSkipEqual) for
+// the ops whose single bit is set: a batch whose upsize policy needs the counts
+// first. Finds are not probed.
+template <int KB, int SB>
+__global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_apply_count(
+    const __grid_constant__ Desc D, const uint8_t *__restrict__ ops, const void *__restrict__ keys,
+    const void *__restrict__ vals, uint32_t vb, uint64_t n, const uint32_t *__restrict__ single,
+    Counters *ctr) {
+    using T = SlotT<KB>;
+    using Gm = Geo<KB, SB>;
+    __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
+    unsigned char *stage = s_stage[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t step = warp_stride();
+    uint32_t n_up = 0, n_er = 0;
+    for (uint64_t base = warp_base(); base < n; base += step) {
+        const uint64_t i = base + lane;
+        typename T::K k = 0;
+        uint8_t op = kOpFind;
+        if (i < n && ((single[i >> 5] >> lane) & 1u)) {
+            op = ops[i];
+            if (op == kOpInsert || op == kOpErase) k = load_key<KB>(keys, i);
+        }
+        const bool act = k != 0;
+        const uint64_t v = act && op == kOpInsert ? load_val(vals, vb, i) : 0ull;
+        const uint32_t hk = fold(k);
+        const Pair p = pair_of(hk, D.d);
+        const char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
+        const KvOut r1 = kv_probe<KB, SB, 1>(p1, k, act, stage);
+        bool hit = act && r1.match >= 0;
+        uint64_t before = r1.value;
+        const bool need2 = act && !hit && (!Gm::kMeta || r1.overflow);
+        if (__any_sync(kFull, need2)) {
+            const char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
+            const KvOut r2 = kv_probe<KB, SB, 1>(p2, k, need2, stage);
+            if (need2 && r2.match >= 0) {
+                hit = true;
+                before = r2.value;
+            }
+        }
+        if (act && op == kOpInsert && (!hit || before != v)) ++n_up;
+        if (act && op == kOpErase && hit) ++n_er;
+    }
+    __shared__ unsigned long long s_sum[2];
+    if (threadIdx.x < 2) s_sum[threadIdx.x] = 0ull;
+    __syncthreads();
+    n_up = __reduce_add_sync(kFull, n_up);
+    n_er = __reduce_add_sync(kFull, n_er);
+    if (lane == 0) {
+        if (n_up) atomicAdd(&s_sum[0], (unsigned long long)n_up);
+        if (n_er) atomicAdd(&s_sum[1], (unsigned long long)n_er);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_sum[0]) atomicAdd(&ctr->nins, s_sum[0]);
+        if (s_sum[1]) atomicAdd(&ctr->erased, s_sum[1]);
     }
 }
 

@@ -1,0 +1,698 @@
+// dyc_bins.cuh -- the repeated keys of a batch, found bin by bin in shared
+// memory (inserts, erases and mixed batches of one table).
+//
+// A chunk's ops are split by a hash of their key into bins of about 1024
+// (k_bin_scatter), and one block per bin finds the keys that occur more than
+// once with a key table in shared memory (k_bin_group). Every other op keeps
+// its bit in a bitmap and is resolved by the probe kernels in op order, with
+// coalesced batch reads and results. The open-addressing table in global
+// memory that this replaces as the first choice took one random L2 or DRAM
+// atomic per op over 64 MB of cells (99-113 us for 2^22 ops), a pass over the
+// cells (23-28 us) and, for mixed batches, a second random read per op (56
+// us); the split is bound by its 8-byte stores to random sectors (36 us, of
+// which 5 us is the bytes) and the grouping by shared-memory atomics (26-39
+// us). 2^24 mixed ops on 2^27 keys: 3.61 -> 2.78 ms a pair of batches.
+//
+// Splitting by the region of a key's first bucket instead, so that a bin's
+// probes fall close together, and probing from the bins in the same kernel,
+// both measured slower: neighbouring lines gained 4 %, and the values, result
+// words and bits at random places cost more than that (312 us against 47 + 39
+// + 187 for 2^22 mixed ops).
+//
+// Up to 16384 ops run as one kernel (k_bin_small): every block reads the whole
+// batch, keeps its bin's ops and resolves them itself, and the last block
+// writes the counters to the host. A mixed batch of 4096 ops took ten
+// kernels, four memsets and two copies: 97 -> 41 us a call.
+//
+// A bin with more ops than its capacity (few keys, each repeated hundreds of
+// times) is left, as a whole, to the general path: its keys meet no key of
+// another bin.
+#pragma once
+
+#include "dyc_apply.cuh"
+
+namespace dyc {
+
+constexpr int kSmallR = kSmallCap / kBlockThreads;  // records per thread (k_bin_small)
+constexpr int kSmallTab = 2 * kSmallCap;            // cells of a bin's key table
+constexpr int kGroupThreads = 512;
+constexpr int kGroupR = kBinCap / kGroupThreads;    // records per thread (k_bin_group)
+constexpr int kGroupTab = 2 * kBinCap;
+
+// An op of a bin: index << 2 | code (2 bits; any other code reads).
+__device__ __forceinline__ uint32_t op_word(uint64_t i, uint8_t op) {
+    return ((uint32_t)i << 2) | (op == kOpInsert ? 1u : op == kOpErase ? 2u : 0u);
+}
+
+template <int KB>
+__device__ __forceinline__ uint32_t bin_of(typename SlotT<KB>::K k, uint32_t nbins) {
+    return __umulhi(cell_hash((uint64_t)k), nbins);
+}
+
+// What a record keeps of its key: a 4-byte key itself, or 32 mixed bits of an
+// 8-byte key (records with the same tag compare their keys in the batch).
+__device__ __forceinline__ uint32_t bin_tag(uint32_t k) { return k; }
+__device__ __forceinline__ uint32_t bin_tag(uint64_t k) {
+    return (uint32_t)k ^ ((uint32_t)(k >> 32) * 0x85EBCA6Bu);
+}
+
+// First cell of a tag in a bin's key table of 2^BITS cells.
+template <int BITS> __device__ __forceinline__ uint32_t bin_cell(uint32_t tag) {
+    return ((tag ^ (tag >> 15)) * 0x9E3779B1u) >> (32 - BITS);
+}
+
+// Zero a chunk's bin counts, the call counters, the batch counters and the
+// result bits; set its single bits.
+template <int KB>
+__global__ void __launch_bounds__(256) k_bin_clear(const __grid_constant__ BinScratch B,
+                                                   unsigned long long *zero, uint32_t nzero,
+                                                   unsigned long long *actr, uint32_t *bits,
+                                                   uint64_t words) {
+    const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = id; i < B.nbins; i += stride) B.count[i] = 0u;
+    if (id < nzero) zero[id] = 0ull;
+    if (actr != nullptr && id < (uint64_t)kCtrSlots) actr[id] = 0ull;
+    if (bits != nullptr)
+        for (uint64_t w = id; w < words; w += stride) bits[w] = 0u;
+    if (B.single != nullptr)
+        for (uint64_t w = id; w < words; w += stride) B.single[w] = 0xffffffffu;
+}
+
+__device__ __forceinline__ void clear_single(const BinScratch &B, uint32_t i) {
+    atomicAnd(&B.single[i >> 5], ~(1u << (i & 31)));
+}
+
+// Split a chunk into its bins: a block takes PER * 512 consecutive ops, counts
+// them per bin in shared memory (each op's place among the block's ops of its
+// bin comes back from the count), takes a range of every bin it has ops for,
+// and writes the ops' records there. Records of one bin come in no order; the
+// op index in the record orders the ops of a key. Ops beyond a bin's capacity
+// are not written (the count tells). Key-0 ops belong to no bin.
+template <int KB, int PER>
+__global__ void __launch_bounds__(512) k_bin_scatter(const __grid_constant__ BinScratch B,
+                                                     const uint8_t *__restrict__ ops,
+                                                     const void *__restrict__ keys, uint64_t n) {
+    using K = typename SlotT<KB>::K;
+    extern __shared__ uint32_t s_cnt[];  // nbins
+    const uint32_t nb = B.nbins;
+    for (uint32_t b = threadIdx.x; b < nb; b += 512) s_cnt[b] = 0u;
+    __syncthreads();
+    static_assert(PER * 512 <= 1 << 13, "a place among the block's ops takes 13 bits");
+    const uint64_t base = (uint64_t)blockIdx.x * (PER * 512) + threadIdx.x;
+    uint32_t tag[PER], at[PER];  // at: place | bin << 13 | op code << 26, ~0 for key 0
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint64_t i = base + (uint64_t)j * 512;
+        const K k = i < n ? load_key<KB>(keys, i) : (K)0;
+        const uint32_t code = op_word(0, (ops != nullptr && i < n) ? ops[i] : (uint8_t)kOpFind);
+        tag[j] = bin_tag(k);
+        at[j] = k != 0 ? bin_of<KB>(k, nb) << 13 | code << 26 : 0xffffffffu;
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+        if (at[j] != 0xffffffffu) at[j] |= atomicAdd(&s_cnt[(at[j] >> 13) & 0x1fffu], 1u);
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < nb; b += 512) {
+        const uint32_t c = s_cnt[b];
+        if (c) s_cnt[b] = atomicAdd(&B.count[b], c);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        if (at[j] == 0xffffffffu) continue;
+        const uint32_t b = (at[j] >> 13) & 0x1fffu;
+        const uint32_t p = s_cnt[b] + (at[j] & 0x1fffu);
+        const uint32_t i = (uint32_t)base + (uint32_t)j * 512u;
+        if (p < (uint32_t)kBinCap)
+            B.rec[(uint64_t)b * kBinCap + p] =
+                (unsigned long long)tag[j] | ((unsigned long long)(i << 2 | at[j] >> 26) << 32);
+        else
+            clear_single(B, i);
+    }
+}
+
+// One block per bin: its ops grouped by key in shared memory. Insert batches
+// keep the single bit of a key's last op, erase batches of its first. In a
+// mixed batch the ops of keys with several ops lose theirs and the keys are
+// listed: id d gets dkey, dcnt and dseg, and its op indexes a range of seg.
+template <int KB, int MODE>
+__global__ void __launch_bounds__(kGroupThreads) k_bin_group(const __grid_constant__ BinScratch B,
+                                                             const __grid_constant__ ApplyScratch A,
+                                                             const void *__restrict__ keys,
+                                                             Counters *ctr) {
+    using K = typename SlotT<KB>::K;
+    __shared__ uint32_t s_tag[kBinCap], s_word[kBinCap], s_cnt[kBinCap], s_tab[kGroupTab];
+    __shared__ uint32_t s_nseg, s_nkey, s_ok;
+    __shared__ unsigned long long s_bseg, s_bkey;
+    const uint32_t tid = threadIdx.x, bin = blockIdx.x;
+    const uint32_t m = B.count[bin];
+    const unsigned long long *rec = B.rec + (uint64_t)bin * kBinCap;
+    if (m > (uint32_t)kBinCap) {  // left to the general path
+        for (uint32_t r = tid; r < (uint32_t)kBinCap; r += kGroupThreads)
+            clear_single(B, (uint32_t)(rec[r] >> 32) >> 2);
+        if (tid == 0) atomicAdd(&ctr->left, (unsigned long long)m);
+        return;
+    }
+    for (uint32_t c = tid; c < (uint32_t)kGroupTab; c += kGroupThreads) s_tab[c] = 0u;
+#pragma unroll
+    for (int q = 0; q < kGroupR; ++q) {
+        const uint32_t r = q * kGroupThreads + tid;
+        s_cnt[r] = MODE == kBinModeErase ? 0xffffffffu : 0u;
+        if (r < m) {
+            const unsigned long long x = rec[r];
+            s_tag[r] = (uint32_t)x;
+            s_word[r] = (uint32_t)(x >> 32);
+        }
+    }
+    if (tid == 0) s_nseg = s_nkey = 0u;
+    __syncthreads();
+    uint32_t lr[kGroupR];  // first record of the key | rank << 16
+#pragma unroll
+    for (int q = 0; q < kGroupR; ++q) {
+        const uint32_t r = q * kGroupThreads + tid;
+        lr[q] = 0u;
+        if (r >= m) continue;
+        const uint32_t tag = s_tag[r], w = s_word[r];
+        uint32_t h = bin_cell<12>(tag), lead;
+        static_assert(kGroupTab == 1 << 12, "bin_cell takes 12 bits");
+        while (true) {  // at most half of the cells are taken: the probe ends
+            const uint32_t old = atomicCAS(&s_tab[h], 0u, r + 1u);
+            lead = old == 0u ? r : old - 1u;
+            if (old == 0u) break;
+            if (s_tag[lead] == tag &&
+                (KB == 4 || load_key<KB>(keys, s_word[lead] >> 2) == load_key<KB>(keys, w >> 2)))
+                break;
+            h = (h + 1u) & (kGroupTab - 1);
+        }
+        if (MODE == kBinModeInsert) atomicMax(&s_cnt[lead], w);
+        else if (MODE == kBinModeErase) atomicMin(&s_cnt[lead], w);
+        else lr[q] = atomicAdd(&s_cnt[lead], 1u) << 16;
+        lr[q] |= lead;
+    }
+    __syncthreads();
+    if constexpr (MODE != kBinModeMixed) {
+#pragma unroll
+        for (int q = 0; q < kGroupR; ++q) {
+            const uint32_t r = q * kGroupThreads + tid;
+            if (r < m && s_cnt[lr[q]] != s_word[r]) clear_single(B, s_word[r] >> 2);
+        }
+    } else {
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < kGroupR; ++q)
+            any |= q * kGroupThreads + tid < m && s_cnt[lr[q] & 0xffffu] > 1u;
+        if (!__syncthreads_or(any)) return;
+        // the table's cells now hold each key's place in its block's ranges
+#pragma unroll
+        for (int q = 0; q < kGroupR; ++q) {
+            const uint32_t r = q * kGroupThreads + tid;
+            if (r < m && (lr[q] & 0xffffu) == r && s_cnt[r] > 1u)
+                s_tab[r] = atomicAdd(&s_nseg, s_cnt[r]) | (atomicAdd(&s_nkey, 1u) << 16);
+        }
+        __syncthreads();
+        if (tid == 0) {
+            s_bkey = atomicAdd(&A.ctr[kCtrDistinct], (unsigned long long)s_nkey);
+            s_bseg = atomicAdd(&A.ctr[kCtrPlaced], (unsigned long long)s_nseg);
+            s_ok = s_bkey + s_nkey <= A.cap_ops && s_bseg + s_nseg <= A.cap_ops;
+            if (!s_ok) note_bad(A);
+        }
+        __syncthreads();
+        if (!s_ok) return;
+#pragma unroll
+        for (int q = 0; q < kGroupR; ++q) {
+            const uint32_t r = q * kGroupThreads + tid, lead = lr[q] & 0xffffu;
+            if (r >= m || s_cnt[lead] <= 1u) continue;
+            const uint32_t i = s_word[r] >> 2;
+            const uint32_t off = (uint32_t)s_bseg + (s_tab[lead] & 0xffffu);
+            A.seg[off + (lr[q] >> 16)] = i;
+            clear_single(B, i);
+            if (lead == r) {
+                const uint32_t d = (uint32_t)s_bkey + (s_tab[lead] >> 16);
+                ((K *)A.dkey)[d] = load_key<KB>(keys, i);
+                A.dcnt[d] = s_cnt[r];
+                A.dseg[d] = (unsigned long long)off << 32;
+            }
+        }
+    }
+}
+
+// Ascending sort of s[0..c) by one warp (mirrored bitonic merges: every
+// compare is ascending, so the places past c, read as larger than any word,
+// need no storage).
+__device__ __forceinline__ void warp_sort_words(uint32_t *s, uint32_t c) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t P = 2;
+    while (P < c) P <<= 1;
+    for (uint32_t k = 2; k <= P; k <<= 1) {
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t q = lane; q < P / 2; q += 32) {
+                // pair q of the stage: t below, u above
+                const uint32_t t = (q / j) * 2 * j + (q % j);
+                const uint32_t u = j == k >> 1 ? (t ^ (k - 1)) : t + j;
+                if (u < c) {
+                    const uint32_t a = s[t], b = s[u];
+                    if (a > b) {
+                        s[t] = b;
+                        s[u] = a;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Results of the sorted op words w[0..c) of one key by one warp, 32 ops a step
+// (as warp_replay): present / value carry the key's state.
+template <bool WRITE>
+__device__ __forceinline__ void warp_replay_words(const uint32_t *w, uint32_t c, bool &present,
+                                                  uint64_t &value, const void *__restrict__ vals,
+                                                  uint32_t vb, void *__restrict__ vals_out,
+                                                  uint32_t *__restrict__ bits_out) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t c0 = 0; c0 < c; c0 += 32) {
+        const bool v = c0 + lane < c;
+        const uint32_t x = v ? w[c0 + lane] : 0u, i = x >> 2, op = x & 3u;
+        const uint64_t myval = (v && op == 1u) ? load_val(vals, vb, i) : 0ull;
+        const unsigned mm = __ballot_sync(kFull, v && op != 0u);
+        const unsigned ins = __ballot_sync(kFull, v && op == 1u);
+        const unsigned before = mm & ((1u << lane) - 1u);
+        const int src = before ? 31 - __clz(before) : -1;
+        const uint64_t srcval = shfl64(myval, src < 0 ? lane : src);
+        bool st_present = present;
+        uint64_t st_value = value;
+        if (src >= 0) {
+            st_present = (ins >> src) & 1u;
+            st_value = st_present ? srcval : 0ull;
+        }
+        if (WRITE && v) {
+            if (vals_out) store_val(vals_out, vb, i, st_present ? st_value : 0ull);
+            if (st_present && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
+        }
+        if (mm) {
+            const int last = 31 - __clz(mm);
+            present = (ins >> last) & 1u;
+            const uint64_t lv = shfl64(myval, last);
+            value = present ? lv : 0ull;
+        }
+    }
+}
+
+constexpr uint32_t kBinShort = 8;   // ops of one key replayed by one lane
+constexpr uint32_t kTailWalk = 64;  // pending entries the last block places itself
+
+template <int KB, int SB> struct BinSmem {
+    alignas(128) unsigned char stage[kWarpsPerBlock][32 * SB];  // the key table before the probes
+    typename SlotT<KB>::K key[kSmallCap];
+    uint32_t word[kSmallCap];
+    uint32_t cnt[kSmallCap];  // per first op of a key: ops, then winner word or count | place << 16
+    uint32_t seg[kSmallCap];
+    uint16_t multi[kSmallCap / 2];
+    uint32_t m, nseg, nmulti, last;
+    unsigned long long sum[6];
+};
+
+// Place the pending entries of list_a (a few) by eviction walks, from the last
+// block of a small batch's kernel.
+template <int KB, int SB>
+__device__ __forceinline__ void tail_walk(const Desc &D, const Scratch &S, Counters *ctr, uint64_t np) {
+    using Sl = typename SlotT<KB>::S;
+    for (uint64_t i = threadIdx.x >> 5; i < np; i += kWarpsPerBlock) {
+        // written by other blocks of this kernel: read past the L1
+        const unsigned long long *src = (const unsigned long long *)((const Sl *)S.list_a + i);
+        Sl e;
+        if constexpr (KB == 4) e = __ldcg(src);
+        else e = Sl{__ldcg(src), __ldcg(src + 1)};
+        const WalkOut<KB> w = walk_lookahead<KB, SB>(D, e, D.max_evict);
+        if ((threadIdx.x & 31) != 0) continue;
+        if (w.steps) atomicAdd(&ctr->evict_steps, (unsigned long long)w.steps);
+        if (w.ok) {
+            atomicAdd(&ctr->inserted, 1ull);
+            atomicAdd(&ctr->size, 1ull);
+        } else {
+            const unsigned long long at = atomicAdd(&ctr->overflow, 1ull);
+            if (at < S.list_cap) ((Sl *)S.list_b)[at] = w.left;
+            else atomicAdd(&ctr->spill, 1ull);
+        }
+    }
+}
+
+// A small batch in one kernel: every block reads the whole batch, keeps the ops
+// of its bin, finds the repeated keys among them in shared memory and probes
+// the table; the last block to finish places the few entries left without a
+// slot and writes the counters to the host.
+template <int KB, int SB, int MODE>
+__global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
+    const __grid_constant__ Desc D, const __grid_constant__ Scratch S,
+    const __grid_constant__ BinScratch B, const uint8_t *__restrict__ ops,
+    const void *__restrict__ keys, const void *__restrict__ vals, uint32_t vb,
+    void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, uint64_t n, uint32_t flags,
+    Counters *ctr, Counters *h_ctr) {
+    using T = SlotT<KB>;
+    using K = typename T::K;
+    using Sl = typename T::S;
+    using Gm = Geo<KB, SB>;
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    BinSmem<KB, SB> &M = *reinterpret_cast<BinSmem<KB, SB> *>(s_raw);
+    uint32_t *tab = reinterpret_cast<uint32_t *>(M.stage);
+    static_assert(kSmallTab == 1 << 11, "bin_cell takes 11 bits");
+    static_assert(sizeof(M.stage) >= kSmallTab * sizeof(uint32_t), "the key table fits the stage");
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    unsigned char *stage = M.stage[tid >> 5];
+    const uint32_t bin = blockIdx.x;
+    uint32_t n_ins = 0, n_upd = 0, n_del = 0, n_sup = 0, n_rej = 0;
+
+    // the bin's records
+    for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kBlockThreads) tab[c] = 0u;
+    for (uint32_t c = tid; c < (uint32_t)kSmallCap; c += kBlockThreads)
+        M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
+    if (tid == 0) M.m = M.nseg = M.nmulti = 0u;
+    if (tid < 6) M.sum[tid] = 0ull;
+    __syncthreads();
+    uint32_t m;
+    {
+        const uint32_t own0 = (uint32_t)(((uint64_t)bin * n) / gridDim.x);
+        const uint32_t own1 = (uint32_t)(((uint64_t)(bin + 1) * n) / gridDim.x);
+#pragma unroll 8
+        for (uint64_t i = tid; i < n; i += kBlockThreads) {
+            const K k = load_key<KB>(keys, i);
+            if (k == 0) {  // belongs to no bin: one block answers it
+                if (i >= own0 && i < own1) {
+                    ++n_rej;
+                    if ((MODE == kBinModeMixed) && vals_out) store_val(vals_out, vb, i, 0ull);
+                }
+            } else if (bin_of<KB>(k, gridDim.x) == bin) {
+                const uint32_t r = atomicAdd(&M.m, 1u);
+                if (r < (uint32_t)kSmallCap) {
+                    M.key[r] = k;
+                    M.word[r] = (uint32_t)i << 2;
+                }
+            }
+        }
+        __syncthreads();
+        m = M.m;
+        if (tid == 0) B.count[bin] = m;
+        if (MODE >= kBinModeMixed && m <= (uint32_t)kSmallCap)
+            for (uint32_t r = tid; r < m; r += kBlockThreads)
+                M.word[r] = op_word(M.word[r] >> 2, ops[M.word[r] >> 2]);
+    }
+    __syncthreads();
+    const bool hot = m > (uint32_t)kSmallCap;  // left to the general path (uniform over the block)
+    if (hot) {
+        if (tid == 0) atomicAdd(&ctr->left, (unsigned long long)m);
+        m = 0u;
+    }
+
+    // group: each record finds its key's first record (lead)
+    K key[kSmallR];
+    uint32_t word[kSmallR], lead[kSmallR], rank[kSmallR];
+#pragma unroll
+    for (int q = 0; q < kSmallR; ++q) {
+        const uint32_t r = q * kBlockThreads + tid;
+        lead[q] = rank[q] = 0u;
+        word[q] = 0u;
+        key[q] = 0;
+        if (r >= m) continue;
+        key[q] = M.key[r];
+        word[q] = M.word[r];
+        uint32_t h = bin_cell<11>(bin_tag(key[q]));
+        // at most kSmallCap of the kSmallTab cells are taken: the probe ends
+        while (true) {
+            const uint32_t old = atomicCAS(&tab[h], 0u, r + 1u);
+            if (old == 0u) {
+                lead[q] = r;
+                break;
+            }
+            if (M.key[old - 1u] == key[q]) {
+                lead[q] = old - 1u;
+                break;
+            }
+            h = (h + 1u) & (kSmallTab - 1);
+        }
+        if (MODE == kBinModeInsert) atomicMax(&M.cnt[lead[q]], word[q]);
+        else if (MODE == kBinModeErase) atomicMin(&M.cnt[lead[q]], word[q]);
+        else rank[q] = atomicAdd(&M.cnt[lead[q]], 1u);
+    }
+    __syncthreads();  // the key table is done: the stage may be used
+
+    // keys with several ops: a range of seg each, their op words listed there
+    bool mine[kSmallR];
+    if constexpr (MODE >= kBinModeMixed) {
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < kSmallR; ++q) {
+            const uint32_t r = q * kBlockThreads + tid;
+            const uint32_t c = r < m ? M.cnt[lead[q]] : 0u;
+            mine[q] = c == 1u;
+            any |= c > 1u;
+        }
+        if (__syncthreads_or(any)) {
+#pragma unroll
+            for (int q = 0; q < kSmallR; ++q) {
+                const uint32_t r = q * kBlockThreads + tid;
+                if (r < m && !mine[q] && lead[q] == r) {
+                    const uint32_t c = M.cnt[r];
+                    M.cnt[r] = c | (atomicAdd(&M.nseg, c) << 16);
+                    M.multi[atomicAdd(&M.nmulti, 1u)] = (uint16_t)r;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < kSmallR; ++q) {
+                const uint32_t r = q * kBlockThreads + tid;
+                if (r < m && !mine[q]) M.seg[(M.cnt[lead[q]] >> 16) + rank[q]] = word[q];
+            }
+            __syncthreads();
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < kSmallR; ++q) {
+            const uint32_t r = q * kBlockThreads + tid;
+            mine[q] = r < m && M.cnt[lead[q]] == word[q];  // op indexes are distinct
+            if (r < m && !mine[q]) ++n_sup;
+        }
+    }
+
+    // keys with one op (the winning op of an insert or erase batch): one probe
+#pragma unroll
+    for (int q = 0; q < kSmallR; ++q) {
+        if ((uint32_t)(q * kBlockThreads) + (tid & ~31u) >= m) break;  // warp-uniform
+        const bool act = mine[q];
+        const uint32_t i = word[q] >> 2;
+        const uint32_t op = MODE == kBinModeInsert ? 1u : MODE == kBinModeErase ? 2u : (word[q] & 3u);
+        const bool ins = act && op == 1u, del = act && op == 2u;
+        Sl e = T::empty();
+        if (ins) e = T::make(key[q], load_val(vals, vb, i));
+        const uint32_t hk = fold(key[q]);
+        const Pair p = pair_of(hk, D.d);
+        char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
+        char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
+        const KvOut r1 = place_probe<KB, SB, false>(p1, key[q], act, p.first, D.d, stage);
+        const bool found1 = act && r1.match >= 0;
+        const bool want_slot = MODE != kBinModeCount && ins && r1.empty == 0u;
+        const bool may2 = !Gm::kMeta || r1.overflow;
+        const bool check2 =
+            act && !found1 && ((may2 && !(MODE == kBinModeInsert && (flags & kBinNewKeys))) || want_slot);
+        KvOut r2{-1, 0ull, false, 0u};
+        if (__any_sync(kFull, check2))
+            r2 = place_probe<KB, SB, false>(p2, key[q], check2, p.second, D.d, stage);
+        const bool found2 = check2 && r2.match >= 0;
+        const bool present = found1 || found2;
+        const uint64_t before = found1 ? r1.value : (found2 ? r2.value : 0ull);
+        if constexpr (MODE == kBinModeCount) {
+            if (ins && (!present || before != T::val(e))) ++n_ins;
+            if (del && present) ++n_del;
+            continue;
+        }
+        bool pend = false;
+        if (ins) {
+            if (present) {
+                if (!(MODE == kBinModeMixed && (flags & kBinSkipEqual) && before == T::val(e))) {
+                    T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match), e);
+                    ++n_upd;
+                }
+            } else {
+                bool ok = claim_empty<KB, SB>(p1, r1.empty, e);
+                if (!ok && check2 && r2.empty) {
+                    mark_overflow<KB, SB>(p1, hk);
+                    ok = claim_empty<KB, SB>(p2, r2.empty, e);
+                }
+                if (ok) ++n_ins;
+                else pend = true;
+            }
+        } else if (del && present) {
+            T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match),
+                     T::empty());
+            ++n_del;
+        }
+        if (MODE == kBinModeMixed && act && vals_out != nullptr) store_val(vals_out, vb, i, before);
+        if (MODE != kBinModeInsert && act && present && bits_out != nullptr)
+            atomicOr(&bits_out[i >> 5], 1u << (i & 31));
+        if constexpr (MODE != kBinModeErase) {
+            __syncwarp();
+            const unsigned long long at = agg_inc(&ctr->pending, pend);
+            if (pend) {
+                if (at < S.list_cap) ((Sl *)S.list_a)[at] = e;
+                else atomicAdd(&ctr->spill, 1ull);
+            }
+        }
+    }
+
+    // keys with several ops: probe, replay the ops in index order, apply the
+    // final state. Key x of the list goes to lane x / 8 of warp x % 8, so a
+    // few long segments spread over the warps.
+    if constexpr (MODE >= kBinModeMixed) {
+        const uint32_t nm = M.nmulti;
+        for (uint32_t x0 = 0; x0 < nm; x0 += kBlockThreads) {
+            const uint32_t x = x0 + lane * kWarpsPerBlock + (tid >> 5);
+            const bool act = x < nm;
+            if (!__any_sync(kFull, act)) continue;
+            const uint32_t r = act ? M.multi[x] : 0u;
+            const K k = act ? M.key[r] : (K)0;
+            const uint32_t c = act ? M.cnt[r] & 0xffffu : 0u, off = act ? M.cnt[r] >> 16 : 0u;
+            const uint32_t hk = fold(k);
+            const Pair p = pair_of(hk, D.d);
+            char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
+            char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
+            const KvOut r1 = place_probe<KB, SB, false>(p1, k, act, p.first, D.d, stage);
+            const bool found1 = act && r1.match >= 0;
+            const bool check2 = act && !found1 && ((!Gm::kMeta || r1.overflow) || r1.empty == 0u);
+            KvOut r2{-1, 0ull, false, 0u};
+            if (__any_sync(kFull, check2))
+                r2 = place_probe<KB, SB, false>(p2, k, check2, p.second, D.d, stage);
+            const bool found2 = check2 && r2.match >= 0;
+            const bool pre = found1 || found2;
+            const uint64_t pre_value = found1 ? r1.value : (found2 ? r2.value : 0ull);
+            bool present = pre;
+            uint64_t value = pre_value;
+            if (act && c <= kBinShort) {
+                uint32_t w[kBinShort];
+#pragma unroll
+                for (uint32_t a = 0; a < kBinShort; ++a) w[a] = a < c ? M.seg[off + a] : 0xffffffffu;
+#pragma unroll
+                for (uint32_t t = 0; t < kBinShort; ++t) {
+#pragma unroll
+                    for (uint32_t a = t & 1u; a + 1 < kBinShort; a += 2) {
+                        const uint32_t lo = min(w[a], w[a + 1]), hi = max(w[a], w[a + 1]);
+                        w[a] = lo;
+                        w[a + 1] = hi;
+                    }
+                }
+#pragma unroll
+                for (uint32_t a = 0; a < kBinShort; ++a) {
+                    if (a >= c) break;
+                    const uint32_t i = w[a] >> 2, op = w[a] & 3u;
+                    const uint64_t in = op == 1u ? load_val(vals, vb, i) : 0ull;
+                    if (MODE == kBinModeMixed) {
+                        if (vals_out) store_val(vals_out, vb, i, present ? value : 0ull);
+                        if (present && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
+                    }
+                    replay_op((uint8_t)op, in, present, value);
+                }
+            }
+            for (unsigned big = __ballot_sync(kFull, c > kBinShort); big; big &= big - 1u) {
+                const int j = __ffs(big) - 1;
+                const uint32_t cj = __shfl_sync(kFull, c, j), oj = __shfl_sync(kFull, off, j);
+                bool pj = __shfl_sync(kFull, present, j);
+                uint64_t vj = shfl64(value, j);
+                __syncwarp();
+                warp_sort_words(M.seg + oj, cj);
+                warp_replay_words<MODE == kBinModeMixed>(M.seg + oj, cj, pj, vj, vals, vb, vals_out,
+                                                     bits_out);
+                if ((int)lane == j) {
+                    present = pj;
+                    value = vj;
+                }
+            }
+            const bool up = act && present && (!pre || value != pre_value);
+            const bool er = act && !present && pre;
+            if constexpr (MODE == kBinModeCount) {
+                n_ins += up ? 1u : 0u;
+                n_del += er ? 1u : 0u;
+                continue;
+            }
+            Sl e = T::empty();
+            bool pend = false;
+            if (up) {
+                e = T::make(k, value);
+                if (pre) {
+                    T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match), e);
+                    ++n_upd;
+                } else {
+                    bool ok = claim_empty<KB, SB>(p1, r1.empty, e);
+                    if (!ok && check2 && r2.empty) {
+                        mark_overflow<KB, SB>(p1, hk);
+                        ok = claim_empty<KB, SB>(p2, r2.empty, e);
+                    }
+                    if (ok) ++n_ins;
+                    else pend = true;
+                }
+            } else if (er) {
+                T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match),
+                         T::empty());
+                ++n_del;
+            }
+            __syncwarp();
+            const unsigned long long at = agg_inc(&ctr->pending, pend);
+            if (pend) {
+                if (at < S.list_cap) ((Sl *)S.list_a)[at] = e;
+                else atomicAdd(&ctr->spill, 1ull);
+            }
+        }
+    }
+
+    // one atomic per counter per block
+    n_ins = __reduce_add_sync(kFull, n_ins);
+    n_upd = __reduce_add_sync(kFull, n_upd);
+    n_del = __reduce_add_sync(kFull, n_del);
+    n_sup = __reduce_add_sync(kFull, n_sup);
+    n_rej = __reduce_add_sync(kFull, n_rej);
+    if (lane == 0) {
+        if (n_ins) atomicAdd(&M.sum[0], (unsigned long long)n_ins);
+        if (n_upd) atomicAdd(&M.sum[1], (unsigned long long)n_upd);
+        if (n_del) atomicAdd(&M.sum[2], (unsigned long long)n_del);
+        if (n_sup) atomicAdd(&M.sum[3], (unsigned long long)n_sup);
+        if (n_rej) atomicAdd(&M.sum[4], (unsigned long long)n_rej);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned long long ins = M.sum[0], upd = M.sum[1], del = M.sum[2];
+        if constexpr (MODE == kBinModeCount) {
+            if (ins) atomicAdd(&ctr->nins, ins);
+            if (del) atomicAdd(&ctr->erased, del);
+        } else {
+            if (ins) atomicAdd(&ctr->inserted, ins);
+            if (upd) atomicAdd(&ctr->updated, upd);
+            if (del) atomicAdd(&ctr->erased, del);
+            const long long net = (long long)ins - (long long)del;
+            if (net) atomicAdd(&ctr->size, (unsigned long long)net);
+        }
+        if (MODE <= kBinModeErase && M.sum[3]) atomicAdd(&ctr->superseded, M.sum[3]);
+        if (MODE == kBinModeInsert && M.sum[4]) atomicAdd(&ctr->rejected, M.sum[4]);
+    }
+    {
+        // the last block sees every other block's lists and counters
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) M.last = atomicAdd(&ctr->ticket, 1ull) == gridDim.x - 1;
+        __syncthreads();
+        if (!M.last) return;
+        __threadfence();
+        if constexpr (MODE != kBinModeErase && MODE != kBinModeCount) {
+            const uint64_t np = *(volatile unsigned long long *)&ctr->pending;
+            if (np && np <= kTailWalk) {
+                tail_walk<KB, SB>(D, S, ctr, np);
+                __threadfence();
+                __syncthreads();
+                if (tid == 0) *(volatile unsigned long long *)&ctr->pending = 0ull;
+                __syncthreads();
+            }
+        }
+        if (tid < sizeof(Counters) / 8)
+            ((volatile unsigned long long *)h_ctr)[tid] = ((volatile unsigned long long *)ctr)[tid];
+        __threadfence_system();
+    }
+}
+
+}  // namespace dyc

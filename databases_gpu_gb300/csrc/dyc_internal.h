@@ -52,8 +52,11 @@ struct Counters {
     unsigned long long spill;  // pending entries a list could not hold (must stay 0)
     unsigned long long pad[2];      // scratch words of dyc_export and dyc_snapshot
     unsigned long long timeouts;    // bounded device waits that gave up (must stay 0)
-    unsigned long long nins;        // scratch word: insert ops of a dyc_apply batch
-    unsigned long long pad2[2];
+    // scratch word: insert ops of a dyc_apply batch (its upserts, from the
+    // counting pass of a batch resolved by bins)
+    unsigned long long nins;
+    unsigned long long left;        // ops of bins that went over (left to the general path)
+    unsigned long long ticket;      // blocks of a small batch's kernel that have finished
 };
 static_assert(sizeof(Counters) == 128, "Counters is one 128-byte block");
 
@@ -74,7 +77,47 @@ struct Scratch {
     // nonzero once the dedup claims met a key twice; while it stays zero
     // every op of the chunk is its key's only op (no winner bits are needed)
     uint32_t *dupseen;
+    // the ops of bins that went over, gathered in index order for the general
+    // path (their keys and values go to list_b): op indexes, codes, result
+    // bits, per-block counts
+    uint32_t *bin_count;  // per bin of a chunk: ops
+    uint32_t *left_idx;
+    uint8_t *left_ops;
+    uint32_t *left_bits;
+    uint32_t *left_cnt;
 };
+
+// A chunk's ops split by key into bins (dyc_bins.cuh): bin b's records are
+// [b * kBinCap, b * kBinCap + min(count[b], kBinCap)), a bin holding kBinMean
+// ops of distinct random keys on average. A bin with more ops than its
+// capacity (few keys, each repeated many times) is left to the general path
+// as a whole. kBinMean * 2 = kBinCap, so the records of a chunk take no more
+// cells than its dedup table. Batches of up to kBinSmallOps ops are split by
+// the kernel that resolves them, into bins of kBinSmallMean ops.
+constexpr int kBinCap = 2048;
+constexpr int kBinMean = 1024;
+constexpr int kSmallCap = 1024;
+constexpr int kBinSmallMean = 192;
+constexpr uint64_t kBinSmallOps = 16384;
+struct BinScratch {
+    unsigned long long *rec;  // key tag | op word << 32 (bin_tag, op_word)
+    uint32_t *count;          // per bin: ops
+    uint32_t nbins, cap;
+    // one bit per op: cleared for the ops of keys with several ops (an insert
+    // or erase batch: all but the op that counts) and of bins that went over
+    uint32_t *single;
+};
+enum : int {
+    kBinModeInsert = 0,  // the last op of a key wins (dyc_insert)
+    kBinModeErase = 1,   // the first op wins (dyc_erase)
+    kBinModeMixed = 2,   // the ops take effect in index order (dyc_apply)
+    kBinModeCount = 3    // as kBinModeMixed, but only counts the upserts and erases
+};
+enum : uint32_t {
+    kBinNewKeys = 1,   // the caller promises absent keys (DYC_FLAG_NEW_KEYS)
+    kBinSkipEqual = 2  // an insert that finds its own value writes and counts nothing
+};
+constexpr int kLeftTile = 2048;  // ops per block of the passes that gather what is left
 
 // Dedup tables of at least this many cells get the winners pass (winbits);
 // smaller ones fit in the L2 beside the bucket lines, so an op of a chunk
@@ -277,12 +320,14 @@ template <int KB> struct Ops {
     // without a slot go to S.list_a, counted in ctr->pending). With a single
     // bitmap (a single_pass batch after its grouping and scatter), only the
     // ops whose bit is set, and their hit bits are ORed in; all ops when
-    // *gate is 0 (no key repeated, so the scatter did not run).
+    // *gate is 0 (no key repeated, so the scatter did not run). flags:
+    // kBinSkipEqual.
     static cudaError_t apply_unique(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                                     const uint8_t *ops, const void *keys, const void *vals,
                                     uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
                                     Counters *ctr, const uint32_t *single = nullptr,
-                                    const unsigned long long *gate = nullptr);
+                                    const unsigned long long *gate = nullptr,
+                                    uint32_t flags = 0u);
     // *count += the INSERT ops among ops[0..n)
     static cudaError_t count_inserts(const LaunchCtx &L, const uint8_t *ops, uint64_t n,
                                      unsigned long long *count);
@@ -335,6 +380,36 @@ template <int KB> struct Ops {
                                 unsigned long long *dst_count, uint64_t dst_cap,
                                 uint32_t max_evict, Counters *gctr, uint64_t max_entries,
                                 unsigned long long *bad);
+    // A chunk of more than kBinSmallOps ops (dyc_bins.cuh): the bin counts,
+    // the call counters (zero, nzero), A.ctr and the result bits zeroed, the
+    // single bits set, the ops split into bins, and the ops of repeated keys
+    // found: their single bits cleared and, for a mixed batch (mode
+    // kBinModeMixed), their keys and segments listed in A as apply_group
+    // lists them. ops is null for the insert and erase modes.
+    static cudaError_t bin_group(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
+                                 int mode, const uint8_t *ops, const void *keys, uint32_t *bits_out,
+                                 uint64_t n, Counters *ctr);
+    // a batch of up to kBinSmallOps ops in one of the kBinMode* modes; the
+    // counters go to h_ctr
+    static cudaError_t bin_small(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
+                                 const BinScratch &B, int mode, const uint8_t *ops,
+                                 const void *keys, const void *vals, uint32_t vb, void *vals_out,
+                                 uint32_t *bits_out, uint64_t n, uint32_t flags, Counters *ctr,
+                                 Counters *h_ctr);
+    // ctr->nins / ctr->erased += the upserts and erases that apply_unique
+    // would make for the ops whose single bit is set
+    static cudaError_t apply_count(const LaunchCtx &L, const Desc &D, int sb, const uint8_t *ops,
+                                   const void *keys, const void *vals, uint32_t vb, uint64_t n,
+                                   const uint32_t *single, Counters *ctr);
+    // the ops of the bins that went over, in index order (S.left_idx, their
+    // keys and values to list_b, codes to S.left_ops), and the way back of
+    // their results
+    static cudaError_t left_gather(const LaunchCtx &L, const Scratch &S, const BinScratch &B,
+                                   const uint8_t *ops, const void *keys, const void *vals,
+                                   uint32_t vb, uint64_t n, void *keys_left, void *vals_left);
+    static cudaError_t left_return(const LaunchCtx &L, const Scratch &S, uint64_t m,
+                                   const void *out, uint32_t vb, void *vals_out,
+                                   uint32_t *bits_out);
     // set every fingerprint bit of every bucket of a subtable
     static cudaError_t mark_all(const LaunchCtx &L, int sb, void *sub, uint32_t nb);
     static cudaError_t export_all(const LaunchCtx &L, const Desc &D, int sb, void *keys,

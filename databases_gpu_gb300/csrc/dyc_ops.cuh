@@ -7,6 +7,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "dyc_left.cuh"
 #include "dyc_set.cuh"
 #include "dyc_kernels.cuh"
 
@@ -157,12 +158,24 @@ cudaError_t Ops<KB>::apply_unique(const LaunchCtx &L, const Desc &D, int sb, con
                                   const uint8_t *ops, const void *keys, const void *vals,
                                   uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
                                   Counters *ctr, const uint32_t *single,
-                                  const unsigned long long *gate) {
+                                  const unsigned long long *gate, uint32_t flags) {
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_apply_unique<KB, SB, true> : k_apply_unique<KB, SB, false>;
         k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, ops, keys, vals, vb, vals_out, bits_out, n,
-                                                  ctr, single, gate);
+                                                  ctr, single, gate, flags);
+    });
+    return cudaGetLastError();
+}
+
+template <int KB>
+cudaError_t Ops<KB>::apply_count(const LaunchCtx &L, const Desc &D, int sb, const uint8_t *ops,
+                                 const void *keys, const void *vals, uint32_t vb, uint64_t n,
+                                 const uint32_t *single, Counters *ctr) {
+    if (n == 0) return cudaSuccess;
+    DYC_SB_DISPATCH(sb, {
+        auto k = k_apply_count<KB, SB>;
+        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, ops, keys, vals, vb, n, single, ctr);
     });
     return cudaGetLastError();
 }
@@ -413,6 +426,26 @@ cudaError_t Ops<KB>::export_all(const LaunchCtx &L, const Desc &D, int sb, void 
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+template <int KB>
+cudaError_t Ops<KB>::left_gather(const LaunchCtx &L, const Scratch &S, const BinScratch &B,
+                                 const uint8_t *ops, const void *keys, const void *vals,
+                                 uint32_t vb, uint64_t n, void *keys_left, void *vals_left) {
+    const unsigned tiles = (unsigned)((n + kLeftTile - 1) / kLeftTile);
+    k_left_count<KB><<<tiles, 256, 0, L.stream>>>(B, S, keys, n);
+    k_left_scan<KB><<<1, 1024, 0, L.stream>>>(S.left_cnt, tiles);
+    k_left_gather<KB><<<tiles, 256, 0, L.stream>>>(B, S, ops, keys, vals, vb, n, keys_left, vals_left);
+    return cudaGetLastError();
+}
+
+template <int KB>
+cudaError_t Ops<KB>::left_return(const LaunchCtx &L, const Scratch &S, uint64_t m, const void *out,
+                                 uint32_t vb, void *vals_out, uint32_t *bits_out) {
+    if (m == 0) return cudaSuccess;
+    k_left_return<KB><<<(unsigned)std::min<uint64_t>((m + 255) / 256, 4096), 256, 0, L.stream>>>(
+        S, m, out, vb, vals_out, bits_out);
+    return cudaGetLastError();
 }
 
 }  // namespace dyc
