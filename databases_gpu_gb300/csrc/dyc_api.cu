@@ -646,10 +646,11 @@ dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64
     return insert_general(t, lk, lv, left, true, new_keys, s);
 }
 
+// old (may be null): the value each removed key had.
 dyc_status erase_pass(dyc_table *t, const Scratch &S, const void *keys, uint64_t n, uint32_t *bits,
-                      bool use_dedup, cudaStream_t s) {
+                      void *old, bool use_dedup, cudaStream_t s) {
     cudaError_t e = KB_CALL(t, erase, ctx(t, s), t->D, t->sb, S, use_dedup, keys, n, bits,
-                            t->d_ctr);
+                            t->d_ctr, old, (uint32_t)t->vb);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "erase kernel: %s", cudaGetErrorString(e));
     TRY(read_counters(t, s));
     t->last.erased += t->h_ctr->erased;
@@ -657,37 +658,53 @@ dyc_status erase_pass(dyc_table *t, const Scratch &S, const void *keys, uint64_t
     return DYC_OK;
 }
 
-dyc_status erase_general(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits,
+dyc_status erase_general(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits, void *old,
                          bool use_dedup, cudaStream_t s) {
     const Scratch S = chunk_scratch(t, n);
     if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepFirst, s));
     else TRY(reset_call_counters(t, s));
-    return erase_pass(t, S, keys, n, bits, use_dedup, s);
+    return erase_pass(t, S, keys, n, bits, old, use_dedup, s);
 }
 
-dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits,
+dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits, void *old,
                        uint32_t flags, cudaStream_t s) {
     const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
-    if (!use_dedup || !bins_ok(t)) return erase_general(t, keys, n, bits, use_dedup, s);
+    if (!use_dedup || !bins_ok(t)) return erase_general(t, keys, n, bits, old, use_dedup, s);
     const dyc::BinScratch B = chunk_bins(t, n, t->S.winbits);
     if (B.single == nullptr) {
-        TRY(bins_small(t, B, dyc::kBinModeErase, nullptr, keys, nullptr, nullptr, bits, n, 0u, s));
+        TRY(bins_small(t, B, dyc::kBinModeErase, nullptr, keys, nullptr, old, bits, n, 0u, s));
         t->last.erased += t->h_ctr->erased;
         t->last.superseded += t->h_ctr->superseded;
     } else {
         TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeErase, nullptr, keys, nullptr, n, s));
-        TRY(erase_pass(t, bins_scratch(t), keys, n, bits, true, s));
+        TRY(erase_pass(t, bins_scratch(t), keys, n, bits, old, true, s));
     }
     const uint64_t left = t->h_ctr->left;
     if (left == 0) return DYC_OK;
-    void *lk, *lv;
+    // the general pass of what is left answers in left_bits (and the freed
+    // list), copied back to the ops' places; it writes only removed keys' values
+    void *lk, *lv, *lo = old ? t->S.list_a : nullptr;
+    uint32_t *lb = (bits || old) ? t->S.left_bits : nullptr;
     TRY(bins_left(t, B, nullptr, keys, nullptr, n, &lk, &lv, s));
-    TRY(erase_general(t, lk, left, bits ? t->S.left_bits : nullptr, true, s));
-    if (bits) {
-        const cudaError_t e = KB_CALL(t, left_return, ctx(t, s), t->S, left, nullptr,
-                                      (uint32_t)t->vb, nullptr, bits);
+    TRY(erase_general(t, lk, left, lb, lo, true, s));
+    if (lb) {
+        const cudaError_t e = KB_CALL(t, left_return, ctx(t, s), t->S, left, lo, (uint32_t)t->vb,
+                                      old, bits);
         if (e != cudaSuccess) return fail(DYC_ECUDA, "return kernel: %s", cudaGetErrorString(e));
         CK(cudaStreamSynchronize(s));
+    }
+    return DYC_OK;
+}
+
+// Erase n keys in chunks, without the downsize that may follow.
+dyc_status erase_chunks(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits, void *old,
+                        uint32_t flags, cudaStream_t s) {
+    const uint64_t chunk = t->chunk;
+    TRY(ensure_scratch(t, n < chunk ? n : chunk));
+    for (uint64_t off = 0; off < n; off += chunk) {
+        const uint64_t m = (n - off) < chunk ? (n - off) : chunk;
+        TRY(erase_chunk(t, (const char *)keys + off * t->kb, m, bits ? bits + off / 32 : nullptr,
+                        old ? (char *)old + off * t->vb : nullptr, flags, s));
     }
     return DYC_OK;
 }
@@ -1008,13 +1025,7 @@ dyc_status dyc_erase(dyc_table *t, const void *d_keys, uint64_t n, uint32_t *d_e
     TRY(settle_held(t, s));
     if (n == 0) return DYC_OK;
     if (!d_keys) return fail(DYC_EINVAL, "null key array");
-    const uint64_t chunk = t->chunk;
-    TRY(ensure_scratch(t, n < chunk ? n : chunk));
-    for (uint64_t off = 0; off < n; off += chunk) {
-        const uint64_t m = (n - off) < chunk ? (n - off) : chunk;
-        TRY(erase_chunk(t, (const char *)d_keys + off * t->kb, m,
-                        d_erased_bits_out ? d_erased_bits_out + off / 32 : nullptr, flags, s));
-    }
+    TRY(erase_chunks(t, d_keys, n, d_erased_bits_out, nullptr, flags, s));
     if (h_erased_count) *h_erased_count = t->last.erased;
     // downsize check after the batch (api.cpp:494-505)
     if (t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE) &&
@@ -2862,6 +2873,46 @@ unsigned wide_grid(dyc_wide *w, uint64_t n) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)w->t->sms * 8));
 }
 
+// Insert m keys whose op that counts S names (use_dedup): the current handles,
+// the staging of the values, and the placement of the new keys. Op i's value
+// is row idx[i] (row i without idx). left: ctr->left as copied to h_ctr before.
+dyc_status wide_insert_pass(dyc_wide *w, const Scratch &S, bool use_dedup, const void *k,
+                            const uint32_t *v, const uint32_t *idx, uint64_t m, uint32_t flags,
+                            cudaStream_t s, uint64_t *left = nullptr) {
+    dyc_table *t = w->t;
+    // current handles of the chunk's keys
+    cudaError_t e = KB_CALL(t, find, ctx(t, s), t->D, t->sb, k, w->pre_h, 4u, w->bits, m);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "wide find: %s", cudaGetErrorString(e));
+    TRY(wide_ensure_heap(w, m, s));
+    CK(cudaMemsetAsync(w->cnt, 0, 2 * sizeof(unsigned long long), s));
+    auto stage = t->kb == 4 ? dyc::k_wide_stage<4> : dyc::k_wide_stage<8>;
+    stage<<<wide_grid(w, m), 256, 0, s>>>(S, use_dedup ? 1 : 0, k, v, idx, w->words, m, w->pre_h,
+                                          w->bits, w->heap, w->stack, w->d_alloc, w->new_keys,
+                                          w->new_h, w->cnt);
+    dyc::k_wide_commit<<<1, 1, 0, s>>>(w->d_alloc, w->cnt);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(w->h_cnt, w->cnt, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    TRY(wide_read_alloc(w, s));
+    if (left) *left = t->h_ctr->left;
+    const uint64_t fresh = w->h_cnt[0];
+    w->last.updated += w->h_cnt[1];
+    if (fresh) {
+        if (t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE)) {
+            int guard = 0;
+            while ((double)(t->size + fresh) > t->cfg.upper_load * (double)t->capacity &&
+                   guard++ < 64)
+                TRY(resize_up_impl(t, s));
+        }
+        t->last = dyc_op_stats{};
+        TRY(insert_chunk(t, w->new_keys, w->new_h, fresh, DYC_FLAG_UNIQUE | DYC_FLAG_NEW_KEYS, s));
+        w->last.inserted += t->last.inserted;
+        w->last.evict_steps += t->last.evict_steps;
+        w->last.overflowed += t->last.overflowed;
+        w->last.resizes_up += t->last.resizes_up;
+    }
+    return DYC_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -2949,47 +3000,29 @@ dyc_status dyc_wide_insert(dyc_wide *w, const void *d_keys, const void *d_vals, 
         const uint64_t m = std::min(chunk, n - off);
         const char *k = (const char *)d_keys + off * t->kb;
         const uint32_t *v = (const uint32_t *)((const char *)d_vals + off * w->vbytes);
-        // current handles of the chunk's keys
-        cudaError_t e = KB_CALL(t, find, ctx(t, s), t->D, t->sb, k, w->pre_h, 4u, w->bits, m);
-        if (e != cudaSuccess) return fail(DYC_ECUDA, "wide find: %s", cudaGetErrorString(e));
         const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && m > 1;
-        const Scratch S = chunk_scratch(t, m);
-        if (use_dedup) {  // clears the chunk's cells first
-            e = KB_CALL(t, dedup, ctx(t, s), S, k, m, dyc::kKeepLast);
-            if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
-        }
-        TRY(wide_ensure_heap(w, m, s));
-        CK(cudaMemsetAsync(w->cnt, 0, 2 * sizeof(unsigned long long), s));
-        const unsigned grid = wide_grid(w, m);
-        if (t->kb == 4)
-            dyc::k_wide_stage<4><<<grid, 256, 0, s>>>(S, use_dedup ? 1 : 0, k, v, w->words, m,
-                                                      w->pre_h, w->bits, w->heap, w->stack,
-                                                      w->d_alloc, w->new_keys, w->new_h, w->cnt,
-                                                      w->cnt + 1);
-        else
-            dyc::k_wide_stage<8><<<grid, 256, 0, s>>>(S, use_dedup ? 1 : 0, k, v, w->words, m,
-                                                      w->pre_h, w->bits, w->heap, w->stack,
-                                                      w->d_alloc, w->new_keys, w->new_h, w->cnt,
-                                                      w->cnt + 1);
-        dyc::k_wide_commit<<<1, 1, 0, s>>>(w->d_alloc);
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(w->h_cnt, w->cnt, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-        TRY(wide_read_alloc(w, s));
-        const uint64_t fresh = w->h_cnt[0];
-        w->last.updated += w->h_cnt[1];
-        if (fresh) {
-            if (t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE)) {
-                int guard = 0;
-                while ((double)(t->size + fresh) > t->cfg.upper_load * (double)t->capacity &&
-                       guard++ < 64)
-                    TRY(resize_up_impl(t, s));
+        if (!use_dedup || !bins_ok(t) || m <= dyc::kBinSmallOps) {
+            const Scratch S = chunk_scratch(t, m);
+            if (use_dedup) {  // clears the chunk's cells first
+                cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, k, m, dyc::kKeepLast);
+                if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
             }
-            t->last = dyc_op_stats{};
-            TRY(insert_chunk(t, w->new_keys, w->new_h, fresh, DYC_FLAG_UNIQUE | DYC_FLAG_NEW_KEYS, s));
-            w->last.inserted += t->last.inserted;
-            w->last.evict_steps += t->last.evict_steps;
-            w->last.overflowed += t->last.overflowed;
-            w->last.resizes_up += t->last.resizes_up;
+            TRY(wide_insert_pass(w, S, use_dedup, k, v, nullptr, m, flags, s));
+            continue;
+        }
+        const dyc::BinScratch B = chunk_bins(t, m, t->S.winbits);
+        TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeInsert, nullptr, k, nullptr, m, s));
+        CK(cudaMemcpyAsync(&t->h_ctr->left, &t->d_ctr->left, sizeof(t->h_ctr->left),
+                           cudaMemcpyDeviceToHost, s));
+        uint64_t left = 0;
+        TRY(wide_insert_pass(w, bins_scratch(t), true, k, v, nullptr, m, flags, s, &left));
+        if (left) {  // keys of bins that went over: by the dedup table
+            void *lk, *lv;
+            TRY(bins_left(t, B, nullptr, k, nullptr, m, &lk, &lv, s));
+            const Scratch S = chunk_scratch(t, left);
+            cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, lk, left, dyc::kKeepLast);
+            if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
+            TRY(wide_insert_pass(w, S, true, lk, v, t->S.left_idx, left, flags, s));
         }
     }
     return DYC_OK;
@@ -3037,19 +3070,18 @@ dyc_status dyc_wide_erase(dyc_wide *w, const void *d_keys, uint64_t n, void *d_v
     for (uint64_t off = 0; off < n; off += chunk) {
         const uint64_t m = std::min(chunk, n - off);
         const char *k = (const char *)d_keys + off * t->kb;
-        // handles before the erase
-        cudaError_t e = KB_CALL(t, find, ctx(t, s), t->D, t->sb, k, w->pre_h, 4u, w->bits, m);
-        if (e != cudaSuccess) return fail(DYC_ECUDA, "wide find: %s", cudaGetErrorString(e));
         uint32_t *eb = d_erased_bits ? d_erased_bits + off / 32 : w->bits;
-        uint64_t cnt = 0;
-        // no downsize inside: the erased bits and handles are read below
-        TRY(dyc_erase(t, k, m, eb, &cnt, flags | DYC_FLAG_NO_RESIZE, s));
-        total += cnt;
+        // the removed keys' handles and erased bits, read below; no downsize
+        t->last = dyc_op_stats{};
+        TRY(settle_held(t, s));
+        TRY(erase_chunks(t, k, m, eb, w->pre_h, flags, s));
+        total += t->last.erased;
+        CK(cudaMemsetAsync(w->cnt, 0, sizeof(unsigned long long), s));
         dyc::k_wide_free<<<wide_grid(w, m), 256, 0, s>>>(
             w->pre_h, eb, m, w->heap, w->words,
             d_vals_out ? (uint32_t *)((char *)d_vals_out + off * w->vbytes) : nullptr, w->stack,
-            w->d_alloc);
-        dyc::k_wide_commit_free<<<1, 1, 0, s>>>(w->d_alloc);
+            w->d_alloc, w->cnt);
+        dyc::k_wide_commit_free<<<1, 1, 0, s>>>(w->d_alloc, w->cnt);
         CK(cudaGetLastError());
         TRY(wide_read_alloc(w, s));
     }

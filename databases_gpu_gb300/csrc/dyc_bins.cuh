@@ -526,7 +526,9 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
                      T::empty());
             ++n_del;
         }
-        if (MODE == kBinModeMixed && act && vals_out != nullptr) store_val(vals_out, vb, i, before);
+        // a mixed op's result; the value an erased key had
+        if ((MODE == kBinModeMixed && act || MODE == kBinModeErase && present) && vals_out != nullptr)
+            store_val(vals_out, vb, i, before);
         if (MODE != kBinModeInsert && act && present && bits_out != nullptr)
             atomicOr(&bits_out[i >> 5], 1u << (i & 31));
         if constexpr (MODE != kBinModeErase) {

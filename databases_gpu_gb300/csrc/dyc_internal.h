@@ -280,9 +280,11 @@ template <int KB> struct Ops {
                             const unsigned long long *src_count, void *dst,
                             unsigned long long *dst_count, uint64_t dst_cap, uint32_t max_evict,
                             bool count_new, Counters *ctr, uint64_t max_entries);
+    // old (may be null): the value each removed key had (vb bytes each; other
+    // ops' words are not written)
     static cudaError_t erase(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                              bool use_dedup, const void *keys, uint64_t n, uint32_t *bits,
-                             Counters *ctr);
+                             Counters *ctr, void *old = nullptr, uint32_t vb = 0u);
     static cudaError_t resize_up(const LaunchCtx &L, int sb, uint32_t t, const void *old_sub,
                                  uint32_t old_nb, void *new_sub);
     // J.n jobs in one launch of J.blocks blocks (job block ranges filled in)

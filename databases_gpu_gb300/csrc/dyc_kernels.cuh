@@ -1004,7 +1004,8 @@ template <int KB, int SB, bool HINT>
 __global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
                                                const __grid_constant__ Scratch S, int use_dedup,
                                                const void *__restrict__ keys, uint64_t n,
-                                               uint32_t *__restrict__ bits, Counters *ctr) {
+                                               uint32_t *__restrict__ bits, void *__restrict__ old,
+                                               uint32_t vb, Counters *ctr) {
     using T = SlotT<KB>;
     using Gm = Geo<KB, SB>;
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
@@ -1036,6 +1037,7 @@ __global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
         bool erased = false;
         if (act && r1.match >= 0) {
             T::store(slot_ptr<KB, SB>(p1, r1.match), T::empty());
+            if (old != nullptr) store_val(old, vb, i, r1.value);
             erased = true;
         }
         const bool need2 = act && r1.match < 0 && (!Gm::kMeta || r1.overflow);
@@ -1044,6 +1046,7 @@ __global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
             const KvOut r2 = kv_probe<KB, SB, 2, HINT>(p2, k, need2, stage, tpol);
             if (need2 && r2.match >= 0) {
                 T::store(slot_ptr<KB, SB>(p2, r2.match), T::empty());
+                if (old != nullptr) store_val(old, vb, i, r2.value);
                 erased = true;
             }
         }

@@ -144,11 +144,12 @@ cudaError_t Ops<KB>::walk(const LaunchCtx &L, const Desc &D, int sb, const void 
 template <int KB>
 cudaError_t Ops<KB>::erase(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                            bool use_dedup, const void *keys, uint64_t n, uint32_t *bits,
-                           Counters *ctr) {
+                           Counters *ctr, void *old, uint32_t vb) {
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_erase<KB, SB, true> : k_erase<KB, SB, false>;
-        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, use_dedup ? 1 : 0, keys, n, bits, ctr);
+        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, use_dedup ? 1 : 0, keys, n, bits, old, vb,
+                                                 ctr);
     });
     return cudaGetLastError();
 }

@@ -11,7 +11,7 @@
 // table; the value itself never moves. No locks, nothing spins.
 #pragma once
 
-#include "dyc_kernels.cuh"
+#include "dyc_apply.cuh"
 
 namespace dyc {
 
@@ -21,9 +21,7 @@ struct WideAlloc {
     uint32_t free_top;  // entries on the free stack
     uint32_t bump;      // first never-used handle
     uint32_t cap;       // heap rows
-    uint32_t taken;     // handles handed out by the current stage kernel
-    uint32_t pushed;    // handles pushed by the current free kernel
-    uint32_t pad[3];
+    uint32_t pad[5];
 };
 
 __device__ __forceinline__ void copy_words(uint32_t *__restrict__ dst,
@@ -41,58 +39,61 @@ __device__ __forceinline__ void copy_words(uint32_t *__restrict__ dst,
 // the never-used range), their value is written, and (key, handle) is listed
 // for placement. Ops on key 0 and ops superseded by a later one in the batch
 // do nothing. The allocator state is only read here (k_wide_commit applies
-// what was handed out).
+// what was handed out: cnt[0] handles). Op i's value is row idx[i] of vals
+// (row i without idx). cnt[0] / cnt[1] += new keys / updates: one atomic per
+// block and step of 256 ops, since atomics on one word pass at ~2 ns each (one
+// per warp and counter: 3e6 32-byte rows took 170 us, now 80).
 template <int KB>
 __global__ void __launch_bounds__(256) k_wide_stage(const __grid_constant__ Scratch S, int use_dedup,
                                                     const void *__restrict__ keys,
                                                     const uint32_t *__restrict__ vals,
+                                                    const uint32_t *__restrict__ idx,
                                                     uint32_t words, uint64_t n,
                                                     const uint32_t *__restrict__ pre_h,
                                                     const uint32_t *__restrict__ pre_bits,
                                                     uint32_t *__restrict__ heap,
                                                     const uint32_t *__restrict__ stack,
-                                                    WideAlloc *A, void *new_keys,
-                                                    uint32_t *new_h,
-                                                    unsigned long long *new_count,
-                                                    unsigned long long *upd_count) {
+                                                    const WideAlloc *__restrict__ A, void *new_keys,
+                                                    uint32_t *new_h, unsigned long long *cnt) {
     using K = typename SlotT<KB>::K;
     const uint32_t free_top = A->free_top, bump = A->bump;
-    const uint64_t step = warp_stride();
-    for (uint64_t base = warp_base(); base < n; base += step) {
-        const uint64_t i = base + (threadIdx.x & 31);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const int slots[2] = {0, 1};
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
+        const uint64_t i = i0 + threadIdx.x;
         bool fresh = false, upd = false;
         K k = 0;
         if (i < n) {
             k = load_key<KB>(keys, i);
             if (k != 0 && (!use_dedup || Dedup<KB>::winner(S, k, (uint32_t)i))) {
-                if ((pre_bits[i >> 5] >> (i & 31)) & 1u) {
-                    copy_words(heap + (uint64_t)pre_h[i] * words, vals + i * words, words);
-                    upd = true;
-                } else {
-                    fresh = true;
-                }
+                upd = (pre_bits[i >> 5] >> (i & 31)) & 1u;
+                fresh = !upd;
             }
         }
-        agg_inc(upd_count, upd);
-        const unsigned long long at = agg_inc(new_count, fresh);
+        uint32_t got[2];  // every thread of the block is here
+        block_alloc<2, 32>(cnt, slots, (unsigned long long)fresh | ((unsigned long long)upd << 32),
+                           got);
+        if (!fresh && !upd) continue;
+        uint32_t h;
         if (fresh) {
-            const uint32_t x = atomicAdd(&A->taken, 1u);
-            const uint32_t h = x < free_top ? stack[free_top - 1 - x] : bump + (x - free_top);
-            copy_words(heap + (uint64_t)h * words, vals + i * words, words);
-            ((K *)new_keys)[at] = k;
-            new_h[at] = h;
+            const uint32_t x = got[0];
+            h = x < free_top ? stack[free_top - 1 - x] : bump + (x - free_top);
+            ((K *)new_keys)[x] = k;
+            new_h[x] = h;
+        } else {
+            h = pre_h[i];
         }
+        copy_words(heap + (uint64_t)h * words, vals + (idx ? (uint64_t)idx[i] : i) * words, words);
     }
 }
 
 // After a stage kernel: the free stack and the never-used range shrink by
 // what it handed out.
-__global__ void k_wide_commit(WideAlloc *A) {
-    const uint32_t t = A->taken;
+__global__ void k_wide_commit(WideAlloc *A, const unsigned long long *cnt) {
+    const uint32_t t = (uint32_t)cnt[0];
     const uint32_t from_stack = t < A->free_top ? t : A->free_top;
     A->free_top -= from_stack;
     A->bump += t - from_stack;
-    A->taken = 0;
 }
 
 // Find: the value of every hit (zeros on a miss; bits == nullptr: all hit).
@@ -112,28 +113,36 @@ __global__ void __launch_bounds__(256) k_wide_gather(const uint32_t *__restrict_
 }
 
 // Erase: every removed key's handle goes back on the free stack, and its
-// value to out (when given; zeros for ops that removed nothing).
+// value to out (when given; zeros for ops that removed nothing). cnt[0] +=
+// handles pushed, one atomic per block and step, as in k_wide_stage (one per
+// warp: 194 us for 3e6 32-byte rows, now 60).
 __global__ void __launch_bounds__(256) k_wide_free(const uint32_t *__restrict__ h,
                                                    const uint32_t *__restrict__ erased,
                                                    uint64_t n, const uint32_t *__restrict__ heap,
                                                    uint32_t words, uint32_t *__restrict__ out,
-                                                   uint32_t *__restrict__ stack, WideAlloc *A) {
+                                                   uint32_t *__restrict__ stack,
+                                                   const WideAlloc *__restrict__ A,
+                                                   unsigned long long *cnt) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const bool e = (erased[i >> 5] >> (i & 31)) & 1u;
-        if (out) {
+    const uint32_t free_top = A->free_top;
+    const int slots[1] = {0};
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
+        const uint64_t i = i0 + threadIdx.x;
+        const bool e = i < n && ((erased[i >> 5] >> (i & 31)) & 1u);
+        uint32_t got[1];  // every thread of the block is here
+        block_alloc<1, 64>(cnt, slots, e ? 1ull : 0ull, got);
+        if (e) stack[free_top + got[0]] = h[i];
+        if (out && i < n) {
             uint32_t *o = out + i * words;
             if (e) copy_words(o, heap + (uint64_t)h[i] * words, words);
             else
                 for (uint32_t w = 0; w < words; ++w) o[w] = 0u;
         }
-        if (e) stack[A->free_top + atomicAdd(&A->pushed, 1u)] = h[i];
     }
 }
 
-__global__ void k_wide_commit_free(WideAlloc *A) {
-    A->free_top += A->pushed;
-    A->pushed = 0;
+__global__ void k_wide_commit_free(WideAlloc *A, const unsigned long long *cnt) {
+    A->free_top += (uint32_t)cnt[0];
 }
 
 }  // namespace dyc

@@ -73,3 +73,37 @@ def test_batches_by_bins_match_oracle(kb, vb, pattern, n):
         assert np.array_equal(dg.unpack_bits(eb, n), eh)
         assert_same_contents(t, m, "erase %d" % step)
     t.close()
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("pattern", ["distinct", "few", "both"])
+@pytest.mark.parametrize("n", [16384, 16385, 100003])
+def test_wide_batches_by_bins(kb, pattern, n):
+    """Rows of 12 bytes: the last row of a key wins, an erase returns it once."""
+    from databases_gpu_gb300.table import DyCuckooWide
+    import databases_gpu_gb300 as dg
+    rng = np.random.default_rng(n + kb)
+    w = DyCuckooWide(2 * n, 12, key_bytes=kb)
+    k = _keys(rng, kb, n, pattern)
+    rows = rng.integers(1, 1 << 30, (n, 3)).astype(np.int32)
+    st = w.insert(to_dev(k), to_dev(rows.view(np.uint32).reshape(-1)))
+    uniq, last = np.unique(k[::-1], return_index=True)  # last occurrence of each key
+    want = {int(a): rows[n - 1 - int(b)] for a, b in zip(uniq, last) if a}
+    assert st["inserted"] == len(want) == w.size
+    v, bits = w.find(to_dev(uniq))
+    hit = dg.unpack_bits(bits, uniq.size)
+    assert np.array_equal(hit, uniq != 0)
+    got = v.cpu().numpy()
+    for a, r in zip(uniq[hit], got[hit]):
+        assert np.array_equal(want[int(a)], r)
+    e = _keys(rng, kb, n, pattern)
+    cnt, ev, eb = w.erase(to_dev(e))
+    first = np.zeros(n, bool)
+    first[np.unique(e, return_index=True)[1]] = True
+    gone = first & np.isin(e, uniq[uniq != 0])
+    assert cnt == int(gone.sum()) and np.array_equal(dg.unpack_bits(eb, n), gone)
+    ev = ev.cpu().numpy()
+    assert not ev[~gone].any()
+    assert all(np.array_equal(want[int(a)], r) for a, r in zip(e[gone], ev[gone]))
+    assert w.size == len(want) - cnt
+    w.close()
