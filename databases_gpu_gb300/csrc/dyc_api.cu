@@ -146,6 +146,7 @@ struct dyc_table {
     size_t scratch_bytes = 0;
     Scratch S{};
     uint64_t chunk = kChunkDefault;
+    uint32_t bins_zero = 0;  // bins whose counts the last chunk left zero (0: not known)
     // mixed-batch scratch (dyc_apply), allocated on first use
     void *apply_buf = nullptr;
     size_t apply_bytes = 0;
@@ -217,31 +218,23 @@ cudaError_t pool_alloc(int device, void **p, size_t bytes, cudaStream_t s) {
 // dispatch on key width
 #define KB_CALL(t, fn, ...) ((t)->kb == 4 ? Ops<4>::fn(__VA_ARGS__) : Ops<8>::fn(__VA_ARGS__))
 
-// Make the scratch lists hold `n` ops (grow only).
-// Dedup cells for a chunk of n ops: a power of two, at most half full, and
-// at most a quarter full while that stays within 2^22 cells (32 MB of 8-byte
-// cells, which stay in the L2 beside the bucket lines). Fewer probes per
-// claim pay there: 2^19-key calls on an L2-resident table went from 5.1 to
-// 5.9 G ops/s (insert) and 8.2 to 8.8 (erase). A larger table at a quarter
-// load spills the L2: 4M-op chunks on a 2^28-key table lost 10 %.
-uint64_t dedup_cells(uint64_t n) {
-    const uint64_t m = n < 16 ? 16 : n;
-    const uint64_t quarter = next_pow2(4 * m);
-    return quarter <= (1ull << 22) ? quarter : next_pow2(2 * m);
+// Bins of a chunk of n ops, and the 32-bit words of their state, counts,
+// starts and cursors.
+uint32_t chunk_nbins(uint64_t n) {
+    return (uint32_t)std::max<uint64_t>(1, n / (uint64_t)dyc::kBinMean);
+}
+uint64_t bin_words(uint64_t nbins) {
+    return dyc::kBinStates + 3 * std::max<uint64_t>(nbins, 128);
 }
 
+// Make the scratch hold chunks of `n` ops (grow only).
 dyc_status ensure_scratch(dyc_table *t, uint64_t n) {
-    const uint64_t cap = dedup_cells(n);
-    const size_t dedup_bytes = (size_t)cap * 8;
-    const size_t idx_bytes = t->kb == 8 ? (size_t)cap * 4 : 0;
+    if (t->scratch && t->S.list_cap >= n) return DYC_OK;
+    const size_t rec_bytes = (size_t)chunk_nbins(n) * dyc::kBinCap * 8;
     const size_t list_bytes = (size_t)n * t->slot_bytes;
     const size_t win_bytes = (size_t)(n / 32 + 1) * 4;
-    const size_t lcnt_bytes = (size_t)(n / dyc::kLeftTile + 1) * 4;
-    const size_t bcnt_bytes = (size_t)(n / dyc::kBinSmallMean + 1) * 4;
-    const size_t need = dedup_bytes + idx_bytes + 2 * list_bytes + 2 * win_bytes + (size_t)n * 5 +
-                        lcnt_bytes + bcnt_bytes + 256 + 10 * 256;
-    if (t->scratch && t->scratch_bytes >= need && t->S.list_cap >= n && t->S.dedup_cap >= cap)
-        return DYC_OK;
+    const size_t word_bytes = (size_t)bin_words(chunk_nbins(n)) * 4;
+    const size_t need = rec_bytes + 2 * list_bytes + win_bytes + word_bytes + 5 * 256;
     if (t->scratch) {
         CK(cudaDeviceSynchronize());
         CK(cudaFree(t->scratch));
@@ -255,19 +248,13 @@ dyc_status ensure_scratch(dyc_table *t, uint64_t n) {
         p += (bytes + 255) & ~(size_t)255;
         return (void *)r;
     };
-    t->S.dedup = carve(dedup_bytes);
-    t->S.dedup_idx = idx_bytes ? (uint32_t *)carve(idx_bytes) : nullptr;
-    t->S.dedup_cap = cap;
+    t->S.rec = (unsigned long long *)carve(rec_bytes);
     t->S.list_a = carve(list_bytes);
     t->S.list_b = carve(list_bytes);
     t->S.list_cap = n;
     t->S.winbits = (uint32_t *)carve(win_bytes);
-    t->S.dupseen = (uint32_t *)carve(4);
-    t->S.bin_count = (uint32_t *)carve(bcnt_bytes);
-    t->S.left_idx = (uint32_t *)carve((size_t)n * 4);
-    t->S.left_ops = (uint8_t *)carve((size_t)n);
-    t->S.left_bits = (uint32_t *)carve(win_bytes);
-    t->S.left_cnt = (uint32_t *)carve(lcnt_bytes);
+    t->S.bin_words = (uint32_t *)carve(word_bytes);
+    t->bins_zero = 0;
     return DYC_OK;
 }
 
@@ -485,54 +472,53 @@ dyc_status drain(dyc_table *t, cudaStream_t s, void *src, unsigned long long *sr
                             kMaxOverflowRounds));
 }
 
-// The table's scratch as one chunk of n ops uses it: the dedup table sized
-// for n (as ensure_scratch sizes it for the largest chunk), so a small call
-// on a table that once took a large batch clears and probes a small table.
-Scratch chunk_scratch(const dyc_table *t, uint64_t n) {
-    Scratch S = t->S;
-    const uint64_t cap = dedup_cells(n);
-    if (cap < S.dedup_cap) S.dedup_cap = cap;
-    return S;
-}
-
-// Batch dedup of one chunk into the dedup buffers of S, on stream s:
-// kKeepLast (insert) names each key's last op, kKeepFirst (erase) its first.
-// One launch clears the chunk's cells and the call counters (what
-// reset_call_counters does), then the claims run.
-dyc_status dedup_chunk(dyc_table *t, const Scratch &S, const void *keys, uint64_t n,
-                       dyc::DedupMode mode, cudaStream_t s) {
-    cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, keys, n, mode, &t->d_ctr->inserted,
-                            (uint32_t)(sizeof(Counters) / 8 - 1));
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
-    return DYC_OK;
-}
-
 // ---- chunks whose keys may repeat, by bins (dyc_bins.cuh) ------------------
-// The records of a chunk take the cells of the dedup table, which the general
-// path fills only after the ops that bins left over have been gathered. The
-// single bits of an insert or erase chunk are the winner bits the place and
-// erase kernels read.
-bool bins_ok(const dyc_table *t) { return t->D.l2_keep == 0u; }  // k_bin_small carries no L2 hints
+// The bins' arrays in one block of words (bin_words).
+void carve_bins(dyc::BinScratch &B, uint32_t *w, uint32_t nbins) {
+    B.state = w;
+    B.count = w + dyc::kBinStates;
+    B.start = B.count + nbins;
+    B.cursor = B.start + nbins;
+    B.nbins = nbins;
+}
 
+// A chunk's bins, its op bits in `single`. The records of bins that went over
+// take list_b, which the eviction walks write later.
 dyc::BinScratch chunk_bins(const dyc_table *t, uint64_t n, uint32_t *single) {
-    const bool small = n <= dyc::kBinSmallOps;
     dyc::BinScratch B{};
-    B.rec = (unsigned long long *)t->S.dedup;
-    B.count = t->S.bin_count;
-    B.nbins = (uint32_t)(small ? (n + dyc::kBinSmallMean - 1) / dyc::kBinSmallMean
-                               : n / dyc::kBinMean);
-    B.cap = small ? dyc::kSmallCap : dyc::kBinCap;
-    B.single = small ? nullptr : single;
+    carve_bins(B, t->S.bin_words, chunk_nbins(n));
+    B.rec = t->S.rec;
+    B.hot = (unsigned long long *)t->S.list_b;
+    B.single = single;
     return B;
 }
 
-// Find the repeated keys of a chunk of more than kBinSmallOps ops.
+// Whether a batch of n ops goes to the small-batch kernel (which carries no L2
+// hints), and its bins.
+bool small_batch(const dyc_table *t, uint64_t n) {
+    return n <= dyc::kBinSmallOps && t->D.l2_keep == 0u;
+}
+dyc::BinScratch small_bins(const dyc_table *t, uint64_t n) {
+    dyc::BinScratch B{};
+    carve_bins(B, t->S.bin_words, (uint32_t)((n + dyc::kBinSmallMean - 1) / dyc::kBinSmallMean));
+    return B;
+}
+
+// Find the repeated keys of a chunk.
 dyc_status bins_group(dyc_table *t, const dyc::BinScratch &B, const dyc::ApplyScratch &A, int mode,
                       const uint8_t *ops, const void *keys, uint32_t *bits_out, uint64_t n,
                       cudaStream_t s) {
+    // the kernels leave the counts zero; another bin count (a chunk of another
+    // size) puts other words there
+    if (t->bins_zero != B.nbins) {
+        t->bins_zero = 0;
+        CK(cudaMemsetAsync(B.state, 0, (dyc::kBinStates + 3 * (size_t)B.nbins) * 4, s));
+    }
+    t->bins_zero = 0;
     const cudaError_t e = KB_CALL(t, bin_group, ctx(t, s), B, A, mode, ops, keys, bits_out, n,
                                   t->d_ctr);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "bin kernels: %s", cudaGetErrorString(e));
+    t->bins_zero = B.nbins;
     return DYC_OK;
 }
 
@@ -545,33 +531,22 @@ dyc_status walk_pending(dyc_table *t, cudaStream_t s) {
     return DYC_OK;
 }
 
-// A batch of up to kBinSmallOps ops: one kernel, which leaves its counters in
-// h_ctr and places a few entries without a slot on its own; more of them take
-// a walk kernel.
-dyc_status bins_small(dyc_table *t, const dyc::BinScratch &B, int mode, const uint8_t *ops,
-                      const void *keys, const void *vals, void *vals_out, uint32_t *bits_out,
-                      uint64_t n, uint32_t flags, cudaStream_t s) {
-    const cudaError_t e = KB_CALL(t, bin_small, ctx(t, s), t->D, t->sb, t->S, B, mode, ops, keys,
-                                  vals, (uint32_t)t->vb, vals_out, bits_out, n, flags, t->d_ctr,
-                                  t->h_ctr);
+// A small batch: one kernel, which leaves its counters in h_ctr and places a
+// few entries without a slot on its own; more of them take a walk kernel.
+// *done is false when a bin did not fit: nothing has been done then.
+dyc_status bins_small(dyc_table *t, int mode, const uint8_t *ops, const void *keys,
+                      const void *vals, void *vals_out, uint32_t *bits_out, uint64_t n,
+                      uint32_t flags, cudaStream_t s, bool *done) {
+    const cudaError_t e = KB_CALL(t, bin_small, ctx(t, s), t->D, t->sb, t->S, small_bins(t, n), mode,
+                                  ops, keys, vals, (uint32_t)t->vb, vals_out, bits_out, n, flags,
+                                  t->d_ctr, t->h_ctr);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "bin kernel: %s", cudaGetErrorString(e));
     CK(cudaStreamSynchronize(s));
     TRY(check_counters(t));
-    if (t->h_ctr->pending == 0) return DYC_OK;
+    *done = t->h_ctr->left == 0;
+    if (!*done || t->h_ctr->pending == 0) return DYC_OK;
     TRY(walk_pending(t, s));
     return read_counters(t, s);
-}
-
-// Gather the ops of the bins that went over, keys and values into list_b
-// (read before the eviction walks write there).
-dyc_status bins_left(dyc_table *t, const dyc::BinScratch &B, const uint8_t *ops, const void *keys,
-                     const void *vals, uint64_t n, void **lk, void **lv, cudaStream_t s) {
-    *lk = t->S.list_b;
-    *lv = (char *)t->S.list_b + (((size_t)t->S.list_cap * t->kb + 7) & ~(size_t)7);
-    const cudaError_t e = KB_CALL(t, left_gather, ctx(t, s), t->S, B, ops, keys, vals,
-                                  (uint32_t)t->vb, n, *lk, *lv);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "gather kernels: %s", cudaGetErrorString(e));
-    return DYC_OK;
 }
 
 // After the counters of an insert pass are in h_ctr: the call's stats, and the
@@ -594,105 +569,52 @@ dyc_status insert_finish(dyc_table *t, cudaStream_t s) {
     return DYC_OK;
 }
 
-// One pass over n ops with the scratch S naming the op of each key that
-// counts (use_dedup) or with distinct keys; `left` ops are not its own.
-dyc_status insert_pass(dyc_table *t, const Scratch &S, const void *keys, const void *vals,
-                       uint64_t n, bool use_dedup, bool new_keys, cudaStream_t s) {
-    cudaError_t e = KB_CALL(t, place, ctx(t, s), t->D, t->sb, S, use_dedup, new_keys, keys,
-                            vals, (uint32_t)t->vb, n, t->d_ctr);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "place kernel: %s", cudaGetErrorString(e));
-    // walks for the ops whose buckets were full: list_a -> list_b
-    TRY(walk_pending(t, s));
-    TRY(read_counters(t, s));
-    t->h_ctr->superseded -= t->h_ctr->left;  // ops of bins that went over won nothing yet
-    return insert_finish(t, s);
-}
-
-// n ops by the batch dedup table, or with distinct keys.
-dyc_status insert_general(dyc_table *t, const void *keys, const void *vals, uint64_t n,
-                          bool use_dedup, bool new_keys, cudaStream_t s) {
-    const Scratch S = chunk_scratch(t, n);
-    if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepLast, s));
-    else TRY(reset_call_counters(t, s));
-    return insert_pass(t, S, keys, vals, n, use_dedup, new_keys, s);
-}
-
-// The scratch with the winner bits the bins left (no dedup table to look at).
-Scratch bins_scratch(const dyc_table *t) {
-    Scratch S = t->S;
-    S.dedup_cap = std::max(S.dedup_cap, dyc::kWinnersMinCap);
-    S.dupseen = nullptr;
-    return S;
-}
-
+// Insert a chunk: the op of each key that counts found first (its bit set in
+// winbits) unless the keys are distinct, then one pass of placement and the
+// walks of what it left without a slot.
 dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64_t n,
                         uint32_t flags, cudaStream_t s) {
     const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
     const bool new_keys = (flags & DYC_FLAG_NEW_KEYS) != 0;
-    if (!use_dedup || !bins_ok(t)) return insert_general(t, keys, vals, n, use_dedup, new_keys, s);
-    const dyc::BinScratch B = chunk_bins(t, n, t->S.winbits);
-    if (B.single == nullptr) {
-        TRY(bins_small(t, B, dyc::kBinModeInsert, nullptr, keys, vals, nullptr, nullptr, n,
-                       new_keys ? (uint32_t)dyc::kBinNewKeys : 0u, s));
-        TRY(insert_finish(t, s));
-    } else {
-        TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeInsert, nullptr, keys, nullptr, n, s));
-        TRY(insert_pass(t, bins_scratch(t), keys, vals, n, true, new_keys, s));
+    if (use_dedup && small_batch(t, n)) {
+        bool done = false;
+        TRY(bins_small(t, dyc::kBinModeInsert, nullptr, keys, vals, nullptr, nullptr, n,
+                       new_keys ? (uint32_t)dyc::kBinNewKeys : 0u, s, &done));
+        if (done) return insert_finish(t, s);
     }
-    const uint64_t left = t->h_ctr->left;
-    if (left == 0) return DYC_OK;
-    void *lk, *lv;
-    TRY(bins_left(t, B, nullptr, keys, vals, n, &lk, &lv, s));
-    return insert_general(t, lk, lv, left, true, new_keys, s);
+    if (use_dedup)
+        TRY(bins_group(t, chunk_bins(t, n, t->S.winbits), dyc::ApplyScratch{}, dyc::kBinModeInsert,
+                       nullptr, keys, nullptr, n, s));
+    else
+        TRY(reset_call_counters(t, s));
+    cudaError_t e = KB_CALL(t, place, ctx(t, s), t->D, t->sb, t->S, use_dedup, new_keys, keys,
+                            vals, (uint32_t)t->vb, n, t->d_ctr);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "place kernel: %s", cudaGetErrorString(e));
+    TRY(walk_pending(t, s));  // the ops whose buckets were full: list_a -> list_b
+    TRY(read_counters(t, s));
+    return insert_finish(t, s);
 }
 
 // old (may be null): the value each removed key had.
-dyc_status erase_pass(dyc_table *t, const Scratch &S, const void *keys, uint64_t n, uint32_t *bits,
-                      void *old, bool use_dedup, cudaStream_t s) {
-    cudaError_t e = KB_CALL(t, erase, ctx(t, s), t->D, t->sb, S, use_dedup, keys, n, bits,
-                            t->d_ctr, old, (uint32_t)t->vb);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "erase kernel: %s", cudaGetErrorString(e));
-    TRY(read_counters(t, s));
-    t->last.erased += t->h_ctr->erased;
-    t->last.superseded += t->h_ctr->superseded - t->h_ctr->left;
-    return DYC_OK;
-}
-
-dyc_status erase_general(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits, void *old,
-                         bool use_dedup, cudaStream_t s) {
-    const Scratch S = chunk_scratch(t, n);
-    if (use_dedup) TRY(dedup_chunk(t, S, keys, n, dyc::kKeepFirst, s));
-    else TRY(reset_call_counters(t, s));
-    return erase_pass(t, S, keys, n, bits, old, use_dedup, s);
-}
-
 dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits, void *old,
                        uint32_t flags, cudaStream_t s) {
     const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
-    if (!use_dedup || !bins_ok(t)) return erase_general(t, keys, n, bits, old, use_dedup, s);
-    const dyc::BinScratch B = chunk_bins(t, n, t->S.winbits);
-    if (B.single == nullptr) {
-        TRY(bins_small(t, B, dyc::kBinModeErase, nullptr, keys, nullptr, old, bits, n, 0u, s));
-        t->last.erased += t->h_ctr->erased;
-        t->last.superseded += t->h_ctr->superseded;
-    } else {
-        TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeErase, nullptr, keys, nullptr, n, s));
-        TRY(erase_pass(t, bins_scratch(t), keys, n, bits, old, true, s));
+    bool done = false;
+    if (use_dedup && small_batch(t, n))
+        TRY(bins_small(t, dyc::kBinModeErase, nullptr, keys, nullptr, old, bits, n, 0u, s, &done));
+    if (!done) {
+        if (use_dedup)
+            TRY(bins_group(t, chunk_bins(t, n, t->S.winbits), dyc::ApplyScratch{},
+                           dyc::kBinModeErase, nullptr, keys, nullptr, n, s));
+        else
+            TRY(reset_call_counters(t, s));
+        cudaError_t e = KB_CALL(t, erase, ctx(t, s), t->D, t->sb, t->S, use_dedup, keys, n, bits,
+                                t->d_ctr, old, (uint32_t)t->vb);
+        if (e != cudaSuccess) return fail(DYC_ECUDA, "erase kernel: %s", cudaGetErrorString(e));
+        TRY(read_counters(t, s));
     }
-    const uint64_t left = t->h_ctr->left;
-    if (left == 0) return DYC_OK;
-    // the general pass of what is left answers in left_bits (and the freed
-    // list), copied back to the ops' places; it writes only removed keys' values
-    void *lk, *lv, *lo = old ? t->S.list_a : nullptr;
-    uint32_t *lb = (bits || old) ? t->S.left_bits : nullptr;
-    TRY(bins_left(t, B, nullptr, keys, nullptr, n, &lk, &lv, s));
-    TRY(erase_general(t, lk, left, lb, lo, true, s));
-    if (lb) {
-        const cudaError_t e = KB_CALL(t, left_return, ctx(t, s), t->S, left, lo, (uint32_t)t->vb,
-                                      old, bits);
-        if (e != cudaSuccess) return fail(DYC_ECUDA, "return kernel: %s", cudaGetErrorString(e));
-        CK(cudaStreamSynchronize(s));
-    }
+    t->last.erased += t->h_ctr->erased;
+    t->last.superseded += t->h_ctr->superseded;
     return DYC_OK;
 }
 
@@ -1285,19 +1207,16 @@ dyc_status dyc_erase_host(dyc_table *t, const void *h_keys, uint64_t n,
 // =============================================================================
 namespace {
 
-// Carve the mixed-batch scratch for `n` ops per chunk (grow only).
-// Carve an ApplyScratch for `ops` ops and `cells` cells out of one device
-// buffer (*buf, grown when too small). ntables > 0 adds the multi-table
-// arrays.
-dyc_status carve_apply(int kb, int vb, uint64_t ops, uint64_t cells, uint32_t ntables,
-                       void **buf, size_t *buf_bytes, dyc::ApplyScratch *out) {
+// Carve an ApplyScratch for `ops` ops out of one device buffer (*buf, grown
+// when too small). ntables > 0 adds the multi-table arrays and the bins of a
+// set batch of nbins bins.
+dyc_status carve_apply(int kb, int vb, uint64_t ops, uint32_t ntables, uint64_t nbins, void **buf,
+                       size_t *buf_bytes, dyc::ApplyScratch *out) {
     const bool multi = ntables > 0;
     const size_t K = (size_t)kb, V = (size_t)vb;
-    const size_t CB = kb == 4 ? 8 : 16;  // cell bytes
     const size_t sizes[] = {
-        cells * CB,                                   // cells
-        ops * 4, ops * 4, ops * K, ops * 4, ops * 8,  // op_cell, op_rank, dkey, dcnt, dseg
-        ops * 4, ops * V, (ops / 32 + 1) * 4,         // seg, pre_val, pre_hit
+        ops * K, ops * 4, ops * 8,                    // dkey, dcnt, dseg
+        ops * 4,                                      // seg
         ops * K, ops * V, ops * K,                    // up_key, up_val, er_key
         dyc::kCtrSlots * 8, ops * 4, ops * 4,         // ctr, wseg, mid
         ops * 4,                                      // sort_tmp
@@ -1305,9 +1224,11 @@ dyc_status carve_apply(int kb, int vb, uint64_t ops, uint64_t cells, uint32_t nt
         multi ? ops * 4 : 0, multi ? ops * 4 : 0,     // up_tid, er_tid
         multi ? (size_t)ntables * 4 : 0,              // tup
         multi ? (size_t)ntables * 4 : 0,              // ter
-        multi ? ((size_t)ntables + 1) * 4 : 0,        // tcell_off
         multi ? (ops / dyc::kTidxStep + 1) * 4 : 0,   // tidx
-        (ops / 32 + 1) * 4};                          // single
+        (ops / 32 + 1) * 4,                           // single
+        multi ? nbins * dyc::kBinCap * 8 : 0,         // rec
+        multi ? (bin_words(nbins) + nbins) * 4 : 0,   // bin_words, and a table per bin
+        multi ? ops * 8 : 0};                         // hot
     size_t need = 0;
     for (size_t b : sizes) need += (b + 255) & ~(size_t)255;
     if (*buf && *buf_bytes < need) {
@@ -1327,15 +1248,10 @@ dyc_status carve_apply(int kb, int vb, uint64_t ops, uint64_t cells, uint32_t nt
         return (void *)r;
     };
     dyc::ApplyScratch A{};
-    A.cells = carve();
-    A.op_cell = (uint32_t *)carve();
-    A.op_rank = (uint32_t *)carve();
     A.dkey = carve();
     A.dcnt = (uint32_t *)carve();
     A.dseg = (unsigned long long *)carve();
     A.seg = (uint32_t *)carve();
-    A.pre_val = carve();
-    A.pre_hit = (uint32_t *)carve();
     A.up_key = carve();
     A.up_val = carve();
     A.er_key = carve();
@@ -1348,12 +1264,14 @@ dyc_status carve_apply(int kb, int vb, uint64_t ops, uint64_t cells, uint32_t nt
     A.er_tid = (uint32_t *)carve();
     A.tup = (uint32_t *)carve();
     A.ter = (uint32_t *)carve();
-    A.tcell_off = (uint32_t *)carve();
     A.tidx = (uint32_t *)carve();
     A.single = (uint32_t *)carve();
+    A.rec = (unsigned long long *)carve();
+    A.bin_words = (uint32_t *)carve();
+    A.hot = (unsigned long long *)carve();
     A.ntables = ntables;
-    A.cap_cells = cells;
     A.cap_ops = ops;
+    A.wide = ops > (1ull << 30) ? 1u : 0u;
     *out = A;
     return DYC_OK;
 }
@@ -1368,7 +1286,7 @@ dyc_status ensure_apply(dyc_table *t, uint64_t n) {
     }
     if (t->apply_buf && t->A.cap_ops >= ops) return DYC_OK;
     if (!t->h_actr) CK(dyc::lib_malloc_host(&t->h_actr, dyc::kCtrSlots * sizeof(unsigned long long)));
-    return carve_apply(t->kb, t->vb, ops, 2 * ops, 0, &t->apply_buf, &t->apply_bytes, &t->A);
+    return carve_apply(t->kb, t->vb, ops, 0, 0, &t->apply_buf, &t->apply_bytes, &t->A);
 }
 
 // Copy D to the device if it changed since the last push. The pinned mirror
@@ -1381,85 +1299,45 @@ dyc_status push_desc(dyc_table *t, cudaStream_t s) {
     return DYC_OK;
 }
 
-dyc_status read_apply_counters(dyc_table *t, cudaStream_t s) {
-    CK(cudaMemcpyAsync(t->h_actr, t->A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
-                       cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    return DYC_OK;
-}
-
-// How a chunk of mixed ops finds its repeated keys, and what resolves the
-// others.
-enum class ApplyPath {
-    kBins,    // k_bin_group lists the repeated keys; the one-pass kernel takes the others
-    kSingle,  // k_apply_group and compaction list them; the one-pass kernel takes the others
-    kAll      // k_apply_group and compaction list every key
-};
-
-// n mixed ops: the keys with several ops listed with their segments, the find
-// of those keys, the replays (dyc_apply.cuh), the one-pass kernel for every
+// n mixed ops: the keys with several ops listed with their segments
+// (dyc_bins.cuh) and replayed (dyc_repeat.cuh), the one-pass kernel for every
 // other op (one probe of its key's buckets; it touches no key the others do),
-// then the erases and upserts of the listed keys and the eviction walks
-// (dyc_set.cuh, with this table's one-entry descriptor array). Every kernel
-// reads its item count on the device, so the host reads the counters once, at
-// the end (in h_ctr when this returns).
-// policy(upserts, erases): the upsize policy where the table must grow before
-// the batch (before); a counting pass over the other ops then runs first and
-// the host reads both kinds' counts. Ops of bins that went over are left
-// untouched, counted in h_ctr->left; with `before` nothing else has been
-// applied then.
+// and the eviction walks (dyc_set.cuh, with this table's one-entry descriptor
+// array). Every kernel reads its item count on the device, so the host reads
+// the counters once, at the end (in h_ctr when this returns).
+// before: policy(upserts, erases), the upsize policy, must run before the batch
+// is applied. The replays then list the repeated keys' upserts and erases, a
+// counting pass takes the others', the host reads both counts, and the lists
+// are applied after the policy.
 template <class F>
-dyc_status apply_kernels(dyc_table *t, ApplyPath path, const dyc::BinScratch &B, const uint8_t *ops,
-                         const void *keys, const void *vals, uint64_t n, void *vals_out,
-                         uint32_t *bits_out, bool before, cudaStream_t s, F &&policy) {
+dyc_status apply_kernels(dyc_table *t, const uint8_t *ops, const void *keys, const void *vals,
+                         uint64_t n, void *vals_out, uint32_t *bits_out, bool before,
+                         cudaStream_t s, F &&policy) {
     const dyc::ApplyScratch &A = t->A;
     const LaunchCtx L = ctx(t, s);
     const uint32_t vb = (uint32_t)t->vb;
-    const bool bins = path == ApplyPath::kBins;
-    dyc::ApplyScratch Ag = A;
-    if (path == ApplyPath::kSingle) {
-        // a batch in which no key repeats (k_apply_group sets the gate) skips
-        // compaction and the scatter; later kernels read counts left at 0
-        Ag.gate = &A.ctr[dyc::kCtrRepeat];
-        Ag.single_pass = 1u;
-    }
     TRY(push_desc(t, s));
-    cudaError_t e = cudaSuccess;
-    if (bins) {
-        TRY(bins_group(t, B, A, dyc::kBinModeMixed, ops, keys, bits_out, n, s));
-    } else {
-        TRY(reset_call_counters(t, s));
-        CK(cudaMemsetAsync(A.cells, 0, (size_t)(2 * n) * (t->kb == 4 ? 8 : 16), s));  // 2n cells used
-        CK(cudaMemsetAsync(A.ctr, 0, dyc::kCtrSlots * sizeof(unsigned long long), s));
-        if (bits_out) CK(cudaMemsetAsync(bits_out, 0, (size_t)((n + 31) / 32) * 4, s));
-        e = KB_CALL(t, apply_group, L, Ag, keys, n);
-    }
-    // state of every listed key before the batch
-    if (e == cudaSuccess)
-        e = KB_CALL(t, set_find, L, t->d_desc, 1u, t->sb, A.dkey, nullptr,
-                    &A.ctr[dyc::kCtrDistinct], n, A.pre_val, vb, A.pre_hit, &A.ctr[dyc::kCtrBad],
-                    t->D.l2_keep != 0u);
-    if (e == cudaSuccess && !bins)
-        e = KB_CALL(t, apply_scatter, L, Ag, n, nullptr, ops, vals, vb, vals_out, bits_out);
-    if (e == cudaSuccess) e = KB_CALL(t, apply_replay, L, Ag, ops, vals, vb, vals_out, bits_out, n, n);
+    TRY(bins_group(t, chunk_bins(t, n, A.single), A, dyc::kBinModeMixed, ops, keys, bits_out, n, s));
+    cudaError_t e = KB_CALL(t, repeat, L, A, t->d_desc, 1u, t->sb, false, ops, vals, vb, vals_out,
+                            bits_out, n, before ? nullptr : t->S.list_a, t->S.list_cap, t->d_ctr);
     if (e == cudaSuccess && before) {
-        if (bins)
-            e = KB_CALL(t, apply_count, L, t->D, t->sb, ops, keys, vals, vb, n, B.single, t->d_ctr);
+        e = KB_CALL(t, apply_count, L, t->D, t->sb, ops, keys, vals, vb, n, A.single, t->d_ctr);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(t->h_actr, A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
                                 cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return fail(DYC_ECUDA, "apply kernels: %s", cudaGetErrorString(e));
         TRY(read_counters(t, s));
-        if (t->h_ctr->left) return DYC_OK;  // the policy needs every op's count
-        TRY(policy(t->h_actr[dyc::kCtrUp] + t->h_ctr->nins, t->h_actr[dyc::kCtrEr] + t->h_ctr->erased));
+        TRY(policy(t->h_actr[dyc::kCtrUp] + t->h_ctr->nins,
+                   t->h_actr[dyc::kCtrEr] + t->h_ctr->erased));
         TRY(push_desc(t, s));
         TRY(reset_call_counters(t, s));
     }
-    if (e == cudaSuccess && path != ApplyPath::kAll)
-        e = KB_CALL(t, apply_unique, L, t->D, t->sb, t->S, ops, keys, vals, vb, vals_out, bits_out,
-                    n, t->d_ctr, bins ? B.single : A.single, Ag.gate,
-                    before ? (uint32_t)dyc::kBinSkipEqual : 0u);
+    // the lists name no upsert of an equal value; neither may the one-pass
+    // kernel where its counts were taken before the batch
     if (e == cudaSuccess)
+        e = KB_CALL(t, apply_unique, L, t->D, t->sb, t->S, ops, keys, vals, vb, vals_out, bits_out,
+                    n, t->d_ctr, A.single, before ? (uint32_t)dyc::kBinSkipEqual : 0u);
+    if (e == cudaSuccess && before)
         e = KB_CALL(t, set_mutate, L, t->d_desc, 1u, t->d_ctr, t->sb, A.er_key, nullptr,
                     &A.ctr[dyc::kCtrEr], A.up_key, A.up_val, vb, nullptr, &A.ctr[dyc::kCtrUp], n,
                     t->S.list_a, nullptr, t->S.list_cap, t->d_ctr, &A.ctr[dyc::kCtrBad], nullptr,
@@ -1479,15 +1357,14 @@ dyc_status apply_kernels(dyc_table *t, ApplyPath path, const dyc::BinScratch &B,
     return DYC_OK;
 }
 
-// A chunk of n mixed ops, by bins (dyc_bins.cuh); ops of bins that went over,
-// and the chunks of tables the bin kernels do not serve, by grouping. The
-// upsize policy (api.cpp:359-369: the size after the batch's erases plus its
-// inserts above upper bound x capacity) needs the batch's upsert and erase
-// counts: where even n inserts keep the table within deferred_fill() of its
-// slots it is applied after the batch with the same counts, so the capacity
-// ends as if it had run first (entries the fuller table could not place
-// take the overflow path); otherwise the counts are taken first, the host
-// reads them and upsizes, and the batch is applied after that.
+// A chunk of n mixed ops. The upsize policy (api.cpp:359-369: the size after
+// the batch's erases plus its inserts above upper bound x capacity) needs the
+// batch's upsert and erase counts: where even n inserts keep the table within
+// deferred_fill() of its slots it is applied after the batch with the same
+// counts, so the capacity ends as if it had run first (entries the fuller
+// table could not place take the overflow path); otherwise the counts are
+// taken first, the host reads them and upsizes, and the batch is applied
+// after that.
 dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const void *vals,
                        uint64_t n, void *vals_out, uint32_t *bits_out, uint32_t flags,
                        cudaStream_t s) {
@@ -1506,66 +1383,32 @@ dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const
         }
         return DYC_OK;
     };
-    dyc_op_stats &St = t->last;
-    const dyc::BinScratch B = chunk_bins(t, n, t->A.single);
-    bool bins = bins_ok(t);
-    if (bins && B.single == nullptr) {  // a small batch
-        if (before) {
-            TRY(bins_small(t, B, dyc::kBinModeCount, ops, keys, vals, nullptr, nullptr, n, 0u, s));
-            if (t->h_ctr->left) bins = false;  // the policy needs every op's count
-            else TRY(policy(t->h_ctr->nins, t->h_ctr->erased));
-        }
-        if (bins)
-            TRY(bins_small(t, B, dyc::kBinModeMixed, ops, keys, vals, vals_out, bits_out, n,
-                           before ? (uint32_t)dyc::kBinSkipEqual : 0u, s));
-    } else if (bins) {
-        TRY(apply_kernels(t, ApplyPath::kBins, B, ops, keys, vals, n, vals_out, bits_out, before, s,
-                          policy));
-        if (before && t->h_ctr->left) bins = false;
+    bool done = small_batch(t, n);
+    if (done && before) {
+        TRY(bins_small(t, dyc::kBinModeCount, ops, keys, vals, nullptr, nullptr, n, 0u, s, &done));
+        if (done) TRY(policy(t->h_ctr->nins, t->h_ctr->erased));
     }
-    if (!bins)
-        TRY(apply_kernels(t, before ? ApplyPath::kAll : ApplyPath::kSingle, B, ops, keys, vals, n,
-                          vals_out, bits_out, before, s, policy));
-    Counters c = *t->h_ctr;
-    if (const uint64_t left = bins ? c.left : 0) {
-        if (c.overflow) {  // its list is used again below
-            St.overflowed += c.overflow;
-            TRY(drain(t, s, t->S.list_b, &t->d_ctr->overflow, t->S.list_a, &t->d_ctr->pending,
-                      t->S.list_cap, true, true));
-            grew = true;
-            c = *t->h_ctr;
-            c.overflow = 0;
-        }
-        void *lk, *lv, *lo = vals_out ? t->S.dedup : nullptr;
-        TRY(bins_left(t, B, ops, keys, vals, n, &lk, &lv, s));
-        TRY(apply_kernels(t, ApplyPath::kSingle, B, t->S.left_ops, lk, lv, left, lo,
-                          bits_out ? t->S.left_bits : nullptr, false, s,
-                          [](uint64_t, uint64_t) { return DYC_OK; }));
-        const cudaError_t e = KB_CALL(t, left_return, ctx(t, s), t->S, left, lo, (uint32_t)t->vb,
-                                      vals_out, bits_out);
-        if (e != cudaSuccess) return fail(DYC_ECUDA, "return kernel: %s", cudaGetErrorString(e));
-        CK(cudaStreamSynchronize(s));
-        c.inserted += t->h_ctr->inserted;
-        c.updated += t->h_ctr->updated;
-        c.erased += t->h_ctr->erased;
-        c.evict_steps += t->h_ctr->evict_steps;
-        c.overflow += t->h_ctr->overflow;
-    }
+    if (done)
+        TRY(bins_small(t, dyc::kBinModeMixed, ops, keys, vals, vals_out, bits_out, n,
+                       before ? (uint32_t)dyc::kBinSkipEqual : 0u, s, &done));
+    if (!done)
+        TRY(apply_kernels(t, ops, keys, vals, n, vals_out, bits_out, before, s, policy));
+    const Counters c = *t->h_ctr;
     // both kinds of keys' upserts and erases of present keys, as the table
     // counted them (an insert of the only op of its key counts as an update
     // even when the value is the same)
     if (!before) TRY(policy(c.inserted + c.updated, c.erased));
+    dyc_op_stats &St = t->last;
     St.inserted += c.inserted;
     St.updated += c.updated;
     St.erased += c.erased;
     St.evict_steps += c.evict_steps;
     St.overflowed += c.overflow;
     if (c.overflow) {
-        const Counters at = *t->h_ctr;
         TRY(drain(t, s, t->S.list_b, &t->d_ctr->overflow, t->S.list_a, &t->d_ctr->pending,
                   t->S.list_cap, true, !grew));
-        St.inserted += t->h_ctr->inserted - at.inserted;
-        St.evict_steps += t->h_ctr->evict_steps - at.evict_steps;
+        St.inserted += t->h_ctr->inserted - c.inserted;
+        St.evict_steps += t->h_ctr->evict_steps - c.evict_steps;
     }
     return DYC_OK;
 }
@@ -1771,6 +1614,7 @@ struct dyc_set {
     void *abuf = nullptr;
     size_t abytes = 0;
     dyc::ApplyScratch A{};
+    dyc::BinScratch bins{};
     void *lbuf = nullptr;
     size_t lbytes = 0;
     void *list_a = nullptr, *list_b = nullptr;
@@ -1792,8 +1636,6 @@ struct dyc_set {
     std::vector<Graph> graphs;
     uint64_t graph_clock = 0;
     cudaStream_t cap_stream = nullptr;  // capture stream (the caller's may be the legacy one)
-    cudaStream_t side = nullptr;        // replays that run beside the main sequence
-    cudaEvent_t fork = nullptr, join = nullptr;
     uint32_t blocks_per_sm = 0;  // launch cap of the set kernels (0: as many as fit)
     uint32_t max_evict_all = 0;  // largest member eviction bound
     dyc_op_stats last{};
@@ -1886,8 +1728,18 @@ dyc_status set_ensure_scratch(dyc_set *s, uint64_t n) {
     const uint64_t ops = n < 128 ? 128 : n;
     if (s->abuf && s->A.cap_ops >= ops) return DYC_OK;
     set_drop_graphs(s);
-    TRY(carve_apply(s->kb, s->vb, ops, 2 * ops, s->ntables, &s->abuf, &s->abytes, &s->A));
-    s->A.single_pass = 1u;  // keys with one op in a batch: k_set_unique in phase B
+    // table t's bins: ops / kBinMean + t (TableBins in dyc_bins.cuh)
+    const uint64_t nbins = ops / dyc::kBinMean + s->ntables + 1;
+    TRY(carve_apply(s->kb, s->vb, ops, s->ntables, nbins, &s->abuf, &s->abytes, &s->A));
+    s->bins = dyc::BinScratch{};
+    carve_bins(s->bins, s->A.bin_words, (uint32_t)nbins);
+    s->bins.tid = s->bins.cursor + nbins;
+    s->bins.rec = s->A.rec;
+    s->bins.hot = s->A.hot;
+    s->bins.single = s->A.single;
+    // a set's bin arrays do not change until the scratch does, and its kernels
+    // leave the counts zero
+    CK(cudaMemset(s->bins.state, 0, (dyc::kBinStates + 3 * nbins) * 4));
     const size_t slot = s->kb == 4 ? 8 : 16;
     const size_t lb = ((ops * slot + 255) & ~(size_t)255) * 2 + ((ops * 4 + 255) & ~(size_t)255) * 2;
     if (s->lbuf) {
@@ -1909,30 +1761,23 @@ dyc_status set_ensure_scratch(dyc_set *s, uint64_t n) {
 
 #define SET_KB_CALL(s, fn, ...) ((s)->kb == 4 ? Ops<4>::fn(__VA_ARGS__) : Ops<8>::fn(__VA_ARGS__))
 
-// Phase A: group, scatter, pre-batch find, replay; counters to the host.
+// Phase A: the repeated keys found, looked up and replayed; counters to the host.
 // Every kernel reads the op count from d_off[ntables] on the device; n (the
 // scratch capacity under a graph) only sizes the grids.
 dyc_status set_phase_a(dyc_set *s, const uint32_t *d_off, const uint8_t *ops, const void *keys,
                        const void *vals, void *out, uint32_t *bits, uint64_t n, bool new_counts,
                        cudaStream_t st) {
     const dyc::ApplyScratch &A = s->A;
-    const LaunchCtx L{s->sms, st, (int)s->blocks_per_sm, s->side, s->fork, s->join};
+    const LaunchCtx L{s->sms, st, (int)s->blocks_per_sm};
     const uint32_t vb = (uint32_t)s->vb;
-    const uint32_t *d_n = d_off + s->ntables;
     // the op count the host's offsets declare, which bounds the device's
     // (a pinned word: a captured graph copies its current value)
     CK(cudaMemcpyAsync(&A.ctr[dyc::kCtrHostN], s->h_hostn, sizeof(unsigned long long),
                        cudaMemcpyHostToDevice, st));
     // also zeroes phase B's counters (nothing between the phases uses them)
-    cudaError_t e = SET_KB_CALL(s, set_group, L, A, d_off, keys, n, bits, s->d_gctr);
+    cudaError_t e = SET_KB_CALL(s, set_group, L, A, s->bins, d_off, ops, keys, n, bits, s->d_gctr);
     if (e == cudaSuccess)
-        e = SET_KB_CALL(s, set_find, L, s->d_desc, s->ntables, s->sb, A.dkey, A.dtid,
-                        &A.ctr[dyc::kCtrDistinct], n, A.pre_val, vb, A.pre_hit,
-                        &A.ctr[dyc::kCtrBad], s->tables[0]->D.l2_keep != 0u);
-    if (e == cudaSuccess)
-        e = SET_KB_CALL(s, apply_scatter, L, A, n, d_n, ops, vals, vb, out, bits);
-    if (e == cudaSuccess)
-        e = SET_KB_CALL(s, apply_replay, L, A, ops, vals, vb, out, bits, n, n, d_n);
+        e = SET_KB_CALL(s, repeat, L, A, s->d_desc, s->ntables, s->sb, true, ops, vals, vb, out, bits, n);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "set phase A kernels: %s", cudaGetErrorString(e));
     if (new_counts)  // each table's upserts, for the upsize decision
     {
@@ -1948,9 +1793,9 @@ dyc_status set_phase_a(dyc_set *s, const uint32_t *d_off, const uint8_t *ops, co
 dyc_status set_phase_b(dyc_set *s, uint64_t n, cudaStream_t st, const uint32_t *hold = nullptr) {
     const dyc::ApplyScratch &A = s->A;
     const LaunchCtx L{s->sms, st, (int)s->blocks_per_sm};
-    cudaError_t e = cudaSuccess;
-    if (A.single_pass)  // keys with one op in the batch, after the policy's upsizes
-        e = SET_KB_CALL(s, set_unique, L, A, s->cur.off, s->d_desc, s->ntables, s->d_tctr, s->sb,
+    // keys with one op in the batch, after the policy's upsizes
+    cudaError_t e =
+        SET_KB_CALL(s, set_unique, L, A, s->cur.off, s->d_desc, s->ntables, s->d_tctr, s->sb,
                         s->cur.ops, s->cur.keys, s->cur.vals, (uint32_t)s->vb, s->cur.out,
                         s->cur.bits, n, s->list_a, s->tid_a, s->list_cap, s->d_gctr, hold,
                         s->tables[0]->D.l2_keep != 0u);
@@ -2227,9 +2072,6 @@ dyc_status dyc_set_create(const dyc_config *cfg, uint32_t ntables, const uint64_
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_hostn, sizeof(unsigned long long));
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_tup, sizeof(uint32_t) * ntables);
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_ter, sizeof(uint32_t) * ntables);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming);
     s->spares = cfg->auto_resize && cfg->device_upsize == 0u;
     if (s->spares) {
         if (e == cudaSuccess) e = dyc::lib_malloc(&s->d_spare, sizeof(dyc::Spare) * ntables);
@@ -2276,9 +2118,6 @@ dyc_status dyc_set_destroy(dyc_set *s) {
     cudaDeviceSynchronize();
     set_drop_graphs(s);
     if (s->cap_stream) cudaStreamDestroy(s->cap_stream);
-    if (s->side) cudaStreamDestroy(s->side);
-    if (s->fork) cudaEventDestroy(s->fork);
-    if (s->join) cudaEventDestroy(s->join);
     for (dyc_table *t : s->tables)
         if (t) dyc_destroy(t);
     if (s->h_spare)
@@ -2385,7 +2224,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
     uint64_t n = 0;
     if (!set_args_ok(s, d_offsets, h_offsets, d_ops, d_keys, d_vals, &n)) return DYC_EINVAL;
     if (n == 0) return DYC_OK;
-    // cells are indexed by 32 bits and a batch uses twice its ops of them
+    // an op's record holds its index in 31 bits
     if (n >= 0x80000000ull) return fail(DYC_EINVAL, "a set batch takes fewer than 2^31 ops");
     cudaStream_t st = (cudaStream_t)stream;
     {
@@ -2873,46 +2712,6 @@ unsigned wide_grid(dyc_wide *w, uint64_t n) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)w->t->sms * 8));
 }
 
-// Insert m keys whose op that counts S names (use_dedup): the current handles,
-// the staging of the values, and the placement of the new keys. Op i's value
-// is row idx[i] (row i without idx). left: ctr->left as copied to h_ctr before.
-dyc_status wide_insert_pass(dyc_wide *w, const Scratch &S, bool use_dedup, const void *k,
-                            const uint32_t *v, const uint32_t *idx, uint64_t m, uint32_t flags,
-                            cudaStream_t s, uint64_t *left = nullptr) {
-    dyc_table *t = w->t;
-    // current handles of the chunk's keys
-    cudaError_t e = KB_CALL(t, find, ctx(t, s), t->D, t->sb, k, w->pre_h, 4u, w->bits, m);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "wide find: %s", cudaGetErrorString(e));
-    TRY(wide_ensure_heap(w, m, s));
-    CK(cudaMemsetAsync(w->cnt, 0, 2 * sizeof(unsigned long long), s));
-    auto stage = t->kb == 4 ? dyc::k_wide_stage<4> : dyc::k_wide_stage<8>;
-    stage<<<wide_grid(w, m), 256, 0, s>>>(S, use_dedup ? 1 : 0, k, v, idx, w->words, m, w->pre_h,
-                                          w->bits, w->heap, w->stack, w->d_alloc, w->new_keys,
-                                          w->new_h, w->cnt);
-    dyc::k_wide_commit<<<1, 1, 0, s>>>(w->d_alloc, w->cnt);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(w->h_cnt, w->cnt, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    TRY(wide_read_alloc(w, s));
-    if (left) *left = t->h_ctr->left;
-    const uint64_t fresh = w->h_cnt[0];
-    w->last.updated += w->h_cnt[1];
-    if (fresh) {
-        if (t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE)) {
-            int guard = 0;
-            while ((double)(t->size + fresh) > t->cfg.upper_load * (double)t->capacity &&
-                   guard++ < 64)
-                TRY(resize_up_impl(t, s));
-        }
-        t->last = dyc_op_stats{};
-        TRY(insert_chunk(t, w->new_keys, w->new_h, fresh, DYC_FLAG_UNIQUE | DYC_FLAG_NEW_KEYS, s));
-        w->last.inserted += t->last.inserted;
-        w->last.evict_steps += t->last.evict_steps;
-        w->last.overflowed += t->last.overflowed;
-        w->last.resizes_up += t->last.resizes_up;
-    }
-    return DYC_OK;
-}
-
 }  // namespace
 
 extern "C" {
@@ -3001,28 +2800,37 @@ dyc_status dyc_wide_insert(dyc_wide *w, const void *d_keys, const void *d_vals, 
         const char *k = (const char *)d_keys + off * t->kb;
         const uint32_t *v = (const uint32_t *)((const char *)d_vals + off * w->vbytes);
         const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && m > 1;
-        if (!use_dedup || !bins_ok(t) || m <= dyc::kBinSmallOps) {
-            const Scratch S = chunk_scratch(t, m);
-            if (use_dedup) {  // clears the chunk's cells first
-                cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, k, m, dyc::kKeepLast);
-                if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
+        if (use_dedup)
+            TRY(bins_group(t, chunk_bins(t, m, t->S.winbits), dyc::ApplyScratch{},
+                           dyc::kBinModeInsert, nullptr, k, nullptr, m, s));
+        // current handles of the chunk's keys
+        cudaError_t e = KB_CALL(t, find, ctx(t, s), t->D, t->sb, k, w->pre_h, 4u, w->bits, m);
+        if (e != cudaSuccess) return fail(DYC_ECUDA, "wide find: %s", cudaGetErrorString(e));
+        TRY(wide_ensure_heap(w, m, s));
+        CK(cudaMemsetAsync(w->cnt, 0, 2 * sizeof(unsigned long long), s));
+        auto stage = t->kb == 4 ? dyc::k_wide_stage<4> : dyc::k_wide_stage<8>;
+        stage<<<wide_grid(w, m), 256, 0, s>>>(t->S, use_dedup ? 1 : 0, k, v, w->words, m, w->pre_h,
+                                              w->bits, w->heap, w->stack, w->d_alloc, w->new_keys,
+                                              w->new_h, w->cnt);
+        dyc::k_wide_commit<<<1, 1, 0, s>>>(w->d_alloc, w->cnt);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(w->h_cnt, w->cnt, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        TRY(wide_read_alloc(w, s));
+        const uint64_t fresh = w->h_cnt[0];
+        w->last.updated += w->h_cnt[1];
+        if (fresh) {
+            if (t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE)) {
+                int guard = 0;
+                while ((double)(t->size + fresh) > t->cfg.upper_load * (double)t->capacity &&
+                       guard++ < 64)
+                    TRY(resize_up_impl(t, s));
             }
-            TRY(wide_insert_pass(w, S, use_dedup, k, v, nullptr, m, flags, s));
-            continue;
-        }
-        const dyc::BinScratch B = chunk_bins(t, m, t->S.winbits);
-        TRY(bins_group(t, B, dyc::ApplyScratch{}, dyc::kBinModeInsert, nullptr, k, nullptr, m, s));
-        CK(cudaMemcpyAsync(&t->h_ctr->left, &t->d_ctr->left, sizeof(t->h_ctr->left),
-                           cudaMemcpyDeviceToHost, s));
-        uint64_t left = 0;
-        TRY(wide_insert_pass(w, bins_scratch(t), true, k, v, nullptr, m, flags, s, &left));
-        if (left) {  // keys of bins that went over: by the dedup table
-            void *lk, *lv;
-            TRY(bins_left(t, B, nullptr, k, nullptr, m, &lk, &lv, s));
-            const Scratch S = chunk_scratch(t, left);
-            cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, lk, left, dyc::kKeepLast);
-            if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
-            TRY(wide_insert_pass(w, S, true, lk, v, t->S.left_idx, left, flags, s));
+            t->last = dyc_op_stats{};
+            TRY(insert_chunk(t, w->new_keys, w->new_h, fresh, DYC_FLAG_UNIQUE | DYC_FLAG_NEW_KEYS, s));
+            w->last.inserted += t->last.inserted;
+            w->last.evict_steps += t->last.evict_steps;
+            w->last.overflowed += t->last.overflowed;
+            w->last.resizes_up += t->last.resizes_up;
         }
     }
     return DYC_OK;

@@ -35,11 +35,15 @@ namespace dyc {
 
 constexpr int kSmallR = kSmallCap / kBlockThreads;  // records per thread (k_bin_small)
 constexpr int kSmallTab = 2 * kSmallCap;            // cells of a bin's key table
+constexpr int kSmallBins = 96;
+static_assert(kBinSmallOps / kBinSmallMean < kSmallBins, "a small batch's bins are counted in one block");
+constexpr int kSplitThreads = 512;
+constexpr uint32_t kSplitBins = 4096;               // bins counted in shared memory (k_bin_scatter)
 constexpr int kGroupThreads = 512;
 constexpr int kGroupR = kBinCap / kGroupThreads;    // records per thread (k_bin_group)
 constexpr int kGroupTab = 2 * kBinCap;
 
-// An op of a bin: index << 2 | code (2 bits; any other code reads).
+// An op of a small batch's bin: index << 2 | code (2 bits; any other code reads).
 __device__ __forceinline__ uint32_t op_word(uint64_t i, uint8_t op) {
     return ((uint32_t)i << 2) | (op == kOpInsert ? 1u : op == kOpErase ? 2u : 0u);
 }
@@ -61,133 +65,464 @@ template <int BITS> __device__ __forceinline__ uint32_t bin_cell(uint32_t tag) {
     return ((tag ^ (tag >> 15)) * 0x9E3779B1u) >> (32 - BITS);
 }
 
-// Zero a chunk's bin counts, the call counters, the batch counters and the
-// result bits; set its single bits.
+// Start of a small batch: the call counters and the result bits zeroed.
 template <int KB>
-__global__ void __launch_bounds__(256) k_bin_clear(const __grid_constant__ BinScratch B,
-                                                   unsigned long long *zero, uint32_t nzero,
-                                                   unsigned long long *actr, uint32_t *bits,
-                                                   uint64_t words) {
+__global__ void __launch_bounds__(256) k_small_clear(unsigned long long *zero, uint32_t nzero,
+                                                     uint32_t *bits, uint64_t words) {
     const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = id; i < B.nbins; i += stride) B.count[i] = 0u;
     if (id < nzero) zero[id] = 0ull;
-    if (actr != nullptr && id < (uint64_t)kCtrSlots) actr[id] = 0ull;
-    if (bits != nullptr)
-        for (uint64_t w = id; w < words; w += stride) bits[w] = 0u;
-    if (B.single != nullptr)
-        for (uint64_t w = id; w < words; w += stride) B.single[w] = 0xffffffffu;
+    for (uint64_t w = id; w < words; w += (uint64_t)gridDim.x * blockDim.x) bits[w] = 0u;
+}
+
+// A record's op word: index << 2 | code, or (batches of 2^30 ops and more,
+// A.wide) index << 1 | insert. The segments of listed keys hold the former, or
+// plain indexes.
+__device__ __forceinline__ uint32_t rec_word(const ApplyScratch &A, uint32_t i, uint32_t code) {
+    return A.wide ? i << 1 | (code & 1u) : i << 2 | code;
+}
+__device__ __forceinline__ uint32_t rec_index(const ApplyScratch &A, uint32_t w) {
+    return A.wide ? w >> 1 : w >> 2;
+}
+__device__ __forceinline__ uint32_t seg_word(const ApplyScratch &A, uint32_t w) {
+    return A.wide ? w >> 1 : w;
 }
 
 __device__ __forceinline__ void clear_single(const BinScratch &B, uint32_t i) {
     atomicAnd(&B.single[i >> 5], ~(1u << (i & 31)));
 }
 
+// A table's bins in a set batch: ops [o0, o1) get bins o0 / kBinMean + t ..
+// o1 / kBinMean + t, so no two tables share one and a bin holds about kBinMean
+// ops. Offsets are clamped to n and the bins to nbins, so device offsets that
+// are out of order (reported by the call) stay inside the scratch.
+struct TableBins {
+    uint32_t first, n;
+};
+__device__ __forceinline__ TableBins table_bins(const BinScratch &B, const uint32_t *off, uint32_t t,
+                                                uint64_t n) {
+    const uint64_t a = __ldg(off + t), b = __ldg(off + t + 1);
+    const uint32_t o0 = (uint32_t)(a < n ? a : n) / kBinMean, o1 = (uint32_t)(b < n ? b : n) / kBinMean;
+    TableBins r{o0 + t, o1 >= o0 ? o1 - o0 + 1u : 1u};
+    if (r.first >= B.nbins) r.first = B.nbins - 1u;
+    if (r.n > B.nbins - r.first) r.n = B.nbins - r.first;
+    return r;
+}
+
+// Where the records of the bins that went over start in `hot`: their counts
+// summed in bin order. Every block of the pass that needs the starts computes
+// them all (the same values, so the writes agree).
+template <int KB> __device__ __noinline__ void plan_hot(const BinScratch &B) {
+    __shared__ uint32_t s_w[kSplitThreads / 32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t per = (B.nbins + kSplitThreads - 1) / kSplitThreads;
+    const uint32_t b0 = threadIdx.x * per, b1 = min(b0 + per, B.nbins);
+    uint32_t sum = 0u;
+    for (uint32_t b = b0; b < b1; ++b) {
+        const uint32_t c = B.count[b];
+        if (c > (uint32_t)kBinCap) sum += c;
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) s_w[w] = x;
+    __syncthreads();
+    uint32_t at = x - sum;
+    for (uint32_t v = 0; v < w; ++v) at += s_w[v];
+    for (uint32_t b = b0; b < b1; ++b) {
+        const uint32_t c = B.count[b];
+        if (c <= (uint32_t)kBinCap) continue;
+        B.start[b] = at;
+        at += c;
+    }
+    __syncthreads();
+}
+
 // Split a chunk into its bins: a block takes PER * 512 consecutive ops, counts
 // them per bin in shared memory (each op's place among the block's ops of its
 // bin comes back from the count), takes a range of every bin it has ops for,
 // and writes the ops' records there. Records of one bin come in no order; the
-// op index in the record orders the ops of a key. Ops beyond a bin's capacity
-// are not written (the count tells). Key-0 ops belong to no bin.
-template <int KB, int PER>
-__global__ void __launch_bounds__(512) k_bin_scatter(const __grid_constant__ BinScratch B,
-                                                     const uint8_t *__restrict__ ops,
-                                                     const void *__restrict__ keys, uint64_t n) {
+// op index in the record orders the ops of a key. Key-0 ops belong to no bin.
+// Ops beyond a bin's capacity are not written, which raises B.state[kBinOver]:
+// the pass HOT then gives all ops of such bins a record in `hot`.
+// SET: the ops of table t are [off[t], off[t + 1]) and go to its own bins; a
+// block's ops then fall into a short range of bins (its records land in long
+// runs), and ops outside a range of kSplitBins take their places one by one.
+// A single table's chunk starts here: the call counters (ctr), A.ctr and the
+// result bits are zeroed and the single bits set (k_set_prep does so for a
+// set). The bin counts, cursors and state are zero on entry: k_bin_group
+// leaves them so.
+template <int KB, int PER, bool SET, bool HOT>
+__global__ void __launch_bounds__(kSplitThreads, 2) k_bin_scatter(
+    const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
+    const uint32_t *__restrict__ off, const uint8_t *__restrict__ ops,
+    const void *__restrict__ keys, uint64_t n, unsigned long long *ctr, uint32_t *bits) {
     using K = typename SlotT<KB>::K;
-    extern __shared__ uint32_t s_cnt[];  // nbins
-    const uint32_t nb = B.nbins;
-    for (uint32_t b = threadIdx.x; b < nb; b += 512) s_cnt[b] = 0u;
-    __syncthreads();
-    static_assert(PER * 512 <= 1 << 13, "a place among the block's ops takes 13 bits");
-    const uint64_t base = (uint64_t)blockIdx.x * (PER * 512) + threadIdx.x;
-    uint32_t tag[PER], at[PER];  // at: place | bin << 13 | op code << 26, ~0 for key 0
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-        const uint64_t i = base + (uint64_t)j * 512;
-        const K k = i < n ? load_key<KB>(keys, i) : (K)0;
-        const uint32_t code = op_word(0, (ops != nullptr && i < n) ? ops[i] : (uint8_t)kOpFind);
-        tag[j] = bin_tag(k);
-        at[j] = k != 0 ? bin_of<KB>(k, nb) << 13 | code << 26 : 0xffffffffu;
+    constexpr uint64_t kTile = (uint64_t)PER * kSplitThreads;
+    static_assert(kTile <= 1 << 13 && kSplitBins <= 1 << 13, "a place and a bin take 13 bits each");
+    __shared__ uint32_t s_cnt[kSplitBins];
+    if (HOT && B.state[kBinOver] == 0u) return;
+    uint32_t *cursor = HOT ? B.cursor : B.count;
+    const uint64_t gid = (uint64_t)blockIdx.x * kSplitThreads + threadIdx.x;
+    if (SET) n = set_op_count(A, off);
+    if (SET && !HOT) {
+        // offsets that disagree with the host's, or are out of order, are
+        // reported (every access below stays inside the scratch either way)
+        if (gid == 0 && ((uint64_t)off[A.ntables] != A.ctr[kCtrHostN] || off[0] != 0u))
+            note_bad(A, kCtrBadOffsets);
+        for (uint64_t t = gid; t < A.ntables; t += (uint64_t)gridDim.x * kSplitThreads)
+            if (off[t] > off[t + 1]) note_bad(A, kCtrBadOffsets);
     }
+    if (!SET && !HOT) {
+        if (gid < sizeof(Counters) / 8 - 1) ctr[gid] = 0ull;
+        if (A.ctr != nullptr && gid < (uint64_t)kCtrSlots) A.ctr[gid] = 0ull;
+    }
+    bool went_over = false, planned = false;
+    auto put = [&](uint32_t b, uint32_t p, uint32_t tag, uint32_t word, uint32_t t) {
+        const unsigned long long r = (unsigned long long)tag | ((unsigned long long)word << 32);
+        if (HOT) {
+            B.hot[(uint64_t)B.start[b] + p] = r;
+            return;
+        }
+        if (SET && p == 0u) B.tid[b] = t;
+        if (p < (uint32_t)kBinCap) B.rec[(uint64_t)b * kBinCap + p] = r;
+        else went_over = true;
+    };
+    for (uint64_t tile = (uint64_t)blockIdx.x * kTile; tile < n; tile += (uint64_t)gridDim.x * kTile) {
+        uint32_t lo = 0u, nb = B.nbins;
+        if (SET) {
+            const uint64_t last = (tile + kTile < n ? tile + kTile : n) - 1;
+            const uint32_t t0 = table_at(A.tidx, off, (uint32_t)tile, (uint32_t)tile);
+            const uint32_t t1 = table_at(A.tidx, off, (uint32_t)last, (uint32_t)last);
+            const TableBins a = table_bins(B, off, t0, n), b = table_bins(B, off, t1, n);
+            lo = a.first;
+            nb = b.first + b.n > lo ? b.first + b.n - lo : 0u;
+            const bool all = nb <= kSplitBins;
+            if (!all) nb = kSplitBins;
+            if (HOT && all) {  // no bin of the tile's tables went over
+                bool any = false;
+                for (uint32_t b2 = threadIdx.x; b2 < nb; b2 += kSplitThreads)
+                    any |= B.count[lo + b2] > (uint32_t)kBinCap;
+                if (!__syncthreads_or(any)) continue;
+            }
+        }
+        if (HOT && !planned) {
+            planned = true;
+            plan_hot<KB>(B);
+        }
+        if (!SET && !HOT) {
+            const uint64_t words = ((tile + kTile < n ? tile + kTile : n) + 31) / 32;
+            for (uint64_t w = tile / 32 + threadIdx.x; w < words; w += kSplitThreads) {
+                B.single[w] = 0xffffffffu;
+                if (bits != nullptr) bits[w] = 0u;
+            }
+        }
+        for (uint32_t b = threadIdx.x; b < nb; b += kSplitThreads) s_cnt[b] = 0u;
+        __syncthreads();
+        // at: place | bin - lo << 13 | op code << 26; ~0: key 0, or done
+        uint32_t tag[PER], at[PER];
 #pragma unroll
-    for (int j = 0; j < PER; ++j)
-        if (at[j] != 0xffffffffu) at[j] |= atomicAdd(&s_cnt[(at[j] >> 13) & 0x1fffu], 1u);
+        for (int j = 0; j < PER; ++j) {
+            const uint64_t i = tile + (uint64_t)j * kSplitThreads + threadIdx.x;
+            const K k = i < n ? load_key<KB>(keys, i) : (K)0;
+            const uint32_t code = op_word(0, (ops != nullptr && i < n) ? ops[i] : (uint8_t)kOpFind);
+            tag[j] = bin_tag(k);
+            at[j] = 0xffffffffu;
+            if (k == 0) continue;
+            uint32_t b, t = 0u;
+            if (SET) {
+                t = table_at(A.tidx, off, (uint32_t)i, (uint32_t)i);
+                const TableBins tb = table_bins(B, off, t, n);
+                b = tb.first + bin_of<KB>(k, tb.n);
+            } else {
+                b = bin_of<KB>(k, nb);
+            }
+            if (HOT && B.count[b] <= (uint32_t)kBinCap) continue;
+            if (!SET || b - lo < nb) at[j] = (b - lo) << 13 | code << 26;
+            else put(b, atomicAdd(&cursor[b], 1u), tag[j], rec_word(A, (uint32_t)i, code), t);
+        }
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+            if (at[j] != 0xffffffffu) at[j] |= atomicAdd(&s_cnt[(at[j] >> 13) & 0x1fffu], 1u);
+        __syncthreads();
+        for (uint32_t b = threadIdx.x; b < nb; b += kSplitThreads) {
+            const uint32_t c = s_cnt[b];
+            if (c) s_cnt[b] = atomicAdd(&cursor[lo + b], c);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            if (at[j] == 0xffffffffu) continue;
+            const uint32_t b = (at[j] >> 13) & 0x1fffu, p = s_cnt[b] + (at[j] & 0x1fffu);
+            const uint32_t i = (uint32_t)tile + (uint32_t)j * kSplitThreads + threadIdx.x;
+            put(lo + b, p, tag[j], rec_word(A, i, at[j] >> 26),
+                (SET && !HOT && p == 0u) ? table_at(A.tidx, off, i, i) : 0u);
+        }
+        __syncthreads();  // the counts are reused by the next tile
+    }
+    if (!HOT && went_over) B.state[kBinOver] = 1u;
+}
+
+// A bin that went over (few keys, each repeated many times, or a skewed
+// batch's most popular ones): the block streams the bin's records twice, first
+// to count each key in a table in shared memory, then to give every op its
+// place. The table takes kHotMax keys; a bin with more is taken in parts by
+// further mixed bits of the key, split again until they fit, so every bin is
+// resolved whatever its keys.
+constexpr uint32_t kHotTab = 2048, kHotMax = 1024;
+
+struct HotSmem {
+    uint32_t first[kHotTab];  // index + 1 of an op with the cell's key
+    uint32_t cnt[kHotTab];    // ops of the key; insert / erase: the op that counts
+    uint32_t off[kHotTab];    // next place in seg (~0: the key has one op)
+    uint16_t id[kHotTab];
+    uint64_t part_mask[72], part[72];  // parts to do (each split adds one)
+    uint32_t top, nkey, nseg, nwarp, nmid, ndist, over, ok;
+    unsigned long long bkey, bseg, bwarp, bmid;
+};
+
+// 64 mixed bits of a key, different for different keys (splitmix64's finalizer).
+__device__ __forceinline__ uint64_t part_bits(uint64_t k) {
+    k = (k ^ (k >> 30)) * 0xBF58476D1CE4E5B9ull;
+    k = (k ^ (k >> 27)) * 0x94D049BB133111EBull;
+    return k ^ (k >> 31);
+}
+
+// List key d (its segment at `at`) by its number of ops, for k_repeat.
+__device__ __forceinline__ void list_long(const ApplyScratch &A, uint32_t d, uint32_t c,
+                                          uint32_t *nwarp, uint32_t *nmid,
+                                          unsigned long long bwarp, unsigned long long bmid) {
+    if (c > kWarpSeg) A.mid[bmid + atomicAdd(nmid, 1u)] = d;
+    else if (c > kShortSeg) A.wseg[bwarp + atomicAdd(nwarp, 1u)] = d;
+}
+
+// A block's ranges of the listed keys, their ops and the long-segment lists;
+// false when they would not fit (counts this batch cannot have produced).
+__device__ __forceinline__ bool take_ranges(const ApplyScratch &A, uint32_t nkey, uint32_t nseg,
+                                            uint32_t nwarp, uint32_t nmid, unsigned long long &bkey,
+                                            unsigned long long &bseg, unsigned long long &bwarp,
+                                            unsigned long long &bmid) {
+    bkey = atomicAdd(&A.ctr[kCtrDistinct], (unsigned long long)nkey);
+    bseg = atomicAdd(&A.ctr[kCtrPlaced], (unsigned long long)nseg);
+    bwarp = nwarp ? atomicAdd(&A.ctr[kCtrWarp], (unsigned long long)nwarp) : 0ull;
+    bmid = nmid ? atomicAdd(&A.ctr[kCtrMid], (unsigned long long)nmid) : 0ull;
+    const bool ok = bkey + nkey <= A.cap_ops && bseg + nseg <= A.cap_ops &&
+                    bwarp + nwarp <= A.cap_ops && bmid + nmid <= A.cap_ops;
+    if (!ok) note_bad(A);
+    return ok;
+}
+
+template <int KB, int MODE, bool SET>
+__device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &A, const void *keys,
+                                       uint32_t bin, uint32_t m, HotSmem &M) {
+    using K = typename SlotT<KB>::K;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, nt = kGroupThreads;
+    const unsigned long long *rec = B.hot + B.start[bin];
+    const uint32_t table = SET ? B.tid[bin] : 0u;
+    // key k's cell; claimed for op i when the key has none yet (claim)
+    auto cell_of = [&](K k, uint32_t i, bool claim) -> uint32_t {
+        uint32_t h = bin_cell<11>(bin_tag(k));
+        static_assert(kHotTab == 1u << 11, "bin_cell takes 11 bits");
+        // claims stop at kHotMax keys, plus one per thread on the way: cells
+        // stay free and the probe ends
+        static_assert(kHotMax + kGroupThreads < kHotTab, "a free cell remains");
+        while (true) {
+            uint32_t f = *(volatile uint32_t *)&M.first[h];
+            if (f == 0u) {
+                if (!claim || *(volatile uint32_t *)&M.over) return h;
+                f = atomicCAS(&M.first[h], 0u, i + 1u);
+                if (f == 0u) {
+                    if (atomicAdd(&M.ndist, 1u) >= kHotMax) *(volatile uint32_t *)&M.over = 1u;
+                    return h;
+                }
+            }
+            if (load_key<KB>(keys, f - 1u) == k) return h;
+            h = (h + 1u) & (kHotTab - 1u);
+        }
+    };
     __syncthreads();
-    for (uint32_t b = threadIdx.x; b < nb; b += 512) {
-        const uint32_t c = s_cnt[b];
-        if (c) s_cnt[b] = atomicAdd(&B.count[b], c);
+    if (tid == 0) {
+        M.top = 1u;
+        M.part_mask[0] = M.part[0] = 0ull;
     }
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-        if (at[j] == 0xffffffffu) continue;
-        const uint32_t b = (at[j] >> 13) & 0x1fffu;
-        const uint32_t p = s_cnt[b] + (at[j] & 0x1fffu);
-        const uint32_t i = (uint32_t)base + (uint32_t)j * 512u;
-        if (p < (uint32_t)kBinCap)
-            B.rec[(uint64_t)b * kBinCap + p] =
-                (unsigned long long)tag[j] | ((unsigned long long)(i << 2 | at[j] >> 26) << 32);
-        else
-            clear_single(B, i);
+    while (M.top != 0u) {
+        const uint32_t top = M.top;
+        const uint64_t mask = M.part_mask[top - 1], part = M.part[top - 1];
+        for (uint32_t c = tid; c < kHotTab; c += nt) {
+            M.first[c] = 0u;
+            M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
+            M.off[c] = 0xffffffffu;
+        }
+        if (tid == 0) M.nkey = M.nseg = M.nwarp = M.nmid = M.ndist = M.over = 0u;
+        __syncthreads();
+        for (uint32_t r0 = 0; r0 < m; r0 += nt) {
+            if (__any_sync(kFull, *(volatile uint32_t *)&M.over != 0u)) break;
+            const uint32_t r = r0 + tid;
+            const uint32_t i = r < m ? rec_index(A, (uint32_t)(rec[r] >> 32)) : 0u;
+            const K k = r < m ? load_key<KB>(keys, i) : (K)0;
+            const bool sel = r < m && (part_bits((uint64_t)k) & mask) == part;
+            const uint32_t h = sel ? cell_of(k, i, true) : 0u;
+            __syncwarp();
+            const unsigned peers = __match_any_sync(kFull, sel ? h : 0x80000000u | lane);
+            if (MODE == kBinModeMixed) {
+                if (sel && __ffs(peers) - 1 == (int)lane) atomicAdd(&M.cnt[h], __popc(peers));
+            } else if (sel) {
+                const uint32_t v = MODE == kBinModeInsert ? __reduce_max_sync(peers, i)
+                                                          : __reduce_min_sync(peers, i);
+                if (__ffs(peers) - 1 == (int)lane) {
+                    if (MODE == kBinModeInsert) atomicMax(&M.cnt[h], v);
+                    else atomicMin(&M.cnt[h], v);
+                }
+            }
+        }
+        __syncthreads();
+        const bool over = M.over != 0u;
+        __syncthreads();
+        if (tid == 0) {
+            if (over) {  // two parts by one more bit; nothing has been written for this one
+                M.part_mask[top - 1] = M.part_mask[top] = 2ull * mask + 1ull;
+                M.part[top] = part | (mask + 1ull);
+                M.top = top + 1u;
+            } else {
+                M.top = top - 1u;
+            }
+        }
+        __syncthreads();
+        if (over) continue;
+        if constexpr (MODE == kBinModeMixed) {
+            for (uint32_t c = tid; c < kHotTab; c += nt) {
+                const uint32_t k = M.cnt[c];
+                if (M.first[c] == 0u || k <= 1u) continue;
+                M.off[c] = atomicAdd(&M.nseg, k);
+                M.id[c] = (uint16_t)atomicAdd(&M.nkey, 1u);
+                if (k > kShortSeg) atomicAdd(k > kWarpSeg ? &M.nmid : &M.nwarp, 1u);
+            }
+            __syncthreads();
+            if (tid == 0) {
+                M.ok = take_ranges(A, M.nkey, M.nseg, M.nwarp, M.nmid, M.bkey, M.bseg, M.bwarp, M.bmid);
+                M.nwarp = M.nmid = 0u;
+            }
+            __syncthreads();
+            if (!M.ok) continue;
+            for (uint32_t c = tid; c < kHotTab; c += nt) {
+                if (M.off[c] == 0xffffffffu) continue;
+                const uint32_t d = (uint32_t)M.bkey + M.id[c], at = (uint32_t)M.bseg + M.off[c];
+                ((K *)A.dkey)[d] = load_key<KB>(keys, M.first[c] - 1u);
+                A.dcnt[d] = M.cnt[c];
+                A.dseg[d] = (unsigned long long)at << 32;
+                if (SET) A.dtid[d] = table;
+                list_long(A, d, M.cnt[c], &M.nwarp, &M.nmid, M.bwarp, M.bmid);
+                M.off[c] = at;
+            }
+            __syncthreads();
+        }
+        uint32_t ins = 0u;
+        for (uint32_t r0 = 0; r0 < m; r0 += nt) {
+            const uint32_t r = r0 + tid;
+            const uint32_t w = r < m ? (uint32_t)(rec[r] >> 32) : 0u, i = rec_index(A, w);
+            const K k = r < m ? load_key<KB>(keys, i) : (K)0;
+            const bool sel = r < m && (part_bits((uint64_t)k) & mask) == part;
+            const uint32_t h = sel ? cell_of(k, i, false) : 0u;
+            if constexpr (MODE == kBinModeMixed) {
+                const bool several = sel && M.cnt[h] > 1u;
+                if (SET && sel && !several) ins += w & 1u;
+                __syncwarp();
+                const unsigned peers = __match_any_sync(kFull, several ? h : 0x80000000u | lane);
+                const int lead = __ffs(peers) - 1;
+                uint32_t at = 0u;
+                if (several && lead == (int)lane) at = atomicAdd(&M.off[h], __popc(peers));
+                at = __shfl_sync(kFull, at, lead) + __popc(peers & ((1u << lane) - 1u));
+                if (several) {
+                    A.seg[at] = seg_word(A, w);
+                    clear_single(B, i);
+                }
+            } else if (sel && M.cnt[h] != i) {
+                clear_single(B, i);
+            }
+        }
+        if (SET && MODE == kBinModeMixed) {
+            ins = __reduce_add_sync(kFull, ins);
+            if (lane == 0 && ins && table < A.ntables) atomicAdd(&A.tup[table], ins);
+        }
+        __syncthreads();
     }
 }
 
 // One block per bin: its ops grouped by key in shared memory. Insert batches
 // keep the single bit of a key's last op, erase batches of its first. In a
 // mixed batch the ops of keys with several ops lose theirs and the keys are
-// listed: id d gets dkey, dcnt and dseg, and its op indexes a range of seg.
-template <int KB, int MODE>
-__global__ void __launch_bounds__(kGroupThreads) k_bin_group(const __grid_constant__ BinScratch B,
-                                                             const __grid_constant__ ApplyScratch A,
-                                                             const void *__restrict__ keys,
-                                                             Counters *ctr) {
+// listed: id d gets dkey, dcnt, dseg and (SET) dtid, and its op indexes a
+// range of seg; ids with more than kShortSeg ops go to wseg or mid as well.
+// SET: the inserts among the other ops are counted as upserts of the bin's
+// table (the upsize policy's insert batch).
+template <int KB, int MODE, bool SET>
+__global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
+    const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
+    const void *__restrict__ keys) {
     using K = typename SlotT<KB>::K;
-    __shared__ uint32_t s_tag[kBinCap], s_word[kBinCap], s_cnt[kBinCap], s_tab[kGroupTab];
-    __shared__ uint32_t s_nseg, s_nkey, s_ok;
-    __shared__ unsigned long long s_bseg, s_bkey;
+    struct Smem {
+        uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kGroupTab];
+    };
+    __shared__ __align__(16) unsigned char s_raw[sizeof(Smem)];
+    static_assert(sizeof(HotSmem) <= sizeof(Smem), "one block of shared memory for both");
+    Smem &M = *reinterpret_cast<Smem *>(s_raw);
+    __shared__ uint32_t s_nseg, s_nkey, s_nwarp, s_nmid, s_ok, s_ins;
+    __shared__ unsigned long long s_bseg, s_bkey, s_bwarp, s_bmid;
     const uint32_t tid = threadIdx.x, bin = blockIdx.x;
     const uint32_t m = B.count[bin];
-    const unsigned long long *rec = B.rec + (uint64_t)bin * kBinCap;
-    if (m > (uint32_t)kBinCap) {  // left to the general path
-        for (uint32_t r = tid; r < (uint32_t)kBinCap; r += kGroupThreads)
-            clear_single(B, (uint32_t)(rec[r] >> 32) >> 2);
-        if (tid == 0) atomicAdd(&ctr->left, (unsigned long long)m);
+    if (m == 0u) {
+        if (bin == 0 && tid < (uint32_t)kBinStates) B.state[tid] = 0u;
         return;
     }
-    for (uint32_t c = tid; c < (uint32_t)kGroupTab; c += kGroupThreads) s_tab[c] = 0u;
+    for (uint32_t c = tid; c < (uint32_t)kGroupTab; c += kGroupThreads) M.tab[c] = 0u;
+    if (tid == 0) s_nseg = s_nkey = s_nwarp = s_nmid = s_ins = 0u;
+    if (m <= (uint32_t)kBinCap) {
+        const unsigned long long *rec = B.rec + (uint64_t)bin * kBinCap;
 #pragma unroll
-    for (int q = 0; q < kGroupR; ++q) {
-        const uint32_t r = q * kGroupThreads + tid;
-        s_cnt[r] = MODE == kBinModeErase ? 0xffffffffu : 0u;
-        if (r < m) {
-            const unsigned long long x = rec[r];
-            s_tag[r] = (uint32_t)x;
-            s_word[r] = (uint32_t)(x >> 32);
+        for (int q = 0; q < kGroupR; ++q) {
+            const uint32_t r = q * kGroupThreads + tid;
+            M.cnt[r] = MODE == kBinModeErase ? 0xffffffffu : 0u;
+            if (r < m) {
+                const unsigned long long x = rec[r];
+                M.tag[r] = (uint32_t)x;
+                M.word[r] = (uint32_t)(x >> 32);
+            }
         }
     }
-    if (tid == 0) s_nseg = s_nkey = 0u;
     __syncthreads();
+    // every thread has read the count: the next batch finds it, and the
+    // split's state, zero
+    if (tid == 0) B.count[bin] = B.cursor[bin] = 0u;
+    if (bin == 0 && tid < (uint32_t)kBinStates) B.state[tid] = 0u;
+    if (m > (uint32_t)kBinCap) {
+        group_hot<KB, MODE, SET>(B, A, keys, bin, m, *reinterpret_cast<HotSmem *>(s_raw));
+        return;
+    }
     uint32_t lr[kGroupR];  // first record of the key | rank << 16
 #pragma unroll
     for (int q = 0; q < kGroupR; ++q) {
         const uint32_t r = q * kGroupThreads + tid;
         lr[q] = 0u;
         if (r >= m) continue;
-        const uint32_t tag = s_tag[r], w = s_word[r];
+        const uint32_t tag = M.tag[r], w = M.word[r];
         uint32_t h = bin_cell<12>(tag), lead;
         static_assert(kGroupTab == 1 << 12, "bin_cell takes 12 bits");
         while (true) {  // at most half of the cells are taken: the probe ends
-            const uint32_t old = atomicCAS(&s_tab[h], 0u, r + 1u);
+            const uint32_t old = atomicCAS(&M.tab[h], 0u, r + 1u);
             lead = old == 0u ? r : old - 1u;
             if (old == 0u) break;
-            if (s_tag[lead] == tag &&
-                (KB == 4 || load_key<KB>(keys, s_word[lead] >> 2) == load_key<KB>(keys, w >> 2)))
+            if (M.tag[lead] == tag &&
+                (KB == 4 || load_key<KB>(keys, rec_index(A, M.word[lead])) ==
+                                load_key<KB>(keys, rec_index(A, w))))
                 break;
             h = (h + 1u) & (kGroupTab - 1);
         }
-        if (MODE == kBinModeInsert) atomicMax(&s_cnt[lead], w);
-        else if (MODE == kBinModeErase) atomicMin(&s_cnt[lead], w);
-        else lr[q] = atomicAdd(&s_cnt[lead], 1u) << 16;
+        if (MODE == kBinModeInsert) atomicMax(&M.cnt[lead], w);
+        else if (MODE == kBinModeErase) atomicMin(&M.cnt[lead], w);
+        else lr[q] = atomicAdd(&M.cnt[lead], 1u) << 16;
         lr[q] |= lead;
     }
     __syncthreads();
@@ -195,45 +530,63 @@ __global__ void __launch_bounds__(kGroupThreads) k_bin_group(const __grid_consta
 #pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
             const uint32_t r = q * kGroupThreads + tid;
-            if (r < m && s_cnt[lr[q]] != s_word[r]) clear_single(B, s_word[r] >> 2);
+            if (r < m && M.cnt[lr[q]] != M.word[r]) clear_single(B, rec_index(A, M.word[r]));
         }
     } else {
         bool any = false;
+        uint32_t ins = 0u;
 #pragma unroll
-        for (int q = 0; q < kGroupR; ++q)
-            any |= q * kGroupThreads + tid < m && s_cnt[lr[q] & 0xffffu] > 1u;
-        if (!__syncthreads_or(any)) return;
+        for (int q = 0; q < kGroupR; ++q) {
+            const uint32_t r = q * kGroupThreads + tid;
+            const bool several = r < m && M.cnt[lr[q] & 0xffffu] > 1u;
+            any |= several;
+            if (SET && r < m && !several) ins += M.word[r] & 1u;
+        }
+        if (SET) {
+            ins = __reduce_add_sync(kFull, ins);
+            if ((tid & 31) == 0 && ins) atomicAdd(&s_ins, ins);
+        }
+        const bool more = __syncthreads_or(any);
+        const uint32_t table = SET ? B.tid[bin] : 0u;
+        if (SET && tid == 0 && s_ins && table < A.ntables) atomicAdd(&A.tup[table], s_ins);
+        if (!more) return;
         // the table's cells now hold each key's place in its block's ranges
 #pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
             const uint32_t r = q * kGroupThreads + tid;
-            if (r < m && (lr[q] & 0xffffu) == r && s_cnt[r] > 1u)
-                s_tab[r] = atomicAdd(&s_nseg, s_cnt[r]) | (atomicAdd(&s_nkey, 1u) << 16);
+            if (r >= m || (lr[q] & 0xffffu) != r) continue;
+            const uint32_t c = M.cnt[r];
+            if (c <= 1u) continue;
+            M.tab[r] = atomicAdd(&s_nseg, c) | (atomicAdd(&s_nkey, 1u) << 16);
+            if (c > kShortSeg) atomicAdd(c > kWarpSeg ? &s_nmid : &s_nwarp, 1u);
         }
         __syncthreads();
         if (tid == 0) {
-            s_bkey = atomicAdd(&A.ctr[kCtrDistinct], (unsigned long long)s_nkey);
-            s_bseg = atomicAdd(&A.ctr[kCtrPlaced], (unsigned long long)s_nseg);
-            s_ok = s_bkey + s_nkey <= A.cap_ops && s_bseg + s_nseg <= A.cap_ops;
-            if (!s_ok) note_bad(A);
+            s_ok = take_ranges(A, s_nkey, s_nseg, s_nwarp, s_nmid, s_bkey, s_bseg, s_bwarp, s_bmid);
+            s_nwarp = s_nmid = 0u;
         }
         __syncthreads();
         if (!s_ok) return;
+        // the ops of the block's segments are put in place in shared memory
+        // (the tags are done) and go out in order
 #pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
             const uint32_t r = q * kGroupThreads + tid, lead = lr[q] & 0xffffu;
-            if (r >= m || s_cnt[lead] <= 1u) continue;
-            const uint32_t i = s_word[r] >> 2;
-            const uint32_t off = (uint32_t)s_bseg + (s_tab[lead] & 0xffffu);
-            A.seg[off + (lr[q] >> 16)] = i;
+            if (r >= m || M.cnt[lead] <= 1u) continue;
+            const uint32_t w = M.word[r], i = rec_index(A, w), place = M.tab[lead] & 0xffffu;
+            M.tag[place + (lr[q] >> 16)] = seg_word(A, w);
             clear_single(B, i);
             if (lead == r) {
-                const uint32_t d = (uint32_t)s_bkey + (s_tab[lead] >> 16);
+                const uint32_t d = (uint32_t)s_bkey + (M.tab[lead] >> 16);
                 ((K *)A.dkey)[d] = load_key<KB>(keys, i);
-                A.dcnt[d] = s_cnt[r];
-                A.dseg[d] = (unsigned long long)off << 32;
+                A.dcnt[d] = M.cnt[r];
+                A.dseg[d] = (unsigned long long)((uint32_t)s_bseg + place) << 32;
+                if (SET) A.dtid[d] = table;
+                list_long(A, d, M.cnt[r], &s_nwarp, &s_nmid, s_bwarp, s_bmid);
             }
         }
+        __syncthreads();
+        for (uint32_t x = tid; x < s_nseg; x += kGroupThreads) A.seg[s_bseg + x] = M.tag[x];
     }
 }
 
@@ -309,7 +662,8 @@ template <int KB, int SB> struct BinSmem {
     uint32_t cnt[kSmallCap];  // per first op of a key: ops, then winner word or count | place << 16
     uint32_t seg[kSmallCap];
     uint16_t multi[kSmallCap / 2];
-    uint32_t m, nseg, nmulti, last;
+    uint32_t nseg, nmulti, last;
+    uint32_t bins[kSmallBins];  // ops per bin of the batch
     unsigned long long sum[6];
 };
 
@@ -367,7 +721,8 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
     for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kBlockThreads) tab[c] = 0u;
     for (uint32_t c = tid; c < (uint32_t)kSmallCap; c += kBlockThreads)
         M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
-    if (tid == 0) M.m = M.nseg = M.nmulti = 0u;
+    if (tid == 0) M.nseg = M.nmulti = 0u;
+    if (tid < (uint32_t)kSmallBins) M.bins[tid] = 0u;
     if (tid < 6) M.sum[tid] = 0ull;
     __syncthreads();
     uint32_t m;
@@ -382,26 +737,28 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
                     ++n_rej;
                     if ((MODE == kBinModeMixed) && vals_out) store_val(vals_out, vb, i, 0ull);
                 }
-            } else if (bin_of<KB>(k, gridDim.x) == bin) {
-                const uint32_t r = atomicAdd(&M.m, 1u);
-                if (r < (uint32_t)kSmallCap) {
+            } else {
+                const uint32_t b = bin_of<KB>(k, gridDim.x);
+                const uint32_t r = atomicAdd(&M.bins[b], 1u);
+                if (b == bin && r < (uint32_t)kSmallCap) {
                     M.key[r] = k;
                     M.word[r] = (uint32_t)i << 2;
                 }
             }
         }
         __syncthreads();
-        m = M.m;
-        if (tid == 0) B.count[bin] = m;
+        m = M.bins[bin];
         if (MODE >= kBinModeMixed && m <= (uint32_t)kSmallCap)
             for (uint32_t r = tid; r < m; r += kBlockThreads)
                 M.word[r] = op_word(M.word[r] >> 2, ops[M.word[r] >> 2]);
     }
     __syncthreads();
-    const bool hot = m > (uint32_t)kSmallCap;  // left to the general path (uniform over the block)
-    if (hot) {
-        if (tid == 0) atomicAdd(&ctr->left, (unsigned long long)m);
+    // every block counted every bin: all agree to leave a batch with a bin
+    // that does not fit to the split kernels, before anything is written
+    if (__syncthreads_or(tid < gridDim.x && M.bins[tid] > (uint32_t)kSmallCap)) {
+        if (bin == 0 && tid == 0) ctr->left = 1ull;
         m = 0u;
+        n_rej = 0u;
     }
 
     // group: each record finds its key's first record (lead)

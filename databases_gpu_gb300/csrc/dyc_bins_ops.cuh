@@ -8,7 +8,7 @@
 #include <set>
 #include <utility>
 
-#include "dyc_bins.cuh"
+#include "dyc_repeat.cuh"
 
 namespace dyc {
 
@@ -26,25 +26,78 @@ inline cudaError_t allow_smem(const void *kernel, int bytes) {
     return e;
 }
 
+// The split, the bins that went over, and the grouping (cap_n sizes the grids;
+// a set's kernels read the op count on the device).
+template <int KB, int MODE, bool SET>
+cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
+                       const uint32_t *off, const uint8_t *ops, const void *keys, uint64_t cap_n,
+                       unsigned long long *ctr, uint32_t *bits) {
+    // 16 ops a thread where that still fills the chip, else 8
+    const uint64_t tile = cap_n >= (1ull << 21) ? 16 * kSplitThreads : 8 * kSplitThreads;
+    const unsigned blocks = (unsigned)((cap_n + tile - 1) / tile);
+    if (tile == 16 * kSplitThreads)
+        k_bin_scatter<KB, 16, SET, false><<<blocks, kSplitThreads, 0, L.stream>>>(
+            B, A, off, ops, keys, cap_n, ctr, bits);
+    else
+        k_bin_scatter<KB, 8, SET, false><<<blocks, kSplitThreads, 0, L.stream>>>(
+            B, A, off, ops, keys, cap_n, ctr, bits);
+    // nothing to do in most batches: a fixed grid of one wave
+    const unsigned some = std::min<unsigned>(blocks, 4u * (unsigned)(L.sms > 0 ? L.sms : 1));
+    k_bin_scatter<KB, 8, SET, true><<<some, kSplitThreads, 0, L.stream>>>(B, A, off, ops, keys, cap_n,
+                                                                          ctr, nullptr);
+    k_bin_group<KB, MODE, SET><<<B.nbins, kGroupThreads, 0, L.stream>>>(B, A, keys);
+    return cudaGetLastError();
+}
+
 template <int KB>
 cudaError_t Ops<KB>::bin_group(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
                                int mode, const uint8_t *ops, const void *keys, uint32_t *bits_out,
                                uint64_t n, Counters *ctr) {
     if (n == 0) return cudaSuccess;
-    const uint64_t words = (n + 31) / 32;
-    k_bin_clear<KB><<<(unsigned)std::min<uint64_t>((words + 255) / 256, 1024), 256, 0, L.stream>>>(
-        B, &ctr->inserted, (uint32_t)(sizeof(Counters) / 8 - 1), A.ctr, bits_out, words);
-    const int smem = (int)B.nbins * 4;
-    // 16 ops a thread where that still fills the chip, else 8
-    if (n >= (1ull << 21))
-        k_bin_scatter<KB, 16><<<(unsigned)((n + 8191) / 8192), 512, smem, L.stream>>>(B, ops, keys, n);
-    else
-        k_bin_scatter<KB, 8><<<(unsigned)((n + 4095) / 4096), 512, smem, L.stream>>>(B, ops, keys, n);
-    auto k = mode == kBinModeInsert  ? k_bin_group<KB, kBinModeInsert>
-             : mode == kBinModeErase ? k_bin_group<KB, kBinModeErase>
-                                     : k_bin_group<KB, kBinModeMixed>;
-    k<<<B.nbins, kGroupThreads, 0, L.stream>>>(B, A, keys, ctr);
+    unsigned long long *c = &ctr->inserted;
+    if (mode == kBinModeInsert)
+        return bin_passes<KB, kBinModeInsert, false>(L, B, A, nullptr, ops, keys, n, c, bits_out);
+    if (mode == kBinModeErase)
+        return bin_passes<KB, kBinModeErase, false>(L, B, A, nullptr, ops, keys, n, c, bits_out);
+    return bin_passes<KB, kBinModeMixed, false>(L, B, A, nullptr, ops, keys, n, c, bits_out);
+}
+
+template <int KB>
+cudaError_t Ops<KB>::set_group(const LaunchCtx &L, const ApplyScratch &A, const BinScratch &B,
+                               const uint32_t *off, const uint8_t *ops, const void *keys,
+                               uint64_t n, uint32_t *bits, Counters *gctr) {
+    const uint64_t work = std::max<uint64_t>(n / 32 + 1, A.ntables);
+    k_set_prep<KB><<<(unsigned)std::min<uint64_t>((work + 255) / 256, 8ull * L.sms), 256, 0, L.stream>>>(
+        A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
+    if (n == 0) return cudaGetLastError();
+    return bin_passes<KB, kBinModeMixed, true>(L, B, A, off, ops, keys, n, nullptr, nullptr);
+}
+
+template <int KB, int SB>
+cudaError_t repeat_launch(const LaunchCtx &L, const ApplyScratch &A, const Desc *descs,
+                          uint32_t ntables, bool set, const uint8_t *ops, const void *vals,
+                          uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
+                          void *list_a, uint64_t list_cap, Counters *gctr) {
+    // a listed key has at least two ops; blocks loop over keys and segments
+    const uint64_t need = (n / 2 + 255) / 256 + 1, wave = 8ull * (uint64_t)(L.sms > 0 ? L.sms : 1);
+    const unsigned grid = (unsigned)std::min<uint64_t>(need, 2 * wave);
+    auto k = set ? k_repeat<KB, SB, true, false>
+                 : list_a ? k_repeat<KB, SB, false, true> : k_repeat<KB, SB, false, false>;
+    k<<<grid, 256, 0, L.stream>>>(A, descs, ntables, ops, vals, vb, vals_out, bits_out, list_a,
+                                  list_cap, gctr);
     return cudaGetLastError();
+}
+
+template <int KB>
+cudaError_t Ops<KB>::repeat(const LaunchCtx &L, const ApplyScratch &A, const Desc *descs,
+                            uint32_t ntables, int sb, bool set, const uint8_t *ops,
+                            const void *vals, uint32_t vb, void *vals_out, uint32_t *bits_out,
+                            uint64_t n, void *list_a, uint64_t list_cap, Counters *gctr) {
+    if (n == 0) return cudaSuccess;
+    const auto f = sb == 32   ? repeat_launch<KB, 32>
+                   : sb == 64 ? repeat_launch<KB, 64>
+                              : repeat_launch<KB, 128>;
+    return f(L, A, descs, ntables, set, ops, vals, vb, vals_out, bits_out, n, list_a, list_cap, gctr);
 }
 
 using BinFn = void (*)(Desc, Scratch, BinScratch, const uint8_t *, const void *, const void *, uint32_t,
@@ -64,8 +117,8 @@ cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const 
                                uint64_t n, uint32_t flags, Counters *ctr, Counters *h_ctr) {
     if (n == 0) return cudaSuccess;
     const uint64_t words = bits_out ? (n + 31) / 32 : 0;
-    k_bin_clear<KB><<<(unsigned)((words + 255) / 256 + 1), 256, 0, L.stream>>>(
-        B, &ctr->inserted, (uint32_t)(sizeof(Counters) / 8 - 1), nullptr, bits_out, words);
+    k_small_clear<KB><<<(unsigned)((words + 255) / 256 + 1), 256, 0, L.stream>>>(
+        &ctr->inserted, (uint32_t)(sizeof(Counters) / 8 - 1), bits_out, words);
     const BinFn k = sb == 32   ? small_kernel<KB, 32>(mode)
                     : sb == 64 ? small_kernel<KB, 64>(mode)
                                : small_kernel<KB, 128>(mode);

@@ -55,58 +55,58 @@ struct Counters {
     // scratch word: insert ops of a dyc_apply batch (its upserts, from the
     // counting pass of a batch resolved by bins)
     unsigned long long nins;
-    unsigned long long left;        // ops of bins that went over (left to the general path)
+    unsigned long long left;        // nonzero: a small batch has a bin that does not fit
     unsigned long long ticket;      // blocks of a small batch's kernel that have finished
 };
 static_assert(sizeof(Counters) == 128, "Counters is one 128-byte block");
 
 enum DedupMode { kKeepLast = 0, kKeepFirst = 1 };
 
-// Scratch lists used by one insert / erase / resize chunk.
-struct Scratch {
-    void *dedup;            // open-addressing table of (key, op index)
-    uint32_t *dedup_idx;    // op index array for 8-byte keys
-    uint64_t dedup_cap;     // power of two
-    void *list_a;           // pending entries (slots)
-    void *list_b;           // overflow entries (slots)
-    uint64_t list_cap;      // entries per list
-    // one bit per op of the chunk, set for the op its key's dedup cell names
-    // (filled from the dedup table after the claims); null: the winner is
-    // looked up in the dedup table by each op
-    uint32_t *winbits;
-    // nonzero once the dedup claims met a key twice; while it stays zero
-    // every op of the chunk is its key's only op (no winner bits are needed)
-    uint32_t *dupseen;
-    // the ops of bins that went over, gathered in index order for the general
-    // path (their keys and values go to list_b): op indexes, codes, result
-    // bits, per-block counts
-    uint32_t *bin_count;  // per bin of a chunk: ops
-    uint32_t *left_idx;
-    uint8_t *left_ops;
-    uint32_t *left_bits;
-    uint32_t *left_cnt;
-};
-
 // A chunk's ops split by key into bins (dyc_bins.cuh): bin b's records are
-// [b * kBinCap, b * kBinCap + min(count[b], kBinCap)), a bin holding kBinMean
-// ops of distinct random keys on average. A bin with more ops than its
-// capacity (few keys, each repeated many times) is left to the general path
-// as a whole. kBinMean * 2 = kBinCap, so the records of a chunk take no more
-// cells than its dedup table. Batches of up to kBinSmallOps ops are split by
-// the kernel that resolves them, into bins of kBinSmallMean ops.
+// [b * kBinCap, b * kBinCap + count[b]), a bin holding kBinMean ops of distinct
+// random keys on average. The ops of a bin with more than kBinCap (few keys,
+// each repeated many times) get records in `hot` instead. kBinMean * 2 =
+// kBinCap, so the records of n ops take 2n words. Batches of up to
+// kBinSmallOps ops are split by the kernel that resolves them, into bins of
+// kBinSmallMean ops.
 constexpr int kBinCap = 2048;
 constexpr int kBinMean = 1024;
 constexpr int kSmallCap = 1024;
 constexpr int kBinSmallMean = 192;
 constexpr uint64_t kBinSmallOps = 16384;
+enum : int {
+    kBinOver = 0,  // nonzero: some bin went over
+    kBinStates = 4
+};
 struct BinScratch {
-    unsigned long long *rec;  // key tag | op word << 32 (bin_tag, op_word)
+    unsigned long long *rec;  // key tag | op word << 32 (rec_word)
+    unsigned long long *hot;  // records of the bins that went over (one per op of the batch)
     uint32_t *count;          // per bin: ops
-    uint32_t nbins, cap;
+    uint32_t *start, *cursor; // per bin that went over: its records in hot; ops written
+    uint32_t *tid;            // set batches: table of a bin
+    uint32_t *state;          // kBinOver
+    uint32_t nbins;
     // one bit per op: cleared for the ops of keys with several ops (an insert
-    // or erase batch: all but the op that counts) and of bins that went over
+    // or erase batch: all but the op that counts)
     uint32_t *single;
 };
+
+// Scratch lists used by one insert / erase / resize chunk.
+struct Scratch {
+    // dyc_erase_noalloc: an open-addressing table of (key, op index), cleared
+    // by the caller; other batches name the op of a key that counts in winbits
+    void *dedup;
+    uint32_t *dedup_idx;    // op index array for 8-byte keys
+    uint64_t dedup_cap;     // power of two
+    void *list_a;           // pending entries (slots)
+    void *list_b;           // overflow entries (slots)
+    uint64_t list_cap;      // entries per list
+    // one bit per op of the chunk, set for the op of its key that counts
+    uint32_t *winbits;
+    unsigned long long *rec;  // records of the chunk's bins (BinScratch)
+    uint32_t *bin_words;      // the bins' state, counts, starts and cursors
+};
+
 enum : int {
     kBinModeInsert = 0,  // the last op of a key wins (dyc_insert)
     kBinModeErase = 1,   // the first op wins (dyc_erase)
@@ -117,65 +117,36 @@ enum : uint32_t {
     kBinNewKeys = 1,   // the caller promises absent keys (DYC_FLAG_NEW_KEYS)
     kBinSkipEqual = 2  // an insert that finds its own value writes and counts nothing
 };
-constexpr int kLeftTile = 2048;  // ops per block of the passes that gather what is left
-
-// Dedup tables of at least this many cells get the winners pass (winbits);
-// smaller ones fit in the L2 beside the bucket lines, so an op of a chunk
-// with repeats looks its winner up in the table instead, and the pass's
-// launch is saved.
-constexpr uint64_t kWinnersMinCap = 1ull << 22;
-__host__ __device__ inline bool winners_pass(const Scratch &S) {
-    return S.winbits != nullptr && S.dedup_cap >= kWinnersMinCap;
-}
 
 // Scratch of one mixed batch of at most `cap_ops` ops. The multi-table
 // fields are null for a single table.
 struct ApplyScratch {
-    // cap_cells cells: 4-byte keys {key, count} in 8 bytes, 8-byte keys
-    // {key, count, pad} in 16; key 0 = free. After compaction the count field
-    // holds the cell's distinct-key id.
-    void *cells;
-    uint32_t *op_cell;         // cell of each op
-    uint32_t *op_rank;         // place of each op inside its key's segment
-    void *dkey;                // distinct keys
-    uint32_t *dcnt;            // per distinct key: ops
-    unsigned long long *dseg;  // per distinct key: segment start << 32
-    uint32_t *seg;             // op indices grouped by key
-    void *pre_val;             // pre-batch value per distinct key
-    uint32_t *pre_hit;         // pre-batch hit bits per distinct key
+    void *dkey;                // keys with several ops in the batch
+    uint32_t *dcnt;            // per such key: ops
+    unsigned long long *dseg;  // per such key: segment start << 32
+    uint32_t *seg;             // ops grouped by key: index << 2 | code, plain indices if wide
+    uint32_t wide;             // batches of 2^30 ops and more
     void *up_key, *up_val;     // upserts to apply
     void *er_key;              // erases to apply
     unsigned long long *ctr;   // see kCtr*
-    uint32_t *wseg;            // distinct ids of segments replayed by a warp
-    uint32_t *mid;             // distinct ids of segments replayed by a block
+    uint32_t *wseg;            // ids of segments replayed by a warp
+    uint32_t *mid;             // ids of segments replayed by a block
     uint32_t *sort_tmp;        // merge scratch of long segments (same offsets as seg)
-    uint64_t cap_cells;        // >= 2 * cap_ops
     uint64_t cap_ops;
+    // bit i set when op i is its key's only op, or a key-0 op: left to the
+    // one-pass kernels
+    uint32_t *single;
     // multi-table batches
-    uint32_t *dtid;            // table of a distinct key
+    uint32_t *dtid;            // table of a listed key
     uint32_t *up_tid, *er_tid; // table of each upsert / erase
     uint32_t *tup;             // per table: upserts listed (the upsize policy's insert batch)
     uint32_t *ter;             // per table: erases listed (keys present before the batch)
-    uint32_t *tcell_off;       // per table: first cell of its region (ntables + 1)
     uint32_t *tidx;            // table of every kTidxStep-th op (cap_ops / kTidxStep + 1)
     uint32_t ntables;
-    // one table's batch (null: none): k_apply_group sets *gate once it meets
-    // a key twice; compaction and the scatter pass run only when it did.
-    unsigned long long *gate;
-    // nonzero: keys with a single op in the batch, and key-0 ops, are left
-    // to the one-pass kernel (k_apply_unique with op_cell / cells), which
-    // runs after the replays. Compaction lists only keys with several ops,
-    // so the find of the distinct keys, the scatter, the replays and the
-    // mutation see those alone.
-    uint32_t single_pass;
-    // single_pass batches: bit i set when op i is left to the one-pass
-    // kernel (written by the scatter, one word per warp, cap_ops / 32 + 1)
-    uint32_t *single;
+    unsigned long long *rec;   // records of the batch's bins (BinScratch); the other bin
+    uint32_t *bin_words;       // arrays; records of bins that went over
+    unsigned long long *hot;
 };
-
-// Cell words after compaction: kIdBit | distinct id. A word without the bit
-// in a single_pass batch is a count of 1 (a key compaction left alone).
-constexpr uint32_t kIdBit = 0x80000000u;
 
 constexpr uint32_t kTidxStep = 64;  // ops per entry of ApplyScratch::tidx
 
@@ -187,7 +158,7 @@ constexpr uint32_t kTidxStep = 64;  // ops per entry of ApplyScratch::tidx
 // disagree with the op count the host declared, kCtrHostN). The host turns
 // either count into an error.
 enum : int {
-    kCtrDistinct = 0,    // distinct keys
+    kCtrDistinct = 0,    // listed keys (several ops each)
     kCtrPlaced = 1,      // ops given a segment slot
     kCtrUp = 2,          // upserts listed
     kCtrEr = 3,          // erases listed
@@ -196,10 +167,8 @@ enum : int {
     kCtrBad = 6,         // device-read counts or ids out of range (must stay 0)
     kCtrBadOffsets = 7,  // set batch: offsets[ntables] != kCtrHostN, or an op outside its table
     kCtrHostN = 8,       // set batch: op count from the host's offsets (copied before the kernels)
-    kCtrRepeat = 9,      // one table's batch: nonzero once k_apply_group met a key twice
     kCtrSlots = 16
 };
-constexpr uint32_t kNoId = 0xffffffffu;  // a cell left without a distinct-key id
 
 
 // Upsizes of many subtables (of different tables) in one launch: job j
@@ -250,10 +219,6 @@ struct LaunchCtx {
     int sms;
     cudaStream_t stream;
     int max_blocks_per_sm = 0;  // 0: as many as fit (else a cap, chosen by a tuner)
-    // optional second stream for launches independent of the main sequence:
-    // forked after `fork` is recorded on `stream`, joined back through `join`
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 // Kernel launchers, one set per key width; `sb` = bucket bytes (32/64/128).
@@ -261,13 +226,9 @@ struct LaunchCtx {
 template <int KB> struct Ops {
     static cudaError_t find(const LaunchCtx &L, const Desc &D, int sb, const void *keys,
                             void *vals, uint32_t vb, uint32_t *hits, uint64_t n);
-    // the batch dedup of a chunk. With the table's own scratch (winbits
-    // set) it first clears the chunk's cells, winner bits and repeat flag,
-    // and `nzero` 64-bit words at `zero` (the call counters), in one launch;
-    // without, the caller has cleared the cells.
+    // erase_noalloc's batch dedup into S.dedup (cleared by the caller)
     static cudaError_t dedup(const LaunchCtx &L, const Scratch &S, const void *keys, uint64_t n,
-                             DedupMode mode, unsigned long long *zero = nullptr,
-                             uint32_t nzero = 0);
+                             DedupMode mode);
     // insert: place or update every op; ops whose two buckets are full go to
     // list_a (counted in pending). new_keys = caller promises absent keys.
     static cudaError_t place(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
@@ -312,50 +273,37 @@ template <int KB> struct Ops {
     static cudaError_t collect(const LaunchCtx &L, int sb, const void *sub, uint32_t nb,
                                void *list, unsigned long long *list_count, uint64_t list_cap,
                                unsigned long long *spill);
-    // mixed batches (dyc_apply.cuh). One table: apply_group (group +
-    // compact), find of the distinct keys, apply_scatter, apply_replay.
-    // Many tables (dyc_set.cuh): set_group replaces apply_group, and
-    // set_find / set_mutate / set_walk replace find / erase + place / walk.
-    static cudaError_t apply_group(const LaunchCtx &L, const ApplyScratch &A, const void *keys,
-                                  uint64_t n);
     // a mixed batch whose keys are all distinct, in one probe pass (ops left
     // without a slot go to S.list_a, counted in ctr->pending). With a single
-    // bitmap (a single_pass batch after its grouping and scatter), only the
-    // ops whose bit is set, and their hit bits are ORed in; all ops when
-    // *gate is 0 (no key repeated, so the scatter did not run). flags:
-    // kBinSkipEqual.
+    // bitmap, only the ops whose bit is set, and their hit bits are ORed in.
+    // flags: kBinSkipEqual.
     static cudaError_t apply_unique(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                                     const uint8_t *ops, const void *keys, const void *vals,
                                     uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
                                     Counters *ctr, const uint32_t *single = nullptr,
-                                    const unsigned long long *gate = nullptr,
                                     uint32_t flags = 0u);
     // *count += the INSERT ops among ops[0..n)
     static cudaError_t count_inserts(const LaunchCtx &L, const uint8_t *ops, uint64_t n,
                                      unsigned long long *count);
-    // after the find of the distinct keys: single-op keys resolved in op
-    // order, the other ops scattered into their keys' segments. n_ptr (many
-    // tables): the op count on the device; n then only sizes grids
-    static cudaError_t apply_scatter(const LaunchCtx &L, const ApplyScratch &A, uint64_t n,
-                                     const uint32_t *n_ptr, const uint8_t *ops, const void *vals,
-                                     uint32_t vb, void *vals_out, uint32_t *bits_out);
-    static cudaError_t apply_replay(const LaunchCtx &L, const ApplyScratch &A, const uint8_t *ops,
-                                   const void *vals, uint32_t vb, void *vals_out,
-                                   uint32_t *bits_out, uint64_t n, uint64_t max_distinct,
-                                   const uint32_t *n_ptr = nullptr);
-    // prep (counters, gctr, result bits, cell regions) + grouping + compaction
-    static cudaError_t set_group(const LaunchCtx &L, const ApplyScratch &A, const uint32_t *off,
-                                 const void *keys, uint64_t n, uint32_t *bits, Counters *gctr);
+    // the listed keys (dyc_repeat.cuh): state before the batch, replay,
+    // results. list_a set (one table, counters in gctr): the final states go
+    // to the table, entries without a slot to list_a; else to A's upsert and
+    // erase lists. n bounds the op count. set: keys carry their table (A.dtid).
+    static cudaError_t repeat(const LaunchCtx &L, const ApplyScratch &A, const Desc *descs,
+                              uint32_t ntables, int sb, bool set, const uint8_t *ops,
+                              const void *vals, uint32_t vb, void *vals_out, uint32_t *bits_out,
+                              uint64_t n, void *list_a = nullptr, uint64_t list_cap = 0,
+                              Counters *gctr = nullptr);
+    // a set batch's prep (counters, gctr, result bits, bin counts) and the
+    // split into bins and grouping (bin_group, per table)
+    static cudaError_t set_group(const LaunchCtx &L, const ApplyScratch &A, const BinScratch &B,
+                                 const uint32_t *off, const uint8_t *ops, const void *keys,
+                                 uint64_t n, uint32_t *bits, Counters *gctr);
     // The set kernels below read their item counts from device memory and
     // clamp them to max_n / max_entries (the capacity of the lists behind
     // them); a table id at or above ntables skips its item. Either event is
     // counted in *bad. hint: the members keep their lines in the L2 (their
     // probes carry L2 eviction-priority hints; plain loads otherwise).
-    static cudaError_t set_find(const LaunchCtx &L, const Desc *descs, uint32_t ntables, int sb,
-                                const void *keys, const uint32_t *tids,
-                                const unsigned long long *n_ptr, uint64_t max_n, void *vals,
-                                uint32_t vb, uint32_t *hits, unsigned long long *bad,
-                                bool hint = false);
     // erases and upserts of a set batch in one launch (max_n: both lists'
     // bound); nothing when *hold is nonzero (the host finishes the policy first)
     static cudaError_t set_mutate(const LaunchCtx &L, const Desc *descs, uint32_t ntables,
@@ -366,7 +314,7 @@ template <int KB> struct Ops {
                                   uint64_t max_n, void *list_a, uint32_t *list_a_tid,
                                   uint64_t list_cap, Counters *gctr, unsigned long long *bad,
                                   const uint32_t *hold = nullptr, bool hint = false);
-    // the ops of a single_pass set batch whose key has no other op in it
+    // the ops of a set batch whose key has no other op in it
     // (and key-0 ops), one probe each (k_set_unique); max_n bounds the grid,
     // the op count is read on the device; nothing when *hold is nonzero
     static cudaError_t set_unique(const LaunchCtx &L, const ApplyScratch &A, const uint32_t *off,
@@ -382,17 +330,16 @@ template <int KB> struct Ops {
                                 unsigned long long *dst_count, uint64_t dst_cap,
                                 uint32_t max_evict, Counters *gctr, uint64_t max_entries,
                                 unsigned long long *bad);
-    // A chunk of more than kBinSmallOps ops (dyc_bins.cuh): the bin counts,
-    // the call counters (zero, nzero), A.ctr and the result bits zeroed, the
-    // single bits set, the ops split into bins, and the ops of repeated keys
-    // found: their single bits cleared and, for a mixed batch (mode
-    // kBinModeMixed), their keys and segments listed in A as apply_group
-    // lists them. ops is null for the insert and erase modes.
+    // A chunk's repeated keys (dyc_bins.cuh): the bin counts, the call counters
+    // (ctr), A.ctr and the result bits zeroed, the single bits set, the ops
+    // split into bins, and the ops of repeated keys found: their single bits
+    // cleared and, for a mixed batch (mode kBinModeMixed), their keys and
+    // segments listed in A. ops is null for the insert and erase modes.
     static cudaError_t bin_group(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
                                  int mode, const uint8_t *ops, const void *keys, uint32_t *bits_out,
                                  uint64_t n, Counters *ctr);
     // a batch of up to kBinSmallOps ops in one of the kBinMode* modes; the
-    // counters go to h_ctr
+    // counters go to h_ctr (left set: nothing done, a bin does not fit)
     static cudaError_t bin_small(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                                  const BinScratch &B, int mode, const uint8_t *ops,
                                  const void *keys, const void *vals, uint32_t vb, void *vals_out,
@@ -403,15 +350,6 @@ template <int KB> struct Ops {
     static cudaError_t apply_count(const LaunchCtx &L, const Desc &D, int sb, const uint8_t *ops,
                                    const void *keys, const void *vals, uint32_t vb, uint64_t n,
                                    const uint32_t *single, Counters *ctr);
-    // the ops of the bins that went over, in index order (S.left_idx, their
-    // keys and values to list_b, codes to S.left_ops), and the way back of
-    // their results
-    static cudaError_t left_gather(const LaunchCtx &L, const Scratch &S, const BinScratch &B,
-                                   const uint8_t *ops, const void *keys, const void *vals,
-                                   uint32_t vb, uint64_t n, void *keys_left, void *vals_left);
-    static cudaError_t left_return(const LaunchCtx &L, const Scratch &S, uint64_t m,
-                                   const void *out, uint32_t vb, void *vals_out,
-                                   uint32_t *bits_out);
     // set every fingerprint bit of every bucket of a subtable
     static cudaError_t mark_all(const LaunchCtx &L, int sb, void *sub, uint32_t nb);
     static cudaError_t export_all(const LaunchCtx &L, const Desc &D, int sb, void *keys,

@@ -412,8 +412,9 @@ __device__ __forceinline__ KvOut place_probe(const char *p, typename SlotT<KB>::
 }
 
 // ----------------------------------------------------------------------------
-// Batch dedup: an open-addressing scratch table maps each key of the batch to
-// its last (insert) or first (erase) op index.
+// The op of a repeated key that counts: a bit per op (Scratch::winbits, from
+// the bins), or for dyc_erase_noalloc an open-addressing table of the batch's
+// keys in its fixed scratch.
 // ----------------------------------------------------------------------------
 template <int KB> struct Dedup;
 
@@ -431,14 +432,12 @@ template <> struct Dedup<4> {
             if ((uint32_t)(old >> 32) == k) {
                 if (mode == kKeepLast) atomicMax(&tab[h], mine);
                 else atomicMin(&tab[h], mine);
-                if (S.dupseen) *(volatile uint32_t *)S.dupseen = 1u;
                 return;
             }
         }
     }
     __device__ static __forceinline__ bool winner(const Scratch &S, uint32_t k, uint32_t i) {
-        if (S.dupseen && *S.dupseen == 0u) return true;  // no key repeats in the chunk
-        if (winners_pass(S)) return (S.winbits[i >> 5] >> (i & 31)) & 1u;
+        if (S.winbits != nullptr) return (S.winbits[i >> 5] >> (i & 31)) & 1u;
         const unsigned long long *tab = (const unsigned long long *)S.dedup;
         const uint64_t mask = S.dedup_cap - 1;
         uint64_t h = mix32(k) & mask;
@@ -463,14 +462,12 @@ template <> struct Dedup<8> {
             if (old == 0ull || old == k) {
                 if (mode == kKeepLast) atomicMax(&S.dedup_idx[h], i);
                 else atomicMin(&S.dedup_idx[h], i);
-                if (old == k && S.dupseen) *(volatile uint32_t *)S.dupseen = 1u;
                 return;
             }
         }
     }
     __device__ static __forceinline__ bool winner(const Scratch &S, uint64_t k, uint32_t i) {
-        if (S.dupseen && *S.dupseen == 0u) return true;  // no key repeats in the chunk
-        if (winners_pass(S)) return (S.winbits[i >> 5] >> (i & 31)) & 1u;
+        if (S.winbits != nullptr) return (S.winbits[i >> 5] >> (i & 31)) & 1u;
         const unsigned long long *tab = (const unsigned long long *)S.dedup;
         const uint64_t mask = S.dedup_cap - 1;
         uint64_t h = mix32(fold(k) ^ (uint32_t)(k >> 32)) & mask;
@@ -483,30 +480,6 @@ template <> struct Dedup<8> {
     }
 };
 
-// Clears one chunk's dedup state in one launch: the key cells (16-byte
-// stores; dedup_cap is a power of two >= 32 and the cells are 256-byte
-// aligned), the op-index cells of 8-byte keys (to idx_fill), win_words
-// winner-bit words, the repeat flag, and nzero 64-bit words at zero.
-template <int KB>
-__global__ void __launch_bounds__(256) k_dedup_clear(const __grid_constant__ Scratch S,
-                                                     uint32_t idx_fill, uint64_t win_words,
-                                                     unsigned long long *zero, uint32_t nzero) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint4 *cells = (uint4 *)S.dedup;
-    const uint64_t n16 = S.dedup_cap / 2;  // two 8-byte cells per store
-    for (uint64_t i = tid; i < n16; i += stride) cells[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (KB == 8 && S.dedup_idx != nullptr) {
-        uint4 *ix = (uint4 *)S.dedup_idx;
-        const uint4 f = make_uint4(idx_fill, idx_fill, idx_fill, idx_fill);
-        for (uint64_t i = tid; i < S.dedup_cap / 4; i += stride) ix[i] = f;
-    }
-    if (S.winbits != nullptr)
-        for (uint64_t i = tid; i < win_words; i += stride) S.winbits[i] = 0u;
-    if (tid == 0 && S.dupseen != nullptr) *S.dupseen = 0u;
-    if (tid < nzero) zero[tid] = 0ull;
-}
-
 template <int KB>
 __global__ void __launch_bounds__(256) k_dedup(const __grid_constant__ Scratch S,
                                                const void *__restrict__ keys, uint64_t n,
@@ -515,27 +488,6 @@ __global__ void __launch_bounds__(256) k_dedup(const __grid_constant__ Scratch S
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         typename SlotT<KB>::K k = load_key<KB>(keys, i);
         if (k != 0) Dedup<KB>::claim(S, k, (uint32_t)i, mode);
-    }
-}
-
-// After the claims: one pass over the dedup cells (sequential reads) sets
-// the winner bit of the op each used cell names (L2 atomics into a bitmap of
-// n bits), so the place and erase kernels read their op's bit coalesced
-// instead of probing the dedup table at random once more (the table of a
-// 4M-op chunk is 64 MB; those probes cost DRAM accesses beside the bucket
-// reads). A chunk whose claims met no key twice skips the pass: every op
-// wins (dupseen).
-template <int KB>
-__global__ void __launch_bounds__(256) k_dedup_winners(const __grid_constant__ Scratch S) {
-    if (S.dupseen && *S.dupseen == 0u) return;  // every op is its key's only one
-    const unsigned long long *tab = (const unsigned long long *)S.dedup;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; h < S.dedup_cap;
-         h += stride) {
-        const unsigned long long c = tab[h];
-        if (c == 0ull) continue;
-        const uint32_t i = KB == 4 ? (uint32_t)c : S.dedup_idx[h];
-        atomicOr(&S.winbits[i >> 5], 1u << (i & 31));
     }
 }
 

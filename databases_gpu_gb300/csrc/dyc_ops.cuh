@@ -7,7 +7,6 @@
 #include <mutex>
 #include <unordered_map>
 
-#include "dyc_left.cuh"
 #include "dyc_set.cuh"
 #include "dyc_kernels.cuh"
 
@@ -27,20 +26,6 @@ inline int tile_grid(const LaunchCtx &L, uint64_t n) {
     const uint64_t one_each = (n + 255) / 256, wave = 8ull * (uint64_t)(L.sms > 0 ? L.sms : 1);
     const uint64_t floor_g = one_each < wave ? one_each : wave;
     if (g < floor_g) g = floor_g;
-    if (L.max_blocks_per_sm > 0) {
-        const uint64_t cap = (uint64_t)L.max_blocks_per_sm * (uint64_t)(L.sms > 0 ? L.sms : 1);
-        if (g > cap) g = cap;
-    }
-    return (int)(g < 1 ? 1 : (g > 0x7fffffffull ? 0x7fffffffull : g));
-}
-
-// Compaction: one block per tile of 256 * kCompactRun cells (a block's tile
-// ends in two barriers and two atomics, so many short blocks keep more tiles
-// in flight than one resident wave looping over them); the tuner's cap
-// applies as for tile_grid.
-inline int compact_grid(const LaunchCtx &L, uint64_t cells) {
-    const uint64_t tile = 256ull * kCompactRun;
-    uint64_t g = (cells + tile - 1) / tile;
     if (L.max_blocks_per_sm > 0) {
         const uint64_t cap = (uint64_t)L.max_blocks_per_sm * (uint64_t)(L.sms > 0 ? L.sms : 1);
         if (g > cap) g = cap;
@@ -97,19 +82,10 @@ cudaError_t Ops<KB>::find(const LaunchCtx &L, const Desc &D, int sb, const void 
 
 template <int KB>
 cudaError_t Ops<KB>::dedup(const LaunchCtx &L, const Scratch &S, const void *keys, uint64_t n,
-                           DedupMode mode, unsigned long long *zero, uint32_t nzero) {
+                           DedupMode mode) {
     if (n == 0) return cudaSuccess;
-    if (S.winbits) {
-        auto c = k_dedup_clear<KB>;
-        c<<<grid_for((const void *)c, L, S.dedup_cap / 2), 256, 0, L.stream>>>(
-            S, mode == kKeepLast ? 0u : 0xFFFFFFFFu, n / 32 + 1, zero, nzero);
-    }
     auto k = k_dedup<KB>;
     k<<<grid_for((const void *)k, L, n), 256, 0, L.stream>>>(S, keys, n, mode);
-    if (winners_pass(S)) {
-        auto w = k_dedup_winners<KB>;
-        w<<<grid_for((const void *)w, L, S.dedup_cap), 256, 0, L.stream>>>(S);
-    }
     return cudaGetLastError();
 }
 
@@ -158,13 +134,12 @@ template <int KB>
 cudaError_t Ops<KB>::apply_unique(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                                   const uint8_t *ops, const void *keys, const void *vals,
                                   uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
-                                  Counters *ctr, const uint32_t *single,
-                                  const unsigned long long *gate, uint32_t flags) {
+                                  Counters *ctr, const uint32_t *single, uint32_t flags) {
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_apply_unique<KB, SB, true> : k_apply_unique<KB, SB, false>;
         k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, ops, keys, vals, vb, vals_out, bits_out, n,
-                                                  ctr, single, gate, flags);
+                                                  ctr, single, flags);
     });
     return cudaGetLastError();
 }
@@ -267,90 +242,6 @@ cudaError_t Ops<KB>::collect(const LaunchCtx &L, int sb, const void *sub, uint32
 }
 
 template <int KB>
-cudaError_t Ops<KB>::apply_group(const LaunchCtx &L, const ApplyScratch &A, const void *keys,
-                                 uint64_t n) {
-    if (n == 0) return cudaSuccess;
-    auto g = k_apply_group<KB>;
-    g<<<tile_grid(L, n), 256, 0, L.stream>>>(A, keys, n);
-    auto c = k_apply_compact<KB>;
-    c<<<compact_grid(L, 2 * n), 256, 0, L.stream>>>(A, 2 * n);
-    return cudaGetLastError();
-}
-
-template <int KB>
-cudaError_t Ops<KB>::apply_scatter(const LaunchCtx &L, const ApplyScratch &A, uint64_t n,
-                                   const uint32_t *n_ptr, const uint8_t *ops, const void *vals,
-                                   uint32_t vb, void *vals_out, uint32_t *bits_out) {
-    if (n == 0) return cudaSuccess;
-    auto sc = k_apply_scatter<KB>;
-    sc<<<tile_grid(L, n), 256, 0, L.stream>>>(A, n, n_ptr, ops, vals, vb, vals_out, bits_out);
-    return cudaGetLastError();
-}
-
-template <int KB>
-cudaError_t Ops<KB>::apply_replay(const LaunchCtx &L, const ApplyScratch &A, const uint8_t *ops,
-                                  const void *vals, uint32_t vb, void *vals_out,
-                                  uint32_t *bits_out, uint64_t n, uint64_t max_distinct,
-                                  const uint32_t *n_ptr) {
-    if (n == 0) return cudaSuccess;
-    auto r = k_apply_replay<KB>;
-    const uint64_t work = n > max_distinct ? n : max_distinct;
-    r<<<tile_grid(L, work), 256, 0, L.stream>>>(A, ops, vals, vb, vals_out, bits_out, n, n_ptr);
-    // the segment classes are disjoint: with a side stream the warp and
-    // block replays run beside the thread replay
-    const bool forked = L.side != nullptr;
-    cudaStream_t s2 = forked ? L.side : L.stream;
-    if (forked) {
-        cudaError_t e = cudaEventRecord(L.fork, L.stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(L.side, L.fork, 0);
-        if (e != cudaSuccess) return e;
-    }
-    auto w = k_apply_replay_warp<KB>;
-    // one warp per kWarpTask warp segments; at most n / (kShortSeg + 1) segments
-    w<<<grid_for((const void *)w, L, (n / (kShortSeg + 1) / kWarpTask + 1) * 32), 256, 0, s2>>>(
-        A, ops, vals, vb, vals_out, bits_out);
-    auto m = k_apply_replay_mid<KB>;
-    // one block per mid segment; at most n / (kWarpSeg + 1) of them
-    m<<<grid_for((const void *)m, L, (n / (kWarpSeg + 1) + 1) * 256), 256, 0, s2>>>(
-        A, ops, vals, vb, vals_out, bits_out);
-    if (forked) {
-        cudaError_t e = cudaEventRecord(L.join, L.side);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(L.stream, L.join, 0);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaGetLastError();
-}
-
-template <int KB>
-cudaError_t Ops<KB>::set_group(const LaunchCtx &L, const ApplyScratch &A, const uint32_t *off,
-                               const void *keys, uint64_t n, uint32_t *bits, Counters *gctr) {
-    auto pr = k_set_prep<KB>;
-    pr<<<grid_for((const void *)pr, L, 2 * n * (cell_bytes<KB>() / 8) + 1), 256, 0, L.stream>>>(
-        A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
-    if (n) {  // n sizes the grids; the kernels read the op count from off[ntables]
-        auto g = k_set_group<KB>;
-        g<<<tile_grid(L, n), 256, 0, L.stream>>>(A, off, keys);
-        auto c = k_apply_compact<KB>;
-        c<<<compact_grid(L, 2 * n), 256, 0, L.stream>>>(A, 0);
-    }
-    return cudaGetLastError();
-}
-
-template <int KB>
-cudaError_t Ops<KB>::set_find(const LaunchCtx &L, const Desc *descs, uint32_t ntables, int sb,
-                              const void *keys, const uint32_t *tids,
-                              const unsigned long long *n_ptr, uint64_t max_n, void *vals,
-                              uint32_t vb, uint32_t *hits, unsigned long long *bad, bool hint) {
-    if (max_n == 0) return cudaSuccess;
-    DYC_SB_DISPATCH(sb, {
-        auto k = hint ? k_set_find<KB, SB, true> : k_set_find<KB, SB, false>;
-        k<<<tile_grid(L, max_n), 256, 0, L.stream>>>(descs, ntables, keys, tids, n_ptr, max_n,
-                                                     vals, vb, hits, bad);
-    });
-    return cudaGetLastError();
-}
-
-template <int KB>
 cudaError_t Ops<KB>::set_mutate(const LaunchCtx &L, const Desc *descs, uint32_t ntables,
                                 Counters *tctr, int sb, const void *er_keys,
                                 const uint32_t *er_tids, const unsigned long long *ne_ptr,
@@ -427,26 +318,6 @@ cudaError_t Ops<KB>::export_all(const LaunchCtx &L, const Desc &D, int sb, void 
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
-}
-
-template <int KB>
-cudaError_t Ops<KB>::left_gather(const LaunchCtx &L, const Scratch &S, const BinScratch &B,
-                                 const uint8_t *ops, const void *keys, const void *vals,
-                                 uint32_t vb, uint64_t n, void *keys_left, void *vals_left) {
-    const unsigned tiles = (unsigned)((n + kLeftTile - 1) / kLeftTile);
-    k_left_count<KB><<<tiles, 256, 0, L.stream>>>(B, S, keys, n);
-    k_left_scan<KB><<<1, 1024, 0, L.stream>>>(S.left_cnt, tiles);
-    k_left_gather<KB><<<tiles, 256, 0, L.stream>>>(B, S, ops, keys, vals, vb, n, keys_left, vals_left);
-    return cudaGetLastError();
-}
-
-template <int KB>
-cudaError_t Ops<KB>::left_return(const LaunchCtx &L, const Scratch &S, uint64_t m, const void *out,
-                                 uint32_t vb, void *vals_out, uint32_t *bits_out) {
-    if (m == 0) return cudaSuccess;
-    k_left_return<KB><<<(unsigned)std::min<uint64_t>((m + 255) / 256, 4096), 256, 0, L.stream>>>(
-        S, m, out, vb, vals_out, bits_out);
-    return cudaGetLastError();
 }
 
 }  // namespace dyc

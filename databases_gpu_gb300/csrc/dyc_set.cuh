@@ -1,7 +1,7 @@
-// dyc_set.cuh -- probe kernels of a multi-table batch (a table set): the find
-// of the distinct keys, one pass for the erases and upserts, and the eviction
-// walks, with the logic of the single-table kernels in dyc_kernels.cuh, but
-// every item carries a table id and reads that
+// dyc_set.cuh -- probe kernels of a multi-table batch (a table set): the ops
+// with a key of their own, one pass for the listed erases and upserts, and the
+// eviction walks, with the logic of the single-table kernels in
+// dyc_kernels.cuh, but every item carries a table id and reads that
 // table's descriptor from a device array, so one grid-stride launch serves
 // the work of every table in the set. Item counts are read on the device
 // (the counters the mixed-batch kernels fill), so a batch's launch sequence
@@ -46,55 +46,6 @@ __device__ __forceinline__ uint32_t checked_tid(const uint32_t *tids, uint64_t i
     atomicAdd(bad, 1ull);
     ok = false;
     return 0u;
-}
-
-// find of keys[i] in table tids[i], i < *n_ptr (k_find per table)
-template <int KB, int SB, bool HINT>
-__global__ void __launch_bounds__(256) k_set_find(const Desc *__restrict__ descs, uint32_t ntables,
-                                                  const void *__restrict__ keys,
-                                                  const uint32_t *__restrict__ tids,
-                                                  const unsigned long long *__restrict__ n_ptr,
-                                                  uint64_t max_n, void *__restrict__ vals,
-                                                  uint32_t vb, uint32_t *__restrict__ hits,
-                                                  unsigned long long *bad) {
-    using T = SlotT<KB>;
-    using Gm = Geo<KB, SB>;
-    __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
-    unsigned char *stage = s_stage[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t n = clamped_count(n_ptr, max_n, bad);
-    const uint64_t step = warp_stride();
-    for (uint64_t base = warp_base(); base < n; base += step) {
-        const uint64_t i = base + lane;
-        typename T::K k = 0;
-        uint32_t tb = 0u;
-        bool ok = true;
-        if (i < n) {
-            k = load_key<KB>(keys, i);
-            tb = checked_tid(tids, i, ntables, bad, ok);
-        }
-        const Desc &D = descs[tb];
-        const bool act = ok && k != 0;
-        const unsigned long long tpol = HINT ? l2_policies(D.l2_keep != 0u).table : 0ull;
-        const uint32_t hk = fold(k);
-        const Pair p = pair_of(hk, D.d);
-        const char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
-        const KvOut r1 = kv_probe<KB, SB, 1, HINT>(p1, k, act, stage, tpol);
-        bool hit = act && r1.match >= 0;
-        uint64_t v = hit ? r1.value : 0ull;
-        const bool need2 = act && !hit && (!Gm::kMeta || r1.overflow);
-        if (__any_sync(kFull, need2)) {
-            const char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
-            const KvOut r2 = kv_probe<KB, SB, 1, HINT>(p2, k, need2, stage, tpol);
-            if (need2 && r2.match >= 0) {
-                hit = true;
-                v = r2.value;
-            }
-        }
-        if (i < n) store_val(vals, vb, i, v);
-        const unsigned m = __ballot_sync(kFull, hit);
-        if (hits != nullptr && lane == 0) hits[base >> 5] = m;
-    }
 }
 
 // erase of unique keys[i] from table tids[i], i in [base, base + 32) and
@@ -272,11 +223,11 @@ __global__ void __launch_bounds__(256) k_set_mutate(
 
 // The ops of a set batch whose key has no other op in it (and key-0 ops),
 // after the device policy's upsizes and before the mutation of the repeated
-// keys (ApplyScratch::single_pass): each resolved in one probe of its
+// keys: each resolved in one probe of its
 // table's buckets, as k_apply_unique does for one table. The result is the
 // key's state before the batch; an insert updates in place or claims an
 // empty slot, else goes to list_a with its table; an erase of a present key
-// clears its slot. Hit bits are ORed in (the scatter and the replays wrote
+// clears its slot. Hit bits are ORed in (the replays wrote
 // the repeated keys' bits). The other phase-B kernels touch only repeated
 // keys, so no key is probed by two kernels at once.
 template <int KB, int SB, bool HINT>
@@ -298,7 +249,7 @@ __global__ void __launch_bounds__(256) k_set_unique(
     uint32_t n_ins = 0, n_upd = 0, n_del = 0;
     for (uint64_t base = warp_base(); base < n; base += step) {
         const uint64_t i = base + lane;
-        bool mine = i < n && ((A.single[i >> 5] >> (i & 31)) & 1u);  // the scatter's bitmap
+        bool mine = i < n && ((A.single[i >> 5] >> (i & 31)) & 1u);  // the grouping's bitmap
         uint32_t tb = 0u;
         typename T::K k = 0;
         uint8_t op = kOpFind;

@@ -39,15 +39,13 @@ __device__ __forceinline__ void copy_words(uint32_t *__restrict__ dst,
 // the never-used range), their value is written, and (key, handle) is listed
 // for placement. Ops on key 0 and ops superseded by a later one in the batch
 // do nothing. The allocator state is only read here (k_wide_commit applies
-// what was handed out: cnt[0] handles). Op i's value is row idx[i] of vals
-// (row i without idx). cnt[0] / cnt[1] += new keys / updates: one atomic per
-// block and step of 256 ops, since atomics on one word pass at ~2 ns each (one
-// per warp and counter: 3e6 32-byte rows took 170 us, now 80).
+// what was handed out: cnt[0] handles). cnt[0] / cnt[1] += new keys / updates:
+// one atomic per block and step of 256 ops, since atomics on one word pass at
+// ~2 ns each (one per warp and counter: 3e6 32-byte rows took 170 us, now 80).
 template <int KB>
 __global__ void __launch_bounds__(256) k_wide_stage(const __grid_constant__ Scratch S, int use_dedup,
                                                     const void *__restrict__ keys,
                                                     const uint32_t *__restrict__ vals,
-                                                    const uint32_t *__restrict__ idx,
                                                     uint32_t words, uint64_t n,
                                                     const uint32_t *__restrict__ pre_h,
                                                     const uint32_t *__restrict__ pre_bits,
@@ -83,7 +81,7 @@ __global__ void __launch_bounds__(256) k_wide_stage(const __grid_constant__ Scra
         } else {
             h = pre_h[i];
         }
-        copy_words(heap + (uint64_t)h * words, vals + (idx ? (uint64_t)idx[i] : i) * words, words);
+        copy_words(heap + (uint64_t)h * words, vals + i * words, words);
     }
 }
 
