@@ -281,6 +281,12 @@ dyc_status read_counters(dyc_table *t, cudaStream_t s) {
     return check_counters(t);
 }
 
+// The same where the call's last kernel has written them to h_ctr (Publish).
+dyc_status published_counters(dyc_table *t, cudaStream_t s) {
+    CK(cudaStreamSynchronize(s));
+    return check_counters(t);
+}
+
 // ---- entries held outside the table after a failed call -------------------
 // An error path (an upsize the pool cannot serve, eviction overflow that
 // outlasts every round) keeps the entries it has not placed: they are copied
@@ -522,13 +528,15 @@ dyc_status bins_group(dyc_table *t, const dyc::BinScratch &B, const dyc::ApplySc
     return DYC_OK;
 }
 
-// Eviction walks of the entries the probe kernels left without a slot.
+// Eviction walks of the entries the probe kernels left without a slot; the
+// counters are in h_ctr when this returns.
 dyc_status walk_pending(dyc_table *t, cudaStream_t s) {
     const cudaError_t e = KB_CALL(t, walk, ctx(t, s), t->D, t->sb, t->S.list_a, &t->d_ctr->pending,
                                   t->S.list_b, &t->d_ctr->overflow, t->S.list_cap,
-                                  t->cfg.max_evictions, true, t->d_ctr, t->S.list_cap);
+                                  t->cfg.max_evictions, true, t->d_ctr, t->S.list_cap,
+                                  dyc::Publish{t->h_ctr, nullptr, nullptr});
     if (e != cudaSuccess) return fail(DYC_ECUDA, "walk kernel: %s", cudaGetErrorString(e));
-    return DYC_OK;
+    return published_counters(t, s);
 }
 
 // A small batch: one kernel, which leaves its counters in h_ctr and places a
@@ -545,8 +553,9 @@ dyc_status bins_small(dyc_table *t, int mode, const uint8_t *ops, const void *ke
     TRY(check_counters(t));
     *done = t->h_ctr->left == 0;
     if (!*done || t->h_ctr->pending == 0) return DYC_OK;
-    TRY(walk_pending(t, s));
-    return read_counters(t, s);
+    // the small kernel's ticket is spent
+    CK(cudaMemsetAsync(&t->d_ctr->ticket, 0, sizeof(unsigned long long), s));
+    return walk_pending(t, s);
 }
 
 // After the counters of an insert pass are in h_ctr: the call's stats, and the
@@ -591,7 +600,6 @@ dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64
                             vals, (uint32_t)t->vb, n, t->d_ctr);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "place kernel: %s", cudaGetErrorString(e));
     TRY(walk_pending(t, s));  // the ops whose buckets were full: list_a -> list_b
-    TRY(read_counters(t, s));
     return insert_finish(t, s);
 }
 
@@ -609,9 +617,10 @@ dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bit
         else
             TRY(reset_call_counters(t, s));
         cudaError_t e = KB_CALL(t, erase, ctx(t, s), t->D, t->sb, t->S, use_dedup, keys, n, bits,
-                                t->d_ctr, old, (uint32_t)t->vb);
+                                t->d_ctr, old, (uint32_t)t->vb,
+                                dyc::Publish{t->h_ctr, nullptr, nullptr});
         if (e != cudaSuccess) return fail(DYC_ECUDA, "erase kernel: %s", cudaGetErrorString(e));
-        TRY(read_counters(t, s));
+        TRY(published_counters(t, s));
     }
     t->last.erased += t->h_ctr->erased;
     t->last.superseded += t->h_ctr->superseded;
@@ -1346,11 +1355,9 @@ dyc_status apply_kernels(dyc_table *t, const uint8_t *ops, const void *keys, con
         e = KB_CALL(t, set_walk, L, t->d_desc, 1u, t->d_ctr, t->sb, t->S.list_a, nullptr,
                     &t->d_ctr->pending, t->S.list_b, nullptr, &t->d_ctr->overflow,
                     t->S.list_cap, t->cfg.max_evictions, t->d_ctr, t->S.list_cap,
-                    &A.ctr[dyc::kCtrBad]);
+                    &A.ctr[dyc::kCtrBad], dyc::Publish{t->h_ctr, A.ctr, t->h_actr});
     if (e != cudaSuccess) return fail(DYC_ECUDA, "apply kernels: %s", cudaGetErrorString(e));
-    CK(cudaMemcpyAsync(t->h_actr, A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
-                       cudaMemcpyDeviceToHost, s));
-    TRY(read_counters(t, s));
+    TRY(published_counters(t, s));
     if (t->h_actr[dyc::kCtrBad])
         return fail(DYC_ECUDA, "mixed batch: %llu device counts or ids out of range",
                     t->h_actr[dyc::kCtrBad]);
@@ -1438,11 +1445,7 @@ dyc_status apply_unique_chunk(dyc_table *t, const uint8_t *ops, const void *keys
     cudaError_t e = KB_CALL(t, apply_unique, ctx(t, s), t->D, t->sb, t->S, ops, keys, vals,
                             (uint32_t)t->vb, vals_out, bits_out, n, t->d_ctr);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "apply kernel: %s", cudaGetErrorString(e));
-    e = KB_CALL(t, walk, ctx(t, s), t->D, t->sb, t->S.list_a, &t->d_ctr->pending, t->S.list_b,
-                &t->d_ctr->overflow, t->S.list_cap, t->cfg.max_evictions, true, t->d_ctr,
-                t->S.list_cap);
-    if (e != cudaSuccess) return fail(DYC_ECUDA, "walk kernel: %s", cudaGetErrorString(e));
-    TRY(read_counters(t, s));
+    TRY(walk_pending(t, s));
     const Counters c = *t->h_ctr;
     dyc_op_stats &St = t->last;
     St.inserted += c.inserted;

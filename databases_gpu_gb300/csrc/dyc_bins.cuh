@@ -33,7 +33,9 @@
 
 namespace dyc {
 
-constexpr int kSmallR = kSmallCap / kBlockThreads;  // records per thread (k_bin_small)
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallR = kSmallCap / kSmallThreads;  // records per thread (k_bin_small)
 constexpr int kSmallTab = 2 * kSmallCap;            // cells of a bin's key table
 constexpr int kSmallBins = 96;
 static_assert(kBinSmallOps / kBinSmallMean < kSmallBins, "a small batch's bins are counted in one block");
@@ -321,6 +323,14 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
     const uint32_t tid = threadIdx.x, lane = tid & 31, nt = kGroupThreads;
     const unsigned long long *rec = B.hot + B.start[bin];
     const uint32_t table = SET ? B.tid[bin] : 0u;
+    // record r: its key, op index and word
+    auto op_at = [&](uint32_t r, K &k, uint32_t &i, uint32_t &w) -> bool {
+        if (r >= m) return false;
+        w = (uint32_t)(rec[r] >> 32);
+        i = rec_index(A, w);
+        k = load_key<KB>(keys, i);
+        return true;
+    };
     // key k's cell; claimed for op i when the key has none yet (claim)
     auto cell_of = [&](K k, uint32_t i, bool claim) -> uint32_t {
         uint32_t h = bin_cell<11>(bin_tag(k));
@@ -360,10 +370,9 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
         __syncthreads();
         for (uint32_t r0 = 0; r0 < m; r0 += nt) {
             if (__any_sync(kFull, *(volatile uint32_t *)&M.over != 0u)) break;
-            const uint32_t r = r0 + tid;
-            const uint32_t i = r < m ? rec_index(A, (uint32_t)(rec[r] >> 32)) : 0u;
-            const K k = r < m ? load_key<KB>(keys, i) : (K)0;
-            const bool sel = r < m && (part_bits((uint64_t)k) & mask) == part;
+            K k = 0;
+            uint32_t i = 0u, w = 0u;
+            const bool sel = op_at(r0 + tid, k, i, w) && (part_bits((uint64_t)k) & mask) == part;
             const uint32_t h = sel ? cell_of(k, i, true) : 0u;
             __syncwarp();
             const unsigned peers = __match_any_sync(kFull, sel ? h : 0x80000000u | lane);
@@ -421,10 +430,9 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
         }
         uint32_t ins = 0u;
         for (uint32_t r0 = 0; r0 < m; r0 += nt) {
-            const uint32_t r = r0 + tid;
-            const uint32_t w = r < m ? (uint32_t)(rec[r] >> 32) : 0u, i = rec_index(A, w);
-            const K k = r < m ? load_key<KB>(keys, i) : (K)0;
-            const bool sel = r < m && (part_bits((uint64_t)k) & mask) == part;
+            K k = 0;
+            uint32_t i = 0u, w = 0u;
+            const bool sel = op_at(r0 + tid, k, i, w) && (part_bits((uint64_t)k) & mask) == part;
             const uint32_t h = sel ? cell_of(k, i, false) : 0u;
             if constexpr (MODE == kBinModeMixed) {
                 const bool several = sel && M.cnt[h] > 1u;
@@ -656,7 +664,7 @@ constexpr uint32_t kBinShort = 8;   // ops of one key replayed by one lane
 constexpr uint32_t kTailWalk = 64;  // pending entries the last block places itself
 
 template <int KB, int SB> struct BinSmem {
-    alignas(128) unsigned char stage[kWarpsPerBlock][32 * SB];  // the key table before the probes
+    alignas(128) unsigned char stage[kSmallWarps][32 * SB];  // the key table before the probes
     typename SlotT<KB>::K key[kSmallCap];
     uint32_t word[kSmallCap];
     uint32_t cnt[kSmallCap];  // per first op of a key: ops, then winner word or count | place << 16
@@ -672,7 +680,7 @@ template <int KB, int SB> struct BinSmem {
 template <int KB, int SB>
 __device__ __forceinline__ void tail_walk(const Desc &D, const Scratch &S, Counters *ctr, uint64_t np) {
     using Sl = typename SlotT<KB>::S;
-    for (uint64_t i = threadIdx.x >> 5; i < np; i += kWarpsPerBlock) {
+    for (uint64_t i = threadIdx.x >> 5; i < np; i += kSmallWarps) {
         // written by other blocks of this kernel: read past the L1
         const unsigned long long *src = (const unsigned long long *)((const Sl *)S.list_a + i);
         Sl e;
@@ -697,7 +705,7 @@ __device__ __forceinline__ void tail_walk(const Desc &D, const Scratch &S, Count
 // the table; the last block to finish places the few entries left without a
 // slot and writes the counters to the host.
 template <int KB, int SB, int MODE>
-__global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
+__global__ void __launch_bounds__(kSmallThreads) k_bin_small(
     const __grid_constant__ Desc D, const __grid_constant__ Scratch S,
     const __grid_constant__ BinScratch B, const uint8_t *__restrict__ ops,
     const void *__restrict__ keys, const void *__restrict__ vals, uint32_t vb,
@@ -718,8 +726,8 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
     uint32_t n_ins = 0, n_upd = 0, n_del = 0, n_sup = 0, n_rej = 0;
 
     // the bin's records
-    for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kBlockThreads) tab[c] = 0u;
-    for (uint32_t c = tid; c < (uint32_t)kSmallCap; c += kBlockThreads)
+    for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kSmallThreads) tab[c] = 0u;
+    for (uint32_t c = tid; c < (uint32_t)kSmallCap; c += kSmallThreads)
         M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
     if (tid == 0) M.nseg = M.nmulti = 0u;
     if (tid < (uint32_t)kSmallBins) M.bins[tid] = 0u;
@@ -730,7 +738,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
         const uint32_t own0 = (uint32_t)(((uint64_t)bin * n) / gridDim.x);
         const uint32_t own1 = (uint32_t)(((uint64_t)(bin + 1) * n) / gridDim.x);
 #pragma unroll 8
-        for (uint64_t i = tid; i < n; i += kBlockThreads) {
+        for (uint64_t i = tid; i < n; i += kSmallThreads) {
             const K k = load_key<KB>(keys, i);
             if (k == 0) {  // belongs to no bin: one block answers it
                 if (i >= own0 && i < own1) {
@@ -749,7 +757,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
         __syncthreads();
         m = M.bins[bin];
         if (MODE >= kBinModeMixed && m <= (uint32_t)kSmallCap)
-            for (uint32_t r = tid; r < m; r += kBlockThreads)
+            for (uint32_t r = tid; r < m; r += kSmallThreads)
                 M.word[r] = op_word(M.word[r] >> 2, ops[M.word[r] >> 2]);
     }
     __syncthreads();
@@ -766,7 +774,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
     uint32_t word[kSmallR], lead[kSmallR], rank[kSmallR];
 #pragma unroll
     for (int q = 0; q < kSmallR; ++q) {
-        const uint32_t r = q * kBlockThreads + tid;
+        const uint32_t r = q * kSmallThreads + tid;
         lead[q] = rank[q] = 0u;
         word[q] = 0u;
         key[q] = 0;
@@ -799,7 +807,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
         bool any = false;
 #pragma unroll
         for (int q = 0; q < kSmallR; ++q) {
-            const uint32_t r = q * kBlockThreads + tid;
+            const uint32_t r = q * kSmallThreads + tid;
             const uint32_t c = r < m ? M.cnt[lead[q]] : 0u;
             mine[q] = c == 1u;
             any |= c > 1u;
@@ -807,7 +815,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
         if (__syncthreads_or(any)) {
 #pragma unroll
             for (int q = 0; q < kSmallR; ++q) {
-                const uint32_t r = q * kBlockThreads + tid;
+                const uint32_t r = q * kSmallThreads + tid;
                 if (r < m && !mine[q] && lead[q] == r) {
                     const uint32_t c = M.cnt[r];
                     M.cnt[r] = c | (atomicAdd(&M.nseg, c) << 16);
@@ -817,7 +825,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
             __syncthreads();
 #pragma unroll
             for (int q = 0; q < kSmallR; ++q) {
-                const uint32_t r = q * kBlockThreads + tid;
+                const uint32_t r = q * kSmallThreads + tid;
                 if (r < m && !mine[q]) M.seg[(M.cnt[lead[q]] >> 16) + rank[q]] = word[q];
             }
             __syncthreads();
@@ -825,7 +833,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
     } else {
 #pragma unroll
         for (int q = 0; q < kSmallR; ++q) {
-            const uint32_t r = q * kBlockThreads + tid;
+            const uint32_t r = q * kSmallThreads + tid;
             mine[q] = r < m && M.cnt[lead[q]] == word[q];  // op indexes are distinct
             if (r < m && !mine[q]) ++n_sup;
         }
@@ -834,7 +842,7 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
     // keys with one op (the winning op of an insert or erase batch): one probe
 #pragma unroll
     for (int q = 0; q < kSmallR; ++q) {
-        if ((uint32_t)(q * kBlockThreads) + (tid & ~31u) >= m) break;  // warp-uniform
+        if ((uint32_t)(q * kSmallThreads) + (tid & ~31u) >= m) break;  // warp-uniform
         const bool act = mine[q];
         const uint32_t i = word[q] >> 2;
         const uint32_t op = MODE == kBinModeInsert ? 1u : MODE == kBinModeErase ? 2u : (word[q] & 3u);
@@ -903,8 +911,8 @@ __global__ void __launch_bounds__(256, SB == 128 ? 4 : 1) k_bin_small(
     // few long segments spread over the warps.
     if constexpr (MODE >= kBinModeMixed) {
         const uint32_t nm = M.nmulti;
-        for (uint32_t x0 = 0; x0 < nm; x0 += kBlockThreads) {
-            const uint32_t x = x0 + lane * kWarpsPerBlock + (tid >> 5);
+        for (uint32_t x0 = 0; x0 < nm; x0 += kSmallThreads) {
+            const uint32_t x = x0 + lane * kSmallWarps + (tid >> 5);
             const bool act = x < nm;
             if (!__any_sync(kFull, act)) continue;
             const uint32_t r = act ? M.multi[x] : 0u;

@@ -127,7 +127,7 @@ cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const 
                                        : sizeof(BinSmem<KB, 128>));
     const cudaError_t e = allow_smem((const void *)k, bytes);
     if (e != cudaSuccess) return e;
-    k<<<B.nbins, 256, bytes, L.stream>>>(D, S, B, ops, keys, vals, vb, vals_out, bits_out, n, flags,
+    k<<<B.nbins, kSmallThreads, bytes, L.stream>>>(D, S, B, ops, keys, vals, vb, vals_out, bits_out, n, flags,
                                          ctr, h_ctr);
     return cudaGetLastError();
 }

@@ -60,6 +60,14 @@ struct Counters {
 };
 static_assert(sizeof(Counters) == 128, "Counters is one 128-byte block");
 
+// Where a call's last kernel writes its counters for the host (pinned memory),
+// instead of a copy behind it; null: nowhere.
+struct Publish {
+    Counters *h_ctr = nullptr;
+    const unsigned long long *actr = nullptr;  // a mixed batch's ApplyScratch::ctr
+    unsigned long long *h_actr = nullptr;
+};
+
 enum DedupMode { kKeepLast = 0, kKeepFirst = 1 };
 
 // A chunk's ops split by key into bins (dyc_bins.cuh): bin b's records are
@@ -72,8 +80,8 @@ enum DedupMode { kKeepLast = 0, kKeepFirst = 1 };
 constexpr int kBinCap = 2048;
 constexpr int kBinMean = 1024;
 constexpr int kSmallCap = 1024;
-constexpr int kBinSmallMean = 192;
-constexpr uint64_t kBinSmallOps = 16384;
+constexpr int kBinSmallMean = 384;
+constexpr uint64_t kBinSmallOps = 32768;
 enum : int {
     kBinOver = 0,  // nonzero: some bin went over
     kBinStates = 4
@@ -240,12 +248,14 @@ template <int KB> struct Ops {
     static cudaError_t walk(const LaunchCtx &L, const Desc &D, int sb, const void *src,
                             const unsigned long long *src_count, void *dst,
                             unsigned long long *dst_count, uint64_t dst_cap, uint32_t max_evict,
-                            bool count_new, Counters *ctr, uint64_t max_entries);
+                            bool count_new, Counters *ctr, uint64_t max_entries,
+                            const Publish &pub = Publish());
     // old (may be null): the value each removed key had (vb bytes each; other
     // ops' words are not written)
     static cudaError_t erase(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                              bool use_dedup, const void *keys, uint64_t n, uint32_t *bits,
-                             Counters *ctr, void *old = nullptr, uint32_t vb = 0u);
+                             Counters *ctr, void *old = nullptr, uint32_t vb = 0u,
+                             const Publish &pub = Publish());
     static cudaError_t resize_up(const LaunchCtx &L, int sb, uint32_t t, const void *old_sub,
                                  uint32_t old_nb, void *new_sub);
     // J.n jobs in one launch of J.blocks blocks (job block ranges filled in)
@@ -329,7 +339,7 @@ template <int KB> struct Ops {
                                 const unsigned long long *src_count, void *dst, uint32_t *dst_tid,
                                 unsigned long long *dst_count, uint64_t dst_cap,
                                 uint32_t max_evict, Counters *gctr, uint64_t max_entries,
-                                unsigned long long *bad);
+                                unsigned long long *bad, const Publish &pub = Publish());
     // A chunk's repeated keys (dyc_bins.cuh): the bin counts, the call counters
     // (ctr), A.ctr and the result bits zeroed, the single bits set, the ops
     // split into bins, and the ops of repeated keys found: their single bits

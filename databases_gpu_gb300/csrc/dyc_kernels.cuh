@@ -40,6 +40,29 @@ __device__ __forceinline__ uint64_t warp_stride() {
     return ((uint64_t)gridDim.x * blockDim.x) & ~31ull;
 }
 
+// Write the counters to the host from the last of `active` blocks to finish
+// (their ticket is ctr->ticket, zero before the call). Every thread of an
+// active block calls it at its end.
+__device__ __forceinline__ void publish_last(const Publish &P, Counters *ctr, uint32_t active) {
+    __shared__ uint32_t s_pub;
+    if (P.h_ctr == nullptr) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_pub = active <= 1u || atomicAdd(&ctr->ticket, 1ull) == active - 1u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_pub) return;
+    if (threadIdx.x < sizeof(Counters) / 8)
+        ((volatile unsigned long long *)P.h_ctr)[threadIdx.x] =
+            ((volatile unsigned long long *)ctr)[threadIdx.x];
+    if (P.h_actr != nullptr && threadIdx.x < (uint32_t)kCtrSlots)
+        ((volatile unsigned long long *)P.h_actr)[threadIdx.x] =
+            ((const volatile unsigned long long *)P.actr)[threadIdx.x];
+    __threadfence_system();
+}
+
 template <int KB, int SB>
 __device__ __forceinline__ typename SlotT<KB>::S *slot_ptr(char *bucket, int j) {
     return reinterpret_cast<typename SlotT<KB>::S *>(bucket + j * SlotT<KB>::kBytes);
@@ -838,7 +861,8 @@ __global__ void __launch_bounds__(256) k_walk(const __grid_constant__ Desc D,
                                               const unsigned long long *src_count, void *dst,
                                               unsigned long long *dst_count, uint64_t dst_cap,
                                               uint32_t max_evict, int count_new, Counters *ctr,
-                                              uint64_t max_entries) {
+                                              uint64_t max_entries,
+                                              const __grid_constant__ Publish pub) {
     using T = SlotT<KB>;
     using Sl = typename T::S;
     __shared__ unsigned long long s_sum[2];
@@ -945,6 +969,10 @@ __global__ void __launch_bounds__(256) k_walk(const __grid_constant__ Desc D,
         }
         if (s_sum[1]) atomicAdd(&ctr->evict_steps, s_sum[1]);
     }
+    // the blocks with entries: a warp each, or 32 entries a warp of a long list
+    const uint64_t aw = n > (uint64_t)kCoopWalk * warps ? (n + 31) / 32 : n;
+    const uint64_t ab = aw < warps ? (aw + kWarpsPerBlock - 1) / kWarpsPerBlock : gridDim.x;
+    if (blockIdx.x < (ab ? ab : 1)) publish_last(pub, ctr, (uint32_t)(ab ? ab : 1));
 }
 
 // ----------------------------------------------------------------------------
@@ -957,7 +985,8 @@ __global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
                                                const __grid_constant__ Scratch S, int use_dedup,
                                                const void *__restrict__ keys, uint64_t n,
                                                uint32_t *__restrict__ bits, void *__restrict__ old,
-                                               uint32_t vb, Counters *ctr) {
+                                               uint32_t vb, Counters *ctr,
+                                               const __grid_constant__ Publish pub) {
     using T = SlotT<KB>;
     using Gm = Geo<KB, SB>;
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
@@ -1025,6 +1054,7 @@ __global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
         }
         if (s_sum[1]) atomicAdd(&ctr->superseded, s_sum[1]);
     }
+    publish_last(pub, ctr, gridDim.x);
 }
 
 // ----------------------------------------------------------------------------

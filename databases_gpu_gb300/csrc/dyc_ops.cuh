@@ -106,13 +106,14 @@ template <int KB>
 cudaError_t Ops<KB>::walk(const LaunchCtx &L, const Desc &D, int sb, const void *src,
                           const unsigned long long *src_count, void *dst,
                           unsigned long long *dst_count, uint64_t dst_cap, uint32_t max_evict,
-                          bool count_new, Counters *ctr, uint64_t max_entries) {
+                          bool count_new, Counters *ctr, uint64_t max_entries,
+                          const Publish &pub) {
     if (max_entries == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_walk<KB, SB>;
         k<<<grid_for((const void *)k, L, max_entries), 256, 0, L.stream>>>(
             D, src, src_count, dst, dst_count, dst_cap, max_evict, count_new ? 1 : 0, ctr,
-            max_entries);
+            max_entries, pub);
     });
     return cudaGetLastError();
 }
@@ -120,12 +121,12 @@ cudaError_t Ops<KB>::walk(const LaunchCtx &L, const Desc &D, int sb, const void 
 template <int KB>
 cudaError_t Ops<KB>::erase(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
                            bool use_dedup, const void *keys, uint64_t n, uint32_t *bits,
-                           Counters *ctr, void *old, uint32_t vb) {
+                           Counters *ctr, void *old, uint32_t vb, const Publish &pub) {
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_erase<KB, SB, true> : k_erase<KB, SB, false>;
         k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, use_dedup ? 1 : 0, keys, n, bits, old, vb,
-                                                 ctr);
+                                                 ctr, pub);
     });
     return cudaGetLastError();
 }
@@ -282,13 +283,14 @@ cudaError_t Ops<KB>::set_walk(const LaunchCtx &L, const Desc *descs, uint32_t nt
                               Counters *tctr, int sb, const void *src, const uint32_t *src_tid,
                               const unsigned long long *src_count, void *dst, uint32_t *dst_tid,
                               unsigned long long *dst_count, uint64_t dst_cap, uint32_t max_evict,
-                              Counters *gctr, uint64_t max_entries, unsigned long long *bad) {
+                              Counters *gctr, uint64_t max_entries, unsigned long long *bad,
+                              const Publish &pub) {
     if (max_entries == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_set_walk<KB, SB>;
         k<<<grid_for((const void *)k, L, max_entries), 256, 0, L.stream>>>(
             descs, ntables, tctr, src, src_tid, src_count, dst, dst_tid, dst_count, dst_cap,
-            max_evict, gctr, max_entries, bad);
+            max_evict, gctr, max_entries, bad, pub);
     });
     return cudaGetLastError();
 }

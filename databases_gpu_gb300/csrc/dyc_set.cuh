@@ -359,7 +359,8 @@ __global__ void __launch_bounds__(256) k_set_walk(const Desc *__restrict__ descs
                                                   uint32_t *dst_tid, unsigned long long *dst_count,
                                                   uint64_t dst_cap, uint32_t max_evict,
                                                   Counters *gctr, uint64_t max_entries,
-                                                  unsigned long long *bad) {
+                                                  unsigned long long *bad,
+                                                  const __grid_constant__ Publish pub) {
     using T = SlotT<KB>;
     using Sl = typename T::S;
     __shared__ unsigned long long s_sum[2];
@@ -489,6 +490,9 @@ __global__ void __launch_bounds__(256) k_set_walk(const Desc *__restrict__ descs
         if (s_sum[0]) atomicAdd(&gctr->inserted, s_sum[0]);
         if (s_sum[1]) atomicAdd(&gctr->evict_steps, s_sum[1]);
     }
+    const uint64_t aw = n > (uint64_t)kCoopWalk * warps ? (n + 31) / 32 : n;
+    const uint64_t ab = aw < warps ? (aw + kWarpsPerBlock - 1) / kWarpsPerBlock : gridDim.x;
+    if (blockIdx.x < (ab ? ab : 1)) publish_last(pub, gctr, (uint32_t)(ab ? ab : 1));
 }
 
 // ----------------------------------------------------------------------------

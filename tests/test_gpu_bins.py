@@ -1,5 +1,5 @@
 """GPU parity of batches resolved by bins (dyc_bins.cuh) against the oracle's
-map: sizes at the edges of the small-batch kernel (16384 ops, bins of 192) and
+map: sizes at the edges of the small-batch kernel (32768 ops, bins of 384) and
 of the split kernels' tiles, batches of distinct keys, of few keys (bins that
 go over their capacity and take the general path) and of both together, key 0,
 and 8-byte keys with equal record tags. Whole numbers: everything is equal."""
@@ -35,7 +35,7 @@ def _keys(rng, kb, n, pattern):
 
 @pytest.mark.parametrize("kb,vb", [(4, 4), (8, 8), (8, 4)])
 @pytest.mark.parametrize("pattern", ["distinct", "few", "both"])
-@pytest.mark.parametrize("n", [1, 2, 193, 4096, 16384, 16385, 40000, 300007])
+@pytest.mark.parametrize("n", [1, 2, 385, 4096, 32768, 32769, 70001, 300007])
 def test_batches_by_bins_match_oracle(kb, vb, pattern, n):
     import databases_gpu_gb300 as dg
     rng = np.random.default_rng(n * 10 + kb)
@@ -77,7 +77,7 @@ def test_batches_by_bins_match_oracle(kb, vb, pattern, n):
 
 @pytest.mark.parametrize("kb", [4, 8])
 @pytest.mark.parametrize("pattern", ["distinct", "few", "both"])
-@pytest.mark.parametrize("n", [16384, 16385, 100003])
+@pytest.mark.parametrize("n", [1024, 32769, 100003])
 def test_wide_batches_by_bins(kb, pattern, n):
     """Rows of 12 bytes: the last row of a key wins, an erase returns it once."""
     from databases_gpu_gb300.table import DyCuckooWide
