@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(256) k_set_prep(const __grid_constant__ ApplyS
                                                   uint32_t *__restrict__ bits,
                                                   unsigned long long *__restrict__ gctr,
                                                   uint32_t gctr_words) {
+    after_previous();
     const uint64_t n = set_op_count(A, off);
     const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(256) k_apply_unique(
     const void *__restrict__ vals, uint32_t vb, void *__restrict__ vals_out,
     uint32_t *__restrict__ bits_out, uint64_t n, Counters *ctr, const uint32_t *single,
     uint32_t flags) {
+    after_previous();
     using T = SlotT<KB>;
     using Sl = typename T::S;
     using Gm = Geo<KB, SB>;
@@ -336,6 +338,7 @@ __global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_apply_count(
     const __grid_constant__ Desc D, const uint8_t *__restrict__ ops, const void *__restrict__ keys,
     const void *__restrict__ vals, uint32_t vb, uint64_t n, const uint32_t *__restrict__ single,
     Counters *ctr) {
+    after_previous();
     using T = SlotT<KB>;
     using Gm = Geo<KB, SB>;
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];

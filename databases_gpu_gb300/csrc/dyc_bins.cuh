@@ -71,6 +71,7 @@ template <int BITS> __device__ __forceinline__ uint32_t bin_cell(uint32_t tag) {
 template <int KB>
 __global__ void __launch_bounds__(256) k_small_clear(unsigned long long *zero, uint32_t nzero,
                                                      uint32_t *bits, uint64_t words) {
+    after_previous();
     const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (id < nzero) zero[id] = 0ull;
     for (uint64_t w = id; w < words; w += (uint64_t)gridDim.x * blockDim.x) bits[w] = 0u;
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_bin_scatter(
     const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
     const uint32_t *__restrict__ off, const uint8_t *__restrict__ ops,
     const void *__restrict__ keys, uint64_t n, unsigned long long *ctr, uint32_t *bits) {
+    after_previous();
     using K = typename SlotT<KB>::K;
     constexpr uint64_t kTile = (uint64_t)PER * kSplitThreads;
     static_assert(kTile <= 1 << 13 && kSplitBins <= 1 << 13, "a place and a bin take 13 bits each");
@@ -470,6 +472,7 @@ template <int KB, int MODE, bool SET>
 __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
     const void *__restrict__ keys) {
+    after_previous();
     using K = typename SlotT<KB>::K;
     struct Smem {
         uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kGroupTab];
@@ -761,6 +764,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_bin_small(
                 M.word[r] = op_word(M.word[r] >> 2, ops[M.word[r] >> 2]);
     }
     __syncthreads();
+    // so far the batch was read and key-0 results written, which the clear
+    // before this kernel does not touch; its grid waited for the ones before it
+    after_previous();
     // every block counted every bin: all agree to leave a batch with a bin
     // that does not fit to the split kernels, before anything is written
     if (__syncthreads_or(tid < gridDim.x && M.bins[tid] > (uint32_t)kSmallCap)) {

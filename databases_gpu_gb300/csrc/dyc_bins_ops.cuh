@@ -36,16 +36,13 @@ cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScrat
     const uint64_t tile = cap_n >= (1ull << 21) ? 16 * kSplitThreads : 8 * kSplitThreads;
     const unsigned blocks = (unsigned)((cap_n + tile - 1) / tile);
     if (tile == 16 * kSplitThreads)
-        k_bin_scatter<KB, 16, SET, false><<<blocks, kSplitThreads, 0, L.stream>>>(
-            B, A, off, ops, keys, cap_n, ctr, bits);
+        launch_after(k_bin_scatter<KB, 16, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits);
     else
-        k_bin_scatter<KB, 8, SET, false><<<blocks, kSplitThreads, 0, L.stream>>>(
-            B, A, off, ops, keys, cap_n, ctr, bits);
+        launch_after(k_bin_scatter<KB, 8, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits);
     // nothing to do in most batches: a fixed grid of one wave
     const unsigned some = std::min<unsigned>(blocks, 4u * (unsigned)(L.sms > 0 ? L.sms : 1));
-    k_bin_scatter<KB, 8, SET, true><<<some, kSplitThreads, 0, L.stream>>>(B, A, off, ops, keys, cap_n,
-                                                                          ctr, nullptr);
-    k_bin_group<KB, MODE, SET><<<B.nbins, kGroupThreads, 0, L.stream>>>(B, A, keys);
+    launch_after(k_bin_scatter<KB, 8, SET, true>, (unsigned)(some), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, nullptr);
+    launch_after(k_bin_group<KB, MODE, SET>, (unsigned)(B.nbins), kGroupThreads, 0, L.stream, B, A, keys);
     return cudaGetLastError();
 }
 
@@ -67,8 +64,7 @@ cudaError_t Ops<KB>::set_group(const LaunchCtx &L, const ApplyScratch &A, const 
                                const uint32_t *off, const uint8_t *ops, const void *keys,
                                uint64_t n, uint32_t *bits, Counters *gctr) {
     const uint64_t work = std::max<uint64_t>(n / 32 + 1, A.ntables);
-    k_set_prep<KB><<<(unsigned)std::min<uint64_t>((work + 255) / 256, 8ull * L.sms), 256, 0, L.stream>>>(
-        A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
+    launch_after(k_set_prep<KB>, (unsigned)((unsigned)std::min<uint64_t>((work + 255) / 256, 8ull * L.sms)), 256, 0, L.stream, A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
     if (n == 0) return cudaGetLastError();
     return bin_passes<KB, kBinModeMixed, true>(L, B, A, off, ops, keys, n, nullptr, nullptr);
 }
@@ -83,8 +79,7 @@ cudaError_t repeat_launch(const LaunchCtx &L, const ApplyScratch &A, const Desc 
     const unsigned grid = (unsigned)std::min<uint64_t>(need, 2 * wave);
     auto k = set ? k_repeat<KB, SB, true, false>
                  : list_a ? k_repeat<KB, SB, false, true> : k_repeat<KB, SB, false, false>;
-    k<<<grid, 256, 0, L.stream>>>(A, descs, ntables, ops, vals, vb, vals_out, bits_out, list_a,
-                                  list_cap, gctr);
+    launch_after(k, (unsigned)(grid), 256, 0, L.stream, A, descs, ntables, ops, vals, vb, vals_out, bits_out, list_a, list_cap, gctr);
     return cudaGetLastError();
 }
 
@@ -117,8 +112,7 @@ cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const 
                                uint64_t n, uint32_t flags, Counters *ctr, Counters *h_ctr) {
     if (n == 0) return cudaSuccess;
     const uint64_t words = bits_out ? (n + 31) / 32 : 0;
-    k_small_clear<KB><<<(unsigned)((words + 255) / 256 + 1), 256, 0, L.stream>>>(
-        &ctr->inserted, (uint32_t)(sizeof(Counters) / 8 - 1), bits_out, words);
+    launch_after(k_small_clear<KB>, (unsigned)((unsigned)((words + 255) / 256 + 1)), 256, 0, L.stream, &ctr->inserted, (uint32_t)(sizeof(Counters) / 8 - 1), bits_out, words);
     const BinFn k = sb == 32   ? small_kernel<KB, 32>(mode)
                     : sb == 64 ? small_kernel<KB, 64>(mode)
                                : small_kernel<KB, 128>(mode);
@@ -127,8 +121,7 @@ cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const 
                                        : sizeof(BinSmem<KB, 128>));
     const cudaError_t e = allow_smem((const void *)k, bytes);
     if (e != cudaSuccess) return e;
-    k<<<B.nbins, kSmallThreads, bytes, L.stream>>>(D, S, B, ops, keys, vals, vb, vals_out, bits_out, n, flags,
-                                         ctr, h_ctr);
+    launch_after(k, (unsigned)(B.nbins), kSmallThreads, bytes, L.stream, D, S, B, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr);
     return cudaGetLastError();
 }
 

@@ -10,6 +10,20 @@
 namespace dyc {
 
 // ----------------------------------------------------------------------------
+// Programmatic dependent launch: a kernel launched with launch_after() may
+// start while the kernel before it in the stream runs its last blocks, which
+// hides the launch latency between the short kernels of a batch (about 1 us
+// each). Such a kernel calls after_previous() before it touches anything the
+// previous kernel reads or writes: it waits until that grid has completed and
+// its writes are visible, and only then lets the next kernel start early. So
+// when a kernel starts, every grid before the previous one has completed.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// ----------------------------------------------------------------------------
 // Hash functions. The same integer mixers as GPU/dyhash/cuckoo.cu:27-64
 // (get_hash1..4: Thomas Wang's 32-bit mix, Bob Jenkins' 6-step mix, an
 // xor-add-mod, and the 0x27d4eb2d multiply-xorshift) and :110-120 (get_hash5,

@@ -229,6 +229,24 @@ struct LaunchCtx {
     int max_blocks_per_sm = 0;  // 0: as many as fit (else a cap, chosen by a tuner)
 };
 
+// Launch a kernel that begins with after_previous() (programmatic dependent
+// launch on the kernel before it in the stream).
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                         cudaStream_t stream, A &&...args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Kernel launchers, one set per key width; `sb` = bucket bytes (32/64/128).
 // All return cudaGetLastError() of their launches.
 template <int KB> struct Ops {

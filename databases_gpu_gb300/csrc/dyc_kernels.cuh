@@ -534,6 +534,7 @@ __global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_find(const __grid_cons
                                               const void *__restrict__ keys,
                                               void *__restrict__ vals, uint32_t vb,
                                               uint32_t *__restrict__ hits, uint64_t n) {
+    after_previous();
     using T = SlotT<KB>;
     using Gm = Geo<KB, SB>;
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
@@ -587,6 +588,7 @@ __global__ void __launch_bounds__(256) k_place(const __grid_constant__ Desc D,
                                                int new_keys, const void *__restrict__ keys,
                                                const void *__restrict__ vals, uint32_t vb,
                                                uint64_t n, Counters *ctr) {
+    after_previous();
     using T = SlotT<KB>;
     using Sl = typename T::S;
     using Gm = Geo<KB, SB>;
@@ -863,6 +865,7 @@ __global__ void __launch_bounds__(256) k_walk(const __grid_constant__ Desc D,
                                               uint32_t max_evict, int count_new, Counters *ctr,
                                               uint64_t max_entries,
                                               const __grid_constant__ Publish pub) {
+    after_previous();
     using T = SlotT<KB>;
     using Sl = typename T::S;
     __shared__ unsigned long long s_sum[2];
@@ -987,6 +990,7 @@ __global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
                                                uint32_t *__restrict__ bits, void *__restrict__ old,
                                                uint32_t vb, Counters *ctr,
                                                const __grid_constant__ Publish pub) {
+    after_previous();
     using T = SlotT<KB>;
     using Gm = Geo<KB, SB>;
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
@@ -1146,6 +1150,7 @@ template <int KB, int SB>
 __global__ void __launch_bounds__(256) k_resize_up_list(const ResizeJob *__restrict__ jobs,
                                                         const SetPolicyOut *__restrict__ out,
                                                         uint32_t max_jobs) {
+    after_previous();
     const uint32_t nj = out->njobs < max_jobs ? out->njobs : max_jobs;
     if (nj == 0) return;
     const uint32_t ntask = out->ntasks;

@@ -75,7 +75,7 @@ cudaError_t Ops<KB>::find(const LaunchCtx &L, const Desc &D, int sb, const void 
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_find<KB, SB, true> : k_find<KB, SB, false>;
-        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, keys, vals, vb, hits, n);
+        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, keys, vals, vb, hits, n);
     });
     return cudaGetLastError();
 }
@@ -96,8 +96,7 @@ cudaError_t Ops<KB>::place(const LaunchCtx &L, const Desc &D, int sb, const Scra
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_place<KB, SB, true> : k_place<KB, SB, false>;
-        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, use_dedup ? 1 : 0, new_keys ? 1 : 0, keys,
-                                                  vals, vb, n, ctr);
+        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, S, use_dedup ? 1 : 0, new_keys ? 1 : 0, keys, vals, vb, n, ctr);
     });
     return cudaGetLastError();
 }
@@ -111,9 +110,7 @@ cudaError_t Ops<KB>::walk(const LaunchCtx &L, const Desc &D, int sb, const void 
     if (max_entries == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_walk<KB, SB>;
-        k<<<grid_for((const void *)k, L, max_entries), 256, 0, L.stream>>>(
-            D, src, src_count, dst, dst_count, dst_cap, max_evict, count_new ? 1 : 0, ctr,
-            max_entries, pub);
+        launch_after(k, (unsigned)(grid_for((const void *)k, L, max_entries)), 256, 0, L.stream, D, src, src_count, dst, dst_count, dst_cap, max_evict, count_new ? 1 : 0, ctr, max_entries, pub);
     });
     return cudaGetLastError();
 }
@@ -125,8 +122,7 @@ cudaError_t Ops<KB>::erase(const LaunchCtx &L, const Desc &D, int sb, const Scra
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_erase<KB, SB, true> : k_erase<KB, SB, false>;
-        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, use_dedup ? 1 : 0, keys, n, bits, old, vb,
-                                                 ctr, pub);
+        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, S, use_dedup ? 1 : 0, keys, n, bits, old, vb, ctr, pub);
     });
     return cudaGetLastError();
 }
@@ -139,8 +135,7 @@ cudaError_t Ops<KB>::apply_unique(const LaunchCtx &L, const Desc &D, int sb, con
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_apply_unique<KB, SB, true> : k_apply_unique<KB, SB, false>;
-        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, S, ops, keys, vals, vb, vals_out, bits_out, n,
-                                                  ctr, single, flags);
+        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, S, ops, keys, vals, vb, vals_out, bits_out, n, ctr, single, flags);
     });
     return cudaGetLastError();
 }
@@ -152,7 +147,7 @@ cudaError_t Ops<KB>::apply_count(const LaunchCtx &L, const Desc &D, int sb, cons
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_apply_count<KB, SB>;
-        k<<<tile_grid(L, n), 256, 0, L.stream>>>(D, ops, keys, vals, vb, n, single, ctr);
+        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, ops, keys, vals, vb, n, single, ctr);
     });
     return cudaGetLastError();
 }
@@ -197,7 +192,8 @@ cudaError_t Ops<KB>::resize_up_list(const LaunchCtx &L, int sb, const ResizeJob 
     DYC_SB_DISPATCH(sb, {
         auto k = k_resize_up_list<KB, SB>;
         // one full wave; blocks loop over the listed tasks
-        k<<<grid_for((const void *)k, L, ~0ull >> 1), 256, 0, L.stream>>>(jobs, out, max_jobs);
+        launch_after(k, (unsigned)grid_for((const void *)k, L, ~0ull >> 1), 256, 0, L.stream, jobs, out,
+                     max_jobs);
     });
     return cudaGetLastError();
 }
@@ -207,7 +203,7 @@ cudaError_t Ops<KB>::set_policy(const LaunchCtx &L, Desc *descs, uint32_t ntable
                                 const Counters *tctr, const uint32_t *tup, const uint32_t *ter,
                                 const Spare *spares, double upper, uint32_t slots, int sb,
                                 ResizeJob *jobs, uint8_t *grew, SetPolicyOut *out) {
-    k_set_policy<KB><<<1, 1024, 0, L.stream>>>(descs, ntables, tctr, tup, ter, spares, upper, slots,
+    launch_after(k_set_policy<KB>, 1u, 1024u, 0, L.stream, descs, ntables, tctr, tup, ter, spares, upper, slots,
                                                (uint32_t)sb / 32u, jobs, grew, out);
     return cudaGetLastError();
 }
@@ -254,7 +250,7 @@ cudaError_t Ops<KB>::set_mutate(const LaunchCtx &L, const Desc *descs, uint32_t 
     if (max_n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = hint ? k_set_mutate<KB, SB, true> : k_set_mutate<KB, SB, false>;
-        k<<<tile_grid(L, max_n + 32), 256, 0, L.stream>>>(
+        launch_after(k, (unsigned)tile_grid(L, max_n + 32), 256, 0, L.stream,
             descs, ntables, tctr, er_keys, er_tids, ne_ptr, up_keys, up_vals, vb, up_tids, nu_ptr,
             max_n, list_a, list_a_tid, list_cap, gctr, bad, hold);
     });
@@ -271,7 +267,7 @@ cudaError_t Ops<KB>::set_unique(const LaunchCtx &L, const ApplyScratch &A, const
     if (max_n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = hint ? k_set_unique<KB, SB, true> : k_set_unique<KB, SB, false>;
-        k<<<tile_grid(L, max_n), 256, 0, L.stream>>>(A, off, descs, ntables, tctr, ops, keys,
+        launch_after(k, (unsigned)tile_grid(L, max_n), 256, 0, L.stream, A, off, descs, ntables, tctr, ops, keys,
                                                       vals, vb, vals_out, bits_out, list_a,
                                                       list_a_tid, list_cap, gctr, hold);
     });
@@ -288,7 +284,7 @@ cudaError_t Ops<KB>::set_walk(const LaunchCtx &L, const Desc *descs, uint32_t nt
     if (max_entries == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_set_walk<KB, SB>;
-        k<<<grid_for((const void *)k, L, max_entries), 256, 0, L.stream>>>(
+        launch_after(k, (unsigned)grid_for((const void *)k, L, max_entries), 256, 0, L.stream,
             descs, ntables, tctr, src, src_tid, src_count, dst, dst_tid, dst_count, dst_cap,
             max_evict, gctr, max_entries, bad, pub);
     });

@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(256, 3) k_repeat(
     const uint8_t *__restrict__ ops, const void *__restrict__ vals, uint32_t vb,
     void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, void *list_a, uint64_t list_cap,
     Counters *gctr) {
+    after_previous();
     constexpr int kStage = 32 * SB * kWarpsPerBlock;
     constexpr int kSort = (int)(kMidSeg * sizeof(uint32_t));
     __shared__ __align__(128) unsigned char s_raw[kStage > kSort ? kStage : kSort];

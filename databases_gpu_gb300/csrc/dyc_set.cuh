@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(256) k_set_mutate(
     const unsigned long long *__restrict__ nu_ptr, uint64_t max_n, void *list_a,
     uint32_t *list_a_tid, uint64_t list_cap, Counters *gctr, unsigned long long *bad,
     const uint32_t *hold) {
+    after_previous();
     if (hold != nullptr && *hold != 0u) return;  // the host applies the rest of the policy first
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
     unsigned char *stage = s_stage[threadIdx.x >> 5];
@@ -237,6 +238,7 @@ __global__ void __launch_bounds__(256) k_set_unique(
     const uint8_t *__restrict__ ops, const void *__restrict__ keys, const void *__restrict__ vals,
     uint32_t vb, void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, void *list_a,
     uint32_t *list_a_tid, uint64_t list_cap, Counters *gctr, const uint32_t *hold) {
+    after_previous();
     using T = SlotT<KB>;
     using Sl = typename T::S;
     using Gm = Geo<KB, SB>;
@@ -361,6 +363,7 @@ __global__ void __launch_bounds__(256) k_set_walk(const Desc *__restrict__ descs
                                                   Counters *gctr, uint64_t max_entries,
                                                   unsigned long long *bad,
                                                   const __grid_constant__ Publish pub) {
+    after_previous();
     using T = SlotT<KB>;
     using Sl = typename T::S;
     __shared__ unsigned long long s_sum[2];
@@ -521,6 +524,7 @@ __global__ void __launch_bounds__(1024) k_set_policy(Desc *__restrict__ descs, u
                                                      ResizeJob *__restrict__ jobs,
                                                      uint8_t *__restrict__ grew,
                                                      SetPolicyOut *__restrict__ out) {
+    after_previous();
     __shared__ uint32_t s_wj[32], s_wt[32];  // per-warp inclusive sums of the tile
     __shared__ uint32_t s_cj, s_ct, s_host;   // jobs / tasks before the tile; host needed
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5, nw = blockDim.x >> 5;
