@@ -1321,7 +1321,7 @@ dyc_status push_desc(dyc_table *t, cudaStream_t s) {
 template <class F>
 dyc_status apply_kernels(dyc_table *t, const uint8_t *ops, const void *keys, const void *vals,
                          uint64_t n, void *vals_out, uint32_t *bits_out, bool before,
-                         cudaStream_t s, F &&policy) {
+                         bool skip_equal, cudaStream_t s, F &&policy) {
     const dyc::ApplyScratch &A = t->A;
     const LaunchCtx L = ctx(t, s);
     const uint32_t vb = (uint32_t)t->vb;
@@ -1341,11 +1341,10 @@ dyc_status apply_kernels(dyc_table *t, const uint8_t *ops, const void *keys, con
         TRY(push_desc(t, s));
         TRY(reset_call_counters(t, s));
     }
-    // the lists name no upsert of an equal value; neither may the one-pass
-    // kernel where its counts were taken before the batch
+    // skip_equal: an insert of the value its key has is no update, as in the lists
     if (e == cudaSuccess)
         e = KB_CALL(t, apply_unique, L, t->D, t->sb, t->S, ops, keys, vals, vb, vals_out, bits_out,
-                    n, t->d_ctr, A.single, before ? (uint32_t)dyc::kBinSkipEqual : 0u);
+                    n, t->d_ctr, A.single, skip_equal ? (uint32_t)dyc::kBinSkipEqual : 0u);
     if (e == cudaSuccess && before)
         e = KB_CALL(t, set_mutate, L, t->d_desc, 1u, t->d_ctr, t->sb, A.er_key, nullptr,
                     &A.ctr[dyc::kCtrEr], A.up_key, A.up_val, vb, nullptr, &A.ctr[dyc::kCtrUp], n,
@@ -1369,14 +1368,17 @@ dyc_status apply_kernels(dyc_table *t, const uint8_t *ops, const void *keys, con
 // batch's upsert and erase counts: where even n inserts keep the table within
 // deferred_fill() of its slots it is applied after the batch with the same
 // counts, so the capacity ends as if it had run first (entries the fuller
-// table could not place take the overflow path); otherwise the counts are
-// taken first, the host reads them and upsizes, and the batch is applied
-// after that.
+// table could not place take the overflow path). Otherwise the batch's inserts
+// are counted first (5 us for 2^22 ops and a host read): where the size plus
+// all of them stays within the bound no upsize can be due. Else the exact
+// counts are taken in a pass over the table (147 us), the host reads them and
+// upsizes, and the batch is applied after that.
 dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const void *vals,
                        uint64_t n, void *vals_out, uint32_t *bits_out, uint32_t flags,
                        cudaStream_t s) {
     const bool resize = t->cfg.auto_resize && !(flags & DYC_FLAG_NO_RESIZE);
-    const bool before = resize && (double)(t->size + n) > deferred_fill(t) * (double)t->capacity;
+    const bool full = resize && (double)(t->size + n) > deferred_fill(t) * (double)t->capacity;
+    bool before = full;
     const uint64_t size0 = t->size;
     bool grew = false;
     // nu upserts and ne erases of present keys
@@ -1397,14 +1399,22 @@ dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const
     }
     if (done)
         TRY(bins_small(t, dyc::kBinModeMixed, ops, keys, vals, vals_out, bits_out, n,
-                       before ? (uint32_t)dyc::kBinSkipEqual : 0u, s, &done));
-    if (!done)
-        TRY(apply_kernels(t, ops, keys, vals, n, vals_out, bits_out, before, s, policy));
+                       full ? (uint32_t)dyc::kBinSkipEqual : 0u, s, &done));
+    if (!done) {
+        if (before && n > dyc::kBinSmallOps) {
+            TRY(reset_call_counters(t, s));
+            const cudaError_t e = KB_CALL(t, count_inserts, ctx(t, s), ops, n, &t->d_ctr->nins);
+            if (e != cudaSuccess) return fail(DYC_ECUDA, "count kernel: %s", cudaGetErrorString(e));
+            TRY(read_counters(t, s));
+            before = (double)(size0 + t->h_ctr->nins) > t->cfg.upper_load * (double)t->capacity;
+        }
+        TRY(apply_kernels(t, ops, keys, vals, n, vals_out, bits_out, before, full, s, policy));
+    }
     const Counters c = *t->h_ctr;
     // both kinds of keys' upserts and erases of present keys, as the table
     // counted them (an insert of the only op of its key counts as an update
     // even when the value is the same)
-    if (!before) TRY(policy(c.inserted + c.updated, c.erased));
+    if (!full) TRY(policy(c.inserted + c.updated, c.erased));
     dyc_op_stats &St = t->last;
     St.inserted += c.inserted;
     St.updated += c.updated;
@@ -1613,6 +1623,7 @@ struct dyc_set {
     Desc *d_desc = nullptr, *h_desc = nullptr;      // per-table descriptors (pinned mirror)
     Counters *d_gctr = nullptr, *h_gctr = nullptr;  // set-wide counters of one call
     unsigned long long *h_actr = nullptr;   // pinned copy of the batch counters (A.ctr)
+    unsigned long long *h_size = nullptr;   // pinned: the members' sizes after a call
     unsigned long long *h_hostn = nullptr;  // pinned: the op count of the current batch
     void *abuf = nullptr;
     size_t abytes = 0;
@@ -1643,11 +1654,10 @@ struct dyc_set {
     uint32_t max_evict_all = 0;  // largest member eviction bound
     dyc_op_stats last{};
     // device half of the upsize policy (cfg.device_upsize == 0, auto_resize):
-    // one upsize target per member, allocated ahead (h_spare, its device copy
-    // d_spare refreshed at every round), the moves k_set_policy lists, which
-    // members it upsized, and the buffers they replaced (freed at the next call)
+    // one upsize target per member, allocated ahead (h_spare), the moves
+    // k_set_policy lists, which members it upsized, and the buffers they replaced (freed at the next call)
     bool spares = false;
-    dyc::Spare *d_spare = nullptr, *h_spare = nullptr;
+    dyc::Spare *h_spare = nullptr;  // pinned, read by the policy kernel
     dyc::ResizeJob *d_jobs = nullptr;
     dyc::SetPolicyOut *d_pout = nullptr, *h_pout = nullptr;
     uint8_t *d_grew = nullptr, *h_grew = nullptr;
@@ -1782,8 +1792,7 @@ dyc_status set_phase_a(dyc_set *s, const uint32_t *d_off, const uint8_t *ops, co
     if (e == cudaSuccess)
         e = SET_KB_CALL(s, repeat, L, A, s->d_desc, s->ntables, s->sb, true, ops, vals, vb, out, bits, n);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "set phase A kernels: %s", cudaGetErrorString(e));
-    if (new_counts)  // each table's upserts, for the upsize decision
-    {
+    if (new_counts) {  // each table's upserts and erases, for the host's upsize decision
         CK(cudaMemcpyAsync(s->h_tup, A.tup, (size_t)s->ntables * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(s->h_ter, A.ter, (size_t)s->ntables * 4, cudaMemcpyDeviceToHost, st));
     }
@@ -1813,11 +1822,19 @@ dyc_status set_phase_b(dyc_set *s, uint64_t n, cudaStream_t st, const uint32_t *
                         &s->d_gctr->overflow, s->list_cap, s->max_evict_all, s->d_gctr,
                         s->list_cap, &A.ctr[dyc::kCtrBad]);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "set phase B kernels: %s", cudaGetErrorString(e));
-    CK(cudaMemcpyAsync(s->h_actr, A.ctr, dyc::kCtrSlots * sizeof(unsigned long long),
-                       cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(s->h_gctr, s->d_gctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(s->h_tctr, s->d_tctr, sizeof(Counters) * s->ntables,
-                       cudaMemcpyDeviceToHost, st));
+    dyc::SetReport R{s->d_gctr, s->h_gctr, A.ctr, s->h_actr, s->d_tctr, s->h_size, s->ntables};
+    if (hold) {  // behind the device policy
+        R.pout = s->d_pout;
+        R.h_pout = s->h_pout;
+        R.grew = s->d_grew;
+        R.h_grew = s->h_grew;
+        R.tup = A.tup;
+        R.ter = A.ter;
+        R.h_tup = s->h_tup;
+        R.h_ter = s->h_ter;
+    }
+    e = SET_KB_CALL(s, set_report, L, R);
+    if (e != cudaSuccess) return fail(DYC_ECUDA, "set report kernel: %s", cudaGetErrorString(e));
     return DYC_OK;
 }
 
@@ -1876,30 +1893,26 @@ void set_fill_spares(dyc_set *s, cudaStream_t st) {
     }
 }
 
-// Spare targets to the device, the policy, the listed upsizes, phase B
-// (held back when the host must finish the policy), and what the policy
-// did back to the host. One capturable sequence.
+// The policy, the listed upsizes, phase B (held back when the host must finish
+// the policy), and what the policy did back to the host. One capturable
+// sequence; the policy reads the spare targets from pinned memory.
 dyc_status set_policy_and_b(dyc_set *s, uint64_t n, cudaStream_t st) {
     const LaunchCtx L{s->sms, st, (int)s->blocks_per_sm};
-    CK(cudaMemcpyAsync(s->d_spare, s->h_spare, sizeof(dyc::Spare) * s->ntables,
-                       cudaMemcpyHostToDevice, st));
     cudaError_t e = SET_KB_CALL(s, set_policy, L, s->d_desc, s->ntables, s->d_tctr, s->A.tup,
-                                s->A.ter, s->d_spare, s->cfg.upper_load,
+                                s->A.ter, s->h_spare, s->cfg.upper_load,
                                 (uint32_t)s->tables[0]->slots, s->sb, s->d_jobs, s->d_grew,
                                 s->d_pout);
     if (e == cudaSuccess)
         e = SET_KB_CALL(s, resize_up_list, L, s->sb, s->d_jobs, s->d_pout, s->ntables);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "set upsize policy: %s", cudaGetErrorString(e));
-    TRY(set_phase_b(s, n, st, &s->d_pout->host));
-    CK(cudaMemcpyAsync(s->h_pout, s->d_pout, sizeof(dyc::SetPolicyOut), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(s->h_grew, s->d_grew, s->ntables, cudaMemcpyDeviceToHost, st));
-    return DYC_OK;
+    return set_phase_b(s, n, st, &s->d_pout->host);
 }
 
 // The members the device upsized: their host descriptors follow the device
 // ones (the spare became subtable ti), the old subtable is freed at the next
 // call, and grew[t] is set as for a host upsize of the policy.
 void set_take_device_upsizes(dyc_set *s, std::vector<uint8_t> &grew) {
+    if (s->h_pout->njobs == 0) return;
     for (uint32_t t = 0; t < s->ntables; ++t) {
         if (!s->h_grew[t]) continue;
         dyc_table *m = s->tables[t];
@@ -2072,12 +2085,12 @@ dyc_status dyc_set_create(const dyc_config *cfg, uint32_t ntables, const uint64_
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_gctr, sizeof(Counters));
     if (e == cudaSuccess)
         e = dyc::lib_malloc_host(&s->h_actr, sizeof(unsigned long long) * dyc::kCtrSlots);
+    if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_size, sizeof(unsigned long long) * ntables);
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_hostn, sizeof(unsigned long long));
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_tup, sizeof(uint32_t) * ntables);
     if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_ter, sizeof(uint32_t) * ntables);
     s->spares = cfg->auto_resize && cfg->device_upsize == 0u;
     if (s->spares) {
-        if (e == cudaSuccess) e = dyc::lib_malloc(&s->d_spare, sizeof(dyc::Spare) * ntables);
         if (e == cudaSuccess) e = dyc::lib_malloc_host(&s->h_spare, sizeof(dyc::Spare) * ntables);
         if (e == cudaSuccess) e = dyc::lib_malloc(&s->d_jobs, sizeof(dyc::ResizeJob) * ntables);
         if (e == cudaSuccess) e = dyc::lib_malloc(&s->d_pout, sizeof(dyc::SetPolicyOut));
@@ -2128,7 +2141,6 @@ dyc_status dyc_set_destroy(dyc_set *s) {
             if (s->h_spare[t].new_sub) cudaFree(s->h_spare[t].new_sub);
     for (const auto &b : s->free_later) cudaFree(b.first);
     for (const auto &b : s->spare_cache) cudaFree(b.second);
-    if (s->d_spare) cudaFree(s->d_spare);
     if (s->h_spare) cudaFreeHost(s->h_spare);
     if (s->d_jobs) cudaFree(s->d_jobs);
     if (s->d_pout) cudaFree(s->d_pout);
@@ -2321,7 +2333,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
         // when a member needs more than its device upsize.
         TRY(set_run(s, gr, 0, st, [&](cudaStream_t cs) {
             return set_phase_a(s, d_offsets, d_ops, d_keys, d_vals, d_vals_out, d_bits_out, ng,
-                               true, cs);
+                               false, cs);
         }));
         TRY(set_release_later(s, st));
         set_fill_spares(s, st);
@@ -2366,7 +2378,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
                     s->h_actr[dyc::kCtrBad]);
     const Counters g = *s->h_gctr;
     if (g.spill) return fail(DYC_EOVERFLOW, "internal list overflow (%llu entries)", g.spill);
-    for (uint32_t t = 0; t < s->ntables; ++t) s->tables[t]->size = s->h_tctr[t].size;
+    for (uint32_t t = 0; t < s->ntables; ++t) s->tables[t]->size = s->h_size[t];
     s->last.inserted = g.inserted;
     s->last.updated = g.updated;
     s->last.erased = g.erased;

@@ -229,6 +229,25 @@ struct LaunchCtx {
     int max_blocks_per_sm = 0;  // 0: as many as fit (else a cap, chosen by a tuner)
 };
 
+// What a set call's last kernel writes to the host (pinned memory): one launch
+// instead of a copy for each. pout and what follows may be null (no device
+// policy in the sequence).
+struct SetReport {
+    const Counters *gctr;
+    Counters *h_gctr;
+    const unsigned long long *actr;
+    unsigned long long *h_actr;
+    const Counters *tctr;           // per table: its size goes to h_size
+    unsigned long long *h_size;
+    uint32_t ntables;
+    const SetPolicyOut *pout;
+    SetPolicyOut *h_pout;
+    const uint8_t *grew;            // written when the policy listed upsizes
+    uint8_t *h_grew;
+    const uint32_t *tup, *ter;      // written when the host must finish the policy
+    uint32_t *h_tup, *h_ter;
+};
+
 // Launch a kernel that begins with after_previous() (programmatic dependent
 // launch on the kernel before it in the stream).
 template <class... P, class... A>
@@ -378,6 +397,7 @@ template <int KB> struct Ops {
     static cudaError_t apply_count(const LaunchCtx &L, const Desc &D, int sb, const uint8_t *ops,
                                    const void *keys, const void *vals, uint32_t vb, uint64_t n,
                                    const uint32_t *single, Counters *ctr);
+    static cudaError_t set_report(const LaunchCtx &L, const SetReport &R);
     // set every fingerprint bit of every bucket of a subtable
     static cudaError_t mark_all(const LaunchCtx &L, int sb, void *sub, uint32_t nb);
     static cudaError_t export_all(const LaunchCtx &L, const Desc &D, int sb, void *keys,

@@ -157,7 +157,7 @@ cudaError_t Ops<KB>::count_inserts(const LaunchCtx &L, const uint8_t *ops, uint6
                                    unsigned long long *count) {
     if (n == 0) return cudaSuccess;
     auto k = k_count_inserts<KB>;
-    k<<<grid_for((const void *)k, L, n), 256, 0, L.stream>>>(ops, n, count);
+    k<<<grid_for((const void *)k, L, n / 16 + 1), 256, 0, L.stream>>>(ops, n, count);
     return cudaGetLastError();
 }
 
@@ -288,6 +288,13 @@ cudaError_t Ops<KB>::set_walk(const LaunchCtx &L, const Desc *descs, uint32_t nt
             descs, ntables, tctr, src, src_tid, src_count, dst, dst_tid, dst_count, dst_cap,
             max_evict, gctr, max_entries, bad, pub);
     });
+    return cudaGetLastError();
+}
+
+template <int KB>
+cudaError_t Ops<KB>::set_report(const LaunchCtx &L, const SetReport &R) {
+    const uint32_t need = (R.ntables + 255u) / 256u;
+    launch_after(k_set_report<KB>, need < 16u ? (need ? need : 1u) : 16u, 256u, 0, L.stream, R);
     return cudaGetLastError();
 }
 

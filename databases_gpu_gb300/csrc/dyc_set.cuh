@@ -510,7 +510,8 @@ __global__ void __launch_bounds__(256) k_set_walk(const Desc *__restrict__ descs
 // member still over the bound after that upsize, or without a fitting
 // spare, sets out->host: phase B's mutate kernel then does nothing and the
 // host applies the rest of the policy before running phase B itself. The
-// capacity and the comparison are the host's, in doubles. One block walks
+// capacity and the comparison are the host's, in doubles. (spares is the host's
+// pinned array: only members over the bound read theirs.) One block walks
 // the members in tiles of blockDim.x (a scan gives each listed move its
 // place and its first task).
 // ----------------------------------------------------------------------------
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(1024) k_set_policy(Desc *__restrict__ descs, u
                                                      const Counters *__restrict__ tctr,
                                                      const uint32_t *__restrict__ tup,
                                                      const uint32_t *__restrict__ ter,
-                                                     const Spare *__restrict__ spares, double upper,
+                                                     const Spare *spares, double upper,
                                                      uint32_t slots, uint32_t chunks_per_bucket,
                                                      ResizeJob *__restrict__ jobs,
                                                      uint8_t *__restrict__ grew,
@@ -617,6 +618,26 @@ __global__ void __launch_bounds__(1024) k_set_policy(Desc *__restrict__ descs, u
         out->host = s_host;
         out->pad = 0u;
     }
+}
+
+template <int KB>
+__global__ void __launch_bounds__(256) k_set_report(const __grid_constant__ SetReport R) {
+    after_previous();
+    const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (id < sizeof(Counters) / 8)
+        ((unsigned long long *)R.h_gctr)[id] = ((const unsigned long long *)R.gctr)[id];
+    if (id < (uint32_t)kCtrSlots) R.h_actr[id] = R.actr[id];
+    for (uint32_t t = id; t < R.ntables; t += stride) R.h_size[t] = R.tctr[t].size;
+    if (R.pout == nullptr) return;
+    const SetPolicyOut o = *R.pout;
+    if (id == 0) *R.h_pout = o;
+    if (o.njobs)
+        for (uint32_t t = id; t < R.ntables; t += stride) R.h_grew[t] = R.grew[t];
+    if (o.host)
+        for (uint32_t t = id; t < R.ntables; t += stride) {
+            R.h_tup[t] = R.tup[t];
+            R.h_ter[t] = R.ter[t];
+        }
 }
 
 }  // namespace dyc
