@@ -267,9 +267,13 @@ cudaError_t Ops<KB>::set_unique(const LaunchCtx &L, const ApplyScratch &A, const
     if (max_n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = hint ? k_set_unique<KB, SB, true> : k_set_unique<KB, SB, false>;
+        // as many bitmap words a warp as leave every warp of a wave some
+        const uint64_t warps = 64ull * (uint64_t)(L.sms > 0 ? L.sms : 1);
+        const uint64_t w = max_n / 32 / warps;
+        const uint32_t words = (uint32_t)(w < 1 ? 1 : w > kUniqueWords ? kUniqueWords : w);
         launch_after(k, (unsigned)tile_grid(L, max_n), 256, 0, L.stream, A, off, descs, ntables, tctr, ops, keys,
                                                       vals, vb, vals_out, bits_out, list_a,
-                                                      list_a_tid, list_cap, gctr, hold);
+                                                      list_a_tid, list_cap, gctr, hold, words);
     });
     return cudaGetLastError();
 }

@@ -231,13 +231,21 @@ __global__ void __launch_bounds__(256) k_set_mutate(
 // clears its slot. Hit bits are ORed in (the replays wrote
 // the repeated keys' bits). The other phase-B kernels touch only repeated
 // keys, so no key is probed by two kernels at once.
+// Bound by the latency of the probes in flight. A warp lists the set bits of
+// up to kUniqueWords bitmap words and probes them 32 at a time: in a round of
+// 2^22 ops over 4096 tables about half the ops repeat a key, and a warp that
+// took one word at a time probed with half its lanes idle (450 us a round,
+// 322 with the list). A small batch takes fewer words to a warp so that the
+// blocks still cover the chip.
+constexpr uint32_t kUniqueWords = 8;  // bitmap words a warp takes at most
+
 template <int KB, int SB, bool HINT>
 __global__ void __launch_bounds__(256) k_set_unique(
     const __grid_constant__ ApplyScratch A, const uint32_t *__restrict__ off,
     const Desc *__restrict__ descs, uint32_t ntables, Counters *__restrict__ tctr,
     const uint8_t *__restrict__ ops, const void *__restrict__ keys, const void *__restrict__ vals,
     uint32_t vb, void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, void *list_a,
-    uint32_t *list_a_tid, uint64_t list_cap, Counters *gctr, const uint32_t *hold) {
+    uint32_t *list_a_tid, uint64_t list_cap, Counters *gctr, const uint32_t *hold, uint32_t words) {
     after_previous();
     using T = SlotT<KB>;
     using Sl = typename T::S;
@@ -245,89 +253,115 @@ __global__ void __launch_bounds__(256) k_set_unique(
     if (hold != nullptr && *hold != 0u) return;  // the host applies the rest of the policy first
     __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
     unsigned char *stage = s_stage[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t n = set_op_count(A, off);
-    const uint64_t step = warp_stride();
     uint32_t n_ins = 0, n_upd = 0, n_del = 0;
-    for (uint64_t base = warp_base(); base < n; base += step) {
-        const uint64_t i = base + lane;
-        bool mine = i < n && ((A.single[i >> 5] >> (i & 31)) & 1u);  // the grouping's bitmap
-        uint32_t tb = 0u;
-        typename T::K k = 0;
-        uint8_t op = kOpFind;
-        Sl e = T::empty();
-        if (mine) {
-            tb = table_at(A.tidx, off, (uint32_t)i, (uint32_t)i);
-            if (tb >= ntables) {
-                note_bad(A);
-                mine = false;
-                tb = 0u;
-            } else {
-                k = load_key<KB>(keys, i);
-                op = ops[i];
-            }
+    // a warp takes `words` bitmap words and probes their ops 32 at a time: the
+    // set bits' places are listed first, so ops of repeated keys cost no lanes
+    __shared__ uint8_t s_op[kWarpsPerBlock][kUniqueWords * 32];
+    __shared__ uint32_t s_bits[kWarpsPerBlock][kUniqueWords];
+    const uint64_t range = 32ull * words;
+    const uint64_t stride = (uint64_t)gridDim.x * kWarpsPerBlock * range;
+    for (uint64_t first = ((uint64_t)blockIdx.x * kWarpsPerBlock + warp) * range; first < n;
+         first += stride) {
+        uint32_t w = 0u;
+        if (lane < words && first + 32ull * lane < n) {
+            const uint64_t left = n - (first + 32ull * lane);
+            w = A.single[(first >> 5) + lane] & (left < 32 ? (1u << left) - 1u : kFull);
         }
-        const Desc &D = descs[tb];
-        const unsigned long long tpol = HINT ? l2_policies(D.l2_keep != 0u).table : 0ull;
-        const bool act = mine && k != 0;  // ops on key 0 miss and change nothing
-        const bool ins = act && op == kOpInsert, del = act && op == kOpErase;
-        if (ins) e = T::make(k, load_val(vals, vb, i));
-        const uint32_t hk = fold(k);
-        const Pair p = pair_of(hk, D.d);
-        char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
-        char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
-        const KvOut r1 = place_probe<KB, SB, HINT>(p1, k, act, p.first, D.d, stage, tpol);
-        const bool found1 = act && r1.match >= 0;
-        const bool check2 =
-            act && !found1 && ((!Gm::kMeta || r1.overflow) || (ins && r1.empty == 0u));
-        KvOut r2{-1, 0ull, false, 0u};
-        if (__any_sync(kFull, check2))
-            r2 = place_probe<KB, SB, HINT>(p2, k, check2, p.second, D.d, stage, tpol);
-        const bool found2 = check2 && r2.match >= 0;
-        const bool present = found1 || found2;
-        const uint64_t before = found1 ? r1.value : (found2 ? r2.value : 0ull);
-        bool pend = false, placed = false, gone = false;
-        if (ins) {
-            if (found1) {
-                T::store(slot_ptr<KB, SB>(p1, r1.match), e);
-                ++n_upd;
-            } else if (found2) {
-                T::store(slot_ptr<KB, SB>(p2, r2.match), e);
-                ++n_upd;
-            } else {
-                bool ok = claim_empty<KB, SB>(p1, r1.empty, e);
-                if (!ok && check2 && r2.empty) {
-                    mark_overflow<KB, SB>(p1, hk);
-                    ok = claim_empty<KB, SB>(p2, r2.empty, e);
-                }
-                if (ok) {
-                    ++n_ins;
-                    placed = true;
-                } else {
-                    pend = true;
-                }
-            }
-        } else if (del && present) {
-            T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match),
-                     T::empty());
-            ++n_del;
-            gone = true;
+        if (lane < words) s_bits[warp][lane] = 0u;
+        uint32_t total = 0u;
+        for (uint32_t x = 0; x < words; ++x) {
+            const uint32_t v = __shfl_sync(kFull, w, x);
+            if ((v >> lane) & 1u)
+                s_op[warp][total + __popc(v & ((1u << lane) - 1u))] = (uint8_t)(x * 32u + lane);
+            total += __popc(v);
         }
-        if (vals_out != nullptr && mine) store_val(vals_out, vb, i, before);
-        const unsigned m = __ballot_sync(kFull, present);
-        if (bits_out != nullptr && lane == 0 && m) atomicOr(&bits_out[base >> 5], m);
         __syncwarp();
-        warp_size_add(tctr, tb, placed, 1);
-        warp_size_add(tctr, tb, gone, -1);
-        const unsigned long long at = agg_inc(&gctr->pending, pend);
-        if (pend) {
-            if (at < list_cap) {
-                ((Sl *)list_a)[at] = e;
-                if (list_a_tid) list_a_tid[at] = tb;
-            } else {
-                atomicAdd(&gctr->spill, 1ull);
+        for (uint32_t at = 0; at < total; at += 32u) {
+            bool mine = at + lane < total;
+            const uint32_t place = mine ? s_op[warp][at + lane] : 0u;
+            const uint64_t i = first + place;
+            uint32_t tb = 0u;
+            typename T::K k = 0;
+            uint8_t op = kOpFind;
+            Sl e = T::empty();
+            if (mine) {
+                tb = table_at(A.tidx, off, (uint32_t)i, (uint32_t)i);
+                if (tb >= ntables) {
+                    note_bad(A);
+                    mine = false;
+                    tb = 0u;
+                } else {
+                    k = load_key<KB>(keys, i);
+                    op = ops[i];
+                }
+            }
+            const Desc &D = descs[tb];
+            const unsigned long long tpol = HINT ? l2_policies(D.l2_keep != 0u).table : 0ull;
+            const bool act = mine && k != 0;  // ops on key 0 miss and change nothing
+            const bool ins = act && op == kOpInsert, del = act && op == kOpErase;
+            if (ins) e = T::make(k, load_val(vals, vb, i));
+            const uint32_t hk = fold(k);
+            const Pair p = pair_of(hk, D.d);
+            char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
+            char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
+            const KvOut r1 = place_probe<KB, SB, HINT>(p1, k, act, p.first, D.d, stage, tpol);
+            const bool found1 = act && r1.match >= 0;
+            const bool check2 =
+                act && !found1 && ((!Gm::kMeta || r1.overflow) || (ins && r1.empty == 0u));
+            KvOut r2{-1, 0ull, false, 0u};
+            if (__any_sync(kFull, check2))
+                r2 = place_probe<KB, SB, HINT>(p2, k, check2, p.second, D.d, stage, tpol);
+            const bool found2 = check2 && r2.match >= 0;
+            const bool present = found1 || found2;
+            const uint64_t before = found1 ? r1.value : (found2 ? r2.value : 0ull);
+            bool pend = false, placed = false, gone = false;
+            if (ins) {
+                if (found1) {
+                    T::store(slot_ptr<KB, SB>(p1, r1.match), e);
+                    ++n_upd;
+                } else if (found2) {
+                    T::store(slot_ptr<KB, SB>(p2, r2.match), e);
+                    ++n_upd;
+                } else {
+                    bool ok = claim_empty<KB, SB>(p1, r1.empty, e);
+                    if (!ok && check2 && r2.empty) {
+                        mark_overflow<KB, SB>(p1, hk);
+                        ok = claim_empty<KB, SB>(p2, r2.empty, e);
+                    }
+                    if (ok) {
+                        ++n_ins;
+                        placed = true;
+                    } else {
+                        pend = true;
+                    }
+                }
+            } else if (del && present) {
+                T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match),
+                         T::empty());
+                ++n_del;
+                gone = true;
+            }
+            if (vals_out != nullptr && mine) store_val(vals_out, vb, i, before);
+            if (present) atomicOr(&s_bits[warp][place >> 5], 1u << (place & 31u));
+            __syncwarp();
+            warp_size_add(tctr, tb, placed, 1);
+            warp_size_add(tctr, tb, gone, -1);
+            const unsigned long long slot = agg_inc(&gctr->pending, pend);
+            if (pend) {
+                if (slot < list_cap) {
+                    ((Sl *)list_a)[slot] = e;
+                    if (list_a_tid) list_a_tid[slot] = tb;
+                } else {
+                    atomicAdd(&gctr->spill, 1ull);
+                }
             }
         }
+        __syncwarp();
+        if (bits_out != nullptr && lane < words && s_bits[warp][lane])
+            atomicOr(&bits_out[(first >> 5) + lane], s_bits[warp][lane]);
+        __syncwarp();  // the list and the bits are reused
     }
     // one atomic per counter per block
     __shared__ unsigned long long s_sum[3];
