@@ -6,12 +6,13 @@
 // once with a key table in shared memory (k_bin_group). Every other op keeps
 // its bit in a bitmap and is resolved by the probe kernels in op order, with
 // coalesced batch reads and results. The open-addressing table in global
-// memory that this replaces as the first choice took one random L2 or DRAM
-// atomic per op over 64 MB of cells (99-113 us for 2^22 ops), a pass over the
-// cells (23-28 us) and, for mixed batches, a second random read per op (56
-// us); the split is bound by its 8-byte stores to random sectors (36 us, of
-// which 5 us is the bytes) and the grouping by shared-memory atomics (26-39
-// us). 2^24 mixed ops on 2^27 keys: 3.61 -> 2.78 ms a pair of batches.
+// memory that this replaces took one random L2 or DRAM atomic per op over 64
+// MB of cells (99-113 us for 2^22 ops), a pass over the cells (23-28 us) and,
+// for mixed batches, a second random read per op (56 us). The split is bound
+// by its 8-byte stores to random sectors (47 us, of which 5 us is the bytes),
+// the grouping by the latency of its steps (19 us for inserts and erases, 27
+// us for mixed ops). 2^24 mixed ops on 2^27 keys: 3.61 -> 2.5 ms a pair of
+// batches.
 //
 // Splitting by the region of a key's first bucket instead, so that a bin's
 // probes fall close together, and probing from the bins in the same kernel,
@@ -19,14 +20,14 @@
 // words and bits at random places cost more than that (312 us against 47 + 39
 // + 187 for 2^22 mixed ops).
 //
-// Up to 16384 ops run as one kernel (k_bin_small): every block reads the whole
-// batch, keeps its bin's ops and resolves them itself, and the last block
-// writes the counters to the host. A mixed batch of 4096 ops took ten
-// kernels, four memsets and two copies: 97 -> 41 us a call.
+// Up to kBinSmallOps ops run as one kernel (k_bin_small): every block reads the
+// whole batch, keeps its bin's ops and resolves them itself, and the last block
+// writes the counters to the host. A mixed batch of 4096 ops took ten kernels,
+// four memsets and two copies: 97 -> 33 us a call.
 //
 // A bin with more ops than its capacity (few keys, each repeated hundreds of
-// times) is left, as a whole, to the general path: its keys meet no key of
-// another bin.
+// times, or a skewed batch's most popular ones) gets a second, exact set of
+// records, which its block streams (group_hot).
 #pragma once
 
 #include "dyc_apply.cuh"
@@ -43,7 +44,8 @@ constexpr int kSplitThreads = 512;
 constexpr uint32_t kSplitBins = 4096;               // bins counted in shared memory (k_bin_scatter)
 constexpr int kGroupThreads = 512;
 constexpr int kGroupR = kBinCap / kGroupThreads;    // records per thread (k_bin_group)
-constexpr int kGroupTab = 2 * kBinCap;
+constexpr int kGroupPre = kBinMean / kGroupThreads; // of them, read along with the count
+constexpr int kGroupTab = 2 * kBinCap;              // cells of a bin's first table, half as many of its second
 
 // An op of a small batch's bin: index << 2 | code (2 bits; any other code reads).
 __device__ __forceinline__ uint32_t op_word(uint64_t i, uint8_t op) {
@@ -153,19 +155,24 @@ template <int KB> __device__ __noinline__ void plan_hot(const BinScratch &B) {
 // SET: the ops of table t are [off[t], off[t + 1]) and go to its own bins; a
 // block's ops then fall into a short range of bins (its records land in long
 // runs), and ops outside a range of kSplitBins take their places one by one.
+// tile_ops (at most PER * 512, a multiple of 512): the ops a block takes, so
+// that the blocks come to whole waves. Loads go out kLoad ops at a time: in a
+// set's split the records it may write kept the compiler from grouping them,
+// and with three blocks an SM a 2^25-op round's split took 189 us, not 297 (a
+// single table's waits for its stores either way: two blocks, 47 us for 2^22).
 // A single table's chunk starts here: the call counters (ctr), A.ctr and the
 // result bits are zeroed and the single bits set (k_set_prep does so for a
 // set). The bin counts, cursors and state are zero on entry: k_bin_group
 // leaves them so.
 template <int KB, int PER, bool SET, bool HOT>
-__global__ void __launch_bounds__(kSplitThreads, 2) k_bin_scatter(
+__global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
     const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
     const uint32_t *__restrict__ off, const uint8_t *__restrict__ ops,
-    const void *__restrict__ keys, uint64_t n, unsigned long long *ctr, uint32_t *bits) {
+    const void *__restrict__ keys, uint64_t n, unsigned long long *ctr, uint32_t *bits,
+    uint32_t tile_ops) {
     after_previous();
     using K = typename SlotT<KB>::K;
-    constexpr uint64_t kTile = (uint64_t)PER * kSplitThreads;
-    static_assert(kTile <= 1 << 13 && kSplitBins <= 1 << 13, "a place and a bin take 13 bits each");
+    static_assert(PER * kSplitThreads <= 1 << 13 && kSplitBins <= 1 << 13, "a place and a bin take 13 bits each");
     __shared__ uint32_t s_cnt[kSplitBins];
     if (HOT && B.state[kBinOver] == 0u) return;
     uint32_t *cursor = HOT ? B.cursor : B.count;
@@ -194,10 +201,10 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_bin_scatter(
         if (p < (uint32_t)kBinCap) B.rec[(uint64_t)b * kBinCap + p] = r;
         else went_over = true;
     };
-    for (uint64_t tile = (uint64_t)blockIdx.x * kTile; tile < n; tile += (uint64_t)gridDim.x * kTile) {
+    for (uint64_t tile = (uint64_t)blockIdx.x * tile_ops; tile < n; tile += (uint64_t)gridDim.x * tile_ops) {
         uint32_t lo = 0u, nb = B.nbins;
         if (SET) {
-            const uint64_t last = (tile + kTile < n ? tile + kTile : n) - 1;
+            const uint64_t last = (tile + tile_ops < n ? tile + tile_ops : n) - 1;
             const uint32_t t0 = table_at(A.tidx, off, (uint32_t)tile, (uint32_t)tile);
             const uint32_t t1 = table_at(A.tidx, off, (uint32_t)last, (uint32_t)last);
             const TableBins a = table_bins(B, off, t0, n), b = table_bins(B, off, t1, n);
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_bin_scatter(
             plan_hot<KB>(B);
         }
         if (!SET && !HOT) {
-            const uint64_t words = ((tile + kTile < n ? tile + kTile : n) + 31) / 32;
+            const uint64_t words = ((tile + tile_ops < n ? tile + tile_ops : n) + 31) / 32;
             for (uint64_t w = tile / 32 + threadIdx.x; w < words; w += kSplitThreads) {
                 B.single[w] = 0xffffffffu;
                 if (bits != nullptr) bits[w] = 0u;
@@ -227,11 +234,23 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_bin_scatter(
         __syncthreads();
         // at: place | bin - lo << 13 | op code << 26; ~0: key 0, or done
         uint32_t tag[PER], at[PER];
+        constexpr int kLoad = 8;
+        K key[kLoad];
+        uint8_t op[kLoad];
+        const uint64_t end = tile + tile_ops < n ? tile + tile_ops : n;
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
+            if (j % kLoad == 0) {  // loads in flight together
+#pragma unroll
+                for (int x = 0; x < kLoad; ++x) {
+                    const uint64_t i = tile + (uint64_t)(j + x) * kSplitThreads + threadIdx.x;
+                    key[x] = i < end ? load_key<KB>(keys, i) : (K)0;
+                    op[x] = (ops != nullptr && i < end) ? ops[i] : (uint8_t)kOpFind;
+                }
+            }
             const uint64_t i = tile + (uint64_t)j * kSplitThreads + threadIdx.x;
-            const K k = i < n ? load_key<KB>(keys, i) : (K)0;
-            const uint32_t code = op_word(0, (ops != nullptr && i < n) ? ops[i] : (uint8_t)kOpFind);
+            const K k = key[j % kLoad];
+            const uint32_t code = op_word(0, op[j % kLoad]);
             tag[j] = bin_tag(k);
             at[j] = 0xffffffffu;
             if (k == 0) continue;
@@ -468,6 +487,13 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
 // range of seg; ids with more than kShortSeg ops go to wseg or mid as well.
 // SET: the inserts among the other ops are counted as upserts of the bin's
 // table (the upsize policy's insert batch).
+// A record leaves its number in its key's cell with a plain store; the record
+// that stays leads the key's group, and most records find themselves there.
+// Only records whose cell another key has claim one in a second table by
+// compare-and-swap, and only a group's further records count themselves in:
+// with one swap and one count for every record 2^22 erases took 26 us (now 19)
+// and 2^22 mixed ops 42 (now 27, of which 7 from fewer barriers and segments
+// written without a stop in shared memory).
 template <int KB, int MODE, bool SET>
 __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
@@ -475,31 +501,42 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     after_previous();
     using K = typename SlotT<KB>::K;
     struct Smem {
-        uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kGroupTab];
+        uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kBinCap];
+        uint16_t first[kGroupTab];
     };
     __shared__ __align__(16) unsigned char s_raw[sizeof(Smem)];
     static_assert(sizeof(HotSmem) <= sizeof(Smem), "one block of shared memory for both");
     Smem &M = *reinterpret_cast<Smem *>(s_raw);
-    __shared__ uint32_t s_nseg, s_nkey, s_nwarp, s_nmid, s_ok, s_ins;
+    __shared__ uint32_t s_place, s_nwarp, s_nmid, s_ok, s_ins;  // place: ops | keys << 16
     __shared__ unsigned long long s_bseg, s_bkey, s_bwarp, s_bmid;
     const uint32_t tid = threadIdx.x, bin = blockIdx.x;
+    // the first kGroupPre rounds of records are read along with their count
+    unsigned long long x[kGroupR];
+#pragma unroll
+    for (int q = 0; q < kGroupPre; ++q) x[q] = B.rec[(uint64_t)bin * kBinCap + q * kGroupThreads + tid];
     const uint32_t m = B.count[bin];
     if (m == 0u) {
         if (bin == 0 && tid < (uint32_t)kBinStates) B.state[tid] = 0u;
         return;
     }
-    for (uint32_t c = tid; c < (uint32_t)kGroupTab; c += kGroupThreads) M.tab[c] = 0u;
-    if (tid == 0) s_nseg = s_nkey = s_nwarp = s_nmid = s_ins = 0u;
+    for (uint32_t c = tid; c < (uint32_t)kBinCap; c += kGroupThreads) M.tab[c] = 0u;
+    if (tid == 0) s_place = s_nwarp = s_nmid = s_ins = 0u;
     if (m <= (uint32_t)kBinCap) {
         const unsigned long long *rec = B.rec + (uint64_t)bin * kBinCap;
 #pragma unroll
+        for (int q = kGroupPre; q < kGroupR; ++q) {
+            const uint32_t r = q * kGroupThreads + tid;
+            if (r < m) x[q] = rec[r];
+        }
+#pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
             const uint32_t r = q * kGroupThreads + tid;
-            M.cnt[r] = MODE == kBinModeErase ? 0xffffffffu : 0u;
             if (r < m) {
-                const unsigned long long x = rec[r];
-                M.tag[r] = (uint32_t)x;
-                M.word[r] = (uint32_t)(x >> 32);
+                const uint32_t tag = (uint32_t)x[q], w = (uint32_t)(x[q] >> 32);
+                M.tag[r] = tag;
+                M.word[r] = w;
+                M.cnt[r] = MODE == kBinModeMixed ? 0u : w;
+                M.first[bin_cell<12>(tag)] = (uint16_t)r;  // one of the cell's records stays
             }
         }
     }
@@ -512,29 +549,36 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
         group_hot<KB, MODE, SET>(B, A, keys, bin, m, *reinterpret_cast<HotSmem *>(s_raw));
         return;
     }
-    uint32_t lr[kGroupR];  // first record of the key | rank << 16
+    uint32_t lr[kGroupR];  // the key's lead record | the op's rank << 16
+    static_assert(kGroupTab == 1 << 12 && kBinCap == 1 << 11, "cells of 12 and 11 bits");
 #pragma unroll
     for (int q = 0; q < kGroupR; ++q) {
         const uint32_t r = q * kGroupThreads + tid;
-        lr[q] = 0u;
+        lr[q] = r;
         if (r >= m) continue;
         const uint32_t tag = M.tag[r], w = M.word[r];
-        uint32_t h = bin_cell<12>(tag), lead;
-        static_assert(kGroupTab == 1 << 12, "bin_cell takes 12 bits");
-        while (true) {  // at most half of the cells are taken: the probe ends
-            const uint32_t old = atomicCAS(&M.tab[h], 0u, r + 1u);
-            lead = old == 0u ? r : old - 1u;
-            if (old == 0u) break;
-            if (M.tag[lead] == tag &&
-                (KB == 4 || load_key<KB>(keys, rec_index(A, M.word[lead])) ==
-                                load_key<KB>(keys, rec_index(A, w))))
-                break;
-            h = (h + 1u) & (kGroupTab - 1);
+        auto same = [&](uint32_t x) {
+            return x == r || (M.tag[x] == tag &&
+                              (KB == 4 || load_key<KB>(keys, rec_index(A, M.word[x])) ==
+                                              load_key<KB>(keys, rec_index(A, w))));
+        };
+        uint32_t lead = M.first[bin_cell<12>(tag)];
+        if (!same(lead)) {
+            // another key has the cell: at most kBinCap - 1 records come here, so
+            // a cell of the second table stays free and the probe ends
+            uint32_t h = bin_cell<23>(tag) & (kBinCap - 1);
+            while (true) {
+                const uint32_t old = atomicCAS(&M.tab[h], 0u, r + 1u);
+                lead = old == 0u ? r : old - 1u;
+                if (old == 0u || same(lead)) break;
+                h = (h + 1u) & (kBinCap - 1);
+            }
         }
+        if (lead == r) continue;
         if (MODE == kBinModeInsert) atomicMax(&M.cnt[lead], w);
         else if (MODE == kBinModeErase) atomicMin(&M.cnt[lead], w);
-        else lr[q] = atomicAdd(&M.cnt[lead], 1u) << 16;
-        lr[q] |= lead;
+        else lr[q] = lead | (atomicAdd(&M.cnt[lead], 1u) + 1u) << 16;
+        if (MODE != kBinModeMixed) lr[q] = lead;
     }
     __syncthreads();
     if constexpr (MODE != kBinModeMixed) {
@@ -544,60 +588,54 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             if (r < m && M.cnt[lr[q]] != M.word[r]) clear_single(B, rec_index(A, M.word[r]));
         }
     } else {
-        bool any = false;
+        // the second table's cells now hold each key's place in its block's ranges
         uint32_t ins = 0u;
 #pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
-            const uint32_t r = q * kGroupThreads + tid;
-            const bool several = r < m && M.cnt[lr[q] & 0xffffu] > 1u;
-            any |= several;
-            if (SET && r < m && !several) ins += M.word[r] & 1u;
+            const uint32_t r = q * kGroupThreads + tid, lead = lr[q] & 0xffffu;
+            if (r >= m) continue;
+            const uint32_t c = M.cnt[lead] + 1u;
+            if (c == 1u) {
+                if (SET) ins += M.word[r] & 1u;
+            } else if (lead == r) {
+                M.tab[r] = atomicAdd(&s_place, c | 1u << 16);
+                if (c > kShortSeg) atomicAdd(c > kWarpSeg ? &s_nmid : &s_nwarp, 1u);
+            }
         }
         if (SET) {
             ins = __reduce_add_sync(kFull, ins);
             if ((tid & 31) == 0 && ins) atomicAdd(&s_ins, ins);
         }
-        const bool more = __syncthreads_or(any);
+        __syncthreads();
         const uint32_t table = SET ? B.tid[bin] : 0u;
         if (SET && tid == 0 && s_ins && table < A.ntables) atomicAdd(&A.tup[table], s_ins);
-        if (!more) return;
-        // the table's cells now hold each key's place in its block's ranges
-#pragma unroll
-        for (int q = 0; q < kGroupR; ++q) {
-            const uint32_t r = q * kGroupThreads + tid;
-            if (r >= m || (lr[q] & 0xffffu) != r) continue;
-            const uint32_t c = M.cnt[r];
-            if (c <= 1u) continue;
-            M.tab[r] = atomicAdd(&s_nseg, c) | (atomicAdd(&s_nkey, 1u) << 16);
-            if (c > kShortSeg) atomicAdd(c > kWarpSeg ? &s_nmid : &s_nwarp, 1u);
-        }
-        __syncthreads();
+        if (s_place == 0u) return;
         if (tid == 0) {
-            s_ok = take_ranges(A, s_nkey, s_nseg, s_nwarp, s_nmid, s_bkey, s_bseg, s_bwarp, s_bmid);
+            s_ok = take_ranges(A, s_place >> 16, s_place & 0xffffu, s_nwarp, s_nmid, s_bkey, s_bseg,
+                               s_bwarp, s_bmid);
             s_nwarp = s_nmid = 0u;
         }
         __syncthreads();
         if (!s_ok) return;
-        // the ops of the block's segments are put in place in shared memory
-        // (the tags are done) and go out in order
 #pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
             const uint32_t r = q * kGroupThreads + tid, lead = lr[q] & 0xffffu;
-            if (r >= m || M.cnt[lead] <= 1u) continue;
-            const uint32_t w = M.word[r], i = rec_index(A, w), place = M.tab[lead] & 0xffffu;
-            M.tag[place + (lr[q] >> 16)] = seg_word(A, w);
+            if (r >= m) continue;
+            const uint32_t c = M.cnt[lead] + 1u;
+            if (c == 1u) continue;
+            const uint32_t w = M.word[r], i = rec_index(A, w);
+            const uint32_t place = (uint32_t)s_bseg + (M.tab[lead] & 0xffffu);
+            A.seg[place + (lr[q] >> 16)] = seg_word(A, w);
             clear_single(B, i);
             if (lead == r) {
                 const uint32_t d = (uint32_t)s_bkey + (M.tab[lead] >> 16);
-                ((K *)A.dkey)[d] = load_key<KB>(keys, i);
-                A.dcnt[d] = M.cnt[r];
-                A.dseg[d] = (unsigned long long)((uint32_t)s_bseg + place) << 32;
+                ((K *)A.dkey)[d] = KB == 4 ? (K)M.tag[r] : load_key<KB>(keys, i);
+                A.dcnt[d] = c;
+                A.dseg[d] = (unsigned long long)place << 32;
                 if (SET) A.dtid[d] = table;
-                list_long(A, d, M.cnt[r], &s_nwarp, &s_nmid, s_bwarp, s_bmid);
+                list_long(A, d, c, &s_nwarp, &s_nmid, s_bwarp, s_bmid);
             }
         }
-        __syncthreads();
-        for (uint32_t x = tid; x < s_nseg; x += kGroupThreads) A.seg[s_bseg + x] = M.tag[x];
     }
 }
 

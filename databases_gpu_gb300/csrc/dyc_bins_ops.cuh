@@ -32,16 +32,21 @@ template <int KB, int MODE, bool SET>
 cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
                        const uint32_t *off, const uint8_t *ops, const void *keys, uint64_t cap_n,
                        unsigned long long *ctr, uint32_t *bits) {
-    // 16 ops a thread where that still fills the chip, else 8
-    const uint64_t tile = cap_n >= (1ull << 21) ? 16 * kSplitThreads : 8 * kSplitThreads;
+    // whole waves of the blocks an SM holds, of at most 16 ops a thread (below
+    // 2^21 ops, where 8 fill the chip, of 8)
+    const uint64_t slots = (SET ? 3u : 2u) * (uint64_t)std::max(L.sms, 1), unit = kSplitThreads;
+    const uint64_t per = cap_n >= (1ull << 21) ? 16 : 8;
+    const uint64_t waves = (cap_n + slots * per * unit - 1) / (slots * per * unit);
+    const uint64_t share = (cap_n + waves * slots - 1) / (waves * slots);
+    const uint32_t tile = (uint32_t)((share + unit - 1) / unit * unit);
     const unsigned blocks = (unsigned)((cap_n + tile - 1) / tile);
-    if (tile == 16 * kSplitThreads)
-        launch_after(k_bin_scatter<KB, 16, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits);
+    if (per == 16)
+        launch_after(k_bin_scatter<KB, 16, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits, tile);
     else
-        launch_after(k_bin_scatter<KB, 8, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits);
+        launch_after(k_bin_scatter<KB, 8, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits, tile);
     // nothing to do in most batches: a fixed grid of one wave
-    const unsigned some = std::min<unsigned>(blocks, 4u * (unsigned)(L.sms > 0 ? L.sms : 1));
-    launch_after(k_bin_scatter<KB, 8, SET, true>, (unsigned)(some), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, nullptr);
+    const unsigned some = (unsigned)std::min<uint64_t>((cap_n + 8 * unit - 1) / (8 * unit), 4u * (uint64_t)std::max(L.sms, 1));
+    launch_after(k_bin_scatter<KB, 8, SET, true>, (unsigned)(some), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, nullptr, 8u * kSplitThreads);
     launch_after(k_bin_group<KB, MODE, SET>, (unsigned)(B.nbins), kGroupThreads, 0, L.stream, B, A, keys);
     return cudaGetLastError();
 }

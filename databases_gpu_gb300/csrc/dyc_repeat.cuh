@@ -306,8 +306,12 @@ __device__ __forceinline__ void list_change(const ApplyScratch &A, const RepKey<
     }
 }
 
+// Bound by the latency of its probes and segment reads. A set's rounds have
+// many segments for a warp each, and a fourth block an SM hides more of them:
+// 2^25 ops over 4096 tables 495 -> 430 us; with five the spilled registers cost
+// as much, and a single table's short segments are faster with three.
 template <int KB, int SB, bool SET, bool MUT>
-__global__ void __launch_bounds__(256, 3) k_repeat(
+__global__ void __launch_bounds__(256, SET ? 4 : 3) k_repeat(
     const __grid_constant__ ApplyScratch A, const Desc *__restrict__ descs, uint32_t ntables,
     const uint8_t *__restrict__ ops, const void *__restrict__ vals, uint32_t vb,
     void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, void *list_a, uint64_t list_cap,

@@ -233,9 +233,9 @@ __global__ void __launch_bounds__(256) k_set_mutate(
 // keys, so no key is probed by two kernels at once.
 // Bound by the latency of the probes in flight. A warp lists the set bits of
 // up to kUniqueWords bitmap words and probes them 32 at a time: in a round of
-// 2^22 ops over 4096 tables about half the ops repeat a key, and a warp that
-// took one word at a time probed with half its lanes idle (450 us a round,
-// 322 with the list). A small batch takes fewer words to a warp so that the
+// 2^25 ops over 4096 tables about half the ops repeat a key, and a warp that
+// took one word at a time probed with half its lanes idle (900 us a round,
+// 645 with the list). A small batch takes fewer words to a warp so that the
 // blocks still cover the chip.
 constexpr uint32_t kUniqueWords = 8;  // bitmap words a warp takes at most
 
