@@ -222,9 +222,12 @@ __device__ __forceinline__ void bitonic_sort(uint32_t *s, uint32_t P, uint32_t t
 // the pass), and an erase clears the key's slot. Ops on different keys run
 // side by side: nothing in the pass moves an entry, so a find never misses a
 // key that is present, and a key's own slot is written only by its own op.
+// Bound by its random lines; five blocks an SM keep more of them in flight than
+// the registers would allow by themselves (2^22 ops: 4-byte keys 185 -> 176 us,
+// 8-byte keys, three blocks, 207 -> 183; six spill: 197 and 198).
 // ----------------------------------------------------------------------------
 template <int KB, int SB, bool HINT>
-__global__ void __launch_bounds__(256) k_apply_unique(
+__global__ void __launch_bounds__(256, 5) k_apply_unique(
     const __grid_constant__ Desc D, const __grid_constant__ Scratch S,
     const uint8_t *__restrict__ ops, const void *__restrict__ keys,
     const void *__restrict__ vals, uint32_t vb, void *__restrict__ vals_out,
@@ -332,9 +335,9 @@ __global__ void __launch_bounds__(256) k_apply_unique(
 
 // The upserts and erases k_apply_unique would make (with kBinSkipEqual) for
 // the ops whose single bit is set: a batch whose upsize policy needs the counts
-// first. Finds are not probed.
+// first. Finds are not probed. (Five blocks an SM: 8-byte keys 149 -> 121 us.)
 template <int KB, int SB>
-__global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_apply_count(
+__global__ void __launch_bounds__(256, 5) k_apply_count(
     const __grid_constant__ Desc D, const uint8_t *__restrict__ ops, const void *__restrict__ keys,
     const void *__restrict__ vals, uint32_t vb, uint64_t n, const uint32_t *__restrict__ single,
     Counters *ctr) {

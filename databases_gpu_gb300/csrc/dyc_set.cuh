@@ -172,9 +172,10 @@ __device__ __forceinline__ void set_place_warp(const Desc *__restrict__ descs, u
 // *nu_ptr) in one grid-stride pass: warp items [0, ceil32(ne)) erase, the
 // rest upsert. The keys of the two lists are distinct, so the two kinds may
 // run concurrently (an upsert only claims empty slots or rewrites its own
-// key; an erase only empties its own key's slot).
+// key; an erase only empties its own key's slot). Six blocks an SM: 97 -> 78 us
+// in a round of 2^25 ops over 4096 tables.
 template <int KB, int SB, bool HINT>
-__global__ void __launch_bounds__(256) k_set_mutate(
+__global__ void __launch_bounds__(256, 6) k_set_mutate(
     const Desc *__restrict__ descs, uint32_t ntables, Counters *__restrict__ tctr,
     const void *__restrict__ er_keys, const uint32_t *__restrict__ er_tids,
     const unsigned long long *__restrict__ ne_ptr, const void *__restrict__ up_keys,
@@ -235,12 +236,13 @@ __global__ void __launch_bounds__(256) k_set_mutate(
 // up to kUniqueWords bitmap words and probes them 32 at a time: in a round of
 // 2^25 ops over 4096 tables about half the ops repeat a key, and a warp that
 // took one word at a time probed with half its lanes idle (900 us a round,
-// 645 with the list). A small batch takes fewer words to a warp so that the
-// blocks still cover the chip.
+// 645 with the list, 604 with five blocks an SM; 8-byte keys spill then, 22.6 us
+// a step of 64 tables for 21.6). A small batch takes fewer words to a warp so
+// that the blocks still cover the chip.
 constexpr uint32_t kUniqueWords = 8;  // bitmap words a warp takes at most
 
 template <int KB, int SB, bool HINT>
-__global__ void __launch_bounds__(256) k_set_unique(
+__global__ void __launch_bounds__(256, KB == 4 ? 5 : 4) k_set_unique(
     const __grid_constant__ ApplyScratch A, const uint32_t *__restrict__ off,
     const Desc *__restrict__ descs, uint32_t ntables, Counters *__restrict__ tctr,
     const uint8_t *__restrict__ ops, const void *__restrict__ keys, const void *__restrict__ vals,
