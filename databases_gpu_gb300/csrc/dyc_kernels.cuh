@@ -303,8 +303,11 @@ struct KvOut {
 constexpr int kBlockThreads = 256;
 constexpr int kWarpsPerBlock = kBlockThreads / 32;
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+template <bool L1> __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    if (L1)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async16_pol(uint32_t dst, const void *src,
                                                unsigned long long pol) {
@@ -321,9 +324,9 @@ template <int SB> __device__ __forceinline__ uint32_t piece_off(int o, int s) {
 // Copy the bucket at p of every active lane into stage (lane-indexed).
 // ALL: every lane is active; otherwise active lanes are served in rank order
 // so few active lanes cost few rounds.
-template <int SB, bool ALL, bool HINT = false>
+template <int SB, bool ALL, bool HINT, bool L1>
 __device__ __forceinline__ void stage_rounds(const char *p, unsigned am, unsigned char *stage,
-                                             unsigned long long pol = 0ull) {
+                                             unsigned long long pol) {
     constexpr int G = SB / 32, RO = 32 / G;
     const int lane = threadIdx.x & 31, g = lane / G, r = lane % G;
     const int nact = ALL ? 32 : __popc(am);
@@ -343,8 +346,8 @@ __device__ __forceinline__ void stage_rounds(const char *p, unsigned am, unsigne
                                polq);
             }
         } else if (have) {
-            cp_async16(base + piece_off<SB>(o, r), (const char *)pq + r * 16);
-            cp_async16(base + piece_off<SB>(o, r + G), (const char *)pq + (r + G) * 16);
+            cp_async16<L1>(base + piece_off<SB>(o, r), (const char *)pq + r * 16);
+            cp_async16<L1>(base + piece_off<SB>(o, r + G), (const char *)pq + (r + G) * 16);
         }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -352,7 +355,7 @@ __device__ __forceinline__ void stage_rounds(const char *p, unsigned am, unsigne
     __syncwarp();  // other lanes' copies are visible after the warp barrier
 }
 
-template <int KB, int SB, bool WANT_EMPTY = false, bool HINT = false>
+template <int KB, int SB, bool WANT_EMPTY, bool HINT, bool L1>
 __device__ __forceinline__ KvOut probe_staged(const char *p, typename SlotT<KB>::K key, bool act,
                                               unsigned char *stage,
                                               unsigned long long pol = 0ull) {
@@ -361,8 +364,8 @@ __device__ __forceinline__ KvOut probe_staged(const char *p, typename SlotT<KB>:
     constexpr int P = SB / 16, SPP = 16 / T::kBytes > 0 ? 16 / T::kBytes : 1;
     const unsigned am = __ballot_sync(kFull, act);
     __syncwarp();  // the previous use of the stage is finished in every lane
-    if (am == kFull) stage_rounds<SB, true, HINT>(p, am, stage, pol);
-    else if (am) stage_rounds<SB, false, HINT>(p, am, stage, pol);
+    if (am == kFull) stage_rounds<SB, true, HINT, L1>(p, am, stage, pol);
+    else if (am) stage_rounds<SB, false, HINT, L1>(p, am, stage, pol);
     KvOut out{-1, 0ull, false, 0u};
     if (!act) return out;
     const int lane = threadIdx.x & 31;
@@ -398,11 +401,11 @@ __device__ __forceinline__ KvOut probe_staged(const char *p, typename SlotT<KB>:
 // buckets; 32-byte buckets (one lane per bucket, a single 256-bit load) read
 // straight into registers, since staging them would split each sector over
 // two 16-byte copies.
-template <int KB, int SB, int MODE, bool HINT = false>
+template <int KB, int SB, int MODE, bool HINT = false, bool L1 = false>
 __device__ __forceinline__ KvOut kv_probe(const char *p, typename SlotT<KB>::K key, bool act,
                                           unsigned char *stage, unsigned long long pol = 0ull) {
     if constexpr (SB >= 64) {
-        return probe_staged<KB, SB, false, HINT>(p, key, act, stage, pol);
+        return probe_staged<KB, SB, false, HINT, L1>(p, key, act, stage, pol);
     } else {
         const ProbeOut<KB> r = probe<KB, SB, MODE, false, false, HINT>(p, key, act, 0u, 0u, pol);
         KvOut o;
@@ -422,7 +425,7 @@ __device__ __forceinline__ KvOut place_probe(const char *p, typename SlotT<KB>::
                                              uint32_t t, uint32_t d, unsigned char *stage,
                                              unsigned long long pol = 0ull) {
     if constexpr (SB >= 64) {
-        return probe_staged<KB, SB, true, HINT>(p, key, act, stage, pol);
+        return probe_staged<KB, SB, true, HINT, false>(p, key, act, stage, pol);
     } else {
         const ProbeOut<KB> r = probe<KB, SB, 2, true, false, HINT>(p, key, act, t, d, pol);
         KvOut o;
@@ -529,20 +532,48 @@ __global__ void __launch_bounds__(256) k_dedup(const __grid_constant__ Scratch S
 // batch) measured 2.5x slower than plain ones (15.6 vs 39.4 G finds/s at
 // Zipf 0.99 on 2^28 keys; uniform 39.3 vs 40.4).
 // ----------------------------------------------------------------------------
-template <int KB, int SB, bool HINT>
-__global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_find(const __grid_constant__ Desc D,
-                                              const void *__restrict__ keys,
-                                              void *__restrict__ vals, uint32_t vb,
-                                              uint32_t *__restrict__ hits, uint64_t n) {
-    after_previous();
+// Buckets skip the L1 unless two of the block's warps have keys that repeat
+// among their first 64, as keys drawn by Zipf 0.99 do on tables of any size and
+// uniform keys only on tables of some ten thousand: many warps then read the
+// same few lines, and the slice of the L2 that holds the hottest one sets the
+// time. With the L1, 12.3 M 8-byte finds at Zipf 0.99 on 2^26 keys (one in ten
+// present) take 260 us, not 332, and 2^24 present keys 361, not 443; uniform
+// finds pay 0.5 % for the sample. Each key leaves its number in a cell of the
+// stage and finds there itself, or an equal key, or, rarely, another. (A choice
+// between the two loads inside one loop costs uniform finds 5 %. 4-byte finds
+// gain as much from the L1, 460 -> 345 us, but their registers are full at five
+// blocks an SM, and with the sample uniform ones took 1 to 4 % more.)
+template <int KB, int SB>
+__device__ __forceinline__ bool repeated_keys(const void *keys, uint64_t n, unsigned char *stage) {
+    using K = typename SlotT<KB>::K;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t i0 = warp_base() + lane, i1 = i0 + warp_stride();
+    const K k0 = i0 < n ? load_key<KB>(keys, i0) : (K)0, k1 = i1 < n ? load_key<KB>(keys, i1) : (K)0;
+    const uint32_t h0 = fold(k0), h1 = fold(k1);
+    volatile unsigned char *c0 = stage + (h0 * 0x9E3779B1u) % (32u * SB);
+    volatile unsigned char *c1 = stage + (h1 * 0x9E3779B1u) % (32u * SB);
+    if (k0 != 0) *c0 = (unsigned char)lane;
+    if (k1 != 0) *c1 = (unsigned char)(32u + lane);
+    __syncwarp();
+    const uint32_t w0 = k0 != 0 ? *c0 : lane, w1 = k1 != 0 ? *c1 : 32u + lane;
+    const uint32_t a0 = __shfl_sync(kFull, h0, w0 & 31u), b0 = __shfl_sync(kFull, h1, w0 & 31u);
+    const uint32_t a1 = __shfl_sync(kFull, h0, w1 & 31u), b1 = __shfl_sync(kFull, h1, w1 & 31u);
+    const bool r0 = w0 != lane && (w0 < 32u ? a0 : b0) == h0;
+    const bool r1 = w1 != 32u + lane && (w1 < 32u ? a1 : b1) == h1;
+    return __syncthreads_count(__any_sync(kFull, r0 || r1)) >= 2 * 32;
+}
+
+template <int KB, int SB, bool HINT, bool L1>
+__device__ __forceinline__ void find_loop(const Desc &D, const void *__restrict__ keys,
+                                          void *__restrict__ vals, uint32_t vb,
+                                          uint32_t *__restrict__ hits, uint64_t n,
+                                          unsigned char *stage) {
     using T = SlotT<KB>;
     using Gm = Geo<KB, SB>;
-    __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
-    unsigned char *stage = s_stage[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t step = warp_stride();
     L2Pol pol{0ull, 0ull};
     if constexpr (HINT) pol = l2_policies(true);
+    const uint64_t step = warp_stride();
     for (uint64_t base = warp_base(); base < n; base += step) {
         const uint64_t i = base + lane;
         typename T::K k = 0;
@@ -554,13 +585,13 @@ __global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_find(const __grid_cons
         const uint32_t hk = fold(k);
         const Pair p = pair_of(hk, D.d);
         const char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
-        const KvOut r1 = kv_probe<KB, SB, 1, HINT>(p1, k, act, stage, pol.table);
+        const KvOut r1 = kv_probe<KB, SB, 1, HINT, L1>(p1, k, act, stage, pol.table);
         bool hit = act && r1.match >= 0;
         uint64_t v = hit ? r1.value : 0ull;
         const bool need2 = act && !hit && (!Gm::kMeta || r1.overflow);
         if (__any_sync(kFull, need2)) {
             const char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
-            const KvOut r2 = kv_probe<KB, SB, 1, HINT>(p2, k, need2, stage, pol.table);
+            const KvOut r2 = kv_probe<KB, SB, 1, HINT, L1>(p2, k, need2, stage, pol.table);
             if (need2 && r2.match >= 0) {
                 hit = true;
                 v = r2.value;
@@ -575,6 +606,22 @@ __global__ void __launch_bounds__(256, KB == 4 ? 5 : 1) k_find(const __grid_cons
             if (hits != nullptr && lane == 0) hits[base >> 5] = m;
         }
     }
+}
+
+// SAMPLE: batches of 8-byte keys of more than six tiles a warp (a shorter one
+// does not get the sample's time back: 4 % of a find of 2^20 keys).
+template <int KB, int SB, bool HINT, bool SAMPLE>
+__global__ void __launch_bounds__(256, KB == 4 ? 5 : 4) k_find(const __grid_constant__ Desc D,
+                                              const void *__restrict__ keys,
+                                              void *__restrict__ vals, uint32_t vb,
+                                              uint32_t *__restrict__ hits, uint64_t n) {
+    after_previous();
+    __shared__ __align__(128) unsigned char s_stage[kWarpsPerBlock][32 * SB];
+    unsigned char *stage = s_stage[threadIdx.x >> 5];
+    if (SAMPLE && repeated_keys<KB, SB>(keys, n, stage))
+        find_loop<KB, SB, HINT, true>(D, keys, vals, vb, hits, n, stage);
+    else
+        find_loop<KB, SB, HINT, false>(D, keys, vals, vb, hits, n, stage);
 }
 
 // ----------------------------------------------------------------------------
@@ -981,10 +1028,11 @@ __global__ void __launch_bounds__(256) k_walk(const __grid_constant__ Desc D,
 // ----------------------------------------------------------------------------
 // erase (cuckoo_delete, cuckoo.cu:524-587): the slot holding the key is
 // cleared with a CAS; the second bucket is only probed when the first one's
-// overflow bit allows the key to be there.
+// overflow bit allows the key to be there. (8-byte keys: 68 registers, three
+// blocks an SM, 184 us for 2^22 erases; five blocks, 170.)
 // ----------------------------------------------------------------------------
 template <int KB, int SB, bool HINT>
-__global__ void __launch_bounds__(256) k_erase(const __grid_constant__ Desc D,
+__global__ void __launch_bounds__(256, KB == 4 ? 4 : 5) k_erase(const __grid_constant__ Desc D,
                                                const __grid_constant__ Scratch S, int use_dedup,
                                                const void *__restrict__ keys, uint64_t n,
                                                uint32_t *__restrict__ bits, void *__restrict__ old,

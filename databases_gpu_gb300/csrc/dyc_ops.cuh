@@ -74,8 +74,11 @@ cudaError_t Ops<KB>::find(const LaunchCtx &L, const Desc &D, int sb, const void 
                           uint32_t vb, uint32_t *hits, uint64_t n) {
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
-        auto k = D.l2_keep ? k_find<KB, SB, true> : k_find<KB, SB, false>;
-        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, keys, vals, vb, hits, n);
+        const unsigned grid = (unsigned)tile_grid(L, n);
+        auto k = D.l2_keep                      ? k_find<KB, SB, true, false>
+                 : n > 6ull * 256u * grid       ? k_find<KB, SB, false, KB == 8 && SB >= 64>
+                                                : k_find<KB, SB, false, false>;
+        launch_after(k, grid, 256, 0, L.stream, D, keys, vals, vb, hits, n);
     });
     return cudaGetLastError();
 }
