@@ -1274,11 +1274,11 @@ dyc_status dyc_erase_host(dyc_table *t, const void *h_keys, uint64_t n,
 
 // =============================================================================
 // dyc_apply: mixed batches of finds, inserts and erases in batch order.
-// The kernels (dyc_apply.cuh) group the ops by key, read every distinct key's
-// state before the batch, replay each key's ops in index order, and leave one
-// list of keys to erase and one of keys to upsert; the table's own erase and
-// insert phases apply those lists (unique keys), so placement, eviction walks,
-// overflow handling and the resize policy are the ones dyc_insert/dyc_erase use.
+// The kernels find the keys with several ops (dyc_bins.cuh), replay each one's
+// ops in index order on its state before the batch (dyc_repeat.cuh), and
+// resolve every other op in one probe (k_apply_unique); placement, eviction
+// walks, overflow handling and the resize policy are the ones dyc_insert and
+// dyc_erase use.
 // =============================================================================
 namespace {
 
