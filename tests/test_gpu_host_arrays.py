@@ -53,3 +53,22 @@ def test_host_arrays_match_oracle(kb, n, kind):
     assert cnt == int(eh.sum()) and np.array_equal(gone, eh.astype(bool))
     assert t.size == len(m)
     t.close()
+
+
+@pytest.mark.parametrize("n", [3 << 22, (3 << 22) + 1])
+def test_long_pinned_finds_match_device_finds(n):
+    """The longest find in place and the shortest one by copies."""
+    import torch
+    import databases_gpu_gb300 as dg
+    from tests.helpers import to_dev, to_host
+    pool = unique_u32(1 << 21, seed=3)
+    t = dg.DyCuckoo(pool.size)
+    t.insert(to_dev(pool[: 1 << 20]), to_dev(pool[: 1 << 20] ^ np.uint32(0x77)))
+    q = pool[np.random.default_rng(n).integers(0, pool.size, n)]
+    out = _host(np.full(n, 7, np.uint32), "pinned")
+    bits = _host(np.full((n + 31) // 32, 0xFFFFFFFF, np.uint32), "pinned")
+    t.find_host(_host(q, "pinned"), out, bits)
+    dv, db = t.find(to_dev(q))
+    assert np.array_equal(out, to_host(dv, 4))
+    assert np.array_equal(bits.view(np.int32), db.cpu().numpy())
+    t.close()
