@@ -26,6 +26,20 @@ inline cudaError_t allow_smem(const void *kernel, int bytes) {
     return e;
 }
 
+template <int KB> cudaError_t Ops<KB>::load_bins() {
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> g(mu);
+    if (done.count(dev)) return cudaSuccess;
+    cudaFuncAttributes a;
+    e = cudaFuncGetAttributes(&a, (const void *)k_bin_group<KB, kBinModeErase, false>);
+    if (e == cudaSuccess) done.insert(dev);
+    return e;
+}
+
 // The split, the bins that went over, and the grouping (cap_n sizes the grids;
 // a set's kernels read the op count on the device).
 template <int KB, int MODE, bool SET>
