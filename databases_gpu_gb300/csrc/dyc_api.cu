@@ -1700,6 +1700,7 @@ struct dyc_set {
     size_t abytes = 0;
     dyc::ApplyScratch A{};
     dyc::BinScratch bins{};
+    bool bins_zero = false;  // the last batch left the bins' counts zero
     void *lbuf = nullptr;
     size_t lbytes = 0;
     void *list_a = nullptr, *list_b = nullptr;
@@ -1821,9 +1822,7 @@ dyc_status set_ensure_scratch(dyc_set *s, uint64_t n) {
     s->bins.rec = s->A.rec;
     s->bins.hot = s->A.hot;
     s->bins.single = s->A.single;
-    // a set's bin arrays do not change until the scratch does, and its kernels
-    // leave the counts zero
-    CK(cudaMemset(s->bins.state, 0, (dyc::kBinStates + 3 * nbins) * 4));
+    s->bins_zero = false;
     const size_t slot = s->kb == 4 ? 8 : 16;
     const size_t lb = ((ops * slot + 255) & ~(size_t)255) * 2 + ((ops * 4 + 255) & ~(size_t)255) * 2;
     if (s->lbuf) {
@@ -2327,6 +2326,11 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
     // them: the kernels must see the current subtables
     TRY(set_refresh_descs(s, st));
     TRY(set_ensure_scratch(s, n));
+    // the kernels leave the bins' counts zero; in new scratch, or after a call
+    // that failed on the way, they are cleared in the order of the batch's stream
+    if (!s->bins_zero)
+        CK(cudaMemsetAsync(s->bins.state, 0, (dyc::kBinStates + 3 * (size_t)s->bins.nbins) * 4, st));
+    s->bins_zero = false;
     *s->h_hostn = n;  // read by the copy at the start of phase A (the last call has synced)
     s->cur = dyc_set::Batch{d_offsets, d_ops, d_keys, d_vals, d_vals_out, d_bits_out};
     dyc_set::Graph *gr = nullptr;
@@ -2440,6 +2444,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
         CK(cudaStreamSynchronize(st));
     }
     if (gr) gr->warm = true;
+    s->bins_zero = true;
     // Device offsets that disagree with h_offsets: the kernels clamped them
     // and the batch ran; the bookkeeping below still follows the device's
     // counters, and the call reports the disagreement at the end.
