@@ -500,6 +500,10 @@ dyc::BinScratch chunk_bins(const dyc_table *t, uint64_t n, uint32_t *single) {
     return B;
 }
 
+bool apart(const void *a, uint64_t na, const void *b, uint64_t nb) {
+    return (const char *)a + na <= (const char *)b || (const char *)b + nb <= (const char *)a;
+}
+
 // Whether a batch of n ops goes to the small-batch kernel (which carries no L2
 // hints), and its bins.
 bool small_batch(const dyc_table *t, uint64_t n) {
@@ -1131,10 +1135,6 @@ void *host_view(const void *h, uint64_t bytes, int align) {
     }
     return (void *)(uintptr_t)dev;
 }
-
-bool apart(const void *a, uint64_t na, const void *b, uint64_t nb) {
-    return (const char *)a + na <= (const char *)b || (const char *)b + nb <= (const char *)a;
-}
 }  // namespace
 
 dyc_status dyc_insert_host(dyc_table *t, const void *h_keys, const void *h_vals, uint64_t n,
@@ -1463,7 +1463,10 @@ dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const
         }
         return DYC_OK;
     };
-    bool done = small_batch(t, n);
+    // every block of the small-batch kernel reads all keys while others write
+    // results, so results written over the keys take the split kernels, where
+    // an op's result is stored after the last read of its key
+    bool done = small_batch(t, n) && apart(keys, n * t->kb, vals_out, vals_out ? n * t->vb : 0);
     if (done && before) {
         TRY(bins_small(t, dyc::kBinModeCount, ops, keys, vals, nullptr, nullptr, n, 0u, s, &done));
         if (done) TRY(policy(t->h_ctr->nins, t->h_ctr->erased));
