@@ -540,13 +540,16 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             }
         }
     }
+    // the records written to `hot`: all of the bin's ops, except where device
+    // offsets that are out of order put ops in bins outside their tile's range
+    const uint32_t nhot = m > (uint32_t)kBinCap ? B.cursor[bin] : 0u;
     __syncthreads();
-    // every thread has read the count: the next batch finds it, and the
+    // every thread has read the counts: the next batch finds them, and the
     // split's state, zero
     if (tid == 0) B.count[bin] = B.cursor[bin] = 0u;
     if (bin == 0 && tid < (uint32_t)kBinStates) B.state[tid] = 0u;
     if (m > (uint32_t)kBinCap) {
-        group_hot<KB, MODE, SET>(B, A, keys, bin, m, *reinterpret_cast<HotSmem *>(s_raw));
+        group_hot<KB, MODE, SET>(B, A, keys, bin, nhot, *reinterpret_cast<HotSmem *>(s_raw));
         return;
     }
     uint32_t lr[kGroupR];  // the key's lead record | the op's rank << 16

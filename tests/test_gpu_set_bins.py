@@ -55,3 +55,37 @@ def test_first_set_call_on_a_side_stream_beside_a_busy_default_stream(kb):
         _check(S, maps, off, ops, k, v, out, bits, "round %d" % r)
     torch.cuda.synchronize()
     S.close()
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+def test_device_offsets_out_of_order_beside_a_hot_key(kb):
+    """Device offsets [0, 4096, 5000, 0, 9000]: the ops from 5000 on fall to
+    table 3, whose bins start below those of table 1, and repeat one key, so
+    the bin of that key goes over its capacity. The tile of ops 4096 to 8191
+    looks for such bins among the ones from table 1's on. The call reports the
+    offsets, and the records it did not write are not read."""
+    import torch
+    import databases_gpu_gb300 as dg
+    from databases_gpu_gb300._lib import DYC_EINVAL
+    kt = np.uint32 if kb == 4 else np.uint64
+    n = 9000
+    host = np.array([0, 4096, 5000, 5000, n], np.uint32)
+    bad = np.array([0, 4096, 5000, 0, n], np.uint32)
+    S = dg.DyCuckooSet([20000] * 4, key_bytes=kb)
+    rng = np.random.default_rng(kb)
+    for r in range(12):  # several keys: the fault needs one in table 3's first bins
+        k = rng.integers(1, 1 << 31, n).astype(kt)
+        k[5000:] = k[0]
+        args = [to_dev(a) for a in (bad, np.ones(n, np.uint8), k, k)]
+        with pytest.raises(dg.DycError) as ei:
+            S.apply(*args, h_offsets=host)
+        assert ei.value.status == DYC_EINVAL, ei.value
+    torch.cuda.synchronize()
+    # the set still serves batches with good offsets
+    S.close()
+    S = dg.DyCuckooSet([20000] * 4, key_bytes=kb)
+    maps = [O.Map() for _ in range(4)]
+    ops = rng.integers(0, 3, n).astype(np.uint8)
+    out, bits = S.apply(to_dev(host), to_dev(ops), to_dev(k), to_dev(k), h_offsets=host)
+    _check(S, maps, host, ops, k, k, out, bits, "good offsets")
+    S.close()
