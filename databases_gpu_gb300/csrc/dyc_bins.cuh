@@ -151,7 +151,8 @@ template <int KB> __device__ __noinline__ void plan_hot(const BinScratch &B) {
 // and writes the ops' records there. Records of one bin come in no order; the
 // op index in the record orders the ops of a key. Key-0 ops belong to no bin.
 // Ops beyond a bin's capacity are not written, which raises B.state[kBinOver]:
-// the pass HOT then gives all ops of such bins a record in `hot`.
+// the pass HOT then gives all ops of such bins a record in `hot` (an insert or
+// erase batch: k_bin_hot).
 // SET: the ops of table t are [off[t], off[t + 1]) and go to its own bins; a
 // block's ops then fall into a short range of bins (its records land in long
 // runs), and ops outside a range of kSplitBins take their places one by one.
@@ -286,6 +287,87 @@ __global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
         __syncthreads();  // the counts are reused by the next tile
     }
     if (!HOT && went_over) B.state[kBinOver] = 1u;
+}
+
+// The pass HOT of an insert or erase batch. Of a key's ops in a tile only one
+// can count in the batch (the last of an insert's, the first of an erase's): the
+// others lose their single bit here and get no record, so the block of a bin
+// that went over streams a record per key and tile, not one per op. Each op
+// leaves its place in its key's cell by a plain store; where another key stays
+// there, its ops all get records. With a record per op that block took nearly
+// all of a call: 2^22 inserts of 8-byte keys, one key 12.7 ms (now 0.15), Zipf
+// 1.2 2.49 (0.21), a tenth of the ops on one key 1.62 (0.28), distinct keys 0.25.
+// Losing bits are cleared a word a warp; by an atomic per op, 1500 keys took 282
+// us for 251.
+template <int KB, int MODE>
+__global__ void __launch_bounds__(kSplitThreads, 2) k_bin_hot(
+    const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
+    const void *__restrict__ keys, uint64_t n) {
+    after_previous();
+    using K = typename SlotT<KB>::K;
+    static_assert(MODE == kBinModeInsert || MODE == kBinModeErase, "one op of a key counts");
+    constexpr int kPer = 8;
+    constexpr uint32_t kTile = kPer * kSplitThreads, kNone = 0xffffffffu;
+    static_assert(kTile == 1u << 12, "a cell per op of the tile, 12 bits");
+    __shared__ uint16_t s_first[kTile];
+    __shared__ uint32_t s_best[kTile];
+    __shared__ uint32_t s_cnt[kSplitBins];  // records per bin, then where they go
+    if (B.state[kBinOver] == 0u) return;
+    plan_hot<KB>(B);
+    for (uint64_t tile = (uint64_t)blockIdx.x * kTile; tile < n; tile += (uint64_t)gridDim.x * kTile) {
+        for (uint32_t c = threadIdx.x; c < kTile; c += kSplitThreads)
+            s_best[c] = MODE == kBinModeInsert ? 0u : kNone;
+        for (uint32_t b = threadIdx.x; b < B.nbins; b += kSplitThreads) s_cnt[b] = 0u;
+        K key[kPer];
+        uint32_t cell[kPer];  // kNone: not an op of a bin that went over
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const uint64_t i = tile + (uint64_t)j * kSplitThreads + threadIdx.x;
+            key[j] = i < n ? load_key<KB>(keys, i) : (K)0;
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            cell[j] = kNone;
+            if (key[j] == 0 || B.count[bin_of<KB>(key[j], B.nbins)] <= (uint32_t)kBinCap) continue;
+            cell[j] = bin_cell<12>(bin_tag(key[j]));
+            s_first[cell[j]] = (uint16_t)(j * kSplitThreads + threadIdx.x);
+        }
+        __syncthreads();
+        bool same[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (cell[j] == kNone) continue;
+            const uint32_t at = j * kSplitThreads + threadIdx.x, lead = s_first[cell[j]];
+            same[j] = lead == at || load_key<KB>(keys, tile + lead) == key[j];
+            if (!same[j]) continue;
+            if (MODE == kBinModeInsert) atomicMax(&s_best[cell[j]], at);
+            else atomicMin(&s_best[cell[j]], at);
+        }
+        __syncthreads();
+        uint32_t at[kPer];  // place among the tile's records of the bin
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const uint32_t x = j * kSplitThreads + threadIdx.x;
+            const bool out = cell[j] != kNone && same[j] && s_best[cell[j]] != x;
+            if (out) cell[j] = kNone;
+            // a warp's ops share a bitmap word, so far all ones
+            const unsigned outs = __ballot_sync(kFull, out);
+            if (outs && (threadIdx.x & 31) == 0) B.single[((uint32_t)tile + x) >> 5] = ~outs;
+            if (cell[j] != kNone) at[j] = atomicAdd(&s_cnt[bin_of<KB>(key[j], B.nbins)], 1u);
+        }
+        __syncthreads();
+        for (uint32_t b = threadIdx.x; b < B.nbins; b += kSplitThreads)
+            if (s_cnt[b]) s_cnt[b] = B.start[b] + atomicAdd(&B.cursor[b], s_cnt[b]);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (cell[j] == kNone) continue;
+            const uint32_t i = (uint32_t)tile + j * kSplitThreads + threadIdx.x;
+            B.hot[(uint64_t)s_cnt[bin_of<KB>(key[j], B.nbins)] + at[j]] =
+                (unsigned long long)bin_tag(key[j]) | ((unsigned long long)rec_word(A, i, 0u) << 32);
+        }
+        __syncthreads();  // the cells are reused by the next tile
+    }
 }
 
 // A bin that went over (few keys, each repeated many times, or a skewed
@@ -540,8 +622,9 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             }
         }
     }
-    // the records written to `hot`: all of the bin's ops, except where device
-    // offsets that are out of order put ops in bins outside their tile's range
+    // the records written to `hot`: all of the bin's ops, except those that
+    // cannot count (k_bin_hot), and where device offsets that are out of order
+    // put ops in bins outside their tile's range
     const uint32_t nhot = m > (uint32_t)kBinCap ? B.cursor[bin] : 0u;
     __syncthreads();
     // every thread has read the counts: the next batch finds them, and the

@@ -60,7 +60,11 @@ cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScrat
         launch_after(k_bin_scatter<KB, 8, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits, tile);
     // nothing to do in most batches: a fixed grid of one wave
     const unsigned some = (unsigned)std::min<uint64_t>((cap_n + 8 * unit - 1) / (8 * unit), 4u * (uint64_t)std::max(L.sms, 1));
-    launch_after(k_bin_scatter<KB, 8, SET, true>, (unsigned)(some), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, nullptr, 8u * kSplitThreads);
+    if constexpr (MODE == kBinModeMixed)
+        launch_after(k_bin_scatter<KB, 8, SET, true>, (unsigned)(some), kSplitThreads, 0, L.stream, B, A, off,
+                     ops, keys, cap_n, ctr, nullptr, 8u * kSplitThreads);
+    else
+        launch_after(k_bin_hot<KB, MODE>, (unsigned)some, kSplitThreads, 0, L.stream, B, A, keys, cap_n);
     launch_after(k_bin_group<KB, MODE, SET>, (unsigned)(B.nbins), kGroupThreads, 0, L.stream, B, A, keys);
     return cudaGetLastError();
 }
