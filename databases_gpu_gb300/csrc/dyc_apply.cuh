@@ -188,28 +188,6 @@ __device__ __forceinline__ void replay_op(uint8_t op, uint64_t inval, bool &pres
     }
 }
 
-// Ascending bitonic sort of s[0..P) (P a power of two) by the threads
-// [t0, t0 + nt) of the caller's group; sync() separates the stages.
-template <class Sync>
-__device__ __forceinline__ void bitonic_sort(uint32_t *s, uint32_t P, uint32_t t0, uint32_t nt,
-                                             Sync sync) {
-    for (uint32_t k = 2; k <= P; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t t = t0; t < P; t += nt) {
-                const uint32_t u = t ^ j;
-                if (u > t) {
-                    const uint32_t a = s[t], b = s[u];
-                    if ((a > b) == ((t & k) == 0)) {
-                        s[t] = b;
-                        s[u] = a;
-                    }
-                }
-            }
-            sync();
-        }
-    }
-}
-
 // ----------------------------------------------------------------------------
 // The ops of a mixed batch that are their keys' only ones: the whole batch
 // when the caller promises distinct keys (DYC_FLAG_UNIQUE), else those whose

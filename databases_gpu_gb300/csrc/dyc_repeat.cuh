@@ -56,13 +56,6 @@ __device__ __forceinline__ RepKey<KB> probe_listed(const ApplyScratch &A, const 
     return x;
 }
 
-// Ops of one key, up to 32 * R of them, by one warp: the op indexes sorted in
-// registers (element e in lane e / R; merges across lanes by shuffles), then
-// each lane takes its R consecutive ops. The op codes and values of all ops
-// are read at once, so a segment costs two dependent memory round trips
-// whatever its length. (Sorted in shared memory and replayed 32 ops a step,
-// the segments of a 4096-table round took 407 us of a warp kernel of their
-// own.)
 // An op word of a segment (SegOps::wide: a plain index).
 struct SegOps {
     const uint8_t *ops;
@@ -74,61 +67,67 @@ struct SegOps {
 };
 static_assert(kOpInsert == 1 && kOpErase == 2, "a segment's op codes are the ops'");
 
-// Replay of the op words idx[0..cnt) (op indices in increasing order) by one
-// warp, 32 ops at a time: each op's state comes from the latest mutation
-// before it in the chunk (a ballot), else from the state carried in.
-__device__ __forceinline__ void warp_replay(const uint32_t *idx, uint32_t cnt, bool &present,
-                                            uint64_t &value, const SegOps &ops,
-                                            const void *__restrict__ vals, uint32_t vb,
-                                            void *__restrict__ vals_out,
-                                            uint32_t *__restrict__ bits_out) {
-    const int lane = threadIdx.x & 31;
-    for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
-        const bool v = c0 + lane < cnt;
-        const uint32_t w = v ? idx[c0 + lane] : 0u, i = ops.index(w);
+// Replay of the op words idx[0..cnt) (op indices in increasing order) by the
+// whole block, an op a thread at a time: an op's state comes from the latest
+// mutation before it in its warp (a ballot), else in the warps before, else
+// from the state carried in; present / value carry the key's state in every
+// thread. (By one warp, 32 ops a step, a batch of 2^22 ops on 5000 keys took 764
+// us, the other warps idle; by all 663.)
+__device__ __forceinline__ void block_replay(const uint32_t *idx, uint32_t cnt, bool &present,
+                                             uint64_t &value, const SegOps &ops,
+                                             const void *__restrict__ vals, uint32_t vb,
+                                             void *__restrict__ vals_out,
+                                             uint32_t *__restrict__ bits_out) {
+    // a warp's latest mutation: 0 none, 1 erase, 2 insert, and its value
+    __shared__ uint32_t s_kind[2][kWarpsPerBlock];
+    __shared__ uint64_t s_val[2][kWarpsPerBlock];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t buf = 0u;
+    for (uint32_t c0 = 0; c0 < cnt; c0 += kBlockThreads, buf ^= 1u) {
+        const bool v = c0 + threadIdx.x < cnt;
+        const uint32_t w = v ? idx[c0 + threadIdx.x] : 0u, i = ops.index(w);
         const uint8_t op = v ? ops.code(w) : (uint8_t)kOpFind;
-        const bool mut = v && (op == kOpInsert || op == kOpErase);  // other codes read
-        const uint64_t myval = (v && op == kOpInsert) ? load_val(vals, vb, i) : 0ull;
+        const bool mut = op == kOpInsert || op == kOpErase;  // other codes read
+        const uint64_t myval = op == kOpInsert ? load_val(vals, vb, i) : 0ull;
         const unsigned mm = __ballot_sync(kFull, mut);
-        const unsigned ins = __ballot_sync(kFull, v && op == kOpInsert);
-        // latest mutation strictly before this lane within the chunk
         const unsigned before = mm & ((1u << lane) - 1u);
-        const int src = before ? 31 - __clz(before) : -1;
-        const uint64_t srcval = shfl64(myval, src < 0 ? lane : src);
-        bool st_present = present;
-        uint64_t st_value = value;
-        if (src >= 0) {
-            st_present = (ins >> src) & 1u;
-            st_value = st_present ? srcval : 0ull;
+        const int src = before ? 31 - __clz(before) : (int)lane;
+        const uint32_t kind = mut ? (op == kOpInsert ? 2u : 1u) : 0u;
+        const uint64_t srcval = shfl64(myval, src);
+        const uint32_t srckind = __shfl_sync(kFull, kind, src);
+        if ((int)lane == (mm ? 31 - __clz(mm) : 0)) {
+            s_kind[buf][warp] = kind;
+            s_val[buf][warp] = myval;
+        }
+        __syncthreads();  // the other buffer is written in the next step
+        bool st = present;
+        uint64_t sval = value;
+#pragma unroll
+        for (uint32_t x = 0; x < (uint32_t)kWarpsPerBlock; ++x) {
+            if (x == warp) {
+                st = present;
+                sval = value;
+            }
+            const uint32_t k = s_kind[buf][x];
+            if (k == 0u) continue;
+            present = k == 2u;
+            value = s_val[buf][x];  // 0 of an erase
+        }
+        if (before) {
+            st = srckind == 2u;
+            sval = srcval;
         }
         if (v) {
-            if (vals_out) store_val(vals_out, vb, i, st_present ? st_value : 0ull);
-            if (st_present && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
-        }
-        // state after the chunk
-        if (mm) {
-            const int last = 31 - __clz(mm);
-            present = (ins >> last) & 1u;
-            const uint64_t lv = shfl64(myval, last);
-            value = present ? lv : 0ull;
+            if (vals_out) store_val(vals_out, vb, i, st ? sval : 0ull);
+            if (st && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
         }
     }
 }
 
-template <int R>
-__device__ __forceinline__ void warp_segment(const uint32_t *__restrict__ seg, uint32_t cnt,
-                                             bool &present, uint64_t &value,
-                                             const SegOps &ops,
-                                             const void *__restrict__ vals, uint32_t vb,
-                                             void *__restrict__ vals_out,
-                                             uint32_t *__restrict__ bits_out) {
+// Ascending sort of a warp's 32 * R words, the word at place lane * R + r in
+// s[r]: a bitonic network in registers, across lanes by shuffles.
+template <int R> __device__ __forceinline__ void warp_sort(uint32_t (&s)[R]) {
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t s[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t e = lane * R + r;
-        s[r] = e < cnt ? seg[e] : 0xffffffffu;
-    }
 #pragma unroll
     for (int k = 2; k <= 32 * R; k <<= 1) {
 #pragma unroll
@@ -153,6 +152,30 @@ __device__ __forceinline__ void warp_segment(const uint32_t *__restrict__ seg, u
             }
         }
     }
+}
+
+// Ops of one key, up to 32 * R of them, by one warp: the op indexes sorted in
+// registers (element e in lane e / R; merges across lanes by shuffles), then
+// each lane takes its R consecutive ops. The op codes and values of all ops
+// are read at once, so a segment costs two dependent memory round trips
+// whatever its length. (Sorted in shared memory and replayed 32 ops a step,
+// the segments of a 4096-table round took 407 us of a warp kernel of their
+// own.)
+template <int R>
+__device__ __forceinline__ void warp_segment(const uint32_t *__restrict__ seg, uint32_t cnt,
+                                             bool &present, uint64_t &value,
+                                             const SegOps &ops,
+                                             const void *__restrict__ vals, uint32_t vb,
+                                             void *__restrict__ vals_out,
+                                             uint32_t *__restrict__ bits_out) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t s[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t e = lane * R + r;
+        s[r] = e < cnt ? seg[e] : 0xffffffffu;
+    }
+    warp_sort<R>(s);
     uint8_t op[R];
     uint64_t in[R];
 #pragma unroll
@@ -195,49 +218,81 @@ __device__ __forceinline__ void warp_segment(const uint32_t *__restrict__ seg, u
     }
 }
 
+// The block's warps sort src[0..cnt) into s in runs of kSortRun words.
+constexpr uint32_t kSortRun = 128;
+__device__ __forceinline__ void sort_runs(const uint32_t *src, uint32_t cnt, uint32_t *s) {
+    constexpr int R = (int)kSortRun / 32;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t first = (threadIdx.x >> 5) * kSortRun; first < cnt; first += kWarpsPerBlock * kSortRun) {
+        uint32_t x[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint32_t e = first + r * 32u + lane;
+            x[r] = e < cnt ? src[e] : 0xffffffffu;
+        }
+        warp_sort<R>(x);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (first + lane * R + r < cnt) s[first + lane * R + r] = x[r];
+    }
+    __syncthreads();
+}
+
+// Sorted runs of w words (the last one shorter) of src[0..cnt) merged in pairs
+// into dst, each word placed by its rank in the other run (op indices are
+// distinct, so ranks are exact). By the whole block.
+__device__ __forceinline__ void merge_runs(const uint32_t *src, uint32_t *dst, uint32_t cnt, uint32_t w) {
+    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+        const uint32_t r0 = i / (2 * w) * (2 * w);
+        const uint32_t mid = r0 + w < cnt ? r0 + w : cnt;
+        const uint32_t end = r0 + 2 * w < cnt ? r0 + 2 * w : cnt;
+        const uint32_t v = src[i];
+        // rank of v in the other run (elements smaller than v)
+        uint32_t lo = i < mid ? mid : r0, hi = i < mid ? end : mid;
+        const uint32_t base = lo;
+        while (lo < hi) {
+            const uint32_t m = (lo + hi) >> 1;
+            if (src[m] < v) lo = m + 1;
+            else hi = m;
+        }
+        const uint32_t own = i < mid ? i - r0 : i - mid;
+        dst[r0 + own + (lo - base)] = v;
+    }
+    __syncthreads();
+}
+
+// Up to kMidSeg words of src sorted by the block in s (2 * kMidSeg words):
+// runs by its warps in registers, then rounds of merges. Returns where they
+// are. (One bitonic network over all words in shared memory, a barrier a
+// stage: 663 us for 2^22 ops on 5000 keys, now 457; on 1500 keys 915, now 590.
+// Runs of up to 512 words a warp spilled 200 bytes.)
+__device__ __forceinline__ uint32_t *mid_sort(const uint32_t *src, uint32_t cnt, uint32_t *s) {
+    sort_runs(src, cnt, s);
+    uint32_t *t = s + kMidSeg;
+    for (uint32_t w = kSortRun; w < cnt; w *= 2) {
+        merge_runs(s, t, cnt, w);
+        uint32_t *x = s;
+        s = t;
+        t = x;
+    }
+    return s;
+}
+
 // Sort the segment of one key with more than kWarpSeg ops by the whole block:
 // in shared memory up to kMidSeg ops, beyond that in kMidSeg chunks merged in
-// global memory, run widths doubling, each element placed by its rank in the
-// other run (op indices are distinct, so ranks are exact), ping-ponging with
-// the scratch copy at the same offsets. Returns the sorted indices.
-__device__ __forceinline__ const uint32_t *block_sort(const ApplyScratch &A, uint32_t off, uint32_t cnt,
+// global memory, run widths doubling, ping-ponging between src and dst. Returns
+// the sorted indices.
+__device__ __forceinline__ const uint32_t *block_sort(uint32_t *src, uint32_t *dst, uint32_t cnt,
                                                       uint32_t *s) {
-    const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    if (cnt <= kMidSeg) {
-        uint32_t P = 2u * kWarpSeg;
-        while (P < cnt) P <<= 1;
-        for (uint32_t j = tid; j < P; j += nt) s[j] = j < cnt ? A.seg[off + j] : 0xffffffffu;
-        __syncthreads();
-        bitonic_sort(s, P, tid, nt, [] { __syncthreads(); });
-        return s;
-    }
-    uint32_t *src = A.seg + off, *dst = A.sort_tmp + off;
+    if (cnt <= kMidSeg) return mid_sort(src, cnt, s);
     for (uint32_t c0 = 0; c0 < cnt; c0 += kMidSeg) {  // sorted chunks, in place
         const uint32_t m = cnt - c0 < kMidSeg ? cnt - c0 : kMidSeg;
-        for (uint32_t j = tid; j < kMidSeg; j += nt) s[j] = j < m ? src[c0 + j] : 0xffffffffu;
-        __syncthreads();
-        bitonic_sort(s, kMidSeg, tid, nt, [] { __syncthreads(); });
-        for (uint32_t j = tid; j < m; j += nt) src[c0 + j] = s[j];
+        const uint32_t *r = mid_sort(src + c0, m, s);
+        for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) src[c0 + j] = r[j];
         __syncthreads();
     }
     for (uint32_t w = kMidSeg; w < cnt; w *= 2) {  // merge runs of w into runs of 2w
-        for (uint32_t i = tid; i < cnt; i += nt) {
-            const uint32_t r0 = i / (2 * w) * (2 * w);
-            const uint32_t mid = r0 + w < cnt ? r0 + w : cnt;
-            const uint32_t end = r0 + 2 * w < cnt ? r0 + 2 * w : cnt;
-            const uint32_t v = src[i];
-            // rank of v in the other run (elements smaller than v)
-            uint32_t lo = i < mid ? mid : r0, hi = i < mid ? end : mid;
-            const uint32_t base = lo;
-            while (lo < hi) {
-                const uint32_t m = (lo + hi) >> 1;
-                if (src[m] < v) lo = m + 1;
-                else hi = m;
-            }
-            const uint32_t own = i < mid ? i - r0 : i - mid;
-            dst[r0 + own + (lo - base)] = v;
-        }
-        __syncthreads();
+        merge_runs(src, dst, cnt, w);
         uint32_t *t = src;
         src = dst;
         dst = t;
@@ -318,7 +373,7 @@ __global__ void __launch_bounds__(256, SET ? 4 : 3) k_repeat(
     Counters *gctr) {
     after_previous();
     constexpr int kStage = 32 * SB * kWarpsPerBlock;
-    constexpr int kSort = (int)(kMidSeg * sizeof(uint32_t));
+    constexpr int kSort = (int)(2 * kMidSeg * sizeof(uint32_t));
     __shared__ __align__(128) unsigned char s_raw[kStage > kSort ? kStage : kSort];
     unsigned char *stage = s_raw + (threadIdx.x >> 5) * (32 * SB);
     const uint32_t tid = threadIdx.x, lane = tid & 31;
@@ -353,17 +408,25 @@ __global__ void __launch_bounds__(256, SET ? 4 : 3) k_repeat(
             if (tid == 0) note_bad(A);
             continue;
         }
-        const uint32_t *sorted = block_sort(A, off, cnt, (uint32_t *)s_raw);
+        const uint32_t *sorted = block_sort(A.seg + off, A.sort_tmp + off, cnt, (uint32_t *)s_raw);
         __syncthreads();
+        // the sorted indices fill the other warps' stages
+        __shared__ __align__(128) unsigned char s_one[SB >= 64 ? 32 * SB : 16];
+        __shared__ uint64_t s_before;
+        __shared__ uint32_t s_present;
+        RepKey<KB> x;
         if (tid < 32) {
-            // the sorted indices fill the other warps' stages
-            __shared__ __align__(128) unsigned char s_one[SB >= 64 ? 32 * SB : 16];
-            const RepKey<KB> x = probe_listed<KB, SB, SET>(A, descs, ntables, d, lane == 0, s_one);
-            bool present = __shfl_sync(kFull, x.pre, 0);
-            uint64_t value = shfl64(x.pre_value, 0);
-            warp_replay(sorted, cnt, present, value, so, vals, vb, vals_out, bits_out);
-            finish(x, lane == 0 && x.k != 0, present, value);
+            x = probe_listed<KB, SB, SET>(A, descs, ntables, d, lane == 0, s_one);
+            if (tid == 0) {
+                s_present = x.pre ? 1u : 0u;
+                s_before = x.pre_value;
+            }
         }
+        __syncthreads();
+        bool present = s_present != 0u;
+        uint64_t value = s_before;
+        block_replay(sorted, cnt, present, value, so, vals, vb, vals_out, bits_out);
+        if (tid < 32) finish(x, lane == 0 && x.k != 0, present, value);
         __syncthreads();  // the sorted indices are reused by the next segment
     }
     // keys with more than kShortSeg: a warp each, kWarpTask of them probed together

@@ -73,3 +73,58 @@ def test_hot_inserts_take_no_more_than_twice_the_time_of_distinct_ones(kb, n, ho
     plain = _us(lambda: t.insert(d, v))
     assert _us(lambda: t.insert(h, v)) < 2.0 * plain
     t.close()
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("bucket_bytes", [32, 64, 128])
+def test_mixed_batches_of_long_segments(kb, bucket_bytes):
+    """Keys with 256 to 20000 ops each (replayed by a block beyond 256, sorted
+    in pieces beyond 4096), among keys with few, through a table and a set."""
+    import databases_gpu_gb300 as dg
+    rng = np.random.default_rng(kb + bucket_bytes)
+    counts = [255, 256, 257, 511, 512, 513, 2000, 4095, 4096, 4097, 8193, 20000] + [1, 2, 9] * 50
+    pool = _pool(kb, len(counts), 3)
+    k = np.repeat(pool, counts)
+    n = k.size
+    kt = k.dtype
+    t = dg.DyCuckoo(4096, key_bytes=kb, value_bytes=kb, bucket_bytes=bucket_bytes)
+    S = dg.DyCuckooSet([2048, 2048], key_bytes=kb, bucket_bytes=bucket_bytes)
+    m, ms = O.Map(), [O.Map(), O.Map()]
+    off = np.array([0, n // 3, n], np.uint32)
+    for step in range(3):
+        k = k[rng.permutation(n)]
+        v = rng.integers(1, 1 << 31, n).astype(kt)
+        ops = rng.choice(np.array([0, 1, 2, 7], np.uint8), size=n, p=[0.5, 0.2, 0.2, 0.1])
+        if step == 1:  # long runs without a mutation
+            ops[rng.random(n) < 0.995] = 0
+        out, bits = t.apply(to_dev(ops), to_dev(k), to_dev(v))
+        ov, oh = m.apply(ops, k.astype(np.uint64), v.astype(np.uint64))
+        assert np.array_equal(dg.unpack_bits(bits, n), oh), step
+        assert np.array_equal(out.cpu().numpy().view(kt).astype(np.uint64), ov), step
+        assert_same_contents(t, m, "step %d" % step)
+        out, bits = S.apply(to_dev(off), to_dev(ops), to_dev(k), to_dev(v), h_offsets=off)
+        hit, val = dg.unpack_bits(bits, n), out.cpu().numpy().view(kt).astype(np.uint64)
+        for i in range(2):
+            a, b = int(off[i]), int(off[i + 1])
+            ov, oh = ms[i].apply(ops[a:b], k[a:b].astype(np.uint64), v[a:b].astype(np.uint64))
+            assert np.array_equal(hit[a:b], oh) and np.array_equal(val[a:b], ov), (step, i)
+            assert_same_contents(S.table(i), ms[i], "step %d table %d" % (step, i))
+    t.close()
+    S.close()
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+def test_mixed_batch_of_long_segments_takes_no_more_than_three_times_distinct_keys(kb):
+    """2^22 ops on 5000 keys: each op's index is sorted and its code and value
+    read in three or four more passes than a distinct key's op; a block must not
+    replay its segment with one warp."""
+    import databases_gpu_gb300 as dg
+    n = 1 << 22
+    rng = np.random.default_rng(4)
+    pool = _pool(kb, n, 6)
+    t = dg.DyCuckoo(4 * n, key_bytes=kb, value_bytes=kb, auto_resize=False)
+    ops, v = to_dev(rng.integers(0, 3, n).astype(np.uint8)), to_dev(pool)
+    d, h = to_dev(pool), to_dev(pool[rng.integers(0, 5000, n)])
+    plain = _us(lambda: t.apply(ops, d, v))
+    assert _us(lambda: t.apply(ops, h, v)) < 3.0 * plain
+    t.close()
