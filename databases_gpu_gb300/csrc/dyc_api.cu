@@ -225,7 +225,7 @@ uint32_t chunk_nbins(uint64_t n) {
     return (uint32_t)std::max<uint64_t>(1, n / (uint64_t)dyc::kBinMean);
 }
 uint64_t bin_words(uint64_t nbins) {
-    return dyc::kBinStates + 3 * std::max<uint64_t>(nbins, 128);
+    return dyc::kBinStates + 3 * nbins;
 }
 
 // Make the scratch hold chunks of `n` ops (grow only).
@@ -505,14 +505,10 @@ bool apart(const void *a, uint64_t na, const void *b, uint64_t nb) {
 }
 
 // Whether a batch of n ops goes to the small-batch kernel (which carries no L2
-// hints), and its bins.
-bool small_batch(const dyc_table *t, uint64_t n) {
-    return n <= dyc::kBinSmallOps && t->D.l2_keep == 0u;
-}
-dyc::BinScratch small_bins(const dyc_table *t, uint64_t n) {
-    dyc::BinScratch B{};
-    carve_bins(B, t->S.bin_words, (uint32_t)((n + dyc::kBinSmallMean - 1) / dyc::kBinSmallMean));
-    return B;
+// hints).
+bool small_batch(const dyc_table *t, uint64_t n, int mode) {
+    return n <= (mode == dyc::kBinModeMixed ? dyc::kBinSmallOps : dyc::kBinSmallUpserts) &&
+           t->D.l2_keep == 0u;
 }
 
 // Find the repeated keys of a chunk.
@@ -546,18 +542,15 @@ dyc_status walk_pending(dyc_table *t, cudaStream_t s) {
 
 // A small batch: one kernel, which leaves its counters in h_ctr and places a
 // few entries without a slot on its own; more of them take a walk kernel.
-// *done is false when a bin did not fit: nothing has been done then.
 dyc_status bins_small(dyc_table *t, int mode, const uint8_t *ops, const void *keys,
                       const void *vals, void *vals_out, uint32_t *bits_out, uint64_t n,
-                      uint32_t flags, cudaStream_t s, bool *done) {
-    const cudaError_t e = KB_CALL(t, bin_small, ctx(t, s), t->D, t->sb, t->S, small_bins(t, n), mode,
-                                  ops, keys, vals, (uint32_t)t->vb, vals_out, bits_out, n, flags,
-                                  t->d_ctr, t->h_ctr);
+                      uint32_t flags, cudaStream_t s) {
+    const cudaError_t e = KB_CALL(t, bin_small, ctx(t, s), t->D, t->sb, t->S, mode, ops, keys, vals,
+                                  (uint32_t)t->vb, vals_out, bits_out, n, flags, t->d_ctr, t->h_ctr);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "bin kernel: %s", cudaGetErrorString(e));
     CK(cudaStreamSynchronize(s));
     TRY(check_counters(t));
-    *done = t->h_ctr->left == 0;
-    if (!*done || t->h_ctr->pending == 0) return DYC_OK;
+    if (t->h_ctr->pending == 0) return DYC_OK;
     // the small kernel's ticket is spent
     CK(cudaMemsetAsync(&t->d_ctr->ticket, 0, sizeof(unsigned long long), s));
     return walk_pending(t, s);
@@ -590,11 +583,10 @@ dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64
                         uint32_t flags, cudaStream_t s) {
     const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
     const bool new_keys = (flags & DYC_FLAG_NEW_KEYS) != 0;
-    if (use_dedup && small_batch(t, n)) {
-        bool done = false;
+    if (use_dedup && small_batch(t, n, dyc::kBinModeInsert)) {
         TRY(bins_small(t, dyc::kBinModeInsert, nullptr, keys, vals, nullptr, nullptr, n,
-                       new_keys ? (uint32_t)dyc::kBinNewKeys : 0u, s, &done));
-        if (done) return insert_finish(t, s);
+                       new_keys ? (uint32_t)dyc::kBinNewKeys : 0u, s));
+        return insert_finish(t, s);
     }
     if (use_dedup)
         TRY(bins_group(t, chunk_bins(t, n, t->S.winbits), dyc::ApplyScratch{}, dyc::kBinModeInsert,
@@ -612,10 +604,9 @@ dyc_status insert_chunk(dyc_table *t, const void *keys, const void *vals, uint64
 dyc_status erase_chunk(dyc_table *t, const void *keys, uint64_t n, uint32_t *bits, void *old,
                        uint32_t flags, cudaStream_t s) {
     const bool use_dedup = !(flags & DYC_FLAG_UNIQUE) && n > 1;
-    bool done = false;
-    if (use_dedup && small_batch(t, n))
-        TRY(bins_small(t, dyc::kBinModeErase, nullptr, keys, nullptr, old, bits, n, 0u, s, &done));
-    if (!done) {
+    if (use_dedup && small_batch(t, n, dyc::kBinModeErase)) {
+        TRY(bins_small(t, dyc::kBinModeErase, nullptr, keys, nullptr, old, bits, n, 0u, s));
+    } else {
         if (use_dedup)
             TRY(bins_group(t, chunk_bins(t, n, t->S.winbits), dyc::ApplyScratch{},
                            dyc::kBinModeErase, nullptr, keys, nullptr, n, s));
@@ -1258,7 +1249,7 @@ dyc_status dyc_erase_host(dyc_table *t, const void *h_keys, uint64_t n,
         CK(cudaMemcpyAsync(dk, (const char *)h_keys + off * t->kb, m * t->kb, cudaMemcpyHostToDevice, t->io_stream));
         uint64_t got = 0;
         // the erase kernel stores whole words of bits (a small batch's ORs them)
-        uint32_t *in_place = view && !small_batch(t, m) ? view + off / 32 : nullptr;
+        uint32_t *in_place = view && !small_batch(t, m, dyc::kBinModeErase) ? view + off / 32 : nullptr;
         uint32_t *bits = in_place ? in_place : h_erased_bits_out ? db : nullptr;
         TRY(dyc_erase(t, dk, m, bits, &got, 0, t->io_stream));
         total += got;
@@ -1466,15 +1457,14 @@ dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const
     // every block of the small-batch kernel reads all keys while others write
     // results, so results written over the keys take the split kernels, where
     // an op's result is stored after the last read of its key
-    bool done = small_batch(t, n) && apart(keys, n * t->kb, vals_out, vals_out ? n * t->vb : 0);
-    if (done && before) {
-        TRY(bins_small(t, dyc::kBinModeCount, ops, keys, vals, nullptr, nullptr, n, 0u, s, &done));
-        if (done) TRY(policy(t->h_ctr->nins, t->h_ctr->erased));
-    }
-    if (done)
+    if (small_batch(t, n, dyc::kBinModeMixed) && apart(keys, n * t->kb, vals_out, vals_out ? n * t->vb : 0)) {
+        if (before) {
+            TRY(bins_small(t, dyc::kBinModeCount, ops, keys, vals, nullptr, nullptr, n, 0u, s));
+            TRY(policy(t->h_ctr->nins, t->h_ctr->erased));
+        }
         TRY(bins_small(t, dyc::kBinModeMixed, ops, keys, vals, vals_out, bits_out, n,
-                       full ? (uint32_t)dyc::kBinSkipEqual : 0u, s, &done));
-    if (!done) {
+                       full ? (uint32_t)dyc::kBinSkipEqual : 0u, s));
+    } else {
         if (before && n > dyc::kBinSmallOps) {
             TRY(reset_call_counters(t, s));
             const cudaError_t e = KB_CALL(t, count_inserts, ctx(t, s), ops, n, &t->d_ctr->nins);

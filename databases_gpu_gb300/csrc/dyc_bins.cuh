@@ -20,14 +20,15 @@
 // words and bits at random places cost more than that (312 us against 47 + 39
 // + 187 for 2^22 mixed ops).
 //
-// Up to kBinSmallOps ops run as one kernel (k_bin_small): every block reads the
-// whole batch, keeps its bin's ops and resolves them itself, and the last block
-// writes the counters to the host. A mixed batch of 4096 ops took ten kernels,
-// four memsets and two copies: 97 -> 33 us a call.
+// A small batch runs as one kernel (k_bin_small): every block reads the whole
+// batch, keeps its bin's ops and resolves them itself, and the last block writes
+// the counters to the host. A mixed batch of 4096 ops took ten kernels, four
+// memsets and two copies: 97 -> 46 us a call on a table of 2^24 keys.
 //
 // A bin with more ops than its capacity (few keys, each repeated hundreds of
 // times, or a skewed batch's most popular ones) gets a second, exact set of
-// records, which its block streams (group_hot).
+// records, which its block streams (group_hot); in a small batch its block reads
+// the batch again.
 #pragma once
 
 #include "dyc_apply.cuh"
@@ -38,8 +39,6 @@ constexpr int kSmallThreads = 512;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallR = kSmallCap / kSmallThreads;  // records per thread (k_bin_small)
 constexpr int kSmallTab = 2 * kSmallCap;            // cells of a bin's key table
-constexpr int kSmallBins = 96;
-static_assert(kBinSmallOps / kBinSmallMean < kSmallBins, "a small batch's bins are counted in one block");
 constexpr int kSplitThreads = 512;
 constexpr uint32_t kSplitBins = 4096;               // bins counted in shared memory (k_bin_scatter)
 constexpr int kGroupThreads = 512;
@@ -725,6 +724,154 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     }
 }
 
+// A lane's key and what the probes of its two buckets found.
+template <int KB> struct RepKey {
+    typename SlotT<KB>::K k;
+    uint32_t tb, hk;
+    char *p1, *p2;
+    KvOut r1, r2;
+    bool found1, found2, pre;
+    uint64_t pre_value;
+};
+
+// Key k of every lane with act in table D (warp-collective).
+template <int KB, int SB>
+__device__ __forceinline__ RepKey<KB> probe_key(const Desc &D, typename SlotT<KB>::K k, bool act,
+                                                unsigned char *stage) {
+    using Gm = Geo<KB, SB>;
+    RepKey<KB> x;
+    x.k = k;
+    x.tb = 0u;
+    x.hk = fold(k);
+    const Pair p = pair_of(x.hk, D.d);
+    x.p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, x.hk));
+    x.p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, x.hk));
+    x.r1 = place_probe<KB, SB, false>(x.p1, k, act, p.first, D.d, stage);
+    x.found1 = act && x.r1.match >= 0;
+    // the second bucket: where the key or an empty slot may be there
+    const bool check2 = act && !x.found1 && ((!Gm::kMeta || x.r1.overflow) || x.r1.empty == 0u);
+    x.r2 = KvOut{-1, 0ull, false, 0u};
+    if (__any_sync(kFull, check2))
+        x.r2 = place_probe<KB, SB, false>(x.p2, k, check2, p.second, D.d, stage);
+    x.found2 = check2 && x.r2.match >= 0;
+    x.pre = x.found1 || x.found2;
+    x.pre_value = x.found1 ? x.r1.value : (x.found2 ? x.r2.value : 0ull);
+    return x;
+}
+
+// An op word of a segment (SegOps::wide: a plain index).
+struct SegOps {
+    const uint8_t *ops;
+    uint32_t wide;
+    __device__ __forceinline__ uint32_t index(uint32_t w) const { return wide ? w : w >> 2; }
+    __device__ __forceinline__ uint8_t code(uint32_t w) const {
+        return wide ? ops[w] : (uint8_t)(w & 3u);  // 1 insert, 2 erase; others read
+    }
+};
+static_assert(kOpInsert == 1 && kOpErase == 2, "a segment's op codes are the ops'");
+
+// Replay of the op words idx[0..cnt) (op indices in increasing order) by the
+// whole block, an op a thread at a time: an op's state comes from the latest
+// mutation before it in its warp (a ballot), else in the warps before, else
+// from the state carried in; present / value carry the key's state in every
+// thread. (By one warp, 32 ops a step, a batch of 2^22 ops on 5000 keys took 764
+// us, the other warps idle; by all 663.)
+template <int THREADS, bool WRITE>
+__device__ __forceinline__ void block_replay(const uint32_t *idx, uint32_t cnt, bool &present,
+                                             uint64_t &value, const SegOps &ops,
+                                             const void *__restrict__ vals, uint32_t vb,
+                                             void *__restrict__ vals_out,
+                                             uint32_t *__restrict__ bits_out) {
+    // a warp's latest mutation: 0 none, 1 erase, 2 insert, and its value
+    constexpr uint32_t kWarps = THREADS / 32;
+    __shared__ uint32_t s_kind[2][kWarps];
+    __shared__ uint64_t s_val[2][kWarps];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t buf = 0u;
+    for (uint32_t c0 = 0; c0 < cnt; c0 += THREADS, buf ^= 1u) {
+        const bool v = c0 + threadIdx.x < cnt;
+        const uint32_t w = v ? idx[c0 + threadIdx.x] : 0u, i = ops.index(w);
+        const uint8_t op = v ? ops.code(w) : (uint8_t)kOpFind;
+        const bool mut = op == kOpInsert || op == kOpErase;  // other codes read
+        const uint64_t myval = op == kOpInsert ? load_val(vals, vb, i) : 0ull;
+        const unsigned mm = __ballot_sync(kFull, mut);
+        const unsigned before = mm & ((1u << lane) - 1u);
+        const int src = before ? 31 - __clz(before) : (int)lane;
+        const uint32_t kind = mut ? (op == kOpInsert ? 2u : 1u) : 0u;
+        const uint64_t srcval = shfl64(myval, src);
+        const uint32_t srckind = __shfl_sync(kFull, kind, src);
+        if ((int)lane == (mm ? 31 - __clz(mm) : 0)) {
+            s_kind[buf][warp] = kind;
+            s_val[buf][warp] = myval;
+        }
+        __syncthreads();  // the other buffer is written in the next step
+        bool st = present;
+        uint64_t sval = value;
+#pragma unroll
+        for (uint32_t x = 0; x < kWarps; ++x) {
+            if (x == warp) {
+                st = present;
+                sval = value;
+            }
+            const uint32_t k = s_kind[buf][x];
+            if (k == 0u) continue;
+            present = k == 2u;
+            value = s_val[buf][x];  // 0 of an erase
+        }
+        if (before) {
+            st = srckind == 2u;
+            sval = srcval;
+        }
+        if (WRITE && v) {
+            if (vals_out) store_val(vals_out, vb, i, st ? sval : 0ull);
+            if (st && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
+        }
+    }
+}
+
+struct RepCounts {
+    uint32_t ins = 0, upd = 0, del = 0;
+};
+
+// The final state of a lane's key (act) to the table; entries without a slot
+// go to list_a. Warp-collective.
+template <int KB, int SB>
+__device__ __forceinline__ void mutate_listed(const RepKey<KB> &x, bool up, bool er, uint64_t value,
+                                              void *list_a, uint64_t list_cap, Counters *gctr,
+                                              RepCounts &n) {
+    using T = SlotT<KB>;
+    typename T::S e = T::empty();
+    bool pend = false;
+    if (up) {
+        e = T::make(x.k, value);
+        if (x.found1) {
+            T::store(slot_ptr<KB, SB>(x.p1, x.r1.match), e);
+            ++n.upd;
+        } else if (x.found2) {
+            T::store(slot_ptr<KB, SB>(x.p2, x.r2.match), e);
+            ++n.upd;
+        } else {
+            bool ok = claim_empty<KB, SB>(x.p1, x.r1.empty, e);
+            if (!ok && x.r2.empty) {
+                mark_overflow<KB, SB>(x.p1, x.hk);
+                ok = claim_empty<KB, SB>(x.p2, x.r2.empty, e);
+            }
+            if (ok) ++n.ins;
+            else pend = true;
+        }
+    } else if (er) {
+        T::store(x.found1 ? slot_ptr<KB, SB>(x.p1, x.r1.match) : slot_ptr<KB, SB>(x.p2, x.r2.match),
+                 T::empty());
+        ++n.del;
+    }
+    __syncwarp();
+    const unsigned long long at = agg_inc(&gctr->pending, pend);
+    if (pend) {
+        if (at < list_cap) ((typename T::S *)list_a)[at] = e;
+        else atomicAdd(&gctr->spill, 1ull);
+    }
+}
+
 // Ascending sort of s[0..c) by one warp (mirrored bitonic merges: every
 // compare is ascending, so the places past c, read as larger than any word,
 // need no storage).
@@ -752,7 +899,7 @@ __device__ __forceinline__ void warp_sort_words(uint32_t *s, uint32_t c) {
 }
 
 // Results of the sorted op words w[0..c) of one key by one warp, 32 ops a step
-// (as warp_replay): present / value carry the key's state.
+// (as block_replay): present / value carry the key's state.
 template <bool WRITE>
 __device__ __forceinline__ void warp_replay_words(const uint32_t *w, uint32_t c, bool &present,
                                                   uint64_t &value, const void *__restrict__ vals,
@@ -788,19 +935,277 @@ __device__ __forceinline__ void warp_replay_words(const uint32_t *w, uint32_t c,
 }
 
 constexpr uint32_t kBinShort = 8;   // ops of one key replayed by one lane
+constexpr uint32_t kSmallLong = 512;  // most ops of one key replayed by one warp (k_bin_small)
 constexpr uint32_t kTailWalk = 64;  // pending entries the last block places itself
 
 template <int KB, int SB> struct BinSmem {
-    alignas(128) unsigned char stage[kSmallWarps][32 * SB];  // the key table before the probes
+    alignas(128) unsigned char stage[kSmallWarps][32 * SB];  // between the probes: tables, bitmaps
     typename SlotT<KB>::K key[kSmallCap];
     uint32_t word[kSmallCap];
-    uint32_t cnt[kSmallCap];  // per first op of a key: ops, then winner word or count | place << 16
-    uint32_t seg[kSmallCap];
-    uint16_t multi[kSmallCap / 2];
-    uint32_t nseg, nmulti, last;
-    uint32_t bins[kSmallBins];  // ops per bin of the batch
+    uint32_t cnt[kSmallCap];  // per first op of a key: the word that counts; mixed: ops | place in seg << 16
+    uint16_t multi[kSmallCap];  // keys with several ops, and those of more than kSmallLong
+    uint16_t longs[kBinSmallOps / kSmallLong];  // each has more ops than that
+    uint64_t part_mask[72], part[72];  // parts of a bin that went over (each split adds one)
+    uint32_t m, nseg, nmulti, nlong, ndist, over, top, last;
+    uint32_t warp_sum[kSmallWarps];
     unsigned long long sum[6];
+    uint32_t seg[kSmallCap];  // the last member: mixed batches of more ops get a word for each
 };
+
+// Bytes of a small batch's BinSmem.
+template <int KB, int SB> constexpr size_t bin_smem(int mode, uint64_t n) {
+    return sizeof(BinSmem<KB, SB>) +
+           (mode >= kBinModeMixed && n > (uint64_t)kSmallCap ? (n - kSmallCap) * sizeof(uint32_t) : 0);
+}
+
+// Key k's cell among the cells `cell` (index + 1 of an op of the cell's key);
+// claimed for op i when it has none yet (claim). A probe of kSmallProbe cells
+// (in a table half full they are one or two) gives its part up (M.over), so
+// the cells never run out.
+constexpr uint32_t kSmallProbe = 256;
+template <int KB, int SB>
+__device__ __forceinline__ uint32_t small_cell(BinSmem<KB, SB> &M, uint32_t *cell, const void *keys,
+                                               typename SlotT<KB>::K k, uint32_t i, bool claim) {
+    static_assert(kSmallTab == 1 << 11, "bin_cell takes 11 bits");
+    uint32_t h = bin_cell<11>(bin_tag(k));
+    for (uint32_t p = 0; p < kSmallProbe; ++p) {
+        uint32_t f = *(volatile uint32_t *)&cell[h];
+        if (f == 0u) {
+            if (!claim) return h;
+            f = atomicCAS(&cell[h], 0u, i + 1u);
+            if (f == 0u) return h;
+        }
+        if (load_key<KB>(keys, f - 1u) == k) return h;
+        h = (h + 1u) & (kSmallTab - 1);
+    }
+    *(volatile uint32_t *)&M.over = 1u;
+    return h;
+}
+
+// f(key, index, bin's own) for the ops of a batch, 32 to a warp, until stop();
+// down: from the last op to the first.
+template <int KB, class F, class Stop>
+__device__ __forceinline__ void stream_batch(const void *keys, uint32_t n, bool down, Stop &&stop, F &&f) {
+    using K = typename SlotT<KB>::K;
+    constexpr int kLoad = 8;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t base = threadIdx.x & ~31u; base < n; base += kLoad * kSmallThreads) {
+        if (stop()) break;
+        K k[kLoad];
+#pragma unroll
+        for (int x = 0; x < kLoad; ++x) {
+            const uint32_t i = base + x * kSmallThreads + lane;
+            k[x] = i < n ? load_key<KB>(keys, down ? n - 1u - i : i) : (K)0;
+        }
+#pragma unroll
+        for (int x = 0; x < kLoad; ++x) {
+            const uint32_t i = base + x * kSmallThreads + lane;
+            f(k[x], down ? n - 1u - i : i, i < n);
+        }
+    }
+}
+
+// After the ops of the next part (top of M.part) of a bin have their cells: the
+// places of a thread's used cells among the part's keys. False, and the part
+// split in two by one more bit of its keys, when they are more than kSmallCap.
+constexpr int kSmallCells = kSmallTab / kSmallThreads;
+template <int KB, int SB>
+__device__ __forceinline__ bool end_part(BinSmem<KB, SB> &M, const uint32_t *cell, uint32_t (&d)[kSmallCells]) {
+    const uint32_t lane = threadIdx.x & 31;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kSmallCells; ++q) {
+        const unsigned m = __ballot_sync(kFull, cell[q * kSmallThreads + threadIdx.x] != 0u);
+        uint32_t at = 0u;
+        if (lane == 0 && m) at = atomicAdd(&M.ndist, (uint32_t)__popc(m));
+        d[q] = __shfl_sync(kFull, at, 0) + __popc(m & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    const bool over = M.over != 0u || M.ndist > (uint32_t)kSmallCap;
+    if (threadIdx.x == 0) {
+        const uint32_t top = M.top;
+        if (over) {
+            const uint64_t mask = M.part_mask[top - 1];
+            M.part[top] = M.part[top - 1] | (mask + 1ull);
+            M.part_mask[top - 1] = M.part_mask[top] = 2ull * mask + 1ull;
+            M.top = top + 1u;
+        } else {
+            M.top = top - 1u;
+        }
+    }
+    return !over;
+}
+
+// An insert or erase batch's bin of more than kSmallCap ops (a popular key, or a
+// few): the keys of its next part to M.key, streamed from the batch again, and
+// the op of each that counts to M.word. Returns their number (0: the part was
+// split). An insert reads the batch from its end: the op met first is then
+// mostly the one that counts, and the others of a popular key only read its
+// cell. n_sup: ops that do not count; n_rej: key-0 ops in [own0, own1), an
+// empty range once they are counted.
+template <int KB, int SB, int MODE>
+__device__ __noinline__ uint32_t gather_keys(BinSmem<KB, SB> &M, const void *keys, uint32_t n,
+                                                uint32_t own0, uint32_t &own1, uint32_t &n_sup,
+                                                uint32_t &n_rej) {
+    using K = typename SlotT<KB>::K;
+    const uint32_t tid = threadIdx.x, bin = blockIdx.x, nbins = gridDim.x;
+    uint32_t *cell = reinterpret_cast<uint32_t *>(M.stage);  // index + 1 of the op that counts so far
+    const uint64_t mask = M.part_mask[M.top - 1], part = M.part[M.top - 1];
+    for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kSmallThreads) cell[c] = 0u;
+    if (tid == 0) M.ndist = M.over = 0u;
+    __syncthreads();
+    uint32_t seen = 0u, rej = 0u;
+    stream_batch<KB>(
+        keys, n, MODE == kBinModeInsert, [&] { return *(volatile uint32_t *)&M.over != 0u; },
+        [&](K k, uint32_t i, bool here) {
+            if (k == 0) {
+                if (here && i >= own0 && i < own1) ++rej;
+                return;
+            }
+            if (bin_of<KB>(k, nbins) != bin) return;
+            if (mask && (part_bits((uint64_t)k) & mask) != part) return;
+            ++seen;
+            const uint32_t h = small_cell<KB, SB>(M, cell, keys, k, i, true);
+            const uint32_t f = *(volatile uint32_t *)&cell[h];
+            if (MODE == kBinModeInsert && f < i + 1u) atomicMax(&cell[h], i + 1u);
+            if (MODE == kBinModeErase && f > i + 1u) atomicMin(&cell[h], i + 1u);
+        });
+    uint32_t d[kSmallCells];
+    const bool done = end_part<KB, SB>(M, cell, d);
+    if (done) {
+        n_sup += seen;
+        n_rej += rej;
+        own1 = own0;
+#pragma unroll
+        for (int q = 0; q < kSmallCells; ++q) {
+            const uint32_t f = cell[q * kSmallThreads + tid];
+            if (f == 0u) continue;
+            M.key[d[q]] = load_key<KB>(keys, f - 1u);
+            M.word[d[q]] = (f - 1u) << 2;
+            --n_sup;
+        }
+    }
+    const uint32_t m = done ? M.ndist : 0u;
+    __syncthreads();
+    return m;
+}
+
+// The same of a mixed batch: the keys of the next part to M.key with their ops,
+// M.cnt the ops | place in seg << 16, M.word the only op of a key with one; the
+// op words of the others in seg, in no order. Returns the number of keys (0:
+// the part was split).
+template <int KB, int SB>
+__device__ __noinline__ uint32_t gather_part(BinSmem<KB, SB> &M, const void *keys, const uint8_t *ops,
+                                             uint32_t n) {
+    using K = typename SlotT<KB>::K;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, bin = blockIdx.x, nbins = gridDim.x;
+    // a cell's ops; then the next place in seg (kNone: its key has one op)
+    constexpr uint32_t kNone = 0xffffffffu;
+    uint32_t *cell = reinterpret_cast<uint32_t *>(M.stage), *cnt = cell + kSmallTab;
+    static_assert(sizeof(M.stage) >= 2 * kSmallTab * sizeof(uint32_t), "two tables fit the stage");
+    const uint64_t mask = M.part_mask[M.top - 1], part = M.part[M.top - 1];
+    for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kSmallThreads) cell[c] = cnt[c] = 0u;
+    if (tid == 0) M.nseg = M.nmulti = M.nlong = M.ndist = M.over = 0u;
+    __syncthreads();
+    auto mine = [&](K k) {
+        return k != 0 && bin_of<KB>(k, nbins) == bin && (!mask || (part_bits((uint64_t)k) & mask) == part);
+    };
+    stream_batch<KB>(
+        keys, n, false, [&] { return __any_sync(kFull, *(volatile uint32_t *)&M.over != 0u) != 0; },
+        [&](K k, uint32_t i, bool) {
+            const bool own = mine(k);
+            if (!__any_sync(kFull, own)) return;
+            const uint32_t h = own ? small_cell<KB, SB>(M, cell, keys, k, i, true) : kNone;
+            __syncwarp();
+            const unsigned peers = __match_any_sync(kFull, h);
+            if (own && __ffs(peers) - 1 == (int)lane) atomicAdd(&cnt[h], (uint32_t)__popc(peers));
+        });
+    uint32_t d[kSmallCells];
+    const bool done = end_part<KB, SB>(M, cell, d);
+    if (done) {
+#pragma unroll
+        for (int q = 0; q < kSmallCells; ++q) {
+            const uint32_t c = q * kSmallThreads + tid, k = cnt[c];
+            if (cell[c] == 0u) continue;
+            const uint32_t i = cell[c] - 1u;
+            M.key[d[q]] = load_key<KB>(keys, i);
+            uint32_t at = 0u;
+            if (k == 1u) {
+                M.word[d[q]] = op_word(i, ops[i]);
+                cnt[c] = kNone;
+            } else {
+                at = atomicAdd(&M.nseg, k);
+                if (k > kSmallLong) M.longs[atomicAdd(&M.nlong, 1u)] = (uint16_t)d[q];
+                else M.multi[atomicAdd(&M.nmulti, 1u)] = (uint16_t)d[q];
+                cnt[c] = at;
+            }
+            M.cnt[d[q]] = k | at << 16;
+        }
+    }
+    const uint32_t m = done ? M.ndist : 0u;
+    __syncthreads();
+    if (M.nseg != 0u)
+        stream_batch<KB>(
+            keys, n, false, [] { return false; },
+            [&](K k, uint32_t i, bool) {
+                const bool own = mine(k);
+                if (!__any_sync(kFull, own)) return;
+                const uint32_t h = own ? small_cell<KB, SB>(M, cell, keys, k, i, false) : 0u;
+                const bool put = own && *(volatile uint32_t *)&cnt[h] != kNone;
+                const uint32_t w = put ? op_word(i, ops[i]) : 0u;
+                __syncwarp();
+                const unsigned peers = __match_any_sync(kFull, put ? h : kNone);
+                const int lead = __ffs(peers) - 1;
+                uint32_t at = 0u;
+                if (put && lead == (int)lane) at = atomicAdd(&cnt[h], (uint32_t)__popc(peers));
+                at = __shfl_sync(kFull, at, lead) + __popc(peers & ((1u << lane) - 1u));
+                if (put) M.seg[at] = w;
+            });
+    __syncthreads();
+    return m;
+}
+
+// The c op words of one key at M.seg[off] into index order by the whole block: a bit per op and two for its code, then the words
+// again from the bits. (Bitonic networks of that length take 100 barriers.)
+template <int KB, int SB>
+__device__ __noinline__ void sort_long(BinSmem<KB, SB> &M, uint32_t off, uint32_t c) {
+    constexpr uint32_t kPer = 2, kWords = kPer * kSmallThreads;
+    static_assert(kWords * 32u >= kBinSmallOps, "a bit for every op");
+    static_assert(sizeof(M.stage) >= 3 * kWords * sizeof(uint32_t), "three bitmaps fit the stage");
+    uint32_t *bits = reinterpret_cast<uint32_t *>(M.stage);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    for (uint32_t w = tid; w < 3u * kWords; w += kSmallThreads) bits[w] = 0u;
+    __syncthreads();
+    for (uint32_t j = tid; j < c; j += kSmallThreads) {
+        const uint32_t w = M.seg[off + j], i = w >> 2, b = 1u << (i & 31u);
+        atomicOr(&bits[i >> 5], b);
+        if (w & 1u) atomicOr(&bits[kWords + (i >> 5)], b);
+        if (w & 2u) atomicOr(&bits[2u * kWords + (i >> 5)], b);
+    }
+    __syncthreads();
+    uint32_t own = 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) own += __popc(bits[tid * kPer + q]);
+    uint32_t incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) M.warp_sum[warp] = incl;
+    __syncthreads();
+    uint32_t at = off + incl - own;
+    for (uint32_t w = 0; w < warp; ++w) at += M.warp_sum[w];
+    for (uint32_t q = 0; q < kPer; ++q) {
+        const uint32_t x = tid * kPer + q, one = bits[kWords + x], two = bits[2u * kWords + x];
+        for (uint32_t b = bits[x]; b; b &= b - 1u) {
+            const uint32_t p = __ffs(b) - 1;
+            M.seg[at++] = (x * 32u + p) << 2 | ((one >> p) & 1u) | ((two >> p) & 1u) << 1;
+        }
+    }
+    __syncthreads();
+}
 
 // Place the pending entries of list_a (a few) by eviction walks, from the last
 // block of a small batch's kernel.
@@ -830,14 +1235,16 @@ __device__ __forceinline__ void tail_walk(const Desc &D, const Scratch &S, Count
 // A small batch in one kernel: every block reads the whole batch, keeps the ops
 // of its bin, finds the repeated keys among them in shared memory and probes
 // the table; the last block to finish places the few entries left without a
-// slot and writes the counters to the host.
+// slot and writes the counters to the host. A bin of more than kSmallCap ops is
+// taken by its block as well, in parts of up to kSmallCap keys (gather_keys,
+// gather_part). It used to leave the batch to the split kernels, after a wait:
+// 8000 inserts on 7 keys 72 -> 41 us, 16000 mixed ops on 7 keys 236 -> 91.
 template <int KB, int SB, int MODE>
-__global__ void __launch_bounds__(kSmallThreads) k_bin_small(
+__global__ void __launch_bounds__(kSmallThreads, 1) k_bin_small(
     const __grid_constant__ Desc D, const __grid_constant__ Scratch S,
-    const __grid_constant__ BinScratch B, const uint8_t *__restrict__ ops,
-    const void *__restrict__ keys, const void *__restrict__ vals, uint32_t vb,
-    void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, uint64_t n, uint32_t flags,
-    Counters *ctr, Counters *h_ctr) {
+    const uint8_t *__restrict__ ops, const void *__restrict__ keys, const void *__restrict__ vals,
+    uint32_t vb, void *__restrict__ vals_out, uint32_t *__restrict__ bits_out, uint64_t n,
+    uint32_t flags, Counters *ctr, Counters *h_ctr) {
     using T = SlotT<KB>;
     using K = typename T::K;
     using Sl = typename T::S;
@@ -845,277 +1252,181 @@ __global__ void __launch_bounds__(kSmallThreads) k_bin_small(
     extern __shared__ __align__(128) unsigned char s_raw[];
     BinSmem<KB, SB> &M = *reinterpret_cast<BinSmem<KB, SB> *>(s_raw);
     uint32_t *tab = reinterpret_cast<uint32_t *>(M.stage);
-    static_assert(kSmallTab == 1 << 11, "bin_cell takes 11 bits");
-    static_assert(sizeof(M.stage) >= kSmallTab * sizeof(uint32_t), "the key table fits the stage");
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     unsigned char *stage = M.stage[tid >> 5];
     const uint32_t bin = blockIdx.x;
     uint32_t n_ins = 0, n_upd = 0, n_del = 0, n_sup = 0, n_rej = 0;
 
-    // the bin's records
+    const uint32_t own0 = (uint32_t)(((uint64_t)bin * n) / gridDim.x);
+    uint32_t own1 = (uint32_t)(((uint64_t)(bin + 1) * n) / gridDim.x);
+    if (tid == 0) {
+        M.m = M.nseg = M.nmulti = M.nlong = 0u;
+        M.top = 1u;
+        M.part_mask[0] = M.part[0] = 0ull;
+    }
+    if (tid < 6) M.sum[tid] = 0ull;
+    // the bin's ops listed, as long as they are at most kSmallCap
     for (uint32_t c = tid; c < (uint32_t)kSmallTab; c += kSmallThreads) tab[c] = 0u;
     for (uint32_t c = tid; c < (uint32_t)kSmallCap; c += kSmallThreads)
         M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
-    if (tid == 0) M.nseg = M.nmulti = 0u;
-    if (tid < (uint32_t)kSmallBins) M.bins[tid] = 0u;
-    if (tid < 6) M.sum[tid] = 0ull;
     __syncthreads();
-    uint32_t m;
-    {
-        const uint32_t own0 = (uint32_t)(((uint64_t)bin * n) / gridDim.x);
-        const uint32_t own1 = (uint32_t)(((uint64_t)(bin + 1) * n) / gridDim.x);
-#pragma unroll 8
-        for (uint64_t i = tid; i < n; i += kSmallThreads) {
-            const K k = load_key<KB>(keys, i);
+    stream_batch<KB>(
+        keys, (uint32_t)n, false,
+        [&] { return MODE < kBinModeMixed && *(volatile uint32_t *)&M.m > (uint32_t)kSmallCap; },
+        [&](K k, uint32_t i, bool here) {
             if (k == 0) {  // belongs to no bin: one block answers it
-                if (i >= own0 && i < own1) {
-                    ++n_rej;
-                    if ((MODE == kBinModeMixed) && vals_out) store_val(vals_out, vb, i, 0ull);
-                }
-            } else {
-                const uint32_t b = bin_of<KB>(k, gridDim.x);
-                const uint32_t r = atomicAdd(&M.bins[b], 1u);
-                if (b == bin && r < (uint32_t)kSmallCap) {
-                    M.key[r] = k;
-                    M.word[r] = (uint32_t)i << 2;
-                }
+                if (!here || i < own0 || i >= own1) return;
+                ++n_rej;
+                if (MODE == kBinModeMixed && vals_out) store_val(vals_out, vb, i, 0ull);
+                return;
             }
-        }
-        __syncthreads();
-        m = M.bins[bin];
-        if (MODE >= kBinModeMixed && m <= (uint32_t)kSmallCap)
-            for (uint32_t r = tid; r < m; r += kSmallThreads)
-                M.word[r] = op_word(M.word[r] >> 2, ops[M.word[r] >> 2]);
+            // a popular key's ops stop counting here once the bin is full
+            if (bin_of<KB>(k, gridDim.x) != bin || *(volatile uint32_t *)&M.m > (uint32_t)kSmallCap) return;
+            const uint32_t r = atomicAdd(&M.m, 1u);
+            if (r < (uint32_t)kSmallCap) {
+                M.key[r] = k;
+                M.word[r] = i << 2;
+            }
+        });
+    __syncthreads();
+    const bool fits = M.m <= (uint32_t)kSmallCap;
+    uint32_t m = fits ? M.m : 0u;  // keys or ops listed
+    if constexpr (MODE >= kBinModeMixed) {
+        for (uint32_t r = tid; r < m; r += kSmallThreads)
+            M.word[r] = op_word(M.word[r] >> 2, ops[M.word[r] >> 2]);
+    } else if (!fits) {
+        n_rej = 0u;  // counted by gather_keys
     }
     __syncthreads();
     // so far the batch was read and key-0 results written, which the clear
     // before this kernel does not touch; its grid waited for the ones before it
     after_previous();
-    // every block counted every bin: all agree to leave a batch with a bin
-    // that does not fit to the split kernels, before anything is written
-    if (__syncthreads_or(tid < gridDim.x && M.bins[tid] > (uint32_t)kSmallCap)) {
-        if (bin == 0 && tid == 0) ctr->left = 1ull;
-        m = 0u;
-        n_rej = 0u;
-    }
 
-    // group: each record finds its key's first record (lead)
-    K key[kSmallR];
-    uint32_t word[kSmallR], lead[kSmallR], rank[kSmallR];
-#pragma unroll
-    for (int q = 0; q < kSmallR; ++q) {
-        const uint32_t r = q * kSmallThreads + tid;
-        lead[q] = rank[q] = 0u;
-        word[q] = 0u;
-        key[q] = 0;
-        if (r >= m) continue;
-        key[q] = M.key[r];
-        word[q] = M.word[r];
-        uint32_t h = bin_cell<11>(bin_tag(key[q]));
-        // at most kSmallCap of the kSmallTab cells are taken: the probe ends
-        while (true) {
-            const uint32_t old = atomicCAS(&tab[h], 0u, r + 1u);
-            if (old == 0u) {
-                lead[q] = r;
-                break;
-            }
-            if (M.key[old - 1u] == key[q]) {
-                lead[q] = old - 1u;
-                break;
-            }
-            h = (h + 1u) & (kSmallTab - 1);
-        }
-        if (MODE == kBinModeInsert) atomicMax(&M.cnt[lead[q]], word[q]);
-        else if (MODE == kBinModeErase) atomicMin(&M.cnt[lead[q]], word[q]);
-        else rank[q] = atomicAdd(&M.cnt[lead[q]], 1u);
-    }
-    __syncthreads();  // the key table is done: the stage may be used
-
-    // keys with several ops: a range of seg each, their op words listed there
-    bool mine[kSmallR];
-    if constexpr (MODE >= kBinModeMixed) {
-        bool any = false;
-#pragma unroll
-        for (int q = 0; q < kSmallR; ++q) {
-            const uint32_t r = q * kSmallThreads + tid;
-            const uint32_t c = r < m ? M.cnt[lead[q]] : 0u;
-            mine[q] = c == 1u;
-            any |= c > 1u;
-        }
-        if (__syncthreads_or(any)) {
+    while (true) {
+        K key[kSmallR];
+        uint32_t word[kSmallR];
+        bool mine[kSmallR];  // the op resolves its key alone
+        if (fits) {
+            // group: each record finds its key's first record (lead)
+            uint32_t lead[kSmallR], rank[kSmallR];
 #pragma unroll
             for (int q = 0; q < kSmallR; ++q) {
                 const uint32_t r = q * kSmallThreads + tid;
-                if (r < m && !mine[q] && lead[q] == r) {
-                    const uint32_t c = M.cnt[r];
-                    M.cnt[r] = c | (atomicAdd(&M.nseg, c) << 16);
-                    M.multi[atomicAdd(&M.nmulti, 1u)] = (uint16_t)r;
+                lead[q] = rank[q] = 0u;
+                word[q] = 0u;
+                key[q] = 0;
+                if (r >= m) continue;
+                key[q] = M.key[r];
+                word[q] = M.word[r];
+                uint32_t h = bin_cell<11>(bin_tag(key[q]));
+                // at most kSmallCap of the kSmallTab cells are taken: the probe ends
+                while (true) {
+                    const uint32_t old = atomicCAS(&tab[h], 0u, r + 1u);
+                    if (old == 0u) {
+                        lead[q] = r;
+                        break;
+                    }
+                    if (M.key[old - 1u] == key[q]) {
+                        lead[q] = old - 1u;
+                        break;
+                    }
+                    h = (h + 1u) & (kSmallTab - 1);
                 }
+                if (MODE == kBinModeInsert) atomicMax(&M.cnt[lead[q]], word[q]);
+                else if (MODE == kBinModeErase) atomicMin(&M.cnt[lead[q]], word[q]);
+                else rank[q] = atomicAdd(&M.cnt[lead[q]], 1u);
             }
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < kSmallR; ++q) {
-                const uint32_t r = q * kSmallThreads + tid;
-                if (r < m && !mine[q]) M.seg[(M.cnt[lead[q]] >> 16) + rank[q]] = word[q];
-            }
-            __syncthreads();
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < kSmallR; ++q) {
-            const uint32_t r = q * kSmallThreads + tid;
-            mine[q] = r < m && M.cnt[lead[q]] == word[q];  // op indexes are distinct
-            if (r < m && !mine[q]) ++n_sup;
-        }
-    }
+            __syncthreads();  // the key table is done: the stage may be used
 
-    // keys with one op (the winning op of an insert or erase batch): one probe
+            // keys with several ops: a range of seg each, their op words listed there
+            if constexpr (MODE >= kBinModeMixed) {
+                bool any = false;
 #pragma unroll
-    for (int q = 0; q < kSmallR; ++q) {
-        if ((uint32_t)(q * kSmallThreads) + (tid & ~31u) >= m) break;  // warp-uniform
-        const bool act = mine[q];
-        const uint32_t i = word[q] >> 2;
-        const uint32_t op = MODE == kBinModeInsert ? 1u : MODE == kBinModeErase ? 2u : (word[q] & 3u);
-        const bool ins = act && op == 1u, del = act && op == 2u;
-        Sl e = T::empty();
-        if (ins) e = T::make(key[q], load_val(vals, vb, i));
-        const uint32_t hk = fold(key[q]);
-        const Pair p = pair_of(hk, D.d);
-        char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
-        char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
-        const KvOut r1 = place_probe<KB, SB, false>(p1, key[q], act, p.first, D.d, stage);
-        const bool found1 = act && r1.match >= 0;
-        const bool want_slot = MODE != kBinModeCount && ins && r1.empty == 0u;
-        const bool may2 = !Gm::kMeta || r1.overflow;
-        const bool check2 =
-            act && !found1 && ((may2 && !(MODE == kBinModeInsert && (flags & kBinNewKeys))) || want_slot);
-        KvOut r2{-1, 0ull, false, 0u};
-        if (__any_sync(kFull, check2))
-            r2 = place_probe<KB, SB, false>(p2, key[q], check2, p.second, D.d, stage);
-        const bool found2 = check2 && r2.match >= 0;
-        const bool present = found1 || found2;
-        const uint64_t before = found1 ? r1.value : (found2 ? r2.value : 0ull);
-        if constexpr (MODE == kBinModeCount) {
-            if (ins && (!present || before != T::val(e))) ++n_ins;
-            if (del && present) ++n_del;
-            continue;
-        }
-        bool pend = false;
-        if (ins) {
-            if (present) {
-                if (!(MODE == kBinModeMixed && (flags & kBinSkipEqual) && before == T::val(e))) {
-                    T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match), e);
-                    ++n_upd;
+                for (int q = 0; q < kSmallR; ++q) {
+                    const uint32_t r = q * kSmallThreads + tid;
+                    const uint32_t c = r < m ? M.cnt[lead[q]] : 0u;
+                    mine[q] = c == 1u;
+                    any |= c > 1u;
+                }
+                if (__syncthreads_or(any)) {
+#pragma unroll
+                    for (int q = 0; q < kSmallR; ++q) {
+                        const uint32_t r = q * kSmallThreads + tid;
+                        if (r < m && !mine[q] && lead[q] == r) {
+                            const uint32_t c = M.cnt[r];
+                            M.cnt[r] = c | (atomicAdd(&M.nseg, c) << 16);
+                            if (c > kSmallLong) M.longs[atomicAdd(&M.nlong, 1u)] = (uint16_t)r;
+                            else M.multi[atomicAdd(&M.nmulti, 1u)] = (uint16_t)r;
+                        }
+                    }
+                    __syncthreads();
+#pragma unroll
+                    for (int q = 0; q < kSmallR; ++q) {
+                        const uint32_t r = q * kSmallThreads + tid;
+                        if (r < m && !mine[q]) M.seg[(M.cnt[lead[q]] >> 16) + rank[q]] = word[q];
+                    }
+                    __syncthreads();
                 }
             } else {
-                bool ok = claim_empty<KB, SB>(p1, r1.empty, e);
-                if (!ok && check2 && r2.empty) {
-                    mark_overflow<KB, SB>(p1, hk);
-                    ok = claim_empty<KB, SB>(p2, r2.empty, e);
+#pragma unroll
+                for (int q = 0; q < kSmallR; ++q) {
+                    const uint32_t r = q * kSmallThreads + tid;
+                    mine[q] = r < m && M.cnt[lead[q]] == word[q];  // op indexes are distinct
+                    if (r < m && !mine[q]) ++n_sup;
                 }
-                if (ok) ++n_ins;
-                else pend = true;
             }
-        } else if (del && present) {
-            T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match),
-                     T::empty());
-            ++n_del;
-        }
-        // a mixed op's result; the value an erased key had
-        if ((MODE == kBinModeMixed && act || MODE == kBinModeErase && present) && vals_out != nullptr)
-            store_val(vals_out, vb, i, before);
-        if (MODE != kBinModeInsert && act && present && bits_out != nullptr)
-            atomicOr(&bits_out[i >> 5], 1u << (i & 31));
-        if constexpr (MODE != kBinModeErase) {
-            __syncwarp();
-            const unsigned long long at = agg_inc(&ctr->pending, pend);
-            if (pend) {
-                if (at < S.list_cap) ((Sl *)S.list_a)[at] = e;
-                else atomicAdd(&ctr->spill, 1ull);
+        } else {
+            if constexpr (MODE >= kBinModeMixed)
+                m = gather_part<KB, SB>(M, keys, ops, (uint32_t)n);
+            else
+                m = gather_keys<KB, SB, MODE>(M, keys, (uint32_t)n, own0, own1, n_sup, n_rej);
+#pragma unroll
+            for (int q = 0; q < kSmallR; ++q) {
+                const uint32_t r = q * kSmallThreads + tid;
+                mine[q] = r < m && (MODE < kBinModeMixed || (M.cnt[r] & 0xffffu) == 1u);
+                key[q] = r < m ? M.key[r] : (K)0;
+                word[q] = mine[q] ? M.word[r] : 0u;
             }
         }
-    }
 
-    // keys with several ops: probe, replay the ops in index order, apply the
-    // final state. Key x of the list goes to lane x / 8 of warp x % 8, so a
-    // few long segments spread over the warps.
-    if constexpr (MODE >= kBinModeMixed) {
-        const uint32_t nm = M.nmulti;
-        for (uint32_t x0 = 0; x0 < nm; x0 += kSmallThreads) {
-            const uint32_t x = x0 + lane * kSmallWarps + (tid >> 5);
-            const bool act = x < nm;
-            if (!__any_sync(kFull, act)) continue;
-            const uint32_t r = act ? M.multi[x] : 0u;
-            const K k = act ? M.key[r] : (K)0;
-            const uint32_t c = act ? M.cnt[r] & 0xffffu : 0u, off = act ? M.cnt[r] >> 16 : 0u;
-            const uint32_t hk = fold(k);
+        // keys with one op (the winning op of an insert or erase batch): one probe
+#pragma unroll
+        for (int q = 0; q < kSmallR; ++q) {
+            if ((uint32_t)(q * kSmallThreads) + (tid & ~31u) >= m) break;  // warp-uniform
+            const bool act = mine[q];
+            const uint32_t i = word[q] >> 2;
+            const uint32_t op = MODE == kBinModeInsert ? 1u : MODE == kBinModeErase ? 2u : (word[q] & 3u);
+            const bool ins = act && op == 1u, del = act && op == 2u;
+            Sl e = T::empty();
+            if (ins) e = T::make(key[q], load_val(vals, vb, i));
+            const uint32_t hk = fold(key[q]);
             const Pair p = pair_of(hk, D.d);
             char *p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, hk));
             char *p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, hk));
-            const KvOut r1 = place_probe<KB, SB, false>(p1, k, act, p.first, D.d, stage);
+            const KvOut r1 = place_probe<KB, SB, false>(p1, key[q], act, p.first, D.d, stage);
             const bool found1 = act && r1.match >= 0;
-            const bool check2 = act && !found1 && ((!Gm::kMeta || r1.overflow) || r1.empty == 0u);
+            const bool want_slot = MODE != kBinModeCount && ins && r1.empty == 0u;
+            const bool may2 = !Gm::kMeta || r1.overflow;
+            const bool check2 =
+                act && !found1 && ((may2 && !(MODE == kBinModeInsert && (flags & kBinNewKeys))) || want_slot);
             KvOut r2{-1, 0ull, false, 0u};
             if (__any_sync(kFull, check2))
-                r2 = place_probe<KB, SB, false>(p2, k, check2, p.second, D.d, stage);
+                r2 = place_probe<KB, SB, false>(p2, key[q], check2, p.second, D.d, stage);
             const bool found2 = check2 && r2.match >= 0;
-            const bool pre = found1 || found2;
-            const uint64_t pre_value = found1 ? r1.value : (found2 ? r2.value : 0ull);
-            bool present = pre;
-            uint64_t value = pre_value;
-            if (act && c <= kBinShort) {
-                uint32_t w[kBinShort];
-#pragma unroll
-                for (uint32_t a = 0; a < kBinShort; ++a) w[a] = a < c ? M.seg[off + a] : 0xffffffffu;
-#pragma unroll
-                for (uint32_t t = 0; t < kBinShort; ++t) {
-#pragma unroll
-                    for (uint32_t a = t & 1u; a + 1 < kBinShort; a += 2) {
-                        const uint32_t lo = min(w[a], w[a + 1]), hi = max(w[a], w[a + 1]);
-                        w[a] = lo;
-                        w[a + 1] = hi;
-                    }
-                }
-#pragma unroll
-                for (uint32_t a = 0; a < kBinShort; ++a) {
-                    if (a >= c) break;
-                    const uint32_t i = w[a] >> 2, op = w[a] & 3u;
-                    const uint64_t in = op == 1u ? load_val(vals, vb, i) : 0ull;
-                    if (MODE == kBinModeMixed) {
-                        if (vals_out) store_val(vals_out, vb, i, present ? value : 0ull);
-                        if (present && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
-                    }
-                    replay_op((uint8_t)op, in, present, value);
-                }
-            }
-            for (unsigned big = __ballot_sync(kFull, c > kBinShort); big; big &= big - 1u) {
-                const int j = __ffs(big) - 1;
-                const uint32_t cj = __shfl_sync(kFull, c, j), oj = __shfl_sync(kFull, off, j);
-                bool pj = __shfl_sync(kFull, present, j);
-                uint64_t vj = shfl64(value, j);
-                __syncwarp();
-                warp_sort_words(M.seg + oj, cj);
-                warp_replay_words<MODE == kBinModeMixed>(M.seg + oj, cj, pj, vj, vals, vb, vals_out,
-                                                     bits_out);
-                if ((int)lane == j) {
-                    present = pj;
-                    value = vj;
-                }
-            }
-            const bool up = act && present && (!pre || value != pre_value);
-            const bool er = act && !present && pre;
+            const bool present = found1 || found2;
+            const uint64_t before = found1 ? r1.value : (found2 ? r2.value : 0ull);
             if constexpr (MODE == kBinModeCount) {
-                n_ins += up ? 1u : 0u;
-                n_del += er ? 1u : 0u;
+                if (ins && (!present || before != T::val(e))) ++n_ins;
+                if (del && present) ++n_del;
                 continue;
             }
-            Sl e = T::empty();
             bool pend = false;
-            if (up) {
-                e = T::make(k, value);
-                if (pre) {
-                    T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match), e);
-                    ++n_upd;
+            if (ins) {
+                if (present) {
+                    if (!(MODE == kBinModeMixed && (flags & kBinSkipEqual) && before == T::val(e))) {
+                        T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match), e);
+                        ++n_upd;
+                    }
                 } else {
                     bool ok = claim_empty<KB, SB>(p1, r1.empty, e);
                     if (!ok && check2 && r2.empty) {
@@ -1125,18 +1436,123 @@ __global__ void __launch_bounds__(kSmallThreads) k_bin_small(
                     if (ok) ++n_ins;
                     else pend = true;
                 }
-            } else if (er) {
+            } else if (del && present) {
                 T::store(found1 ? slot_ptr<KB, SB>(p1, r1.match) : slot_ptr<KB, SB>(p2, r2.match),
                          T::empty());
                 ++n_del;
             }
-            __syncwarp();
-            const unsigned long long at = agg_inc(&ctr->pending, pend);
-            if (pend) {
-                if (at < S.list_cap) ((Sl *)S.list_a)[at] = e;
-                else atomicAdd(&ctr->spill, 1ull);
+            // a mixed op's result; the value an erased key had
+            if ((MODE == kBinModeMixed && act || MODE == kBinModeErase && present) && vals_out != nullptr)
+                store_val(vals_out, vb, i, before);
+            if (MODE != kBinModeInsert && act && present && bits_out != nullptr)
+                atomicOr(&bits_out[i >> 5], 1u << (i & 31));
+            if constexpr (MODE != kBinModeErase) {
+                __syncwarp();
+                const unsigned long long at = agg_inc(&ctr->pending, pend);
+                if (pend) {
+                    if (at < S.list_cap) ((Sl *)S.list_a)[at] = e;
+                    else atomicAdd(&ctr->spill, 1ull);
+                }
             }
         }
+
+        // keys with several ops: probe, replay the ops in index order, apply the
+        // final state
+        if constexpr (MODE >= kBinModeMixed) {
+            RepCounts rc;
+            auto finish = [&](const RepKey<KB> &x, bool act, bool present, uint64_t value) {
+                const bool up = act && present && (!x.pre || value != x.pre_value);
+                const bool er = act && !present && x.pre;
+                if constexpr (MODE == kBinModeCount) {
+                    rc.ins += up ? 1u : 0u;
+                    rc.del += er ? 1u : 0u;
+                } else {
+                    mutate_listed<KB, SB>(x, up, er, value, S.list_a, S.list_cap, ctr, rc);
+                }
+            };
+            // Key x of the list goes to lane x / 16 of warp x % 16, so a few long
+            // segments spread over the warps.
+            const uint32_t nm = M.nmulti;
+            for (uint32_t x0 = 0; x0 < nm; x0 += kSmallThreads) {
+                const uint32_t y = x0 + lane * kSmallWarps + (tid >> 5);
+                const bool act = y < nm;
+                if (!__any_sync(kFull, act)) continue;
+                const uint32_t r = act ? M.multi[y] : 0u;
+                const uint32_t c = act ? M.cnt[r] & 0xffffu : 0u, off = act ? M.cnt[r] >> 16 : 0u;
+                const RepKey<KB> x = probe_key<KB, SB>(D, act ? M.key[r] : (K)0, act, stage);
+                bool present = x.pre;
+                uint64_t value = x.pre_value;
+                if (act && c <= kBinShort) {
+                    uint32_t w[kBinShort];
+#pragma unroll
+                    for (uint32_t a = 0; a < kBinShort; ++a) w[a] = a < c ? M.seg[off + a] : 0xffffffffu;
+#pragma unroll
+                    for (uint32_t t = 0; t < kBinShort; ++t) {
+#pragma unroll
+                        for (uint32_t a = t & 1u; a + 1 < kBinShort; a += 2) {
+                            const uint32_t lo = min(w[a], w[a + 1]), hi = max(w[a], w[a + 1]);
+                            w[a] = lo;
+                            w[a + 1] = hi;
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t a = 0; a < kBinShort; ++a) {
+                        if (a >= c) break;
+                        const uint32_t i = w[a] >> 2, op = w[a] & 3u;
+                        const uint64_t in = op == 1u ? load_val(vals, vb, i) : 0ull;
+                        if (MODE == kBinModeMixed) {
+                            if (vals_out) store_val(vals_out, vb, i, present ? value : 0ull);
+                            if (present && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
+                        }
+                        replay_op((uint8_t)op, in, present, value);
+                    }
+                }
+                for (unsigned big = __ballot_sync(kFull, c > kBinShort); big; big &= big - 1u) {
+                    const int j = __ffs(big) - 1;
+                    const uint32_t cj = __shfl_sync(kFull, c, j), oj = __shfl_sync(kFull, off, j);
+                    bool pj = __shfl_sync(kFull, present, j);
+                    uint64_t vj = shfl64(value, j);
+                    __syncwarp();
+                    warp_sort_words(M.seg + oj, cj);
+                    warp_replay_words<MODE == kBinModeMixed>(M.seg + oj, cj, pj, vj, vals, vb, vals_out,
+                                                             bits_out);
+                    if ((int)lane == j) {
+                        present = pj;
+                        value = vj;
+                    }
+                }
+                finish(x, act, present, value);
+            }
+            // keys with more than kSmallLong ops: the whole block each
+            const uint32_t nl = M.nlong;
+            for (uint32_t y = 0; y < nl; ++y) {
+                const uint32_t r = M.longs[y], c = M.cnt[r] & 0xffffu, off = M.cnt[r] >> 16;
+                sort_long<KB, SB>(M, off, c);
+                __shared__ uint64_t s_before;
+                __shared__ uint32_t s_present;
+                RepKey<KB> x;
+                if (tid < 32) {
+                    x = probe_key<KB, SB>(D, M.key[r], lane == 0, stage);
+                    if (tid == 0) {
+                        s_present = x.pre ? 1u : 0u;
+                        s_before = x.pre_value;
+                    }
+                }
+                __syncthreads();
+                bool present = s_present != 0u;
+                uint64_t value = s_before;
+                block_replay<kSmallThreads, MODE == kBinModeMixed>(M.seg + off, c, present, value,
+                                                                   SegOps{ops, 0u}, vals, vb, vals_out,
+                                                                   bits_out);
+                if (tid < 32) finish(x, lane == 0, present, value);
+                __syncthreads();
+            }
+            n_ins += rc.ins;
+            n_upd += rc.upd;
+            n_del += rc.del;
+        }
+        if (fits || M.top == 0u) break;
+        __syncthreads();  // the lists are reused by the next part
     }
 
     // one atomic per counter per block
@@ -1149,7 +1565,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_bin_small(
         if (n_ins) atomicAdd(&M.sum[0], (unsigned long long)n_ins);
         if (n_upd) atomicAdd(&M.sum[1], (unsigned long long)n_upd);
         if (n_del) atomicAdd(&M.sum[2], (unsigned long long)n_del);
-        if (n_sup) atomicAdd(&M.sum[3], (unsigned long long)n_sup);
+        if (n_sup) atomicAdd(&M.sum[3], (unsigned long long)(long long)(int32_t)n_sup);  // may be below 0
         if (n_rej) atomicAdd(&M.sum[4], (unsigned long long)n_rej);
     }
     __syncthreads();

@@ -5,7 +5,7 @@ template cudaError_t dyc::Ops<8>::bin_group(const LaunchCtx &, const BinScratch 
                                             const ApplyScratch &, int, const uint8_t *,
                                             const void *, uint32_t *, uint64_t, Counters *);
 template cudaError_t dyc::Ops<8>::bin_small(const LaunchCtx &, const Desc &, int, const Scratch &,
-                                            const BinScratch &, int, const uint8_t *, const void *,
+                                            int, const uint8_t *, const void *,
                                             const void *, uint32_t, void *, uint32_t *, uint64_t,
                                             uint32_t, Counters *, Counters *);
 template cudaError_t dyc::Ops<8>::set_group(const LaunchCtx &, const ApplyScratch &,

@@ -118,7 +118,7 @@ cudaError_t Ops<KB>::repeat(const LaunchCtx &L, const ApplyScratch &A, const Des
     return f(L, A, descs, ntables, set, ops, vals, vb, vals_out, bits_out, n, list_a, list_cap, gctr);
 }
 
-using BinFn = void (*)(Desc, Scratch, BinScratch, const uint8_t *, const void *, const void *, uint32_t,
+using BinFn = void (*)(Desc, Scratch, const uint8_t *, const void *, const void *, uint32_t,
                        void *, uint32_t *, uint64_t, uint32_t, Counters *, Counters *);
 
 template <int KB, int SB> BinFn small_kernel(int mode) {
@@ -130,21 +130,21 @@ template <int KB, int SB> BinFn small_kernel(int mode) {
 
 template <int KB>
 cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
-                               const BinScratch &B, int mode, const uint8_t *ops, const void *keys,
-                               const void *vals, uint32_t vb, void *vals_out, uint32_t *bits_out,
-                               uint64_t n, uint32_t flags, Counters *ctr, Counters *h_ctr) {
+                               int mode, const uint8_t *ops, const void *keys, const void *vals,
+                               uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
+                               uint32_t flags, Counters *ctr, Counters *h_ctr) {
     if (n == 0) return cudaSuccess;
     const uint64_t words = bits_out ? (n + 31) / 32 : 0;
-    launch_after(k_small_clear<KB>, (unsigned)((unsigned)((words + 255) / 256 + 1)), 256, 0, L.stream, &ctr->inserted, (uint32_t)(sizeof(Counters) / 8 - 1), bits_out, words);
+    launch_after(k_small_clear<KB>, (unsigned)((words + 255) / 256 + 1), 256, 0, L.stream, &ctr->inserted,
+                 (uint32_t)(sizeof(Counters) / 8 - 1), bits_out, words);
     const BinFn k = sb == 32   ? small_kernel<KB, 32>(mode)
                     : sb == 64 ? small_kernel<KB, 64>(mode)
                                : small_kernel<KB, 128>(mode);
-    const int bytes = (int)(sb == 32   ? sizeof(BinSmem<KB, 32>)
-                            : sb == 64 ? sizeof(BinSmem<KB, 64>)
-                                       : sizeof(BinSmem<KB, 128>));
-    const cudaError_t e = allow_smem((const void *)k, bytes);
+    const auto bytes = sb == 32 ? bin_smem<KB, 32> : sb == 64 ? bin_smem<KB, 64> : bin_smem<KB, 128>;
+    const cudaError_t e = allow_smem((const void *)k, (int)bytes(mode, kBinSmallOps));
     if (e != cudaSuccess) return e;
-    launch_after(k, (unsigned)(B.nbins), kSmallThreads, bytes, L.stream, D, S, B, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr);
+    launch_after(k, (unsigned)((n + kBinSmallMean - 1) / kBinSmallMean), kSmallThreads, bytes(mode, n), L.stream,
+                 D, S, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr);
     return cudaGetLastError();
 }
 

@@ -55,8 +55,8 @@ struct Counters {
     // scratch word: insert ops of a dyc_apply batch (its upserts, from the
     // counting pass of a batch resolved by bins)
     unsigned long long nins;
-    unsigned long long left;        // nonzero: a small batch has a bin that does not fit
-    unsigned long long ticket;      // blocks of a small batch's kernel that have finished
+    unsigned long long ticket;      // blocks of a call's last kernel that have finished
+    unsigned long long pad2;
 };
 static_assert(sizeof(Counters) == 128, "Counters is one 128-byte block");
 
@@ -75,13 +75,22 @@ enum DedupMode { kKeepLast = 0, kKeepFirst = 1 };
 // random keys on average. The ops of a bin with more than kBinCap (few keys,
 // each repeated many times) get records in `hot` instead. kBinMean * 2 =
 // kBinCap, so the records of n ops take 2n words. Batches of up to
-// kBinSmallOps ops are split by the kernel that resolves them, into bins of
-// kBinSmallMean ops.
+// kBinSmallOps mixed ops, or kBinSmallUpserts inserts or erases, are split by
+// the kernel that resolves them (k_bin_small), into bins of kBinSmallMean ops.
+// The lines lie where the split kernels get as fast, in us of a call on a table
+// of 2^24 4-byte keys, one kernel / split:
+//   mixed ops       8000       16000       24000       32768
+//     distinct     47 / 49     50 / 52     54 / 53     56 / 54
+//     7 keys       70 / 86     91 / 106   112 / 118   134 / 152
+//     100 keys     55 / 80     65 / 122   116 / 130   134 / 84
+//   inserts         8000       12000       16000       32768
+//     distinct     37 / 38     39 / 38     40 / 39     45 / 40
+//     7 keys       41 / 44     44 / 45     47 / 45     60 / 47
 constexpr int kBinCap = 2048;
 constexpr int kBinMean = 1024;
 constexpr int kSmallCap = 1024;
 constexpr int kBinSmallMean = 384;
-constexpr uint64_t kBinSmallOps = 32768;
+constexpr uint64_t kBinSmallOps = 24576, kBinSmallUpserts = 8192;
 enum : int {
     kBinOver = 0,  // nonzero: some bin went over
     kBinStates = 4
@@ -388,13 +397,13 @@ template <int KB> struct Ops {
     static cudaError_t bin_group(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
                                  int mode, const uint8_t *ops, const void *keys, uint32_t *bits_out,
                                  uint64_t n, Counters *ctr);
-    // a batch of up to kBinSmallOps ops in one of the kBinMode* modes; the
-    // counters go to h_ctr (left set: nothing done, a bin does not fit)
+    // a batch of up to kBinSmallOps ops in one kernel, in one of the kBinMode*
+    // modes; the
+    // counters go to h_ctr
     static cudaError_t bin_small(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,
-                                 const BinScratch &B, int mode, const uint8_t *ops,
-                                 const void *keys, const void *vals, uint32_t vb, void *vals_out,
-                                 uint32_t *bits_out, uint64_t n, uint32_t flags, Counters *ctr,
-                                 Counters *h_ctr);
+                                 int mode, const uint8_t *ops, const void *keys, const void *vals,
+                                 uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
+                                 uint32_t flags, Counters *ctr, Counters *h_ctr);
     // ctr->nins / ctr->erased += the upserts and erases that apply_unique
     // would make for the ops whose single bit is set
     static cudaError_t apply_count(const LaunchCtx &L, const Desc &D, int sb, const uint8_t *ops,

@@ -9,22 +9,11 @@
 
 namespace dyc {
 
-// A lane's key and what the probes of its two buckets found.
-template <int KB> struct RepKey {
-    typename SlotT<KB>::K k;
-    uint32_t tb, hk;
-    char *p1, *p2;
-    KvOut r1, r2;
-    bool found1, found2, pre;
-    uint64_t pre_value;
-};
-
 // Key d of every lane with act (warp-collective).
 template <int KB, int SB, bool SET>
 __device__ __forceinline__ RepKey<KB> probe_listed(const ApplyScratch &A, const Desc *__restrict__ descs,
                                                    uint32_t ntables, uint32_t d, bool act,
                                                    unsigned char *stage) {
-    using Gm = Geo<KB, SB>;
     RepKey<KB> x;
     x.k = 0;
     x.tb = 0u;
@@ -37,91 +26,10 @@ __device__ __forceinline__ RepKey<KB> probe_listed(const ApplyScratch &A, const 
             x.k = 0;
         }
     }
-    act = act && x.k != 0;
-    const Desc &D = descs[x.tb];
-    x.hk = fold(x.k);
-    const Pair p = pair_of(x.hk, D.d);
-    x.p1 = bucket_ptr<KB, SB>(D, p.first, bucket_index(D, p.first, x.hk));
-    x.p2 = bucket_ptr<KB, SB>(D, p.second, bucket_index(D, p.second, x.hk));
-    x.r1 = place_probe<KB, SB>(x.p1, x.k, act, p.first, D.d, stage);
-    x.found1 = act && x.r1.match >= 0;
-    // the second bucket: where the key or an empty slot may be there
-    const bool check2 = act && !x.found1 && ((!Gm::kMeta || x.r1.overflow) || x.r1.empty == 0u);
-    x.r2 = KvOut{-1, 0ull, false, 0u};
-    if (__any_sync(kFull, check2))
-        x.r2 = place_probe<KB, SB>(x.p2, x.k, check2, p.second, D.d, stage);
-    x.found2 = check2 && x.r2.match >= 0;
-    x.pre = x.found1 || x.found2;
-    x.pre_value = x.found1 ? x.r1.value : (x.found2 ? x.r2.value : 0ull);
+    const uint32_t tb = x.tb;
+    x = probe_key<KB, SB>(descs[tb], x.k, act && x.k != 0, stage);
+    x.tb = tb;
     return x;
-}
-
-// An op word of a segment (SegOps::wide: a plain index).
-struct SegOps {
-    const uint8_t *ops;
-    uint32_t wide;
-    __device__ __forceinline__ uint32_t index(uint32_t w) const { return wide ? w : w >> 2; }
-    __device__ __forceinline__ uint8_t code(uint32_t w) const {
-        return wide ? ops[w] : (uint8_t)(w & 3u);  // 1 insert, 2 erase; others read
-    }
-};
-static_assert(kOpInsert == 1 && kOpErase == 2, "a segment's op codes are the ops'");
-
-// Replay of the op words idx[0..cnt) (op indices in increasing order) by the
-// whole block, an op a thread at a time: an op's state comes from the latest
-// mutation before it in its warp (a ballot), else in the warps before, else
-// from the state carried in; present / value carry the key's state in every
-// thread. (By one warp, 32 ops a step, a batch of 2^22 ops on 5000 keys took 764
-// us, the other warps idle; by all 663.)
-__device__ __forceinline__ void block_replay(const uint32_t *idx, uint32_t cnt, bool &present,
-                                             uint64_t &value, const SegOps &ops,
-                                             const void *__restrict__ vals, uint32_t vb,
-                                             void *__restrict__ vals_out,
-                                             uint32_t *__restrict__ bits_out) {
-    // a warp's latest mutation: 0 none, 1 erase, 2 insert, and its value
-    __shared__ uint32_t s_kind[2][kWarpsPerBlock];
-    __shared__ uint64_t s_val[2][kWarpsPerBlock];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t buf = 0u;
-    for (uint32_t c0 = 0; c0 < cnt; c0 += kBlockThreads, buf ^= 1u) {
-        const bool v = c0 + threadIdx.x < cnt;
-        const uint32_t w = v ? idx[c0 + threadIdx.x] : 0u, i = ops.index(w);
-        const uint8_t op = v ? ops.code(w) : (uint8_t)kOpFind;
-        const bool mut = op == kOpInsert || op == kOpErase;  // other codes read
-        const uint64_t myval = op == kOpInsert ? load_val(vals, vb, i) : 0ull;
-        const unsigned mm = __ballot_sync(kFull, mut);
-        const unsigned before = mm & ((1u << lane) - 1u);
-        const int src = before ? 31 - __clz(before) : (int)lane;
-        const uint32_t kind = mut ? (op == kOpInsert ? 2u : 1u) : 0u;
-        const uint64_t srcval = shfl64(myval, src);
-        const uint32_t srckind = __shfl_sync(kFull, kind, src);
-        if ((int)lane == (mm ? 31 - __clz(mm) : 0)) {
-            s_kind[buf][warp] = kind;
-            s_val[buf][warp] = myval;
-        }
-        __syncthreads();  // the other buffer is written in the next step
-        bool st = present;
-        uint64_t sval = value;
-#pragma unroll
-        for (uint32_t x = 0; x < (uint32_t)kWarpsPerBlock; ++x) {
-            if (x == warp) {
-                st = present;
-                sval = value;
-            }
-            const uint32_t k = s_kind[buf][x];
-            if (k == 0u) continue;
-            present = k == 2u;
-            value = s_val[buf][x];  // 0 of an erase
-        }
-        if (before) {
-            st = srckind == 2u;
-            sval = srcval;
-        }
-        if (v) {
-            if (vals_out) store_val(vals_out, vb, i, st ? sval : 0ull);
-            if (st && bits_out) atomicOr(&bits_out[i >> 5], 1u << (i & 31));
-        }
-    }
 }
 
 // Ascending sort of a warp's 32 * R words, the word at place lane * R + r in
@@ -300,50 +208,7 @@ __device__ __forceinline__ const uint32_t *block_sort(uint32_t *src, uint32_t *d
     return src;
 }
 
-struct RepCounts {
-    uint32_t ins = 0, upd = 0, del = 0;
-};
-
-// The final state of a lane's key (act) to the table; entries without a slot
-// go to list_a. Warp-collective.
-template <int KB, int SB>
-__device__ __forceinline__ void mutate_listed(const RepKey<KB> &x, bool up, bool er, uint64_t value,
-                                              void *list_a, uint64_t list_cap, Counters *gctr,
-                                              RepCounts &n) {
-    using T = SlotT<KB>;
-    typename T::S e = T::empty();
-    bool pend = false;
-    if (up) {
-        e = T::make(x.k, value);
-        if (x.found1) {
-            T::store(slot_ptr<KB, SB>(x.p1, x.r1.match), e);
-            ++n.upd;
-        } else if (x.found2) {
-            T::store(slot_ptr<KB, SB>(x.p2, x.r2.match), e);
-            ++n.upd;
-        } else {
-            bool ok = claim_empty<KB, SB>(x.p1, x.r1.empty, e);
-            if (!ok && x.r2.empty) {
-                mark_overflow<KB, SB>(x.p1, x.hk);
-                ok = claim_empty<KB, SB>(x.p2, x.r2.empty, e);
-            }
-            if (ok) ++n.ins;
-            else pend = true;
-        }
-    } else if (er) {
-        T::store(x.found1 ? slot_ptr<KB, SB>(x.p1, x.r1.match) : slot_ptr<KB, SB>(x.p2, x.r2.match),
-                 T::empty());
-        ++n.del;
-    }
-    __syncwarp();
-    const unsigned long long at = agg_inc(&gctr->pending, pend);
-    if (pend) {
-        if (at < list_cap) ((typename T::S *)list_a)[at] = e;
-        else atomicAdd(&gctr->spill, 1ull);
-    }
-}
-
-// The same to the lists, at place u (upserts) or e (erases).
+// A lane's key (act) to the lists of changes, at place u (upserts) or e (erases).
 template <int KB>
 __device__ __forceinline__ void list_change(const ApplyScratch &A, const RepKey<KB> &x, bool up,
                                             bool er, uint64_t value, uint32_t vb,
@@ -425,7 +290,7 @@ __global__ void __launch_bounds__(256, SET ? 4 : 3) k_repeat(
         __syncthreads();
         bool present = s_present != 0u;
         uint64_t value = s_before;
-        block_replay(sorted, cnt, present, value, so, vals, vb, vals_out, bits_out);
+        block_replay<kBlockThreads, true>(sorted, cnt, present, value, so, vals, vb, vals_out, bits_out);
         if (tid < 32) finish(x, lane == 0 && x.k != 0, present, value);
         __syncthreads();  // the sorted indices are reused by the next segment
     }

@@ -45,6 +45,72 @@ def test_inserts_and_erases_of_hot_keys(kb, n, hot, share):
     t.close()
 
 
+def _bin(keys, nbins):
+    """The bin of each key among nbins (bin_of in dyc_bins.cuh)."""
+    k = keys.astype(np.uint64)
+    lo, hi = (k & np.uint64(0xFFFFFFFF)).astype(np.uint32), (k >> np.uint64(32)).astype(np.uint32)
+    with np.errstate(over="ignore"):
+        x = lo if keys.itemsize == 4 else (lo ^ hi ^ (np.uint32(0x9E3779B9) * hi)) ^ hi
+        x = x ^ (x >> np.uint32(16))
+        x = x * np.uint32(0x7FEB352D)
+        x = x ^ (x >> np.uint32(15))
+        x = x * np.uint32(0x846CA68B)
+        x = x ^ (x >> np.uint32(16))
+    return (x.astype(np.uint64) * np.uint64(nbins)) >> np.uint64(32)
+
+
+@pytest.mark.parametrize("kb", [4, 8])
+@pytest.mark.parametrize("bucket_bytes", [32, 64, 128])
+@pytest.mark.parametrize("mix", ["one", "seven", "tenth", "hundred", "bin", "bin twice"])
+@pytest.mark.parametrize("n", [1025, 2049, 8192, 24576])
+def test_small_batches_with_a_bin_over_its_capacity(kb, bucket_bytes, mix, n):
+    """Batches of one kernel in which a bin gets more than 1024 ops: a few keys,
+    a tenth of the ops on one key, or distinct keys all of one bin (more than
+    1024 of them: the bin is taken in parts), once and repeated."""
+    import torch
+    import databases_gpu_gb300 as dg
+    rng = np.random.default_rng(n + kb)
+    pool = _pool(kb, 1 << 20, n)
+    nbins = (n + 383) // 384
+    if mix.startswith("bin"):
+        pool = np.concatenate([pool, _pool(kb, 3 << 20, n + 1)])
+        pool = np.unique(pool[_bin(pool, nbins) == nbins // 2])
+    draw = {"one": lambda: pool[np.zeros(n, np.int64)],
+            "seven": lambda: pool[rng.integers(0, 7, n)],
+            "hundred": lambda: pool[rng.integers(0, 100, n)],
+            "tenth": lambda: np.where(rng.random(n) < 0.1, pool[0], pool[rng.integers(0, pool.size, n)]),
+            "bin": lambda: pool[rng.permutation(pool.size)[np.arange(n) % pool.size]],
+            "bin twice": lambda: pool[rng.integers(0, min(n // 2, pool.size), n)]}[mix]
+    t = dg.DyCuckoo(2 * n, key_bytes=kb, value_bytes=kb, bucket_bytes=bucket_bytes)
+    m = O.Map()
+    for step in range(2):
+        k = draw().copy()
+        k[rng.random(n) < 0.001] = 0
+        kt = k.dtype
+        v = rng.integers(1, 1 << 31, n).astype(kt)
+        before = len(m)
+        st = t.insert(to_dev(k), to_dev(v))
+        m.insert(k.astype(np.uint64), v.astype(np.uint64))
+        distinct = np.unique(k[k != 0]).size
+        assert st["inserted"] == len(m) - before and st["updated"] == distinct - st["inserted"]
+        assert st["superseded"] == int((k != 0).sum()) - distinct and st["rejected"] == int((k == 0).sum())
+        assert_same_contents(t, m, "insert %d" % step)
+        k, v = draw(), rng.integers(1, 1 << 31, n).astype(kt)
+        ops = rng.choice(np.array([0, 1, 2, 9], np.uint8), size=n, p=[0.4, 0.3, 0.2, 0.1])
+        out, bits = t.apply(to_dev(ops), to_dev(k), to_dev(v))
+        ov, oh = m.apply(ops, k.astype(np.uint64), v.astype(np.uint64))
+        assert np.array_equal(dg.unpack_bits(bits, n), oh), step
+        assert np.array_equal(out.cpu().numpy().view(kt).astype(np.uint64), ov), step
+        assert_same_contents(t, m, "apply %d" % step)
+        e = draw()
+        eb = torch.full(((n + 31) // 32,), -1, dtype=torch.int32, device="cuda")
+        got = t.erase(to_dev(e), erased_bits=eb)
+        _, eh = m.erase(e.astype(np.uint64))
+        assert got == int(eh.sum()) and np.array_equal(dg.unpack_bits(eb, n), eh)
+        assert_same_contents(t, m, "erase %d" % step)
+    t.close()
+
+
 def _us(f, reps=9):
     import time
 
@@ -60,7 +126,7 @@ def _us(f, reps=9):
 
 
 @pytest.mark.parametrize("kb", [4, 8])
-@pytest.mark.parametrize("n", [100000, 1 << 20])
+@pytest.mark.parametrize("n", [8192, 32768, 100000, 1 << 20])
 @pytest.mark.parametrize("hot", [1, 7, 100])
 def test_hot_inserts_take_no_more_than_twice_the_time_of_distinct_ones(kb, n, hot):
     """The split and the grouping read as many ops either way and the probes are
