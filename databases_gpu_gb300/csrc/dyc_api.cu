@@ -1298,8 +1298,9 @@ dyc_status carve_apply(int kb, int vb, uint64_t ops, uint32_t ntables, uint64_t 
         multi ? (ops / dyc::kTidxStep + 1) * 4 : 0,   // tidx
         (ops / 32 + 1) * 4,                           // single
         multi ? nbins * dyc::kBinCap * 8 : 0,         // rec
-        multi ? (bin_words(nbins) + nbins) * 4 : 0,   // bin_words, and a table per bin
-        multi ? ops * 8 : 0};                         // hot
+        multi ? bin_words(nbins) * 4 : 0,             // bin_words
+        multi ? ops * 8 : 0,                          // hot
+        multi ? nbins * sizeof(uint2) : 0};           // bin_tables
     size_t need = 0;
     for (size_t b : sizes) need += (b + 255) & ~(size_t)255;
     if (*buf && *buf_bytes < need) {
@@ -1340,6 +1341,7 @@ dyc_status carve_apply(int kb, int vb, uint64_t ops, uint32_t ntables, uint64_t 
     A.rec = (unsigned long long *)carve();
     A.bin_words = (uint32_t *)carve();
     A.hot = (unsigned long long *)carve();
+    A.bin_tables = (uint2 *)carve();
     A.ntables = ntables;
     A.cap_ops = ops;
     A.wide = ops > (1ull << 30) ? 1u : 0u;
@@ -1806,14 +1808,13 @@ dyc_status set_ensure_scratch(dyc_set *s, uint64_t n) {
     const uint64_t ops = n < 128 ? 128 : n;
     if (s->abuf && s->A.cap_ops >= ops) return DYC_OK;
     set_drop_graphs(s);
-    // table t's bins: ops / kBinMean + t (TableBins in dyc_bins.cuh)
-    const uint64_t nbins = ops / dyc::kBinMean + s->ntables + 1;
+    const uint64_t nbins = dyc::set_nbins(ops);
     TRY(carve_apply(s->kb, s->vb, ops, s->ntables, nbins, &s->abuf, &s->abytes, &s->A));
     s->bins = dyc::BinScratch{};
     carve_bins(s->bins, s->A.bin_words, (uint32_t)nbins);
-    s->bins.tid = s->bins.cursor + nbins;
     s->bins.rec = s->A.rec;
     s->bins.hot = s->A.hot;
+    s->bins.tables = s->A.bin_tables;
     s->bins.single = s->A.single;
     s->bins_zero = false;
     const size_t slot = s->kb == 4 ? 8 : 16;
@@ -1839,10 +1840,10 @@ dyc_status set_ensure_scratch(dyc_set *s, uint64_t n) {
 
 // Phase A: the repeated keys found, looked up and replayed; counters to the host.
 // Every kernel reads the op count from d_off[ntables] on the device; n (the
-// scratch capacity under a graph) only sizes the grids.
+// scratch capacity under a graph, not sized) only sizes the grids.
 dyc_status set_phase_a(dyc_set *s, const uint32_t *d_off, const uint8_t *ops, const void *keys,
-                       const void *vals, void *out, uint32_t *bits, uint64_t n, bool new_counts,
-                       cudaStream_t st) {
+                       const void *vals, void *out, uint32_t *bits, uint64_t n, bool sized,
+                       bool new_counts, cudaStream_t st) {
     const dyc::ApplyScratch &A = s->A;
     const LaunchCtx L{s->sms, st, (int)s->blocks_per_sm};
     const uint32_t vb = (uint32_t)s->vb;
@@ -1851,7 +1852,8 @@ dyc_status set_phase_a(dyc_set *s, const uint32_t *d_off, const uint8_t *ops, co
     CK(cudaMemcpyAsync(&A.ctr[dyc::kCtrHostN], s->h_hostn, sizeof(unsigned long long),
                        cudaMemcpyHostToDevice, st));
     // also zeroes phase B's counters (nothing between the phases uses them)
-    cudaError_t e = SET_KB_CALL(s, set_group, L, A, s->bins, d_off, ops, keys, n, bits, s->d_gctr);
+    cudaError_t e = SET_KB_CALL(s, set_group, L, A, s->bins, d_off, ops, keys, n, sized, bits,
+                                s->d_gctr);
     if (e == cudaSuccess)
         e = SET_KB_CALL(s, repeat, L, A, s->d_desc, s->ntables, s->sb, true, ops, vals, vb, out, bits, n);
     if (e != cudaSuccess) return fail(DYC_ECUDA, "set phase A kernels: %s", cudaGetErrorString(e));
@@ -2401,7 +2403,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
         // when a member needs more than its device upsize.
         TRY(set_run(s, gr, 0, st, [&](cudaStream_t cs) {
             return set_phase_a(s, d_offsets, d_ops, d_keys, d_vals, d_vals_out, d_bits_out, ng,
-                               false, cs);
+                               !gr, false, cs);
         }));
         TRY(set_release_later(s, st));
         set_fill_spares(s, st);
@@ -2419,7 +2421,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
     } else if (deferred) {
         TRY(set_run(s, gr, 2, st, [&](cudaStream_t cs) {
             TRY(set_phase_a(s, d_offsets, d_ops, d_keys, d_vals, d_vals_out, d_bits_out, ng,
-                            resize, cs));
+                            !gr, resize, cs));
             return set_phase_b(s, ng, cs);
         }));
         CK(cudaStreamSynchronize(st));
@@ -2428,7 +2430,7 @@ dyc_status dyc_set_apply(dyc_set *s, const uint32_t *d_offsets, const uint32_t *
         s->last.split_phases = 1;
         TRY(set_run(s, gr, 0, st, [&](cudaStream_t cs) {
             return set_phase_a(s, d_offsets, d_ops, d_keys, d_vals, d_vals_out, d_bits_out, ng,
-                               true, cs);
+                               !gr, true, cs);
         }));
         CK(cudaStreamSynchronize(st));
         TRY(upsize_policy());

@@ -97,7 +97,8 @@ __device__ __forceinline__ uint32_t table_at(const uint32_t *__restrict__ tidx,
 // Start of a set batch of off[ntables] ops, in one launch: zero the batch
 // counters (all but kCtrHostN, copied in before this kernel), the probe
 // phase's counters (gctr, gctr_words words), the result bits and the per-
-// table new-key counts; set the single bits; fill the op index.
+// table new-key counts; set the single bits; fill the op index and the bins'
+// tables.
 template <int KB>
 __global__ void __launch_bounds__(256) k_set_prep(const __grid_constant__ ApplyScratch A,
                                                   const uint32_t *__restrict__ off,
@@ -111,8 +112,14 @@ __global__ void __launch_bounds__(256) k_set_prep(const __grid_constant__ ApplyS
     if (id < (uint64_t)kCtrSlots && id != (uint64_t)kCtrHostN) A.ctr[id] = 0ull;
     if (gctr != nullptr && id < gctr_words) gctr[id] = 0ull;
     for (uint64_t t = id; t < A.ntables; t += stride) A.tup[t] = A.ter[t] = 0u;
-    for (uint64_t b = id; b * kTidxStep < n; b += stride)
-        A.tidx[b] = table_of(off, A.ntables, (uint32_t)(b * kTidxStep));
+    for (uint64_t b = id; b * kTidxStep < n; b += stride) {
+        const uint32_t i = (uint32_t)(b * kTidxStep), t = table_of(off, A.ntables, i);
+        A.tidx[b] = t;
+        if (i % kSetBinMean != 0u) continue;
+        // a bin starts here: its first table, and whether it is the only one
+        const uint32_t end = (uint32_t)(n - i < kSetBinMean ? n : i + kSetBinMean);
+        A.bin_tables[i / kSetBinMean] = make_uint2(t, off[t + 1] >= end ? 1u : 0u);
+    }
     for (uint64_t w = id; w < (n + 31) / 32; w += stride) {
         if (bits != nullptr) bits[w] = 0u;
         A.single[w] = 0xffffffffu;

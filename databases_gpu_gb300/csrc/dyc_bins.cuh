@@ -44,6 +44,7 @@ constexpr uint32_t kSplitBins = 4096;               // bins counted in shared me
 constexpr int kGroupThreads = 512;
 constexpr int kGroupR = kBinCap / kGroupThreads;    // records per thread (k_bin_group)
 constexpr int kGroupPre = kBinMean / kGroupThreads; // of them, read along with the count
+constexpr uint32_t kBinOffs = 64;                   // tables of a set batch's bin told apart in shared memory
 constexpr int kGroupTab = 2 * kBinCap;              // cells of a bin's first table, half as many of its second
 
 // An op of a small batch's bin: index << 2 | code (2 bits; any other code reads).
@@ -95,31 +96,33 @@ __device__ __forceinline__ void clear_single(const BinScratch &B, uint32_t i) {
     atomicAnd(&B.single[i >> 5], ~(1u << (i & 31)));
 }
 
-// A table's bins in a set batch: ops [o0, o1) get bins o0 / kBinMean + t ..
-// o1 / kBinMean + t, so no two tables share one and a bin holds about kBinMean
-// ops. Offsets are clamped to n and the bins to nbins, so device offsets that
-// are out of order (reported by the call) stay inside the scratch.
-struct TableBins {
-    uint32_t first, n;
-};
-__device__ __forceinline__ TableBins table_bins(const BinScratch &B, const uint32_t *off, uint32_t t,
-                                                uint64_t n) {
+// The bin of a set batch's op: its table's ops are [o0, o1), its key's hash names
+// a place among them, and a bin holds the ops of kSetBinMean places (tables with
+// few ops share one, and no bin belongs to a table without any). So a bin gets
+// kSetBinMean ops of distinct keys on average, whatever the tables are, and its
+// ops belong to the tables that have ops at its places. Offsets are clamped to
+// n, so device offsets that are out of order (reported by the call) stay inside
+// the scratch. (With bins of its own every table took 16 KB of records: 1.6 GB
+// of scratch for a 1000-op batch over 100000 tables.)
+static_assert(kSetBinMean % kTidxStep == 0, "the table of a bin's first place is in tidx");
+__device__ __forceinline__ uint32_t set_bin(const uint32_t *off, uint32_t t, uint32_t hash, uint64_t n) {
     const uint64_t a = __ldg(off + t), b = __ldg(off + t + 1);
-    const uint32_t o0 = (uint32_t)(a < n ? a : n) / kBinMean, o1 = (uint32_t)(b < n ? b : n) / kBinMean;
-    TableBins r{o0 + t, o1 >= o0 ? o1 - o0 + 1u : 1u};
-    if (r.first >= B.nbins) r.first = B.nbins - 1u;
-    if (r.n > B.nbins - r.first) r.n = B.nbins - r.first;
-    return r;
+    const uint32_t o0 = (uint32_t)(a < n ? a : n - 1), o1 = (uint32_t)(b < n ? b : n);
+    return (o0 + (o1 > o0 ? __umulhi(hash, o1 - o0) : 0u)) / kSetBinMean;
 }
+
+// A record's tag in a set batch: the same key in different tables of a bin has
+// different tags.
+__device__ __forceinline__ uint32_t table_mix(uint32_t t) { return t * 0x9E3779B1u; }
 
 // Where the records of the bins that went over start in `hot`: their counts
 // summed in bin order. Every block of the pass that needs the starts computes
 // them all (the same values, so the writes agree).
-template <int KB> __device__ __noinline__ void plan_hot(const BinScratch &B) {
+template <int KB> __device__ __noinline__ void plan_hot(const BinScratch &B, uint32_t nbins) {
     __shared__ uint32_t s_w[kSplitThreads / 32];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t per = (B.nbins + kSplitThreads - 1) / kSplitThreads;
-    const uint32_t b0 = threadIdx.x * per, b1 = min(b0 + per, B.nbins);
+    const uint32_t per = (nbins + kSplitThreads - 1) / kSplitThreads;
+    const uint32_t b0 = threadIdx.x * per, b1 = min(b0 + per, nbins);
     uint32_t sum = 0u;
     for (uint32_t b = b0; b < b1; ++b) {
         const uint32_t c = B.count[b];
@@ -152,8 +155,8 @@ template <int KB> __device__ __noinline__ void plan_hot(const BinScratch &B) {
 // Ops beyond a bin's capacity are not written, which raises B.state[kBinOver]:
 // the pass HOT then gives all ops of such bins a record in `hot` (an insert or
 // erase batch: k_bin_hot).
-// SET: the ops of table t are [off[t], off[t + 1]) and go to its own bins; a
-// block's ops then fall into a short range of bins (its records land in long
+// SET: the ops of table t are [off[t], off[t + 1]) and go to bins of its range;
+// a block's ops then fall into a short range of bins (its records land in long
 // runs), and ops outside a range of kSplitBins take their places one by one.
 // tile_ops (at most PER * 512, a multiple of 512): the ops a block takes, so
 // that the blocks come to whole waves. Loads go out kLoad ops at a time: in a
@@ -191,13 +194,12 @@ __global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
         if (A.ctr != nullptr && gid < (uint64_t)kCtrSlots) A.ctr[gid] = 0ull;
     }
     bool went_over = false, planned = false;
-    auto put = [&](uint32_t b, uint32_t p, uint32_t tag, uint32_t word, uint32_t t) {
+    auto put = [&](uint32_t b, uint32_t p, uint32_t tag, uint32_t word) {
         const unsigned long long r = (unsigned long long)tag | ((unsigned long long)word << 32);
         if (HOT) {
             B.hot[(uint64_t)B.start[b] + p] = r;
             return;
         }
-        if (SET && p == 0u) B.tid[b] = t;
         if (p < (uint32_t)kBinCap) B.rec[(uint64_t)b * kBinCap + p] = r;
         else went_over = true;
     };
@@ -207,9 +209,9 @@ __global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
             const uint64_t last = (tile + tile_ops < n ? tile + tile_ops : n) - 1;
             const uint32_t t0 = table_at(A.tidx, off, (uint32_t)tile, (uint32_t)tile);
             const uint32_t t1 = table_at(A.tidx, off, (uint32_t)last, (uint32_t)last);
-            const TableBins a = table_bins(B, off, t0, n), b = table_bins(B, off, t1, n);
-            lo = a.first;
-            nb = b.first + b.n > lo ? b.first + b.n - lo : 0u;
+            const uint32_t hi = set_bin(off, t1, 0xffffffffu, n);
+            lo = set_bin(off, t0, 0u, n);
+            nb = hi >= lo ? hi - lo + 1u : 0u;
             const bool all = nb <= kSplitBins;
             if (!all) nb = kSplitBins;
             if (HOT && all) {  // no bin of the tile's tables went over
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
         }
         if (HOT && !planned) {
             planned = true;
-            plan_hot<KB>(B);
+            plan_hot<KB>(B, SET ? (uint32_t)set_nbins(n) : B.nbins);
         }
         if (!SET && !HOT) {
             const uint64_t words = ((tile + tile_ops < n ? tile + tile_ops : n) + 31) / 32;
@@ -254,17 +256,17 @@ __global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
             tag[j] = bin_tag(k);
             at[j] = 0xffffffffu;
             if (k == 0) continue;
-            uint32_t b, t = 0u;
+            uint32_t b;
             if (SET) {
-                t = table_at(A.tidx, off, (uint32_t)i, (uint32_t)i);
-                const TableBins tb = table_bins(B, off, t, n);
-                b = tb.first + bin_of<KB>(k, tb.n);
+                const uint32_t t = table_at(A.tidx, off, (uint32_t)i, (uint32_t)i);
+                b = set_bin(off, t, cell_hash((uint64_t)k), n);
+                tag[j] ^= table_mix(t);
             } else {
                 b = bin_of<KB>(k, nb);
             }
             if (HOT && B.count[b] <= (uint32_t)kBinCap) continue;
             if (!SET || b - lo < nb) at[j] = (b - lo) << 13 | code << 26;
-            else put(b, atomicAdd(&cursor[b], 1u), tag[j], rec_word(A, (uint32_t)i, code), t);
+            else put(b, atomicAdd(&cursor[b], 1u), tag[j], rec_word(A, (uint32_t)i, code));
         }
 #pragma unroll
         for (int j = 0; j < PER; ++j)
@@ -280,8 +282,7 @@ __global__ void __launch_bounds__(kSplitThreads, SET ? 3 : 2) k_bin_scatter(
             if (at[j] == 0xffffffffu) continue;
             const uint32_t b = (at[j] >> 13) & 0x1fffu, p = s_cnt[b] + (at[j] & 0x1fffu);
             const uint32_t i = (uint32_t)tile + (uint32_t)j * kSplitThreads + threadIdx.x;
-            put(lo + b, p, tag[j], rec_word(A, i, at[j] >> 26),
-                (SET && !HOT && p == 0u) ? table_at(A.tidx, off, i, i) : 0u);
+            put(lo + b, p, tag[j], rec_word(A, i, at[j] >> 26));
         }
         __syncthreads();  // the counts are reused by the next tile
     }
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_bin_hot(
     __shared__ uint32_t s_best[kTile];
     __shared__ uint32_t s_cnt[kSplitBins];  // records per bin, then where they go
     if (B.state[kBinOver] == 0u) return;
-    plan_hot<KB>(B);
+    plan_hot<KB>(B, B.nbins);
     for (uint64_t tile = (uint64_t)blockIdx.x * kTile; tile < n; tile += (uint64_t)gridDim.x * kTile) {
         for (uint32_t c = threadIdx.x; c < kTile; c += kSplitThreads)
             s_best[c] = MODE == kBinModeInsert ? 0u : kNone;
@@ -418,24 +419,38 @@ __device__ __forceinline__ bool take_ranges(const ApplyScratch &A, uint32_t nkey
     return ok;
 }
 
+// The table of op i of a set batch's bin (bin_tables: its first table, and 1
+// when that is the only one).
+__device__ __forceinline__ uint32_t bin_table(const ApplyScratch &A, const uint32_t *off, uint2 tables,
+                                              uint32_t i) {
+    return tables.y ? tables.x : table_at(A.tidx, off, i, i);
+}
+
 template <int KB, int MODE, bool SET>
 __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &A, const void *keys,
-                                       uint32_t bin, uint32_t m, HotSmem &M) {
+                                       uint32_t bin, uint32_t m, const uint32_t *off, HotSmem &M) {
     using K = typename SlotT<KB>::K;
     const uint32_t tid = threadIdx.x, lane = tid & 31, nt = kGroupThreads;
     const unsigned long long *rec = B.hot + B.start[bin];
-    const uint32_t table = SET ? B.tid[bin] : 0u;
-    // record r: its key, op index and word
-    auto op_at = [&](uint32_t r, K &k, uint32_t &i, uint32_t &w) -> bool {
+    const uint2 tables = SET ? B.tables[bin] : make_uint2(0u, 1u);
+    auto table_of_op = [&](uint32_t i) { return bin_table(A, off, tables, i); };
+    // record r, of a key of the part: its key, table, tag, op index and word. (A
+    // bin's tables are at most kSetBinMean, so that many of its keys share one
+    // of these sums at most, and a part of one sum fits.)
+    static_assert(kSetBinMean <= kHotMax, "a part that cannot be split further fits");
+    uint64_t mask = 0ull, part = 0ull;
+    auto op_at = [&](uint32_t r, K &k, uint32_t &t, uint32_t &tag, uint32_t &i, uint32_t &w) -> bool {
         if (r >= m) return false;
+        tag = (uint32_t)rec[r];
         w = (uint32_t)(rec[r] >> 32);
         i = rec_index(A, w);
         k = load_key<KB>(keys, i);
-        return true;
+        t = SET ? table_of_op(i) : 0u;
+        return (part_bits((uint64_t)k + (uint64_t)t * 0x9E3779B97F4A7C15ull) & mask) == part;
     };
-    // key k's cell; claimed for op i when the key has none yet (claim)
-    auto cell_of = [&](K k, uint32_t i, bool claim) -> uint32_t {
-        uint32_t h = bin_cell<11>(bin_tag(k));
+    // the cell of key k of table t; claimed for op i when it has none yet (claim)
+    auto cell_of = [&](K k, uint32_t t, uint32_t tag, uint32_t i, bool claim) -> uint32_t {
+        uint32_t h = bin_cell<11>(tag);
         static_assert(kHotTab == 1u << 11, "bin_cell takes 11 bits");
         // claims stop at kHotMax keys, plus one per thread on the way: cells
         // stay free and the probe ends
@@ -450,7 +465,7 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
                     return h;
                 }
             }
-            if (load_key<KB>(keys, f - 1u) == k) return h;
+            if (load_key<KB>(keys, f - 1u) == k && (!SET || tables.y || table_of_op(f - 1u) == t)) return h;
             h = (h + 1u) & (kHotTab - 1u);
         }
     };
@@ -462,7 +477,8 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
     __syncthreads();
     while (M.top != 0u) {
         const uint32_t top = M.top;
-        const uint64_t mask = M.part_mask[top - 1], part = M.part[top - 1];
+        mask = M.part_mask[top - 1];
+        part = M.part[top - 1];
         for (uint32_t c = tid; c < kHotTab; c += nt) {
             M.first[c] = 0u;
             M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
@@ -473,9 +489,9 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
         for (uint32_t r0 = 0; r0 < m; r0 += nt) {
             if (__any_sync(kFull, *(volatile uint32_t *)&M.over != 0u)) break;
             K k = 0;
-            uint32_t i = 0u, w = 0u;
-            const bool sel = op_at(r0 + tid, k, i, w) && (part_bits((uint64_t)k) & mask) == part;
-            const uint32_t h = sel ? cell_of(k, i, true) : 0u;
+            uint32_t t = 0u, tag = 0u, i = 0u, w = 0u;
+            const bool sel = op_at(r0 + tid, k, t, tag, i, w);
+            const uint32_t h = sel ? cell_of(k, t, tag, i, true) : 0u;
             __syncwarp();
             const unsigned peers = __match_any_sync(kFull, sel ? h : 0x80000000u | lane);
             if (MODE == kBinModeMixed) {
@@ -493,7 +509,10 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
         const bool over = M.over != 0u;
         __syncthreads();
         if (tid == 0) {
-            if (over) {  // two parts by one more bit; nothing has been written for this one
+            if (over && mask == ~0ull) {  // only with offsets that are out of order
+                note_bad(A);
+                M.top = top - 1u;
+            } else if (over) {  // two parts by one more bit; nothing has been written for this one
                 M.part_mask[top - 1] = M.part_mask[top] = 2ull * mask + 1ull;
                 M.part[top] = part | (mask + 1ull);
                 M.top = top + 1u;
@@ -524,7 +543,7 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
                 ((K *)A.dkey)[d] = load_key<KB>(keys, M.first[c] - 1u);
                 A.dcnt[d] = M.cnt[c];
                 A.dseg[d] = (unsigned long long)at << 32;
-                if (SET) A.dtid[d] = table;
+                if (SET) A.dtid[d] = table_of_op(M.first[c] - 1u);
                 list_long(A, d, M.cnt[c], &M.nwarp, &M.nmid, M.bwarp, M.bmid);
                 M.off[c] = at;
             }
@@ -533,12 +552,15 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
         uint32_t ins = 0u;
         for (uint32_t r0 = 0; r0 < m; r0 += nt) {
             K k = 0;
-            uint32_t i = 0u, w = 0u;
-            const bool sel = op_at(r0 + tid, k, i, w) && (part_bits((uint64_t)k) & mask) == part;
-            const uint32_t h = sel ? cell_of(k, i, false) : 0u;
+            uint32_t t = 0u, tag = 0u, i = 0u, w = 0u;
+            const bool sel = op_at(r0 + tid, k, t, tag, i, w);
+            const uint32_t h = sel ? cell_of(k, t, tag, i, false) : 0u;
             if constexpr (MODE == kBinModeMixed) {
                 const bool several = sel && M.cnt[h] > 1u;
-                if (SET && sel && !several) ins += w & 1u;
+                if (SET && sel && !several && (w & 1u)) {
+                    if (tables.y) ++ins;
+                    else atomicAdd(&A.tup[t], 1u);
+                }
                 __syncwarp();
                 const unsigned peers = __match_any_sync(kFull, several ? h : 0x80000000u | lane);
                 const int lead = __ffs(peers) - 1;
@@ -555,7 +577,7 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
         }
         if (SET && MODE == kBinModeMixed) {
             ins = __reduce_add_sync(kFull, ins);
-            if (lane == 0 && ins && table < A.ntables) atomicAdd(&A.tup[table], ins);
+            if (lane == 0 && ins) atomicAdd(&A.tup[tables.x], ins);
         }
         __syncthreads();
     }
@@ -566,8 +588,8 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
 // mixed batch the ops of keys with several ops lose theirs and the keys are
 // listed: id d gets dkey, dcnt, dseg and (SET) dtid, and its op indexes a
 // range of seg; ids with more than kShortSeg ops go to wseg or mid as well.
-// SET: the inserts among the other ops are counted as upserts of the bin's
-// table (the upsize policy's insert batch).
+// SET: the inserts among the other ops are counted as upserts of their tables
+// (the upsize policy's insert batch); sized: the grid is the batch's bins.
 // A record leaves its number in its key's cell with a plain store; the record
 // that stays leads the key's group, and most records find themselves there.
 // Only records whose cell another key has claim one in a second table by
@@ -578,12 +600,17 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
 template <int KB, int MODE, bool SET>
 __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     const __grid_constant__ BinScratch B, const __grid_constant__ ApplyScratch A,
-    const void *__restrict__ keys) {
+    const uint32_t *__restrict__ off, const void *__restrict__ keys, bool sized) {
     after_previous();
     using K = typename SlotT<KB>::K;
     struct Smem {
         uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kBinCap];
         uint16_t first[kGroupTab];
+        // in a bin of several tables: a record's table (its id from the first
+        // one's on; kBinOffs: looked up by op), where the tables end, and the
+        // inserts that count for each
+        uint8_t table[SET ? kBinCap : 1];
+        uint32_t off[SET ? kBinOffs : 1], ins[SET ? kBinOffs : 1];
     };
     __shared__ __align__(16) unsigned char s_raw[sizeof(Smem)];
     static_assert(sizeof(HotSmem) <= sizeof(Smem), "one block of shared memory for both");
@@ -591,6 +618,10 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     __shared__ uint32_t s_place, s_nwarp, s_nmid, s_ok, s_ins;  // place: ops | keys << 16
     __shared__ unsigned long long s_bseg, s_bkey, s_bwarp, s_bmid;
     const uint32_t tid = threadIdx.x, bin = blockIdx.x;
+    // nothing there, and no counts to zero
+    if (SET && !sized && bin >= set_nbins(set_op_count(A, off))) return;
+    const uint2 tables = SET ? B.tables[bin] : make_uint2(0u, 1u);
+    const bool one = tables.y != 0u;
     // the first kGroupPre rounds of records are read along with their count
     unsigned long long x[kGroupR];
 #pragma unroll
@@ -620,6 +651,11 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
                 M.first[bin_cell<12>(tag)] = (uint16_t)r;  // one of the cell's records stays
             }
         }
+        if (SET && !one && tid < kBinOffs) {
+            const uint32_t t = tables.x + 1u + tid;
+            M.off[tid] = off[t < A.ntables ? t : A.ntables];
+            M.ins[tid] = 0u;
+        }
     }
     // the records written to `hot`: all of the bin's ops, except those that
     // cannot count (k_bin_hot), and where device offsets that are out of order
@@ -631,10 +667,26 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     if (tid == 0) B.count[bin] = B.cursor[bin] = 0u;
     if (bin == 0 && tid < (uint32_t)kBinStates) B.state[tid] = 0u;
     if (m > (uint32_t)kBinCap) {
-        group_hot<KB, MODE, SET>(B, A, keys, bin, nhot, *reinterpret_cast<HotSmem *>(s_raw));
+        group_hot<KB, MODE, SET>(B, A, keys, bin, nhot, off, *reinterpret_cast<HotSmem *>(s_raw));
         return;
     }
+    if (SET && !one) {
+        for (uint32_t r = tid; r < m; r += kGroupThreads) {
+            const uint32_t i = rec_index(A, M.word[r]);
+            uint32_t t = 0u;  // ends up to and with i
+#pragma unroll
+            for (uint32_t w = kBinOffs / 2; w; w >>= 1)
+                if (M.off[t + w - 1u] <= i) t += w;
+            M.table[r] = (uint8_t)(t + (M.off[t] <= i ? 1u : 0u));
+        }
+        __syncthreads();
+    }
     uint32_t lr[kGroupR];  // the key's lead record | the op's rank << 16
+    // the table of record r, op i
+    auto table_rec = [&](uint32_t r, uint32_t i) -> uint32_t {
+        if (!SET || one) return tables.x;
+        return M.table[r] == kBinOffs ? table_at(A.tidx, off, i, i) : tables.x + M.table[r];
+    };
     static_assert(kGroupTab == 1 << 12 && kBinCap == 1 << 11, "cells of 12 and 11 bits");
 #pragma unroll
     for (int q = 0; q < kGroupR; ++q) {
@@ -643,9 +695,14 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
         if (r >= m) continue;
         const uint32_t tag = M.tag[r], w = M.word[r];
         auto same = [&](uint32_t x) {
-            return x == r || (M.tag[x] == tag &&
-                              (KB == 4 || load_key<KB>(keys, rec_index(A, M.word[x])) ==
-                                              load_key<KB>(keys, rec_index(A, w))));
+            if (x == r) return true;
+            if (M.tag[x] != tag) return false;
+            if (KB == 4 && (!SET || one)) return true;
+            const uint32_t i = rec_index(A, w), j = rec_index(A, M.word[x]);
+            if (KB != 4 && load_key<KB>(keys, j) != load_key<KB>(keys, i)) return false;
+            if (!SET || one || M.table[x] != M.table[r]) return !SET || one;
+            // 4-byte keys: tag and table give the key
+            return M.table[r] != kBinOffs || table_rec(x, j) == table_rec(r, i);
         };
         uint32_t lead = M.first[bin_cell<12>(tag)];
         if (!same(lead)) {
@@ -681,7 +738,11 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             if (r >= m) continue;
             const uint32_t c = M.cnt[lead] + 1u;
             if (c == 1u) {
-                if (SET) ins += M.word[r] & 1u;
+                if (SET && (M.word[r] & 1u)) {
+                    if (one) ++ins;
+                    else if (M.table[r] != kBinOffs) atomicAdd(&M.ins[M.table[r]], 1u);
+                    else atomicAdd(&A.tup[table_rec(r, rec_index(A, M.word[r]))], 1u);
+                }
             } else if (lead == r) {
                 M.tab[r] = atomicAdd(&s_place, c | 1u << 16);
                 if (c > kShortSeg) atomicAdd(c > kWarpSeg ? &s_nmid : &s_nwarp, 1u);
@@ -692,8 +753,8 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             if ((tid & 31) == 0 && ins) atomicAdd(&s_ins, ins);
         }
         __syncthreads();
-        const uint32_t table = SET ? B.tid[bin] : 0u;
-        if (SET && tid == 0 && s_ins && table < A.ntables) atomicAdd(&A.tup[table], s_ins);
+        if (SET && tid == 0 && s_ins) atomicAdd(&A.tup[tables.x], s_ins);
+        if (SET && !one && tid < kBinOffs && M.ins[tid]) atomicAdd(&A.tup[tables.x + tid], M.ins[tid]);
         if (s_place == 0u) return;
         if (tid == 0) {
             s_ok = take_ranges(A, s_place >> 16, s_place & 0xffffu, s_nwarp, s_nmid, s_bkey, s_bseg,
@@ -714,10 +775,11 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             clear_single(B, i);
             if (lead == r) {
                 const uint32_t d = (uint32_t)s_bkey + (M.tab[lead] >> 16);
-                ((K *)A.dkey)[d] = KB == 4 ? (K)M.tag[r] : load_key<KB>(keys, i);
+                const uint32_t t = table_rec(r, i);
+                ((K *)A.dkey)[d] = KB == 4 ? (K)(M.tag[r] ^ table_mix(t)) : load_key<KB>(keys, i);
                 A.dcnt[d] = c;
                 A.dseg[d] = (unsigned long long)place << 32;
-                if (SET) A.dtid[d] = table;
+                if (SET) A.dtid[d] = t;
                 list_long(A, d, c, &s_nwarp, &s_nmid, s_bwarp, s_bmid);
             }
         }

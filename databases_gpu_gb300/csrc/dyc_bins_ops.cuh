@@ -41,11 +41,11 @@ template <int KB> cudaError_t Ops<KB>::load_bins() {
 }
 
 // The split, the bins that went over, and the grouping (cap_n sizes the grids;
-// a set's kernels read the op count on the device).
+// a set's kernels read the op count on the device, and it is cap_n if sized).
 template <int KB, int MODE, bool SET>
 cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
                        const uint32_t *off, const uint8_t *ops, const void *keys, uint64_t cap_n,
-                       unsigned long long *ctr, uint32_t *bits) {
+                       unsigned long long *ctr, uint32_t *bits, bool sized = true) {
     // whole waves of the blocks an SM holds, of at most 16 ops a thread (below
     // 2^21 ops, where 8 fill the chip, of 8)
     const uint64_t slots = (SET ? 3u : 2u) * (uint64_t)std::max(L.sms, 1), unit = kSplitThreads;
@@ -65,7 +65,8 @@ cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScrat
                      ops, keys, cap_n, ctr, nullptr, 8u * kSplitThreads);
     else
         launch_after(k_bin_hot<KB, MODE>, (unsigned)some, kSplitThreads, 0, L.stream, B, A, keys, cap_n);
-    launch_after(k_bin_group<KB, MODE, SET>, (unsigned)(B.nbins), kGroupThreads, 0, L.stream, B, A, keys);
+    launch_after(k_bin_group<KB, MODE, SET>, SET ? (unsigned)set_nbins(cap_n) : B.nbins, kGroupThreads, 0,
+                 L.stream, B, A, off, keys, sized);
     return cudaGetLastError();
 }
 
@@ -85,11 +86,11 @@ cudaError_t Ops<KB>::bin_group(const LaunchCtx &L, const BinScratch &B, const Ap
 template <int KB>
 cudaError_t Ops<KB>::set_group(const LaunchCtx &L, const ApplyScratch &A, const BinScratch &B,
                                const uint32_t *off, const uint8_t *ops, const void *keys,
-                               uint64_t n, uint32_t *bits, Counters *gctr) {
+                               uint64_t n, bool sized, uint32_t *bits, Counters *gctr) {
     const uint64_t work = std::max<uint64_t>(n / 32 + 1, A.ntables);
     launch_after(k_set_prep<KB>, (unsigned)((unsigned)std::min<uint64_t>((work + 255) / 256, 8ull * L.sms)), 256, 0, L.stream, A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
     if (n == 0) return cudaGetLastError();
-    return bin_passes<KB, kBinModeMixed, true>(L, B, A, off, ops, keys, n, nullptr, nullptr);
+    return bin_passes<KB, kBinModeMixed, true>(L, B, A, off, ops, keys, n, nullptr, nullptr, sized);
 }
 
 template <int KB, int SB>
