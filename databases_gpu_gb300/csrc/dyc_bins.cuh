@@ -583,6 +583,17 @@ __device__ __noinline__ void group_hot(const BinScratch &B, const ApplyScratch &
     }
 }
 
+template <bool SET> struct GroupSmem {
+    uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kBinCap];
+    uint16_t first[kGroupTab];
+    // in a bin of several tables: a record's table (its id from the first
+    // one's on; kBinOffs: looked up by op), where the tables end, and the
+    // inserts that count for each
+    uint8_t table[SET ? kBinCap : 1];
+    uint32_t off[SET ? kBinOffs : 1], ins[SET ? kBinOffs : 1];
+};
+template <bool SET> constexpr size_t kGroupSmem = sizeof(GroupSmem<SET>);
+
 // One block per bin: its ops grouped by key in shared memory. Insert batches
 // keep the single bit of a key's last op, erase batches of its first. In a
 // mixed batch the ops of keys with several ops lose theirs and the keys are
@@ -603,15 +614,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     const uint32_t *__restrict__ off, const void *__restrict__ keys, bool sized) {
     after_previous();
     using K = typename SlotT<KB>::K;
-    struct Smem {
-        uint32_t tag[kBinCap], word[kBinCap], cnt[kBinCap], tab[kBinCap];
-        uint16_t first[kGroupTab];
-        // in a bin of several tables: a record's table (its id from the first
-        // one's on; kBinOffs: looked up by op), where the tables end, and the
-        // inserts that count for each
-        uint8_t table[SET ? kBinCap : 1];
-        uint32_t off[SET ? kBinOffs : 1], ins[SET ? kBinOffs : 1];
-    };
+    using Smem = GroupSmem<SET>;
     __shared__ __align__(16) unsigned char s_raw[sizeof(Smem)];
     static_assert(sizeof(HotSmem) <= sizeof(Smem), "one block of shared memory for both");
     Smem &M = *reinterpret_cast<Smem *>(s_raw);
@@ -1004,7 +1007,8 @@ template <int KB, int SB> struct BinSmem {
     alignas(128) unsigned char stage[kSmallWarps][32 * SB];  // between the probes: tables, bitmaps
     typename SlotT<KB>::K key[kSmallCap];
     uint32_t word[kSmallCap];
-    uint32_t cnt[kSmallCap];  // per first op of a key: the word that counts; mixed: ops | place in seg << 16
+    // per first op of a key: the word that counts; mixed: its ops | place in seg << 16
+    uint32_t cnt[kSmallCap];
     uint16_t multi[kSmallCap];  // keys with several ops, and those of more than kSmallLong
     uint16_t longs[kBinSmallOps / kSmallLong];  // each has more ops than that
     uint64_t part_mask[72], part[72];  // parts of a bin that went over (each split adds one)

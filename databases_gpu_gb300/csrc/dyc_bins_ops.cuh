@@ -40,6 +40,21 @@ template <int KB> cudaError_t Ops<KB>::load_bins() {
     return e;
 }
 
+// A grid within a tuner's cap on the resident blocks.
+inline unsigned capped(const LaunchCtx &L, uint64_t blocks) {
+    const uint64_t cap = (uint64_t)std::max(L.max_blocks_per_sm, 0) * (uint64_t)std::max(L.sms, 1);
+    return (unsigned)(cap && blocks > cap ? cap : std::max<uint64_t>(blocks, 1));
+}
+
+// The same for a kernel with a block for every bin: dynamic shared memory that
+// leaves an SM room for no more blocks (`used` bytes each) than the cap.
+constexpr size_t kSmemPerSm = 228 << 10;
+inline size_t cap_pad(const LaunchCtx &L, size_t used) {
+    if (L.max_blocks_per_sm <= 0) return 0;
+    const size_t bytes = kSmemPerSm / (size_t)(L.max_blocks_per_sm + 1) + 16;
+    return bytes > used ? bytes - used : 0;
+}
+
 // The split, the bins that went over, and the grouping (cap_n sizes the grids;
 // a set's kernels read the op count on the device, and it is cap_n if sized).
 template <int KB, int MODE, bool SET>
@@ -53,20 +68,25 @@ cudaError_t bin_passes(const LaunchCtx &L, const BinScratch &B, const ApplyScrat
     const uint64_t waves = (cap_n + slots * per * unit - 1) / (slots * per * unit);
     const uint64_t share = (cap_n + waves * slots - 1) / (waves * slots);
     const uint32_t tile = (uint32_t)((share + unit - 1) / unit * unit);
-    const unsigned blocks = (unsigned)((cap_n + tile - 1) / tile);
-    if (per == 16)
-        launch_after(k_bin_scatter<KB, 16, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits, tile);
-    else
-        launch_after(k_bin_scatter<KB, 8, SET, false>, (unsigned)(blocks), kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits, tile);
+    const unsigned blocks = capped(L, (cap_n + tile - 1) / tile);
+    auto split = per == 16 ? k_bin_scatter<KB, 16, SET, false> : k_bin_scatter<KB, 8, SET, false>;
+    launch_after(split, blocks, kSplitThreads, 0, L.stream, B, A, off, ops, keys, cap_n, ctr, bits, tile);
     // nothing to do in most batches: a fixed grid of one wave
-    const unsigned some = (unsigned)std::min<uint64_t>((cap_n + 8 * unit - 1) / (8 * unit), 4u * (uint64_t)std::max(L.sms, 1));
+    const unsigned some = capped(L, std::min<uint64_t>((cap_n + 8 * unit - 1) / (8 * unit),
+                                                       4u * (uint64_t)std::max(L.sms, 1)));
     if constexpr (MODE == kBinModeMixed)
-        launch_after(k_bin_scatter<KB, 8, SET, true>, (unsigned)(some), kSplitThreads, 0, L.stream, B, A, off,
-                     ops, keys, cap_n, ctr, nullptr, 8u * kSplitThreads);
+        launch_after(k_bin_scatter<KB, 8, SET, true>, some, kSplitThreads, 0, L.stream, B, A, off, ops, keys,
+                     cap_n, ctr, nullptr, 8u * kSplitThreads);
     else
-        launch_after(k_bin_hot<KB, MODE>, (unsigned)some, kSplitThreads, 0, L.stream, B, A, keys, cap_n);
-    launch_after(k_bin_group<KB, MODE, SET>, SET ? (unsigned)set_nbins(cap_n) : B.nbins, kGroupThreads, 0,
-                 L.stream, B, A, off, keys, sized);
+        launch_after(k_bin_hot<KB, MODE>, some, kSplitThreads, 0, L.stream, B, A, keys, cap_n);
+    auto group = k_bin_group<KB, MODE, SET>;
+    const size_t pad = cap_pad(L, kGroupSmem<SET>);
+    if (pad) {
+        const cudaError_t e = allow_smem((const void *)group, (int)(kSmemPerSm / 2));
+        if (e != cudaSuccess) return e;
+    }
+    launch_after(group, SET ? (unsigned)set_nbins(cap_n) : B.nbins, kGroupThreads, pad, L.stream, B, A, off,
+                 keys, sized);
     return cudaGetLastError();
 }
 
@@ -88,7 +108,8 @@ cudaError_t Ops<KB>::set_group(const LaunchCtx &L, const ApplyScratch &A, const 
                                const uint32_t *off, const uint8_t *ops, const void *keys,
                                uint64_t n, bool sized, uint32_t *bits, Counters *gctr) {
     const uint64_t work = std::max<uint64_t>(n / 32 + 1, A.ntables);
-    launch_after(k_set_prep<KB>, (unsigned)((unsigned)std::min<uint64_t>((work + 255) / 256, 8ull * L.sms)), 256, 0, L.stream, A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
+    launch_after(k_set_prep<KB>, capped(L, std::min<uint64_t>((work + 255) / 256, 8ull * L.sms)), 256, 0,
+                 L.stream, A, off, bits, (unsigned long long *)gctr, (uint32_t)(sizeof(Counters) / 8));
     if (n == 0) return cudaGetLastError();
     return bin_passes<KB, kBinModeMixed, true>(L, B, A, off, ops, keys, n, nullptr, nullptr, sized);
 }
@@ -100,10 +121,11 @@ cudaError_t repeat_launch(const LaunchCtx &L, const ApplyScratch &A, const Desc 
                           void *list_a, uint64_t list_cap, Counters *gctr) {
     // a listed key has at least two ops; blocks loop over keys and segments
     const uint64_t need = (n / 2 + 255) / 256 + 1, wave = 8ull * (uint64_t)(L.sms > 0 ? L.sms : 1);
-    const unsigned grid = (unsigned)std::min<uint64_t>(need, 2 * wave);
+    const unsigned grid = capped(L, std::min<uint64_t>(need, 2 * wave));
     auto k = set ? k_repeat<KB, SB, true, false>
                  : list_a ? k_repeat<KB, SB, false, true> : k_repeat<KB, SB, false, false>;
-    launch_after(k, (unsigned)(grid), 256, 0, L.stream, A, descs, ntables, ops, vals, vb, vals_out, bits_out, list_a, list_cap, gctr);
+    launch_after(k, grid, 256, 0, L.stream, A, descs, ntables, ops, vals, vb, vals_out, bits_out, list_a,
+                 list_cap, gctr);
     return cudaGetLastError();
 }
 
@@ -144,8 +166,8 @@ cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const 
     const auto bytes = sb == 32 ? bin_smem<KB, 32> : sb == 64 ? bin_smem<KB, 64> : bin_smem<KB, 128>;
     const cudaError_t e = allow_smem((const void *)k, (int)bytes(mode, kBinSmallOps));
     if (e != cudaSuccess) return e;
-    launch_after(k, (unsigned)((n + kBinSmallMean - 1) / kBinSmallMean), kSmallThreads, bytes(mode, n), L.stream,
-                 D, S, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr);
+    launch_after(k, (unsigned)((n + kBinSmallMean - 1) / kBinSmallMean), kSmallThreads, bytes(mode, n),
+                 L.stream, D, S, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr);
     return cudaGetLastError();
 }
 

@@ -99,7 +99,8 @@ cudaError_t Ops<KB>::place(const LaunchCtx &L, const Desc &D, int sb, const Scra
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_place<KB, SB, true> : k_place<KB, SB, false>;
-        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, S, use_dedup ? 1 : 0, new_keys ? 1 : 0, keys, vals, vb, n, ctr);
+        launch_after(k, (unsigned)tile_grid(L, n), 256, 0, L.stream, D, S, use_dedup ? 1 : 0,
+                     new_keys ? 1 : 0, keys, vals, vb, n, ctr);
     });
     return cudaGetLastError();
 }
@@ -113,7 +114,8 @@ cudaError_t Ops<KB>::walk(const LaunchCtx &L, const Desc &D, int sb, const void 
     if (max_entries == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_walk<KB, SB>;
-        launch_after(k, (unsigned)(grid_for((const void *)k, L, max_entries)), 256, 0, L.stream, D, src, src_count, dst, dst_count, dst_cap, max_evict, count_new ? 1 : 0, ctr, max_entries, pub);
+        launch_after(k, (unsigned)grid_for((const void *)k, L, max_entries), 256, 0, L.stream, D, src, src_count,
+                     dst, dst_count, dst_cap, max_evict, count_new ? 1 : 0, ctr, max_entries, pub);
     });
     return cudaGetLastError();
 }
@@ -125,7 +127,8 @@ cudaError_t Ops<KB>::erase(const LaunchCtx &L, const Desc &D, int sb, const Scra
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_erase<KB, SB, true> : k_erase<KB, SB, false>;
-        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, S, use_dedup ? 1 : 0, keys, n, bits, old, vb, ctr, pub);
+        launch_after(k, (unsigned)tile_grid(L, n), 256, 0, L.stream, D, S, use_dedup ? 1 : 0, keys, n, bits,
+                     old, vb, ctr, pub);
     });
     return cudaGetLastError();
 }
@@ -138,7 +141,8 @@ cudaError_t Ops<KB>::apply_unique(const LaunchCtx &L, const Desc &D, int sb, con
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = D.l2_keep ? k_apply_unique<KB, SB, true> : k_apply_unique<KB, SB, false>;
-        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, S, ops, keys, vals, vb, vals_out, bits_out, n, ctr, single, flags);
+        launch_after(k, (unsigned)tile_grid(L, n), 256, 0, L.stream, D, S, ops, keys, vals, vb, vals_out,
+                     bits_out, n, ctr, single, flags);
     });
     return cudaGetLastError();
 }
@@ -150,7 +154,7 @@ cudaError_t Ops<KB>::apply_count(const LaunchCtx &L, const Desc &D, int sb, cons
     if (n == 0) return cudaSuccess;
     DYC_SB_DISPATCH(sb, {
         auto k = k_apply_count<KB, SB>;
-        launch_after(k, (unsigned)(tile_grid(L, n)), 256, 0, L.stream, D, ops, keys, vals, vb, n, single, ctr);
+        launch_after(k, (unsigned)tile_grid(L, n), 256, 0, L.stream, D, ops, keys, vals, vb, n, single, ctr);
     });
     return cudaGetLastError();
 }
@@ -274,9 +278,8 @@ cudaError_t Ops<KB>::set_unique(const LaunchCtx &L, const ApplyScratch &A, const
         const uint64_t warps = 64ull * (uint64_t)(L.sms > 0 ? L.sms : 1);
         const uint64_t w = max_n / 32 / warps;
         const uint32_t words = (uint32_t)(w < 1 ? 1 : w > kUniqueWords ? kUniqueWords : w);
-        launch_after(k, (unsigned)tile_grid(L, max_n), 256, 0, L.stream, A, off, descs, ntables, tctr, ops, keys,
-                                                      vals, vb, vals_out, bits_out, list_a,
-                                                      list_a_tid, list_cap, gctr, hold, words);
+        launch_after(k, (unsigned)tile_grid(L, max_n), 256, 0, L.stream, A, off, descs, ntables, tctr, ops,
+                     keys, vals, vb, vals_out, bits_out, list_a, list_a_tid, list_cap, gctr, hold, words);
     });
     return cudaGetLastError();
 }
