@@ -19,9 +19,11 @@ LIB = os.path.join(PKG, "libdycuckoo.so")
 
 SOURCES = ["dyc_ops4.cu", "dyc_ops8.cu", "dyc_bins4.cu", "dyc_bins8.cu",
            "dyc_api.cu", "dyc_server.cu"]
+# one module per key width and bucket size: a process loads those it uses
+SOURCES += [("dyc_bins_sb.cu", kb, sb) for kb in (4, 8) for sb in (32, 64, 128)]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # Device code uncompressed: unpacking it took 10 ms of the first use of a key
-# width's bin kernels (now 1.4 ms); the library is 33 MB for it, not 15.
+# width's bin kernels (0.8 without); the library is 38 MB for it.
 NVCC_FLAGS = ARCH + ["--compress-mode=none", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
                      "-I", INCLUDE, "-I", CSRC]
 
@@ -54,9 +56,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     procs = []
     objs = []
     for src in SOURCES:
-        obj = os.path.join(BUILD_DIR, src.replace(".cu", ".o"))
+        name, defs = src, []
+        if not isinstance(src, str):
+            src, kb, sb = src
+            name, defs = "dyc_bins_sb%d_%d.cu" % (kb, sb), ["-DDYC_KB=%d" % kb, "-DDYC_SB=%d" % sb]
+        obj = os.path.join(BUILD_DIR, name.replace(".cu", ".o"))
         objs.append(obj)
-        cmd = [cc] + NVCC_FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [cc] + NVCC_FLAGS + defs + ["-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             print(" ".join(cmd))
         procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE,

@@ -827,8 +827,7 @@ dyc_status create_impl(const dyc_config *cfg, Counters *ext_d, Counters *ext_h, 
         t->capacity += (uint64_t)nb * t->slots;
     }
     refresh_l2(t);
-    cudaError_t e = KB_CALL(t, load_bins);
-    if (e != cudaSuccess) return undo(fail(DYC_ECUDA, "bin kernels: %s", cudaGetErrorString(e)));
+    cudaError_t e = cudaSuccess;
     if (ext_d) {
         t->owns_ctr = false;
         t->d_ctr = ext_d;

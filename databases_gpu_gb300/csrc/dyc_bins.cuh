@@ -1050,10 +1050,9 @@ __device__ __forceinline__ uint32_t small_cell(BinSmem<KB, SB> &M, uint32_t *cel
 
 // f(key, index, bin's own) for the ops of a batch, 32 to a warp, until stop();
 // down: from the last op to the first.
-template <int KB, class F, class Stop>
+template <int KB, int kLoad, class F, class Stop>
 __device__ __forceinline__ void stream_batch(const void *keys, uint32_t n, bool down, Stop &&stop, F &&f) {
     using K = typename SlotT<KB>::K;
-    constexpr int kLoad = 8;
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t base = threadIdx.x & ~31u; base < n; base += kLoad * kSmallThreads) {
         if (stop()) break;
@@ -1121,7 +1120,7 @@ __device__ __noinline__ uint32_t gather_keys(BinSmem<KB, SB> &M, const void *key
     if (tid == 0) M.ndist = M.over = 0u;
     __syncthreads();
     uint32_t seen = 0u, rej = 0u;
-    stream_batch<KB>(
+    stream_batch<KB, 4>(
         keys, n, MODE == kBinModeInsert, [&] { return *(volatile uint32_t *)&M.over != 0u; },
         [&](K k, uint32_t i, bool here) {
             if (k == 0) {
@@ -1176,7 +1175,7 @@ __device__ __noinline__ uint32_t gather_part(BinSmem<KB, SB> &M, const void *key
     auto mine = [&](K k) {
         return k != 0 && bin_of<KB>(k, nbins) == bin && (!mask || (part_bits((uint64_t)k) & mask) == part);
     };
-    stream_batch<KB>(
+    stream_batch<KB, 4>(
         keys, n, false, [&] { return __any_sync(kFull, *(volatile uint32_t *)&M.over != 0u) != 0; },
         [&](K k, uint32_t i, bool) {
             const bool own = mine(k);
@@ -1211,7 +1210,7 @@ __device__ __noinline__ uint32_t gather_part(BinSmem<KB, SB> &M, const void *key
     const uint32_t m = done ? M.ndist : 0u;
     __syncthreads();
     if (M.nseg != 0u)
-        stream_batch<KB>(
+        stream_batch<KB, 4>(
             keys, n, false, [] { return false; },
             [&](K k, uint32_t i, bool) {
                 const bool own = mine(k);
@@ -1336,7 +1335,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_bin_small(
     for (uint32_t c = tid; c < (uint32_t)kSmallCap; c += kSmallThreads)
         M.cnt[c] = MODE == kBinModeErase ? 0xffffffffu : 0u;
     __syncthreads();
-    stream_batch<KB>(
+    stream_batch<KB, 8>(
         keys, (uint32_t)n, false,
         [&] { return MODE < kBinModeMixed && *(volatile uint32_t *)&M.m > (uint32_t)kSmallCap; },
         [&](K k, uint32_t i, bool here) {

@@ -1,6 +1,5 @@
 // Bin kernels and launchers for 4-byte keys.
 #include "dyc_bins_ops.cuh"
-template cudaError_t dyc::Ops<4>::load_bins();
 template cudaError_t dyc::Ops<4>::bin_group(const LaunchCtx &, const BinScratch &,
                                             const ApplyScratch &, int, const uint8_t *,
                                             const void *, uint32_t *, uint64_t, Counters *);

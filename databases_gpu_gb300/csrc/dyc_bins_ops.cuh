@@ -1,6 +1,6 @@
 // dyc_bins_ops.cuh -- host launchers of the bin kernels (dyc_bins.cuh) for one
 // key width. Included by dyc_bins4.cu and dyc_bins8.cu, which compile beside
-// dyc_ops4.cu and dyc_ops8.cu.
+// dyc_ops4.cu and dyc_ops8.cu, and by dyc_bins_sb.cuh.
 #pragma once
 
 #include <algorithm>
@@ -8,7 +8,7 @@
 #include <set>
 #include <utility>
 
-#include "dyc_repeat.cuh"
+#include "dyc_bins.cuh"
 
 namespace dyc {
 
@@ -23,20 +23,6 @@ inline cudaError_t allow_smem(const void *kernel, int bytes) {
     if (done.count({dev, kernel})) return cudaSuccess;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) done.insert({dev, kernel});
-    return e;
-}
-
-template <int KB> cudaError_t Ops<KB>::load_bins() {
-    static std::mutex mu;
-    static std::set<int> done;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> g(mu);
-    if (done.count(dev)) return cudaSuccess;
-    cudaFuncAttributes a;
-    e = cudaFuncGetAttributes(&a, (const void *)k_bin_group<KB, kBinModeErase, false>);
-    if (e == cudaSuccess) done.insert(dev);
     return e;
 }
 
@@ -114,20 +100,9 @@ cudaError_t Ops<KB>::set_group(const LaunchCtx &L, const ApplyScratch &A, const 
     return bin_passes<KB, kBinModeMixed, true>(L, B, A, off, ops, keys, n, nullptr, nullptr, sized);
 }
 
-template <int KB, int SB>
-cudaError_t repeat_launch(const LaunchCtx &L, const ApplyScratch &A, const Desc *descs,
-                          uint32_t ntables, bool set, const uint8_t *ops, const void *vals,
-                          uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n,
-                          void *list_a, uint64_t list_cap, Counters *gctr) {
-    // a listed key has at least two ops; blocks loop over keys and segments
-    const uint64_t need = (n / 2 + 255) / 256 + 1, wave = 8ull * (uint64_t)(L.sms > 0 ? L.sms : 1);
-    const unsigned grid = capped(L, std::min<uint64_t>(need, 2 * wave));
-    auto k = set ? k_repeat<KB, SB, true, false>
-                 : list_a ? k_repeat<KB, SB, false, true> : k_repeat<KB, SB, false, false>;
-    launch_after(k, grid, 256, 0, L.stream, A, descs, ntables, ops, vals, vb, vals_out, bits_out, list_a,
-                 list_cap, gctr);
-    return cudaGetLastError();
-}
+// The launchers of a bucket size (BinsSb).
+#define DYC_BINS_SB(sb, call) \
+    (sb == 32 ? BinsSb<KB, 32>::call : sb == 64 ? BinsSb<KB, 64>::call : BinsSb<KB, 128>::call)
 
 template <int KB>
 cudaError_t Ops<KB>::repeat(const LaunchCtx &L, const ApplyScratch &A, const Desc *descs,
@@ -135,20 +110,8 @@ cudaError_t Ops<KB>::repeat(const LaunchCtx &L, const ApplyScratch &A, const Des
                             const void *vals, uint32_t vb, void *vals_out, uint32_t *bits_out,
                             uint64_t n, void *list_a, uint64_t list_cap, Counters *gctr) {
     if (n == 0) return cudaSuccess;
-    const auto f = sb == 32   ? repeat_launch<KB, 32>
-                   : sb == 64 ? repeat_launch<KB, 64>
-                              : repeat_launch<KB, 128>;
-    return f(L, A, descs, ntables, set, ops, vals, vb, vals_out, bits_out, n, list_a, list_cap, gctr);
-}
-
-using BinFn = void (*)(Desc, Scratch, const uint8_t *, const void *, const void *, uint32_t,
-                       void *, uint32_t *, uint64_t, uint32_t, Counters *, Counters *);
-
-template <int KB, int SB> BinFn small_kernel(int mode) {
-    if (mode == kBinModeInsert) return k_bin_small<KB, SB, kBinModeInsert>;
-    if (mode == kBinModeErase) return k_bin_small<KB, SB, kBinModeErase>;
-    if (mode == kBinModeMixed) return k_bin_small<KB, SB, kBinModeMixed>;
-    return k_bin_small<KB, SB, kBinModeCount>;
+    return DYC_BINS_SB(sb, repeat(L, A, descs, ntables, set, ops, vals, vb, vals_out, bits_out, n, list_a,
+                                  list_cap, gctr));
 }
 
 template <int KB>
@@ -160,15 +123,7 @@ cudaError_t Ops<KB>::bin_small(const LaunchCtx &L, const Desc &D, int sb, const 
     const uint64_t words = bits_out ? (n + 31) / 32 : 0;
     launch_after(k_small_clear<KB>, (unsigned)((words + 255) / 256 + 1), 256, 0, L.stream, &ctr->inserted,
                  (uint32_t)(sizeof(Counters) / 8 - 1), bits_out, words);
-    const BinFn k = sb == 32   ? small_kernel<KB, 32>(mode)
-                    : sb == 64 ? small_kernel<KB, 64>(mode)
-                               : small_kernel<KB, 128>(mode);
-    const auto bytes = sb == 32 ? bin_smem<KB, 32> : sb == 64 ? bin_smem<KB, 64> : bin_smem<KB, 128>;
-    const cudaError_t e = allow_smem((const void *)k, (int)bytes(mode, kBinSmallOps));
-    if (e != cudaSuccess) return e;
-    launch_after(k, (unsigned)((n + kBinSmallMean - 1) / kBinSmallMean), kSmallThreads, bytes(mode, n),
-                 L.stream, D, S, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr);
-    return cudaGetLastError();
+    return DYC_BINS_SB(sb, small(L, D, S, mode, ops, keys, vals, vb, vals_out, bits_out, n, flags, ctr, h_ctr));
 }
 
 }  // namespace dyc

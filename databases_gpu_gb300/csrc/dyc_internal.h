@@ -281,6 +281,19 @@ cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, si
     return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
+// Launchers of the bin kernels that probe buckets of SB bytes (dyc_bins_sb.cuh),
+// behind Ops::repeat and Ops::bin_small.
+template <int KB, int SB> struct BinsSb {
+    static cudaError_t repeat(const LaunchCtx &L, const ApplyScratch &A, const Desc *descs,
+                              uint32_t ntables, bool set, const uint8_t *ops, const void *vals,
+                              uint32_t vb, void *vals_out, uint32_t *bits_out, uint64_t n, void *list_a,
+                              uint64_t list_cap, Counters *gctr);
+    static cudaError_t small(const LaunchCtx &L, const Desc &D, const Scratch &S, int mode,
+                             const uint8_t *ops, const void *keys, const void *vals, uint32_t vb,
+                             void *vals_out, uint32_t *bits_out, uint64_t n, uint32_t flags,
+                             Counters *ctr, Counters *h_ctr);
+};
+
 // Kernel launchers, one set per key width; `sb` = bucket bytes (32/64/128).
 // All return cudaGetLastError() of their launches.
 template <int KB> struct Ops {
@@ -397,9 +410,6 @@ template <int KB> struct Ops {
     // split into bins, and the ops of repeated keys found: their single bits
     // cleared and, for a mixed batch (mode kBinModeMixed), their keys and
     // segments listed in A. ops is null for the insert and erase modes.
-    // The bin kernels' code brought to the current device, once a process, when
-    // its first table is made: left to the first batch it took 1.4 ms of it.
-    static cudaError_t load_bins();
     static cudaError_t bin_group(const LaunchCtx &L, const BinScratch &B, const ApplyScratch &A,
                                  int mode, const uint8_t *ops, const void *keys, uint32_t *bits_out,
                                  uint64_t n, Counters *ctr);
