@@ -376,7 +376,9 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_bin_hot(
 // place. The table takes kHotMax keys; a bin with more is taken in parts by
 // further mixed bits of the key, split again until they fit, so every bin is
 // resolved whatever its keys.
-constexpr uint32_t kHotTab = 2048, kHotMax = 1024;
+// kHotMax is above a bin's ordinary keys (kBinMean and some), or a bin with one
+// popular key more would be split in two half of the time.
+constexpr uint32_t kHotTab = 2048, kHotMax = 1472;
 
 struct HotSmem {
     uint32_t first[kHotTab];  // index + 1 of an op with the cell's key
@@ -629,19 +631,27 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
     unsigned long long x[kGroupR];
 #pragma unroll
     for (int q = 0; q < kGroupPre; ++q) x[q] = B.rec[(uint64_t)bin * kBinCap + q * kGroupThreads + tid];
-    const uint32_t m = B.count[bin];
-    if (m == 0u) {
+    const uint32_t count = B.count[bin];
+    if (count == 0u) {
         if (bin == 0 && tid < (uint32_t)kBinStates) B.state[tid] = 0u;
         return;
     }
+    // the records written to `hot`: all of the bin's ops, except those that
+    // cannot count (k_bin_hot), and where device offsets that are out of order
+    // put ops in bins outside their tile's range
+    const uint32_t nhot = count > (uint32_t)kBinCap ? B.cursor[bin] : 0u;
+    // with one record a key and tile most bins that went over fit after all
+    // (32768 inserts, a tenth of them on one key: 61 us by group_hot, 47 here)
+    const bool again = MODE != kBinModeMixed && count > (uint32_t)kBinCap && nhot <= (uint32_t)kBinCap;
+    const uint32_t m = again ? nhot : count;
     for (uint32_t c = tid; c < (uint32_t)kBinCap; c += kGroupThreads) M.tab[c] = 0u;
     if (tid == 0) s_place = s_nwarp = s_nmid = s_ins = 0u;
     if (m <= (uint32_t)kBinCap) {
-        const unsigned long long *rec = B.rec + (uint64_t)bin * kBinCap;
+        const unsigned long long *rec = again ? B.hot + B.start[bin] : B.rec + (uint64_t)bin * kBinCap;
 #pragma unroll
-        for (int q = kGroupPre; q < kGroupR; ++q) {
+        for (int q = 0; q < kGroupR; ++q) {
             const uint32_t r = q * kGroupThreads + tid;
-            if (r < m) x[q] = rec[r];
+            if (r < m && (q >= kGroupPre || again)) x[q] = rec[r];
         }
 #pragma unroll
         for (int q = 0; q < kGroupR; ++q) {
@@ -660,10 +670,6 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_bin_group(
             M.ins[tid] = 0u;
         }
     }
-    // the records written to `hot`: all of the bin's ops, except those that
-    // cannot count (k_bin_hot), and where device offsets that are out of order
-    // put ops in bins outside their tile's range
-    const uint32_t nhot = m > (uint32_t)kBinCap ? B.cursor[bin] : 0u;
     __syncthreads();
     // every thread has read the counts: the next batch finds them, and the
     // split's state, zero
