@@ -1434,7 +1434,7 @@ dyc_status apply_kernels(dyc_table *t, const uint8_t *ops, const void *keys, con
 // table could not place take the overflow path). Otherwise the batch's inserts
 // are counted first (5 us for 2^22 ops and a host read): where the size plus
 // all of them stays within the bound no upsize can be due. Else the exact
-// counts are taken in a pass over the table (147 us), the host reads them and
+// counts are taken in a pass over the table (121 us), the host reads them and
 // upsizes, and the batch is applied after that.
 dyc_status apply_chunk(dyc_table *t, const uint8_t *ops, const void *keys, const void *vals,
                        uint64_t n, void *vals_out, uint32_t *bits_out, uint32_t flags,
@@ -1655,7 +1655,7 @@ extern "C" dyc_status dyc_erase_noalloc(dyc_table *t, const void *d_keys, uint64
         // the array keeps the previous call's cells: clear the ones this call uses
         CK(cudaMemsetAsync(S.dedup, 0, (size_t)S.dedup_cap * 8, s));
         if (S.dedup_idx) CK(cudaMemsetAsync(S.dedup_idx, 0xFF, (size_t)S.dedup_cap * 4, s));
-        cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, d_keys, n, dyc::kKeepFirst);
+        cudaError_t e = KB_CALL(t, dedup, ctx(t, s), S, d_keys, n);
         if (e != cudaSuccess) return fail(DYC_ECUDA, "dedup kernel: %s", cudaGetErrorString(e));
     }
     cudaError_t e = KB_CALL(t, erase, ctx(t, s), t->D, t->sb, S, use_dedup, d_keys, n,

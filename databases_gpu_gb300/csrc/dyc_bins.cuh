@@ -1,5 +1,5 @@
 // dyc_bins.cuh -- the repeated keys of a batch, found bin by bin in shared
-// memory (inserts, erases and mixed batches of one table).
+// memory (inserts, erases and mixed batches of a table, and batches of a set).
 //
 // A chunk's ops are split by a hash of their key into bins of about 1024
 // (k_bin_scatter), and one block per bin finds the keys that occur more than
@@ -11,7 +11,7 @@
 // for mixed batches, a second random read per op (56 us). The split is bound
 // by its 8-byte stores to random sectors (47 us, of which 5 us is the bytes),
 // the grouping by the latency of its steps (19 us for inserts and erases, 27
-// us for mixed ops). 2^24 mixed ops on 2^27 keys: 3.61 -> 2.5 ms a pair of
+// us for mixed ops). 2^24 mixed ops on 2^27 keys: 3.64 -> 2.31 ms a pair of
 // batches.
 //
 // Splitting by the region of a key's first bucket instead, so that a bin's

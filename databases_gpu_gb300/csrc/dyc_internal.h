@@ -68,8 +68,6 @@ struct Publish {
     unsigned long long *h_actr = nullptr;
 };
 
-enum DedupMode { kKeepLast = 0, kKeepFirst = 1 };
-
 // A chunk's ops split by key into bins (dyc_bins.cuh): bin b's records are
 // [b * kBinCap, b * kBinCap + count[b]), a bin holding kBinMean ops of distinct
 // random keys on average. The ops of a bin with more than kBinCap (few keys,
@@ -93,7 +91,7 @@ constexpr int kBinSmallMean = 384;
 constexpr uint64_t kBinSmallOps = 24576, kBinSmallUpserts = 8192;
 enum : int {
     kBinOver = 0,  // nonzero: some bin went over
-    kBinStates = 4
+    kBinStates = 1
 };
 struct BinScratch {
     unsigned long long *rec;  // key tag | op word << 32 (rec_word)
@@ -299,9 +297,9 @@ template <int KB, int SB> struct BinsSb {
 template <int KB> struct Ops {
     static cudaError_t find(const LaunchCtx &L, const Desc &D, int sb, const void *keys,
                             void *vals, uint32_t vb, uint32_t *hits, uint64_t n);
-    // erase_noalloc's batch dedup into S.dedup (cleared by the caller)
-    static cudaError_t dedup(const LaunchCtx &L, const Scratch &S, const void *keys, uint64_t n,
-                             DedupMode mode);
+    // erase_noalloc's batch dedup into S.dedup (cleared by the caller): each
+    // key's first op
+    static cudaError_t dedup(const LaunchCtx &L, const Scratch &S, const void *keys, uint64_t n);
     // insert: place or update every op; ops whose two buckets are full go to
     // list_a (counted in pending). new_keys = caller promises absent keys.
     static cudaError_t place(const LaunchCtx &L, const Desc &D, int sb, const Scratch &S,

@@ -446,8 +446,7 @@ template <int KB> struct Dedup;
 
 template <> struct Dedup<4> {
     // one 64-bit cell: key << 32 | op index; 0 = free
-    __device__ static __forceinline__ void claim(const Scratch &S, uint32_t k, uint32_t i,
-                                                 DedupMode mode) {
+    __device__ static __forceinline__ void claim(const Scratch &S, uint32_t k, uint32_t i) {
         unsigned long long *tab = (unsigned long long *)S.dedup;
         const uint64_t mask = S.dedup_cap - 1;
         const unsigned long long mine = ((unsigned long long)k << 32) | i;
@@ -456,8 +455,7 @@ template <> struct Dedup<4> {
             unsigned long long old = atomicCAS(&tab[h], 0ull, mine);
             if (old == 0ull) return;
             if ((uint32_t)(old >> 32) == k) {
-                if (mode == kKeepLast) atomicMax(&tab[h], mine);
-                else atomicMin(&tab[h], mine);
+                atomicMin(&tab[h], mine);
                 return;
             }
         }
@@ -478,16 +476,14 @@ template <> struct Dedup<4> {
 
 template <> struct Dedup<8> {
     // key array + op-index array; key 0 = free
-    __device__ static __forceinline__ void claim(const Scratch &S, uint64_t k, uint32_t i,
-                                                 DedupMode mode) {
+    __device__ static __forceinline__ void claim(const Scratch &S, uint64_t k, uint32_t i) {
         unsigned long long *tab = (unsigned long long *)S.dedup;
         const uint64_t mask = S.dedup_cap - 1;
         uint64_t h = mix32(fold(k) ^ (uint32_t)(k >> 32)) & mask;
         for (uint64_t probe = 0; probe <= mask; ++probe, h = (h + 1) & mask) {
             unsigned long long old = atomicCAS(&tab[h], 0ull, (unsigned long long)k);
             if (old == 0ull || old == k) {
-                if (mode == kKeepLast) atomicMax(&S.dedup_idx[h], i);
-                else atomicMin(&S.dedup_idx[h], i);
+                atomicMin(&S.dedup_idx[h], i);
                 return;
             }
         }
@@ -508,12 +504,11 @@ template <> struct Dedup<8> {
 
 template <int KB>
 __global__ void __launch_bounds__(256) k_dedup(const __grid_constant__ Scratch S,
-                                               const void *__restrict__ keys, uint64_t n,
-                                               DedupMode mode) {
+                                               const void *__restrict__ keys, uint64_t n) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         typename SlotT<KB>::K k = load_key<KB>(keys, i);
-        if (k != 0) Dedup<KB>::claim(S, k, (uint32_t)i, mode);
+        if (k != 0) Dedup<KB>::claim(S, k, (uint32_t)i);
     }
 }
 

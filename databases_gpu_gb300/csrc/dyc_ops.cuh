@@ -84,11 +84,10 @@ cudaError_t Ops<KB>::find(const LaunchCtx &L, const Desc &D, int sb, const void 
 }
 
 template <int KB>
-cudaError_t Ops<KB>::dedup(const LaunchCtx &L, const Scratch &S, const void *keys, uint64_t n,
-                           DedupMode mode) {
+cudaError_t Ops<KB>::dedup(const LaunchCtx &L, const Scratch &S, const void *keys, uint64_t n) {
     if (n == 0) return cudaSuccess;
     auto k = k_dedup<KB>;
-    k<<<grid_for((const void *)k, L, n), 256, 0, L.stream>>>(S, keys, n, mode);
+    k<<<grid_for((const void *)k, L, n), 256, 0, L.stream>>>(S, keys, n);
     return cudaGetLastError();
 }
 
