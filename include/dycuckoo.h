@@ -242,8 +242,8 @@ dyc_status dyc_erase_host(dyc_table *t, const void *h_keys, uint64_t n,
  * An op sees the latest earlier op on its key in the batch, else the table
  * as it was before the call. Ops on key 0 miss and change nothing.
  * d_vals is read only for INSERT ops but must hold n values; d_vals_out and
- * d_bits_out (ceil(n/32) words) are optional. Ops other than 0/1/2 are
- * treated as FIND. Inserts may upsize first (projected load above
+ * d_bits_out (ceil(n/32) words) are optional; d_vals_out may be d_keys where
+ * both widths are equal. Ops other than 0/1/2 are treated as FIND. Inserts may upsize first (projected load above
  * upper_load); the batch may downsize after (load below lower_load), unless
  * DYC_FLAG_NO_RESIZE. Returns after the batch is in the table.
  * DYC_FLAG_UNIQUE (no key repeats in the batch): every op is resolved and
@@ -362,7 +362,7 @@ dyc_status dyc_set_destroy(dyc_set *s);
 
 /* Launch and table parameters, typically chosen by a tuner per table-size
  * class (databases_gpu_gb300/tune.py): blocks_per_sm caps the resident
- * blocks per SM of the set's launches (0: as many as fit); max_evictions
+ * blocks per SM of the set's batch kernels (0: as many as fit); max_evictions
  * (NULL: unchanged) gives every member its own eviction bound. */
 dyc_status dyc_set_configure(dyc_set *s, uint32_t blocks_per_sm, const uint32_t *max_evictions);
 
