@@ -1089,10 +1089,10 @@ dyc_status ensure_io(dyc_table *t, size_t bytes) {
     return DYC_OK;
 }
 
-// Where the device sees a host array that its kernels may use in place: memory
-// of cudaHostAlloc (pinned and mapped) that holds all of it, aligned to its
-// elements. Else null, and the array is copied: pageable memory, memory that a
-// program registered itself (it may be read-only to the device).
+// Where the device sees a host array that its kernels may use in place: pinned
+// and mapped memory (of cudaHostAlloc or cudaHostRegister) that holds all of it,
+// which the device may write, aligned to its elements. Else null, and the array
+// is copied: pageable and managed memory.
 // A find of 2,000,006 pinned keys took 140 us by copies in, kernel and copies
 // out one after another, 111 us in the best number of overlapped pieces (three;
 // pageable arrays lost 40 us by it) and takes 87 in place, 100,000 keys 19 us
@@ -1109,14 +1109,15 @@ void *host_view(const void *h, uint64_t bytes, int align) {
     }();
     if (!query || (uintptr_t)h % (uintptr_t)align != 0) return nullptr;
     unsigned int type = 0, flags = 0;
+    unsigned long long access = 0;
     CUdeviceptr dev = 0, start = 0;
     size_t size = 0;
     CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
-                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
-                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-    void *to[] = {&type, &dev, &start, &size};
-    if (query(4, what, to, (CUdeviceptr)(uintptr_t)h) != CUDA_SUCCESS) return nullptr;
-    if (type != CU_MEMORYTYPE_HOST || dev == 0 || dev < start || size < bytes ||
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                  CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void *to[] = {&type, &dev, &start, &size, &access};
+    if (query(5, what, to, (CUdeviceptr)(uintptr_t)h) != CUDA_SUCCESS) return nullptr;
+    if (type != CU_MEMORYTYPE_HOST || access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE || dev == 0 || dev < start || size < bytes ||
         dev - start > size - bytes)
         return nullptr;
     if (cudaHostGetFlags(&flags, (void *)h) != cudaSuccess) {

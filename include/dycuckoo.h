@@ -214,9 +214,9 @@ dyc_status dyc_export(dyc_table *t, void *d_keys_out, void *d_vals_out, uint64_t
 dyc_status dyc_last_stats(dyc_table *t, dyc_op_stats *out);
 
 /* Host-buffer forms: the signatures of hashAPI::hash_insert / hash_search /
- * hash_delete (api.cpp:184-303). Arrays in memory of cudaHostAlloc (pinned)
- * are used in place where a kernel reads or writes them once, in order; others
- * go through device buffers owned by the table. They return when the results
+ * hash_delete (api.cpp:184-303). Pinned arrays (cudaHostAlloc or
+ * cudaHostRegister) are used in place where a kernel reads or writes them once,
+ * in order; others go through device buffers owned by the table. They return when the results
  * are in host memory. */
 dyc_status dyc_insert_host(dyc_table *t, const void *h_keys, const void *h_vals, uint64_t n,
                            uint32_t flags);
